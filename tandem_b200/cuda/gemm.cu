@@ -44,7 +44,7 @@ namespace {
 
 constexpr int BK = 64;
 constexpr int SMEM_BUDGET = 192 * 1024;   // operand ring
-constexpr int EPI_STAGING = 8 * 4096;     // per epilogue warp: a 32-row x 128-byte block for coalescing its stores
+constexpr int EPI_STAGING = 8 * 4096 + 8 * 128;  // per epilogue warp: two 32-row x 64-byte blocks on their way out, 32 bias values
 
 enum EpilogueFlags {
   EPI_BIAS = 1,        // + bias[col]
@@ -64,7 +64,6 @@ struct GemmArgs {
   const __nv_bfloat16* aux_in;   // residual, or the saved gelu' factors, [M, ldc]
   __nv_bfloat16* aux_out;        // gelu'(pre-activation) out for EPI_GELU, [M, ldc]
   int* error;                    // host-mapped; set to 1 when a wait runs out
-  int tma_store;                 // map_out (and map_pre) are valid: bf16 output blocks leave through TMA stores
   // Split-K of the last wave.  Output tiles [0, whole_tiles) -- as many full rounds of one tile per CTA as there are --
   // are computed whole.  The remaining tiles, too few to occupy the SMs, have their reduction cut into `splits`
   // parts and each (tile, part) is a work item: parts 1 .. splits-1 ("producers") park their raw fp32 accumulator
@@ -77,7 +76,30 @@ struct GemmArgs {
   int whole_tiles;        // tiles computed by one item each (0 when every tile is split)
   float* partials;        // [split tile][splits - 1][column quad][row][4] floats
   unsigned* split_flags;  // [split tile][splits - 1][8 epilogue warps], zero between launches (the consumer resets them)
+  int group_m;            // rows of tiles per raster group (tile_coords)
+  int kind;               // EpilogueKind; all but KIND_DIRECT leave through TMA stores (map_out and map_pre are valid)
 };
+
+// Output tile `tile` -> its tile row and column.  The first `whole` tiles are swept in groups of `group_m` tile rows, column
+// by column within a group, so that the tiles in flight at one time cover a block of the output that is roughly square and
+// each operand panel is read by several of them; the tiles of an unfinished column and the split ones behind
+// them come in column order.  Sweeping all of it by columns lets every tile in flight read an A panel of its own, and A,
+// larger than L2 at 16384 tokens, comes from memory once per column of tiles.  Measured at 16384 x 2048 x 8192 (bf16, cold
+// L2): 1245 -> 1515 TFLOP/s on 128 x 256 tiles, 1420 -> 1600 on 256 x 256 tiles; groups of 4 to 16 rows of tiles
+// are within 3 % of one another.
+__device__ __forceinline__ void tile_coords(int tile, int tiles_m, int whole, int group_m, int* mi, int* ni) {
+  const int columns = whole / tiles_m;
+  if (tile >= columns * tiles_m) {
+    *mi = tile % tiles_m;
+    *ni = tile / tiles_m;
+    return;
+  }
+  const int per_group = group_m * columns;
+  const int first = tile / per_group * group_m, in = tile % per_group;
+  const int size = tiles_m - first < group_m ? tiles_m - first : group_m;
+  *mi = first + in % size;
+  *ni = in / size;
+}
 
 // All-gather fused into the GEMM (B operand = a weight whose flat bytes are sharded over the ranks).
 // Two extra warps per CTA pull the weight, chunk by chunk, from the owners' shard memory (plain 16-byte
@@ -126,21 +148,81 @@ __device__ __forceinline__ bool wait_chunks(const uint32_t* ready, int c_lo, int
   return true;
 }
 
-// Exact (erf) GELU and its derivative from one evaluation:  erf through Abramowitz & Stegun 7.1.26 (absolute error
-// below 1.5e-7, far inside a bf16 rounding), whose exp(-z^2) with z = |x| / sqrt(2) is the very exp(-x^2 / 2) that the
-// density needs.  One ex2 and one reciprocal on the special-function unit plus a dozen FMAs, against erff + expf before;
-// the element-wise epilogue is what bounds the K = 768 GEMMs.
+// Two fp32 values per register pair: the Blackwell f32x2 instructions do two IEEE operations per issue slot.
+typedef unsigned long long f32x2;
+__device__ __forceinline__ f32x2 pair2(float a, float b) {
+  f32x2 r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
+  return r;
+}
+__device__ __forceinline__ void split2(f32x2 v, float* a, float* b) { asm("mov.b64 {%0, %1}, %2;" : "=f"(*a), "=f"(*b) : "l"(v)); }
+__device__ __forceinline__ f32x2 add2(f32x2 a, f32x2 b) {
+  f32x2 r;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+__device__ __forceinline__ f32x2 mul2(f32x2 a, f32x2 b) {
+  f32x2 r;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+__device__ __forceinline__ f32x2 fma2(f32x2 a, f32x2 b, f32x2 c) {
+  f32x2 r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+  return r;
+}
+__device__ __forceinline__ uint32_t bf16_pair(f32x2 v) {
+  float a, b;
+  split2(v, &a, &b);
+  const __nv_bfloat162 h = __floats2bfloat162_rn(a, b);
+  return *reinterpret_cast<const uint32_t*>(&h);
+}
+__device__ __forceinline__ f32x2 from_bf16_pair(uint32_t v) { return pair2(__uint_as_float(v << 16), __uint_as_float(v & 0xffff0000u)); }
+
+// 1 / d of two values given as -d, 1 <= d, correctly rounded: the special-function unit's approximation (1 ulp) and one
+// Newton step on the residual that an FMA leaves exact (Markstein, IBM J. Res. Dev. 34, 1990).  Above 1e30 it
+// answers 1e-30, which the caller multiplies by exp(-x^2 / 2) = 0.  __frcp_rn's range checks cost a third of the GELU epilogue.
+__device__ __forceinline__ f32x2 reciprocal2(f32x2 minus_d) {
+  float d0, d1, r0, r1;
+  split2(minus_d, &d0, &d1);
+  d0 = fmaxf(d0, -1e30f);
+  d1 = fmaxf(d1, -1e30f);
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r0) : "f"(-d0));
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r1) : "f"(-d1));
+  const f32x2 r = pair2(r0, r1);
+  return fma2(r, fma2(pair2(d0, d1), r, pair2(1.f, 1.f)), r);
+}
+
+// Exact (erf) GELU and its derivative from one evaluation, two values at a time:  erf through Abramowitz & Stegun 7.1.26
+// (absolute error below 1.5e-7, far inside a bf16 rounding), whose exp(-z^2) with z = |x| / sqrt(2) is the very
+// exp(-x^2 / 2) that the density needs.  Element-wise work is what bounds the K = 768 GEMM with GELU, so everything but
+// the special-function unit's part is packed.
 //   gelu(x)  = x * Phi(x)          Phi(x) = (1 + erf(x / sqrt 2)) / 2
 //   gelu'(x) = Phi(x) + x * phi(x)  phi(x) = exp(-x^2 / 2) / sqrt(2 pi)
+__device__ __forceinline__ void gelu_and_grad2(f32x2 x, f32x2* g, f32x2* dg) {
+  auto both = [](float v) { return pair2(v, v); };
+  float x0, x1, a0, a1;
+  split2(x, &x0, &x1);
+  const f32x2 z = mul2(pair2(fabsf(x0), fabsf(x1)), both(0.70710678118654752440f));
+  const f32x2 t = reciprocal2(fma2(both(-0.3275911f), z, both(-1.f)));
+  split2(mul2(mul2(both(-0.72134752044448170368f), x), x), &a0, &a1);  // log2 of exp(-x^2 / 2)
+  const f32x2 e = pair2(ex2_approx(a0), ex2_approx(a1));
+  f32x2 p = fma2(t, both(-1.061405429f), both(1.453152027f));  // the polynomial with its sign turned
+  p = fma2(t, p, both(-1.421413741f));
+  p = fma2(t, p, both(0.284496736f));
+  p = fma2(t, p, both(-0.254829592f));
+  float r0, r1;
+  split2(fma2(mul2(t, p), e, both(1.f)), &r0, &r1);  // erf(|x| / sqrt 2)
+  const f32x2 cdf = mul2(both(0.5f), add2(both(1.f), pair2(copysignf(r0, x0), copysignf(r1, x1))));
+  *g = mul2(x, cdf);
+  *dg = fma2(mul2(x, both(0.39894228040143267794f)), e, cdf);
+}
 __device__ __forceinline__ void gelu_and_grad(float x, float* g, float* dg) {
-  const float z = fabsf(x) * 0.70710678118654752440f;
-  const float t = __frcp_rn(fmaf(0.3275911f, z, 1.f));
-  const float e = ex2_approx(-0.72134752044448170368f * x * x);  // exp(-x^2 / 2)
-  const float poly = t * fmaf(t, fmaf(t, fmaf(t, fmaf(t, 1.061405429f, -1.453152027f), 1.421413741f), -0.284496736f), 0.254829592f);
-  const float erf_abs = fmaf(-poly, e, 1.f);
-  const float cdf = 0.5f * (1.f + copysignf(erf_abs, x));
-  *g = x * cdf;
-  *dg = fmaf(x * 0.39894228040143267794f, e, cdf);
+  f32x2 g2, d2;
+  gelu_and_grad2(pair2(x, x), &g2, &d2);
+  float unused;
+  split2(g2, g, &unused);
+  split2(d2, dg, &unused);
 }
 
 // ------------------------------------------------------------------------------------------ kernel
@@ -231,169 +313,151 @@ __device__ __forceinline__ void epilogue_chunk_generic(const uint32_t (&raw)[32]
   }
 }
 
-// The same for a chunk that lies wholly inside the matrix with 16-byte-aligned rows: no per-element
-// bounds checks, bias fetched as four 16-byte vectors.
-__device__ __forceinline__ void epilogue_chunk_interior(const uint32_t (&raw)[32], int row, int col0, const GemmArgs& g, void* out,
-                                                        bool out_f32, bool bias_vec) {
-  const size_t base = (size_t)row * g.ldc + col0;
+// What a tile's accumulators become on the way out (chosen by the host).
+enum EpilogueKind {
+  KIND_DIRECT = 0,  // anything else: each thread stores its row (fp32 outputs, unaligned rows, rare flag combinations)
+  KIND_PLAIN = 1,   // (+ bias)
+  KIND_ADD = 2,     // (+ bias) + aux_in
+  KIND_MUL = 3,     // (+ bias) * aux_in
+  KIND_GELU = 4,    // gelu(+ bias), and gelu' to aux_out if it is wanted
+};
+
+// Eight columns of a lane's row of a 32-row x 32-column bf16 block in shared memory: rows of 64 bytes, 16-byte slots
+// XOR-swizzled as TMA's 64-byte swizzle does, which also spreads a warp's writes (lane = row) over all banks.
+__device__ __forceinline__ void put8(uint8_t* block, int lane, int slot, uint4 v) {
+  *reinterpret_cast<uint4*>(block + lane * 64 + ((slot ^ ((lane >> 1) & 3)) << 4)) = v;
+}
+
+__device__ __forceinline__ void bulk_store_2d(const CUtensorMap* map, const uint8_t* block, int x, int y) {
+  asm volatile("cp.async.bulk.tensor.2d.global.shared::cta.bulk_group [%0, {%2, %3}], [%1];" ::"l"(map), "r"(smem_u32(block)), "r"(x), "r"(y)
+               : "memory");
+}
+
+// One warp's share of a finished tile: 32 rows x columns [32 * c_begin, 32 * c_end), 32 columns at a time.
+// TMEM -> registers -> element-wise work -> a swizzled 2 KB block in shared memory -> one bulk tensor store, which clips
+// rows >= M and columns >= N.  Two blocks per warp: the store of one chunk reads its block while the next chunk is computed
+// (GELU needs both at once, for its output and its derivative).  The stores never pass through the load/store unit, whose
+// global stores (measured on B200) slow the MMA/TMA traffic of the main loop several times more than their size
+// would suggest.  What this loop costs is instruction fetch: with every flag tested in one body unrolled over 64
+// columns it took 1100 cycles per 64 columns to convert and store plain results, 3400 with a bias and 12000 with GELU.
+// So there is one body per kind, the loop over chunks stays rolled, the bias passes through shared memory (one
+// coalesced load per chunk instead of a load per column), and a chunk's aux_in is fetched one chunk ahead.
+template <int KIND, typename Release>
+__device__ __forceinline__ void store_tile(uint32_t taddr, int c_begin, int c_end, int n0, int row0, int lane, uint8_t* stage, float* bias_sm,
+                                           const GemmArgs& g, const __nv_bfloat16* aux, const CUtensorMap* out_map,
+                                           const CUtensorMap* pre_map, Release release) {
+  const int left = g.N - n0;  // columns of the matrix from here on
+  if (32 * c_end > left) c_end = (left + 31) / 32;
+  if (row0 >= g.M || c_begin >= c_end) {
+    release();
+    return;
+  }
+  const bool has_bias = g.flags & EPI_BIAS, keep_pre = KIND == KIND_GELU && g.aux_out != nullptr;
+  constexpr bool HAS_AUX = KIND == KIND_ADD || KIND == KIND_MUL;
+  const bool row_ok = row0 + lane < g.M;
+  const __nv_bfloat16* aux_row = HAS_AUX ? aux + (size_t)(row_ok ? row0 + lane : row0) * g.ldc + n0 : nullptr;
+  uint4 next_aux[4];
+  float next_bias = 0.f;
+  auto fetch = [&](int c) {
+    if (has_bias) next_bias = c * 32 + lane < left ? __bfloat162float(g.bias[n0 + c * 32 + lane]) : 0.f;
+    if (HAS_AUX) {
 #pragma unroll
-  for (int v8 = 0; v8 < 4; ++v8) {
-    float x[8];
-#pragma unroll
-    for (int j = 0; j < 8; ++j) x[j] = __uint_as_float(raw[v8 * 8 + j]);
-    if (g.flags & EPI_BIAS) {
-      __nv_bfloat16 bv[8];
-      if (bias_vec) {
-        *reinterpret_cast<uint4*>(bv) = __ldg(reinterpret_cast<const uint4*>(g.bias + col0 + v8 * 8));
-      } else {
-#pragma unroll
-        for (int j = 0; j < 8; ++j) bv[j] = g.bias[col0 + v8 * 8 + j];
-      }
-#pragma unroll
-      for (int j = 0; j < 8; ++j) x[j] += __bfloat162float(bv[j]);
+      for (int v = 0; v < 4; ++v)
+        if (c * 32 + v * 8 < left) next_aux[v] = *reinterpret_cast<const uint4*>(aux_row + c * 32 + v * 8);
     }
-    if (g.flags & (EPI_RESIDUAL | EPI_DGELU)) {
-      __nv_bfloat16 aux[8];
-      *reinterpret_cast<uint4*>(aux) = *reinterpret_cast<const uint4*>(g.aux_in + base + v8 * 8);
+  };
+  fetch(c_begin);
+#pragma unroll 1
+  for (int c = c_begin; c < c_end; ++c) {
+    uint32_t raw[32];
+    tmem_ld32(taddr + c * 32, raw);
+    if (has_bias) bias_sm[lane] = next_bias;
+    uint4 cur_aux[4];
+    if (HAS_AUX) {
 #pragma unroll
-      for (int j = 0; j < 8; ++j) {
-        const float a = __bfloat162float(aux[j]);
-        x[j] = (g.flags & EPI_RESIDUAL) ? x[j] + a : x[j] * a;
+      for (int v = 0; v < 4; ++v) cur_aux[v] = next_aux[v];
+    }
+    if (c + 1 < c_end) fetch(c + 1);
+    uint8_t* block = stage + (KIND == KIND_GELU ? 0 : (c & 1) * 2048);
+    if (elect_one()) {  // the store that last used this block has read it
+      if (KIND == KIND_GELU) asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
+      else asm volatile("cp.async.bulk.wait_group.read 1;" ::: "memory");
+    }
+    __syncwarp();
+    tmem_ld_wait();
+    if (c + 1 == c_end) release();  // the accumulator is in registers
+    f32x2 x[16];
+#pragma unroll
+    for (int j = 0; j < 16; ++j) x[j] = pair2(__uint_as_float(raw[2 * j]), __uint_as_float(raw[2 * j + 1]));
+    if (has_bias) {
+#pragma unroll
+      for (int v = 0; v < 8; ++v) {
+        const float4 b = *reinterpret_cast<const float4*>(bias_sm + 4 * v);
+        x[2 * v] = add2(x[2 * v], pair2(b.x, b.y));
+        x[2 * v + 1] = add2(x[2 * v + 1], pair2(b.z, b.w));
       }
     }
-    if (g.flags & EPI_GELU) {
-      float dg[8];
 #pragma unroll
-      for (int j = 0; j < 8; ++j) gelu_and_grad(x[j], &x[j], &dg[j]);
-      if (g.aux_out != nullptr) {
-        __nv_bfloat162 pre[4];
+    for (int v = 0; v < 4; ++v) {
+      uint32_t y[4], dy[4];
+      const uint32_t a[4] = {cur_aux[v].x, cur_aux[v].y, cur_aux[v].z, cur_aux[v].w};
 #pragma unroll
-        for (int j = 0; j < 4; ++j) pre[j] = __floats2bfloat162_rn(dg[2 * j], dg[2 * j + 1]);
-        *reinterpret_cast<uint4*>(g.aux_out + base + v8 * 8) = *reinterpret_cast<const uint4*>(pre);
+      for (int j = 0; j < 4; ++j) {
+        f32x2 w = x[4 * v + j];
+        if (KIND == KIND_ADD) w = add2(w, from_bf16_pair(a[j]));
+        if (KIND == KIND_MUL) w = mul2(w, from_bf16_pair(a[j]));
+        if (KIND == KIND_GELU) {
+          f32x2 slope;
+          gelu_and_grad2(w, &w, &slope);
+          dy[j] = bf16_pair(slope);
+        }
+        y[j] = bf16_pair(w);
       }
+      put8(block, lane, v, make_uint4(y[0], y[1], y[2], y[3]));
+      if (keep_pre) put8(block + 2048, lane, v, make_uint4(dy[0], dy[1], dy[2], dy[3]));
     }
-    if (out_f32) {
-      float* o = reinterpret_cast<float*>(out) + base + v8 * 8;
-      float4 lo = make_float4(x[0], x[1], x[2], x[3]), hi = make_float4(x[4], x[5], x[6], x[7]);
-      if (g.flags & EPI_ACCUMULATE) {
-        const float4 a = *reinterpret_cast<const float4*>(o), b = *reinterpret_cast<const float4*>(o + 4);
-        lo.x += a.x; lo.y += a.y; lo.z += a.z; lo.w += a.w;
-        hi.x += b.x; hi.y += b.y; hi.z += b.z; hi.w += b.w;
-      }
-      *reinterpret_cast<float4*>(o) = lo;
-      *reinterpret_cast<float4*>(o + 4) = hi;
-    } else {
-      __nv_bfloat16* o = reinterpret_cast<__nv_bfloat16*>(out) + base + v8 * 8;
-      if (g.flags & EPI_ACCUMULATE) {
-        __nv_bfloat16 y[8];
-        *reinterpret_cast<uint4*>(y) = *reinterpret_cast<const uint4*>(o);
-#pragma unroll
-        for (int j = 0; j < 8; ++j) x[j] += __bfloat162float(y[j]);
-      }
-      __nv_bfloat162 y2[4];
-#pragma unroll
-      for (int j = 0; j < 4; ++j) y2[j] = __floats2bfloat162_rn(x[2 * j], x[2 * j + 1]);
-      *reinterpret_cast<uint4*>(o) = *reinterpret_cast<const uint4*>(y2);
+    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");  // generic-proxy writes, then the async proxy's read
+    __syncwarp();
+    if (elect_one()) {
+      bulk_store_2d(out_map, block, n0 + c * 32, row0);
+      if (keep_pre) bulk_store_2d(pre_map, block + 2048, n0 + c * 32, row0);
+      asm volatile("cp.async.bulk.commit_group;" ::: "memory");
     }
   }
 }
 
-// Writes a warp's 32-row x 64-column bf16 block (lane = row, `v` = that row's 128 bytes as eight 16-byte
-// vectors) to row-major global memory through a 4 KB shared-memory block.  The 16-byte slots are
-// XOR-swizzled by row, which is both conflict-free for the writes (lane = row) and the 128-byte swizzle
-// of a TMA tile.
-//   map != nullptr: one cp.async.bulk.tensor store of the block {64 columns, 32 rows} at (col0, row0); the
-//     tensor map clips rows >= M and columns >= N.  Shared memory carries the bytes once in and once out, and
-//     the stores never pass through the load/store unit, whose global stores (measured on B200) slow the
-//     MMA/TMA traffic of the main loop several times more than their size would suggest.
-//   map == nullptr: the warp reads the block back and stores complete 128-byte lines itself.
-__device__ __forceinline__ void store_block(uint8_t* stage, const uint4 (&v)[8], const CUtensorMap* map, __nv_bfloat16* out, size_t ldc,
-                                            int row0, int rows_valid, int col0, int lane) {
-  if (map != nullptr) {
-    if (lane == 0) asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");  // the previous store has read the block
-    __syncwarp();
-#pragma unroll
-    for (int sgm = 0; sgm < 8; ++sgm) *reinterpret_cast<uint4*>(stage + lane * 128 + ((sgm ^ (lane & 7)) << 4)) = v[sgm];
-    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");  // generic-proxy writes, then the async proxy's read
-    __syncwarp();
-    if (lane == 0) {
-      asm volatile("cp.async.bulk.tensor.2d.global.shared::cta.bulk_group [%0, {%2, %3}], [%1];" ::"l"(map), "r"(smem_u32(stage)),
-                   "r"(col0), "r"(row0)
-                   : "memory");
-      asm volatile("cp.async.bulk.commit_group;" ::: "memory");
+template <typename Release>
+__device__ __forceinline__ void epilogue_tile(uint32_t taddr, int c_begin, int c_end, int n0, int row0, int lane, uint8_t* stage,
+                                              float* bias_sm, const GemmArgs& g, const CUtensorMap* out_map, const CUtensorMap* pre_map,
+                                              Release release) {
+  switch (g.kind) {
+    case KIND_PLAIN:
+      return store_tile<KIND_PLAIN>(taddr, c_begin, c_end, n0, row0, lane, stage, bias_sm, g, nullptr, out_map, pre_map, release);
+    case KIND_ADD:  // gradient accumulation adds the output's old value
+      return store_tile<KIND_ADD>(taddr, c_begin, c_end, n0, row0, lane, stage, bias_sm, g,
+                                  g.flags & EPI_ACCUMULATE ? reinterpret_cast<const __nv_bfloat16*>(g.out) : g.aux_in, out_map, pre_map, release);
+    case KIND_MUL:
+      return store_tile<KIND_MUL>(taddr, c_begin, c_end, n0, row0, lane, stage, bias_sm, g, g.aux_in, out_map, pre_map, release);
+    case KIND_GELU:
+      return store_tile<KIND_GELU>(taddr, c_begin, c_end, n0, row0, lane, stage, bias_sm, g, nullptr, out_map, pre_map, release);
+    default: {
+#pragma unroll 1
+      for (int c = c_begin; c < c_end; ++c) {
+        uint32_t raw[32];
+        tmem_ld32(taddr + c * 32, raw);
+        tmem_ld_wait();
+        epilogue_chunk_generic(raw, row0 + lane, n0 + c * 32, g, g.out, g.flags & EPI_OUT_F32);
+      }
+      release();
     }
-    return;
-  }
-  __syncwarp();
-#pragma unroll
-  for (int sgm = 0; sgm < 8; ++sgm) *reinterpret_cast<uint4*>(stage + lane * 128 + ((sgm ^ (lane & 7)) << 4)) = v[sgm];
-  __syncwarp();
-  const int sgm = lane & 7;
-#pragma unroll
-  for (int i = 0; i < 8; ++i) {
-    const int r = (lane >> 3) + 4 * i;
-    const uint4 x = *reinterpret_cast<const uint4*>(stage + r * 128 + ((sgm ^ (r & 7)) << 4));
-    if (r < rows_valid) *reinterpret_cast<uint4*>(out + (size_t)(row0 + r) * ldc + col0 + sgm * 8) = x;
   }
 }
 
 // Before an epilogue warp leaves: its bulk stores have read their shared-memory blocks (the writes themselves
 // complete with the grid).
-__device__ __forceinline__ void drain_stores(int lane) {
-  if (lane == 0) asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
+__device__ __forceinline__ void drain_stores() {
+  if (elect_one()) asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
   __syncwarp();
-}
-
-// Two adjacent 32-column chunks (64 columns) of an interior tile with a bf16 output: element-wise
-// work in registers, then coalesced stores of the result (and of the pre-activation, if kept).
-__device__ __forceinline__ void epilogue_pair_interior(const uint32_t (&ra)[32], const uint32_t (&rb)[32], uint8_t* stage, int row,
-                                                       int row0, int rows_valid, int col0, const GemmArgs& g, void* out, bool bias_vec,
-                                                       int lane, const CUtensorMap* map_out, const CUtensorMap* map_pre) {
-  uint4 outv[8], prev[8];
-  const bool keep_pre = (g.flags & EPI_GELU) && g.aux_out != nullptr;
-  const bool row_ok = row < g.M;
-  const size_t base = (size_t)(row_ok ? row : row0) * g.ldc + col0;  // rows past M only feed the staging shuffle
-#pragma unroll
-  for (int v8 = 0; v8 < 8; ++v8) {
-    float x[8];
-#pragma unroll
-    for (int j = 0; j < 8; ++j) x[j] = __uint_as_float(v8 < 4 ? ra[v8 * 8 + j] : rb[(v8 - 4) * 8 + j]);
-    if (g.flags & EPI_BIAS) {
-      __nv_bfloat16 bv[8];
-      if (bias_vec) {
-        *reinterpret_cast<uint4*>(bv) = __ldg(reinterpret_cast<const uint4*>(g.bias + col0 + v8 * 8));
-      } else {
-#pragma unroll
-        for (int j = 0; j < 8; ++j) bv[j] = g.bias[col0 + v8 * 8 + j];
-      }
-#pragma unroll
-      for (int j = 0; j < 8; ++j) x[j] += __bfloat162float(bv[j]);
-    }
-    if (g.flags & (EPI_RESIDUAL | EPI_DGELU | EPI_ACCUMULATE)) {
-      __nv_bfloat16 aux[8];
-      const __nv_bfloat16* src = (g.flags & EPI_ACCUMULATE) && !(g.flags & (EPI_RESIDUAL | EPI_DGELU))
-                                     ? reinterpret_cast<const __nv_bfloat16*>(out) : g.aux_in;
-      *reinterpret_cast<uint4*>(aux) = *reinterpret_cast<const uint4*>(src + base + v8 * 8);
-#pragma unroll
-      for (int j = 0; j < 8; ++j) {
-        const float a = __bfloat162float(aux[j]);
-        x[j] = (g.flags & EPI_DGELU) ? x[j] * a : x[j] + a;
-      }
-    }
-    if (g.flags & EPI_GELU) {
-      float dg[8];
-#pragma unroll
-      for (int j = 0; j < 8; ++j) gelu_and_grad(x[j], &x[j], &dg[j]);
-      __nv_bfloat162* pp = reinterpret_cast<__nv_bfloat162*>(&prev[v8]);
-#pragma unroll
-      for (int j = 0; j < 4; ++j) pp[j] = __floats2bfloat162_rn(dg[2 * j], dg[2 * j + 1]);
-    }
-    __nv_bfloat162* oo = reinterpret_cast<__nv_bfloat162*>(&outv[v8]);
-#pragma unroll
-    for (int j = 0; j < 4; ++j) oo[j] = __floats2bfloat162_rn(x[2 * j], x[2 * j + 1]);
-  }
-  store_block(stage, outv, map_out, reinterpret_cast<__nv_bfloat16*>(out), g.ldc, row0, rows_valid, col0, lane);
-  if (keep_pre) store_block(stage, prev, map_pre, g.aux_out, g.ldc, row0, rows_valid, col0, lane);
 }
 
 // Tile shapes.  BM = 128: one 128-row accumulator per tile, two of them in TMEM so the next tile's
@@ -407,6 +471,7 @@ struct SmemLayout {
   static constexpr int STAGE_BYTES = A_BYTES + B_BYTES;
   static constexpr int STAGES = SMEM_BUDGET / STAGE_BYTES > 8 ? 8 : SMEM_BUDGET / STAGE_BYTES;
   static constexpr int TOTAL = STAGES * STAGE_BYTES + EPI_STAGING + 1024 /* alignment slack */ + 256 /* barriers */;
+  static_assert(TOTAL <= 227 * 1024, "shared memory of one SM");
   static constexpr int THREADS = 64 + 256;  // producer warp, MMA warp, eight epilogue warps
 };
 
@@ -414,8 +479,6 @@ template <int BM, int BN, bool A_MN, bool B_MN, bool GATHER = false>
 __global__ void __launch_bounds__(GATHER ? 448 : 320, 1)
 k_gemm(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b, const __grid_constant__ CUtensorMap map_out,
        const __grid_constant__ CUtensorMap map_pre, const GemmArgs g, const GatherArgs ga) {
-  const CUtensorMap* out_map = g.tma_store ? &map_out : nullptr;
-  const CUtensorMap* pre_map = g.tma_store ? &map_pre : nullptr;
   extern __shared__ uint8_t smem_raw[];
   using L = SmemLayout<BM, BN>;
   constexpr int STAGES = L::STAGES;
@@ -427,7 +490,7 @@ k_gemm(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtens
   uint64_t* acc_empty = acc_full + 2;
   uint32_t* tmem_holder = reinterpret_cast<uint32_t*>(acc_empty + 2);
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;  // warp: known to be uniform
   const int tiles_m = (g.M + BM - 1) / BM, tiles_n = (g.N + BN - 1) / BN;
   const int splits = g.splits > 1 ? g.splits : 1;
   const int out_tiles = tiles_m * tiles_n;
@@ -445,13 +508,13 @@ k_gemm(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtens
   };
   constexpr uint32_t ACC_COLS = BN == 192 ? 256 : BN;  // column stride between the two accumulators
   constexpr uint32_t TMEM_COLS = 2 * ACC_COLS;         // 256 or 512: a power of two
-  // Tile t -> (m0, n0).  m runs fastest, so the CTAs sweep one weight panel at a time; with GATHER the panels
-  // are visited starting from the one this rank's own shard feeds, the order in which the chunks arrive.
+  // Item -> (m0, n0).  With GATHER m runs fastest, so the CTAs sweep one weight panel at a time, starting from the one
+  // this rank's own shard feeds: the order in which the chunks arrive.
   auto tile_origin = [&](int item, int* m0, int* n0) {
-    const int tile = tile_of(item);
-    int n_idx = tile / tiles_m;
+    int m_idx, n_idx;
+    tile_coords(tile_of(item), tiles_m, whole, GATHER ? tiles_m : g.group_m, &m_idx, &n_idx);
     if (GATHER) n_idx = (n_idx + ga.n_start) % tiles_n;
-    *m0 = (tile % tiles_m) * BM;
+    *m0 = m_idx * BM;
     *n0 = n_idx * BN;
   };
 
@@ -465,7 +528,7 @@ k_gemm(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtens
     } else if (lane == STAGES + 2) {
       prefetch_tensormap(&map_a);
       prefetch_tensormap(&map_b);
-      if (g.tma_store) prefetch_tensormap(&map_out);
+      if (g.kind != KIND_DIRECT) prefetch_tensormap(&map_out);
     }
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
@@ -482,24 +545,23 @@ k_gemm(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtens
 
   if (warp == 0) {
     // ------------------------------------------------------------------ TMA producer
-    if (lane == 0) {
-      uint32_t it = 0;
-      bool ok = true;
-      for (int tile = blockIdx.x; tile < num_tiles && ok; tile += gridDim.x) {
-        int m0, n0;
-        tile_origin(tile, &m0, &n0);
-        if (GATHER) {  // the panel's bytes must have arrived (they are row-contiguous: rows n0 .. n0+BN of [N, K])
-          const long long lo = (long long)n0 * g.K * 2;
-          long long hi = (long long)(n0 + BN < g.N ? n0 + BN : g.N) * g.K * 2;
-          if (!(ok = wait_chunks(ga.ready, (int)(lo / ga.chunk_bytes), (int)((hi - 1) / ga.chunk_bytes), ga.epoch, g.error))) break;
-          asm volatile("fence.proxy.async;" ::: "memory");  // the fetchers' generic-proxy stores, then TMA's async-proxy loads
-        }
-        int kb0, kb1;
-        k_range(tile, &kb0, &kb1);
-        for (int kb = kb0; kb < kb1; ++kb, ++it) {
-          const int s = it % STAGES;
-          const uint32_t phase = (it / STAGES) & 1;
-          if (!(ok = mbar_wait(&empty[s], phase ^ 1, g.error))) break;
+    uint32_t s = 0, phase = 1;  // ring slot and the parity of its next `empty`
+    bool ok = true;
+    for (int tile = blockIdx.x; tile < num_tiles && ok; tile += gridDim.x) {
+      int m0, n0;
+      tile_origin(tile, &m0, &n0);
+      if (GATHER) {  // the panel's bytes must have arrived (they are row-contiguous: rows n0 .. n0+BN of [N, K])
+        const long long lo = (long long)n0 * g.K * 2;
+        long long hi = (long long)(n0 + BN < g.N ? n0 + BN : g.N) * g.K * 2;
+        ok = wait_chunks(ga.ready, (int)(lo / ga.chunk_bytes), (int)((hi - 1) / ga.chunk_bytes), ga.epoch, g.error);
+        if (!(ok = __all_sync(0xffffffffu, ok))) break;
+        asm volatile("fence.proxy.async;" ::: "memory");  // the fetchers' generic-proxy stores, then TMA's async-proxy loads
+      }
+      int kb0, kb1;
+      k_range(tile, &kb0, &kb1);
+      for (int kb = kb0; kb < kb1; ++kb) {
+        if (!(ok = mbar_wait_all(&empty[s], phase, g.error))) break;
+        if (elect_one()) {
           uint8_t* a_dst = smem + s * L::STAGE_BYTES;
           uint8_t* b_dst = a_dst + L::A_BYTES;
           mbar_expect_tx(&full[s], L::STAGE_BYTES);
@@ -517,41 +579,40 @@ k_gemm(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtens
             for (int j = 0; j < BN / 64; ++j) tma_load_2d(b_dst + j * 8192, &map_b, &full[s], n0 + j * 64, k0);
           }
         }
+        if (++s == STAGES) s = 0, phase ^= 1;
       }
     }
   } else if (warp == 1) {
     // ------------------------------------------------------------------ MMA issuer
-    if (lane == 0) {
-      constexpr uint32_t idesc = instr_desc(128, BN, A_MN, B_MN);
-      constexpr int HALVES = BM / 128;
-      uint32_t it = 0, local_tile = 0;
-      bool ok = true;
-      for (int tile = blockIdx.x; tile < num_tiles && ok; tile += gridDim.x, ++local_tile) {
-        // BM = 128: accumulators alternate between the two TMEM regions.  BM = 256: region h holds rows [128h, 128h+128).
-        const uint32_t first_buf = HALVES == 1 ? (local_tile & 1) : 0;
-        const uint32_t acc_phase = HALVES == 1 ? ((local_tile >> 1) & 1) : (local_tile & 1);
-        int kb0, kb1;
-        k_range(tile, &kb0, &kb1);
-        for (int kb = kb0; kb < kb1 && ok; ++kb, ++it) {
-          const int s = it % STAGES;
-          const uint32_t phase = (it / STAGES) & 1;
-          if (!(ok = mbar_wait(&full[s], phase, g.error))) break;
-          tc_fence_after();
-          const uint32_t a_addr = smem_u32(smem + s * L::STAGE_BYTES);
-          const uint32_t b_addr = a_addr + L::A_BYTES;
-          // K-major: rows of 128 B, 8-row groups 1024 B apart; one K=16 step is 32 B along the row.
-          // MN-major: 64-wide strips 8192 B apart (LBO), 8 k-rows 1024 B apart (SBO); one K=16 step is 16 rows = 2048 B.
-          const uint64_t b_desc = B_MN ? smem_desc(b_addr, 8192, 1024) : smem_desc(b_addr, 16, 1024);
+    constexpr uint32_t idesc = instr_desc(128, BN, A_MN, B_MN);
+    constexpr int HALVES = BM / 128;
+    uint32_t s = 0, phase = 0, local_tile = 0;
+    bool ok = true;
+    for (int tile = blockIdx.x; tile < num_tiles && ok; tile += gridDim.x, ++local_tile) {
+      // BM = 128: accumulators alternate between the two TMEM regions.  BM = 256: region h holds rows [128h, 128h+128).
+      const uint32_t first_buf = HALVES == 1 ? (local_tile & 1) : 0;
+      const uint32_t acc_phase = HALVES == 1 ? ((local_tile >> 1) & 1) : (local_tile & 1);
+      int kb0, kb1;
+      k_range(tile, &kb0, &kb1);
+      for (int kb = kb0; kb < kb1 && ok; ++kb) {
+        if (!(ok = mbar_wait_all(&full[s], phase, g.error))) break;
+        tc_fence_after();
+        const uint32_t a_addr = smem_u32(smem + s * L::STAGE_BYTES);
+        const uint32_t b_addr = a_addr + L::A_BYTES;
+        // K-major: rows of 128 B, 8-row groups 1024 B apart; one K=16 step is 32 B along the row.
+        // MN-major: 64-wide strips 8192 B apart (LBO), 8 k-rows 1024 B apart (SBO); one K=16 step is 16 rows = 2048 B.
+        const uint64_t b_desc = B_MN ? smem_desc(b_addr, 8192, 1024) : smem_desc(b_addr, 16, 1024);
 #pragma unroll
-          for (int h = 0; h < HALVES; ++h) {
-            const uint32_t buf = first_buf + h;
-            if (kb == kb0) {  // the epilogue has drained this accumulator
-              if (!(ok = mbar_wait(&acc_empty[buf], acc_phase ^ 1, g.error))) break;
-              tc_fence_after();
-            }
-            const uint32_t d_tmem = tmem_base + buf * ACC_COLS;
-            const uint32_t a_half = a_addr + h * 16384;  // 128 rows x 128 B, or two 64-wide strips
-            const uint64_t a_desc = A_MN ? smem_desc(a_half, 8192, 1024) : smem_desc(a_half, 16, 1024);
+        for (int h = 0; h < HALVES; ++h) {
+          const uint32_t buf = first_buf + h;
+          if (kb == kb0) {  // the epilogue has drained this accumulator
+            if (!(ok = mbar_wait_all(&acc_empty[buf], acc_phase ^ 1, g.error))) break;
+            tc_fence_after();
+          }
+          const uint32_t d_tmem = tmem_base + buf * ACC_COLS;
+          const uint32_t a_half = a_addr + h * 16384;  // 128 rows x 128 B, or two 64-wide strips
+          const uint64_t a_desc = A_MN ? smem_desc(a_half, 8192, 1024) : smem_desc(a_half, 16, 1024);
+          if (elect_one()) {
 #pragma unroll
             for (int k = 0; k < BK / 16; ++k) {
               const uint64_t a_k = a_desc + (uint64_t)((A_MN ? 2048 : 32) * k >> 4);
@@ -559,12 +620,13 @@ k_gemm(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtens
               mma_bf16(d_tmem, a_k, b_k, idesc, (kb > kb0 || k > 0) ? 1u : 0u);
             }
           }
-          if (ok) mma_commit(&empty[s]);  // the stage may be refilled once these MMAs have read it
         }
-        if (ok) {
+        if (ok && elect_one()) mma_commit(&empty[s]);  // the stage may be refilled once these MMAs have read it
+        if (++s == STAGES) s = 0, phase ^= 1;
+      }
+      if (ok && elect_one()) {
 #pragma unroll
-          for (int h = 0; h < HALVES; ++h) mma_commit(&acc_full[first_buf + h]);
-        }
+        for (int h = 0; h < HALVES; ++h) mma_commit(&acc_full[first_buf + h]);
       }
     }
   } else if (GATHER && warp >= 10) {
@@ -614,7 +676,8 @@ k_gemm(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtens
     const int half = BM == 128 ? 0 : group;
     uint32_t local_tile = 0;
     bool ok = true;
-    const bool out_f32 = g.flags & EPI_OUT_F32;  // split-K: the host passes "store the fp32 partial tile" as the flags
+    uint8_t* stage = staging + (warp - 2) * 4096;
+    float* bias_sm = reinterpret_cast<float*>(staging + 8 * 4096 + (warp - 2) * 128);
     if (GATHER && (g.flags & EPI_BIAS) && ga.tail_bytes > 0) {
       // the bias sits right behind the weight in the flat buffer and is fetched with it: wait for its chunks
       const long long lo = (long long)g.N * g.K * 2, hi = lo + ga.tail_bytes;
@@ -624,7 +687,6 @@ k_gemm(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtens
     for (int tile = blockIdx.x; tile < num_tiles && ok; tile += gridDim.x, ++local_tile) {
       int m0, n0;
       tile_origin(tile, &m0, &n0);
-      void* out = g.out;
       const int part = part_of(tile), split_tile = tile_of(tile) - whole;
       // this warp's share of the parked partial tiles of its output tile: [part - 1][column quad][row][4]
       float* parked = part >= 0 ? g.partials + (size_t)split_tile * (splits - 1) * (BM * BN) : nullptr;
@@ -649,83 +711,72 @@ k_gemm(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtens
       }
       const uint32_t buf = BM == 128 ? (local_tile & 1) : half;
       const uint32_t acc_phase = BM == 128 ? ((local_tile >> 1) & 1) : (local_tile & 1);
-      ok = mbar_wait_warp(&acc_full[buf], acc_phase, g.error);
+      ok = mbar_wait_all(&acc_full[buf], acc_phase, g.error);
       if (!ok) break;
       tc_fence_after();
-      const int row = m0 + half * 128 + quarter * 32 + lane;
       const uint32_t taddr = tmem_base + ((uint32_t)(quarter * 32) << 16) + buf * ACC_COLS;
-      // Chunks of 32 columns, the TMEM load of the next one in flight while this one is processed.
-      const bool interior_rows = row < g.M && (g.ldc & 7) == 0 && (reinterpret_cast<uintptr_t>(out) & 15) == 0;
-      const bool bias_vec = (g.flags & EPI_BIAS) && (reinterpret_cast<uintptr_t>(g.bias) & 15) == 0;
+      // BM = 128: the two warp groups split the columns; BN / 64 chunks of 32 columns each
       constexpr int CHUNKS = BN / 32;
-      // BM = 128: the two warp groups split the columns (BN = 192: four chunks and two, so each takes whole pairs)
-      const int c_split = BN == 192 ? 4 : CHUNKS / 2;
-      const int c_begin = BM == 128 ? group * c_split : 0;
-      const int c_end = BM == 128 ? (group == 0 ? c_split : CHUNKS) : CHUNKS;
-      {
-        uint32_t ra[32], rb[32];
-        uint8_t* stage = staging + (warp - 2) * 4096;
-        const int row0 = m0 + half * 128 + quarter * 32;           // first row of this warp's block
-        const int rows_valid = g.M - row0 < 32 ? g.M - row0 : 32;   // may be <= 0 on the last tile row
-        // bf16 outputs whose rows are 16-byte aligned go through the coalescing path; accumulate-with-aux combinations
-        // and fp32 outputs take the direct path.
-        const bool pair_ok = !out_f32 && (g.ldc & 7) == 0 && (reinterpret_cast<uintptr_t>(out) & 15) == 0 && rows_valid > 0 &&
-                             !((g.flags & EPI_ACCUMULATE) && (g.flags & (EPI_RESIDUAL | EPI_DGELU)));
+      const int c_begin = BM == 128 ? group * (CHUNKS / 2) : 0;
+      const int c_end = BM == 128 ? c_begin + CHUNKS / 2 : CHUNKS;
+      const int row0 = m0 + half * 128 + quarter * 32;  // first row of this warp's block
+      auto release = [&]() {
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&acc_empty[buf]);
+      };
+      // Parked layout: [part - 1][column quad][row][4 floats].  A lane's four consecutive columns are one 16-byte
+      // vector and consecutive lanes (rows) are consecutive vectors, so a warp moves 512 contiguous bytes per
+      // instruction, 8 instructions per 32 columns.
+      if (part > 0) {  // producer: park the raw accumulator
 #pragma unroll 1
-        for (int c = c_begin; c < c_end; c += 2) {  // c_end - c_begin is even: 2 or 4 or 8 chunks
-          tmem_ld32(taddr + c * 32, ra);
-          tmem_ld32(taddr + (c + 1) * 32, rb);
+        for (int c = c_begin; c < c_end; ++c) {
+          uint32_t raw[32];
+          tmem_ld32(taddr + c * 32, raw);
           tmem_ld_wait();
-          const int col0 = n0 + c * 32;
-          // Parked layout: [part - 1][column quad][row][4 floats].  A lane's four consecutive columns are one 16-byte
-          // vector and consecutive lanes (rows) are consecutive vectors, so a warp moves 512 contiguous bytes per
-          // instruction, 16 instructions per 64 columns.
-          if (part > 0) {  // producer: park the raw accumulator
-            float4* dst = reinterpret_cast<float4*>(parked + (size_t)(part - 1) * (BM * BN)) + (size_t)c * 8 * BM + tile_row;
+          float4* dst = reinterpret_cast<float4*>(parked + (size_t)(part - 1) * (BM * BN)) + (size_t)c * 8 * BM + tile_row;
 #pragma unroll
-            for (int q = 0; q < 8; ++q) {
-              __stcg(dst + (size_t)q * BM, make_float4(__uint_as_float(ra[4 * q]), __uint_as_float(ra[4 * q + 1]),
-                                                       __uint_as_float(ra[4 * q + 2]), __uint_as_float(ra[4 * q + 3])));
-              __stcg(dst + (size_t)(8 + q) * BM, make_float4(__uint_as_float(rb[4 * q]), __uint_as_float(rb[4 * q + 1]),
-                                                             __uint_as_float(rb[4 * q + 2]), __uint_as_float(rb[4 * q + 3])));
-            }
-            continue;
-          }
-          if (part == 0) {  // consumer: fold the parked tiles in, in part order
-            if (!ok) continue;
-            for (int p = 0; p < splits - 1; ++p) {
-              const float4* src = reinterpret_cast<const float4*>(parked + (size_t)p * (BM * BN)) + (size_t)c * 8 * BM + tile_row;
-              // all sixteen loads of a part are issued before the first add: one trip to L2 per part, not one per batch
-              // the compiler happens to pick (volatile asm statements keep their order)
+          for (int q = 0; q < 8; ++q)
+            __stcg(dst + (size_t)q * BM, make_float4(__uint_as_float(raw[4 * q]), __uint_as_float(raw[4 * q + 1]),
+                                                     __uint_as_float(raw[4 * q + 2]), __uint_as_float(raw[4 * q + 3])));
+        }
+        release();
+      } else {
+        if (part == 0) {  // consumer: fold the parked tiles into the accumulator, in part order
+#pragma unroll 1
+          for (int c = c_begin; c < c_end; ++c) {
+            uint32_t raw[32];
+            tmem_ld32(taddr + c * 32, raw);
+            tmem_ld_wait();
+            const float4* src = reinterpret_cast<const float4*>(parked) + (size_t)c * 8 * BM + tile_row;
+            // two parts per trip: all sixteen loads are issued before the first add (volatile asm statements keep
+            // their order), so that a trip to L2 is paid once for both
+            for (int p = 0; p < splits - 1; p += 2) {
+              const bool two = p + 1 < splits - 1;
               float4 v[16];
 #pragma unroll
               for (int q = 0; q < 16; ++q)
-                asm volatile("ld.global.cg.v4.f32 {%0, %1, %2, %3}, [%4];"
-                             : "=f"(v[q].x), "=f"(v[q].y), "=f"(v[q].z), "=f"(v[q].w)
-                             : "l"(src + (size_t)q * BM)
-                             : "memory");
+                if (q < 8 || two)
+                  asm volatile("ld.global.cg.v4.f32 {%0, %1, %2, %3}, [%4];"
+                               : "=f"(v[q].x), "=f"(v[q].y), "=f"(v[q].z), "=f"(v[q].w)
+                               : "l"(src + (size_t)(p + (q >> 3)) * (BM * BN / 4) + (size_t)(q & 7) * BM)
+                               : "memory");
 #pragma unroll
-              for (int q = 0; q < 8; ++q) {
-                ra[4 * q] = __float_as_uint(__uint_as_float(ra[4 * q]) + v[q].x);
-                ra[4 * q + 1] = __float_as_uint(__uint_as_float(ra[4 * q + 1]) + v[q].y);
-                ra[4 * q + 2] = __float_as_uint(__uint_as_float(ra[4 * q + 2]) + v[q].z);
-                ra[4 * q + 3] = __float_as_uint(__uint_as_float(ra[4 * q + 3]) + v[q].w);
-                rb[4 * q] = __float_as_uint(__uint_as_float(rb[4 * q]) + v[8 + q].x);
-                rb[4 * q + 1] = __float_as_uint(__uint_as_float(rb[4 * q + 1]) + v[8 + q].y);
-                rb[4 * q + 2] = __float_as_uint(__uint_as_float(rb[4 * q + 2]) + v[8 + q].z);
-                rb[4 * q + 3] = __float_as_uint(__uint_as_float(rb[4 * q + 3]) + v[8 + q].w);
+              for (int q = 0; q < 16; ++q) {
+                if (q < 8 || two) {
+                  uint32_t* r = raw + 4 * (q & 7);
+                  r[0] = __float_as_uint(__uint_as_float(r[0]) + v[q].x);
+                  r[1] = __float_as_uint(__uint_as_float(r[1]) + v[q].y);
+                  r[2] = __float_as_uint(__uint_as_float(r[2]) + v[q].z);
+                  r[3] = __float_as_uint(__uint_as_float(r[3]) + v[q].w);
+                }
               }
             }
+            tmem_st32(taddr + c * 32, raw);
           }
-          if (pair_ok && col0 + 64 <= g.N) {
-            epilogue_pair_interior(ra, rb, stage, row, row0, rows_valid, col0, g, out, bias_vec, lane, out_map, pre_map);
-          } else {
-            if (interior_rows && col0 + 32 <= g.N) epilogue_chunk_interior(ra, row, col0, g, out, out_f32, bias_vec);
-            else epilogue_chunk_generic(ra, row, col0, g, out, out_f32);
-            if (interior_rows && col0 + 64 <= g.N) epilogue_chunk_interior(rb, row, col0 + 32, g, out, out_f32, bias_vec);
-            else epilogue_chunk_generic(rb, row, col0 + 32, g, out, out_f32);
-          }
+          tmem_st_wait();
         }
+        epilogue_tile(taddr, c_begin, c_end, n0, row0, lane, stage, bias_sm, g, &map_out, &map_pre, release);
       }
       if (part > 0) {  // the parked share is complete: publish it
         __threadfence();
@@ -735,11 +786,8 @@ k_gemm(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtens
         __syncwarp();
         if (lane < splits - 1) my_flags[lane * 8] = 0u;
       }
-      tc_fence_before();
-      __syncwarp();
-      if (lane == 0) mbar_arrive(&acc_empty[buf]);
     }
-    drain_stores(lane);
+    drain_stores();
   }
 
   // ------------------------------------------------------------------ teardown
@@ -771,6 +819,7 @@ struct PairLayout {
   static constexpr int STAGE_BYTES = A_BYTES + B_BYTES;
   static constexpr int STAGES = SMEM_BUDGET / STAGE_BYTES > 8 ? 8 : SMEM_BUDGET / STAGE_BYTES;
   static constexpr int TOTAL = STAGES * STAGE_BYTES + EPI_STAGING + 1024 /* alignment slack */ + 256 /* barriers */;
+  static_assert(TOTAL <= 227 * 1024, "shared memory of one SM");
   static constexpr int THREADS = 64 + 256;
 };
 
@@ -778,8 +827,6 @@ template <int BN, bool A_MN, bool B_MN>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(320, 1)
 k_gemm_pair(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b, const __grid_constant__ CUtensorMap map_out,
             const __grid_constant__ CUtensorMap map_pre, const GemmArgs g) {
-  const CUtensorMap* out_map = g.tma_store ? &map_out : nullptr;
-  const CUtensorMap* pre_map = g.tma_store ? &map_pre : nullptr;
   extern __shared__ uint8_t smem_raw[];
   using L = PairLayout<BN>;
   constexpr int STAGES = L::STAGES;
@@ -791,7 +838,7 @@ k_gemm_pair(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ C
   uint64_t* acc_empty = acc_full + 2;
   uint32_t* tmem_holder = reinterpret_cast<uint32_t*>(acc_empty + 2);
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;  // warp: known to be uniform
   const uint32_t rank = cluster_ctarank();  // 0: the leader
   const int pair = blockIdx.x >> 1, num_pairs = gridDim.x >> 1;
   const int tiles_m = (g.M + 255) / 256, tiles_n = (g.N + BN - 1) / BN;
@@ -823,16 +870,16 @@ k_gemm_pair(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ C
 
   if (warp == 0) {
     // ------------------------------------------------------------------ TMA producer (both CTAs)
-    if (lane == 0) {
-      uint32_t it = 0;
-      bool ok = true;
-      for (int tile = pair; tile < num_tiles && ok; tile += num_pairs) {
-        const int m0 = (tile % tiles_m) * 256 + (int)rank * 128;
-        const int n0 = (tile / tiles_m) * BN + (int)rank * (BN / 2);
-        for (int kb = 0; kb < k_blocks; ++kb, ++it) {
-          const int s = it % STAGES;
-          const uint32_t phase = (it / STAGES) & 1;
-          if (!(ok = mbar_wait(&empty[s], phase ^ 1, g.error))) break;
+    uint32_t s = 0, phase = 1;
+    bool ok = true;
+    for (int tile = pair; tile < num_tiles && ok; tile += num_pairs) {
+      int m_idx, n_idx;
+      tile_coords(tile, tiles_m, num_tiles, g.group_m, &m_idx, &n_idx);
+      const int m0 = m_idx * 256 + (int)rank * 128;
+      const int n0 = n_idx * BN + (int)rank * (BN / 2);
+      for (int kb = 0; kb < k_blocks; ++kb) {
+        if (!(ok = mbar_wait_all(&empty[s], phase, g.error))) break;
+        if (elect_one()) {
           uint8_t* a_dst = smem + s * L::STAGE_BYTES;
           uint8_t* b_dst = a_dst + L::A_BYTES;
           if (rank == 0) mbar_expect_tx(&full[s], 2 * L::STAGE_BYTES);
@@ -851,24 +898,23 @@ k_gemm_pair(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ C
             for (int j = 0; j < BN / 128; ++j) tma_load_2d_pair(b_dst + j * 8192, &map_b, bar, n0 + j * 64, k0);
           }
         }
+        if (++s == STAGES) s = 0, phase ^= 1;
       }
     }
   } else if (warp == 1) {
     // ------------------------------------------------------------------ MMA issuer (leader only)
-    if (lane == 0 && rank == 0) {
+    if (rank == 0) {
       constexpr uint32_t idesc = instr_desc(256, BN, A_MN, B_MN);
-      uint32_t it = 0, local_tile = 0;
+      uint32_t s = 0, phase = 0, local_tile = 0;
       bool ok = true;
       for (int tile = pair; tile < num_tiles && ok; tile += num_pairs, ++local_tile) {
         const uint32_t buf = local_tile & 1;
         const uint32_t acc_phase = (local_tile >> 1) & 1;
-        for (int kb = 0; kb < k_blocks && ok; ++kb, ++it) {
-          const int s = it % STAGES;
-          const uint32_t phase = (it / STAGES) & 1;
-          if (!(ok = mbar_wait(&full[s], phase, g.error))) break;
+        for (int kb = 0; kb < k_blocks && ok; ++kb) {
+          if (!(ok = mbar_wait_all(&full[s], phase, g.error))) break;
           tc_fence_after();
           if (kb == 0) {  // both CTAs' epilogues have drained this accumulator
-            if (!(ok = mbar_wait(&acc_empty[buf], acc_phase ^ 1, g.error))) break;
+            if (!(ok = mbar_wait_all(&acc_empty[buf], acc_phase ^ 1, g.error))) break;
             tc_fence_after();
           }
           const uint32_t a_addr = smem_u32(smem + s * L::STAGE_BYTES);
@@ -876,15 +922,18 @@ k_gemm_pair(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ C
           const uint64_t a_desc = A_MN ? smem_desc(a_addr, 8192, 1024) : smem_desc(a_addr, 16, 1024);
           const uint64_t b_desc = B_MN ? smem_desc(b_addr, 8192, 1024) : smem_desc(b_addr, 16, 1024);
           const uint32_t d_tmem = tmem_base + buf * BN;
+          if (elect_one()) {
 #pragma unroll
-          for (int k = 0; k < BK / 16; ++k) {
-            const uint64_t a_k = a_desc + (uint64_t)((A_MN ? 2048 : 32) * k >> 4);
-            const uint64_t b_k = b_desc + (uint64_t)((B_MN ? 2048 : 32) * k >> 4);
-            mma_bf16_pair(d_tmem, a_k, b_k, idesc, (kb > 0 || k > 0) ? 1u : 0u);
+            for (int k = 0; k < BK / 16; ++k) {
+              const uint64_t a_k = a_desc + (uint64_t)((A_MN ? 2048 : 32) * k >> 4);
+              const uint64_t b_k = b_desc + (uint64_t)((B_MN ? 2048 : 32) * k >> 4);
+              mma_bf16_pair(d_tmem, a_k, b_k, idesc, (kb > 0 || k > 0) ? 1u : 0u);
+            }
+            mma_commit_pair(&empty[s], 3);  // both CTAs may refill the stage once these MMAs have read it
           }
-          mma_commit_pair(&empty[s], 3);  // both CTAs may refill the stage once these MMAs have read it
+          if (++s == STAGES) s = 0, phase ^= 1;
         }
-        if (ok) mma_commit_pair(&acc_full[buf], 3);
+        if (ok && elect_one()) mma_commit_pair(&acc_full[buf], 3);
       }
     }
   } else {
@@ -893,49 +942,29 @@ k_gemm_pair(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ C
     const int group = (warp - 2) >> 2;
     uint32_t local_tile = 0;
     bool ok = true;
-    const bool out_f32 = g.flags & EPI_OUT_F32;
+    uint8_t* stage = staging + (warp - 2) * 4096;
+    float* bias_sm = reinterpret_cast<float*>(staging + 8 * 4096 + (warp - 2) * 128);
     for (int tile = pair; tile < num_tiles && ok; tile += num_pairs, ++local_tile) {
-      const int m0 = (tile % tiles_m) * 256 + (int)rank * 128;
-      const int n0 = (tile / tiles_m) * BN;
+      int m_idx, n_idx;
+      tile_coords(tile, tiles_m, num_tiles, g.group_m, &m_idx, &n_idx);
+      const int m0 = m_idx * 256 + (int)rank * 128;
+      const int n0 = n_idx * BN;
       const uint32_t buf = local_tile & 1;
       const uint32_t acc_phase = (local_tile >> 1) & 1;
-      ok = mbar_wait_warp(&acc_full[buf], acc_phase, g.error);
+      ok = mbar_wait_all(&acc_full[buf], acc_phase, g.error);
       if (!ok) break;
       tc_fence_after();
-      const int row = m0 + quarter * 32 + lane;
       const uint32_t taddr = tmem_base + ((uint32_t)(quarter * 32) << 16) + buf * BN;
-      const bool interior_rows = row < g.M && (g.ldc & 7) == 0 && (reinterpret_cast<uintptr_t>(g.out) & 15) == 0;
-      const bool bias_vec = (g.flags & EPI_BIAS) && (reinterpret_cast<uintptr_t>(g.bias) & 15) == 0;
       constexpr int CHUNKS = BN / 32;
       const int c_begin = group * (CHUNKS / 2), c_end = c_begin + CHUNKS / 2;
-      {
-        uint32_t ra[32], rb[32];
-        uint8_t* stage = staging + (warp - 2) * 4096;
-        const int row0 = m0 + quarter * 32;
-        const int rows_valid = g.M - row0 < 32 ? g.M - row0 : 32;
-        const bool pair_ok = !out_f32 && (g.ldc & 7) == 0 && (reinterpret_cast<uintptr_t>(g.out) & 15) == 0 && rows_valid > 0 &&
-                             !((g.flags & EPI_ACCUMULATE) && (g.flags & (EPI_RESIDUAL | EPI_DGELU)));
-#pragma unroll 1
-        for (int c = c_begin; c < c_end; c += 2) {
-          tmem_ld32(taddr + c * 32, ra);
-          tmem_ld32(taddr + (c + 1) * 32, rb);
-          tmem_ld_wait();
-          const int col0 = n0 + c * 32;
-          if (pair_ok && col0 + 64 <= g.N) {
-            epilogue_pair_interior(ra, rb, stage, row, row0, rows_valid, col0, g, g.out, bias_vec, lane, out_map, pre_map);
-          } else {
-            if (interior_rows && col0 + 32 <= g.N) epilogue_chunk_interior(ra, row, col0, g, g.out, out_f32, bias_vec);
-            else epilogue_chunk_generic(ra, row, col0, g, g.out, out_f32);
-            if (interior_rows && col0 + 64 <= g.N) epilogue_chunk_interior(rb, row, col0 + 32, g, g.out, out_f32, bias_vec);
-            else epilogue_chunk_generic(rb, row, col0 + 32, g, g.out, out_f32);
-          }
-        }
-      }
-      tc_fence_before();
-      __syncwarp();
-      if (lane == 0) mbar_arrive_cluster(map_to_cta(smem_u32(&acc_empty[buf]), 0));
+      auto release = [&]() {
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive_cluster(map_to_cta(smem_u32(&acc_empty[buf]), 0));
+      };
+      epilogue_tile(taddr, c_begin, c_end, n0, m0 + quarter * 32, lane, stage, bias_sm, g, &map_out, &map_pre, release);
     }
-    drain_stores(lane);
+    drain_stores();
   }
 
   // ------------------------------------------------------------------ teardown
@@ -970,7 +999,8 @@ EncodeTiled encoder() {
 char g_map_error[256] = "";
 
 // A 2-D bf16 tensor map: `inner` contiguous elements per row, `outer` rows of `row_stride` elements.
-int make_map(CUtensorMap* map, const void* ptr, long long inner, long long outer, long long row_stride, int box_inner, int box_outer) {
+int make_map(CUtensorMap* map, const void* ptr, long long inner, long long outer, long long row_stride, int box_inner, int box_outer,
+             CUtensorMapSwizzle swizzle = CU_TENSOR_MAP_SWIZZLE_128B) {
   // cuTensorMapEncodeTiled is a driver entry point: it needs this thread to have a current context, which a
   // thread that has so far only been handed cached allocations (an autograd worker) may not have yet.
   static thread_local bool context_ready = false;
@@ -985,7 +1015,7 @@ int make_map(CUtensorMap* map, const void* ptr, long long inner, long long outer
   cuuint32_t box[2] = {(cuuint32_t)box_inner, (cuuint32_t)box_outer};
   cuuint32_t elem[2] = {1, 1};
   CUresult r = enc(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void*>(ptr), dims, strides, box, elem,
-                   CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+                   CU_TENSOR_MAP_INTERLEAVE_NONE, swizzle, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
                    CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   if (r != CUDA_SUCCESS)
     snprintf(g_map_error, sizeof(g_map_error), "cuTensorMapEncodeTiled -> %d (ptr %p, dims %lld x %lld, row stride %lld el, box %d x %d)",
@@ -993,18 +1023,21 @@ int make_map(CUtensorMap* map, const void* ptr, long long inner, long long outer
   return r == CUDA_SUCCESS ? 0 : -11;
 }
 
-// Tensor maps for the epilogue's TMA stores: 32-row x 64-column bf16 blocks of out (and of the kept pre-activation).
-// Returns 1 if the output qualifies (bf16, 16-byte aligned rows), 0 if the epilogue must store by itself.
+// The epilogue of this call, with the tensor maps of its TMA stores: 32-row x 32-column bf16 blocks of out (and of the kept
+// gelu' factors).
 int g_tma_store_enabled = 1;
-int make_store_maps(CUtensorMap* mo, CUtensorMap* mp, void* out, void* aux_out, int M, int N, int ldc, int flags) {
+int plan_epilogue(CUtensorMap* mo, CUtensorMap* mp, void* out, void* aux_out, int M, int N, int ldc, int flags) {
   memset(mo, 0, sizeof(*mo));
   memset(mp, 0, sizeof(*mp));
-  if (!g_tma_store_enabled || (flags & EPI_OUT_F32) || (ldc & 7) || ((uintptr_t)out & 15) || N < 64 || M < 32) return 0;
+  const int work = flags & (EPI_GELU | EPI_RESIDUAL | EPI_DGELU | EPI_ACCUMULATE);
+  const int kind = work == 0 ? KIND_PLAIN : work == EPI_RESIDUAL || work == EPI_ACCUMULATE ? KIND_ADD : work == EPI_DGELU ? KIND_MUL
+                   : work == EPI_GELU ? KIND_GELU : KIND_DIRECT;
+  if (!g_tma_store_enabled || (flags & EPI_OUT_F32) || (ldc & 7) || ((uintptr_t)out & 15) || N < 64 || M < 32) return KIND_DIRECT;
   const bool keep_pre = (flags & EPI_GELU) && aux_out != nullptr;
-  if (keep_pre && ((uintptr_t)aux_out & 15)) return 0;
-  if (make_map(mo, out, N, M, ldc, 64, 32)) return 0;
-  if (keep_pre && make_map(mp, aux_out, N, M, ldc, 64, 32)) return 0;
-  return 1;
+  if (keep_pre && ((uintptr_t)aux_out & 15)) return KIND_DIRECT;
+  if (make_map(mo, out, N, M, ldc, 32, 32, CU_TENSOR_MAP_SWIZZLE_64B)) return KIND_DIRECT;
+  if (keep_pre && make_map(mp, aux_out, N, M, ldc, 32, 32, CU_TENSOR_MAP_SWIZZLE_64B)) return KIND_DIRECT;
+  return kind;
 }
 
 int* g_error_host = nullptr;
@@ -1188,9 +1221,10 @@ int tb_gemm_bf16(const void* A, const void* B, void* out, int M, int N, int K, i
   else rc = make_map(&mb, B, N, K, ldb, 64, 64);
   if (rc) return rc;
   CUtensorMap mo, mp;
-  const int tma_store = make_store_maps(&mo, &mp, out, aux_out, M, N, ldc, flags);
-  GemmArgs g{M, N, K, ldc, flags, out, (const __nv_bfloat16*)bias, (const __nv_bfloat16*)aux_in, (__nv_bfloat16*)aux_out, g_error_dev, tma_store,
-             splits, splits > 1 ? plan.whole_tiles : 0, (float*)workspace, split_flags};
+  const int kind = plan_epilogue(&mo, &mp, out, aux_out, M, N, ldc, flags);
+  const int group_m = BM == 128 ? 8 : 4;  // 1024 rows
+  GemmArgs g{M, N, K, ldc, flags, out, (const __nv_bfloat16*)bias, (const __nv_bfloat16*)aux_in, (__nv_bfloat16*)aux_out, g_error_dev,
+             splits, splits > 1 ? plan.whole_tiles : 0, (float*)workspace, split_flags, group_m, kind};
   tb_note_launch(1);
 #define GO2(BN_) \
   do { \
@@ -1283,9 +1317,9 @@ int tb_gemm_gathered(const void* A, void* out, int M, int N, int K, int lda, int
   rc = make_map(&mb, (const char*)full + w_off, K, N, K, 64, BN);
   if (rc) return rc;
   CUtensorMap mo, mp;
-  const int tma_store = make_store_maps(&mo, &mp, out, aux_out, M, N, ldc, flags);
-  GemmArgs g{M, N, K, ldc, flags, out, (const __nv_bfloat16*)bias, (const __nv_bfloat16*)aux_in, (__nv_bfloat16*)aux_out, g_error_dev, tma_store,
-             1, 0, nullptr, nullptr};
+  const int kind = plan_epilogue(&mo, &mp, out, aux_out, M, N, ldc, flags);
+  GemmArgs g{M, N, K, ldc, flags, out, (const __nv_bfloat16*)bias, (const __nv_bfloat16*)aux_in, (__nv_bfloat16*)aux_out, g_error_dev,
+             1, 0, nullptr, nullptr, 1, kind};
   GatherArgs ga{};
   for (int q = 0; q < n_ranks; ++q) {
     ga.shard[q] = (const char*)shards[q];

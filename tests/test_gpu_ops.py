@@ -119,6 +119,53 @@ def test_gemm_split_k(M, N, K, splits, tile, force_tile):
         lib().tb_gemm_force_splits(0)
 
 
+@pytest.mark.parametrize("tile", [0, 1, 2, 3, 4, 5])
+@pytest.mark.parametrize("M,N,K", [(2300, 1100, 136), (1281, 3000, 64), (4224, 4200, 72)])
+def test_gemm_raster_and_edges(M, N, K, tile, force_tile):
+    """Several raster groups, the last one short, and an unfinished last column of tiles; rows and columns that fit no tile, chunks
+    that start beyond the last column, bias and aux at the edges.  Sums of at most 136 products: fp32 order is far below the
+    bf16 rounding that `close` allows for."""
+    from tandem_b200.ops import gemm as G
+    from tandem_b200.ops._lib import empty_padded
+
+    force_tile(tile)
+    x, w, bias = rnd(M, K, scale=0.5), rnd(N, K, scale=0.5), rnd(N)
+    res = empty_padded(M, N, torch.bfloat16, "cuda")
+    res.copy_(rnd(M, N))
+    ref = x.float() @ w.float().t() + bias.float()
+    close(G.gemm(x, w, M, N, K, K, K, False, False, G.BIAS, bias), ref)
+    out = empty_padded(M, N, torch.bfloat16, "cuda")
+    close(G.gemm(x, w, M, N, K, K, K, False, False, G.BIAS | G.RESIDUAL, bias, res, out=out), ref + res.float())
+    close(G.gemm(x, w, M, N, K, K, K, False, False, G.DGELU, None, res, out=out), (ref - bias.float()) * res.float())
+    slope = empty_padded(M, N, torch.bfloat16, "cuda")
+    close(G.gemm(x, w, M, N, K, K, K, False, False, G.BIAS | G.GELU, bias, None, slope, out=out), torch.nn.functional.gelu(ref))
+    close(slope, gelu_slope(ref))
+
+
+def test_gelu_epilogue_at_the_extremes(force_tile):
+    """GELU and its derivative where the reciprocal and the exponential saturate, and for infinities and NaN."""
+    from tandem_b200.ops import gemm as G
+
+    M, N, K = 128, 128, 64
+    values = torch.tensor([0.0, 1e-20, 0.5, 3.0, 9.0, 60.0, 1e4, 1e20, 3e38, float("inf"), float("nan")], device="cuda").bfloat16()
+    values = torch.cat([values, -values])
+    x = torch.zeros(M, K, device="cuda", dtype=torch.bfloat16)
+    w = torch.zeros(N, K, device="cuda", dtype=torch.bfloat16)
+    bias = torch.zeros(N, device="cuda", dtype=torch.bfloat16)
+    bias[:values.numel()] = values
+    slope = torch.empty(M, N, device="cuda", dtype=torch.bfloat16)
+    out = G.gemm(x, w, M, N, K, K, K, False, False, G.BIAS | G.GELU, bias, None, slope)
+    v = values.double()
+    cdf = 0.5 * torch.special.erfc(-v / 2**0.5)
+    want, want_slope = v * cdf, cdf + v * torch.exp(-v * v / 2) / (2 * torch.pi) ** 0.5
+    got, got_slope = out[5, :v.numel()].double(), slope[5, :v.numel()].double()
+    finite = v.isfinite()
+    # the formula's 1.5e-7 absolute error, times |x| for gelu, and one bf16 rounding
+    assert ((got - want).abs()[finite] <= 2.0**-8 * want.abs()[finite] + 2e-7 * v.abs()[finite].clamp(min=1)).all()
+    assert ((got_slope - want_slope).abs()[finite] <= 2.0**-8 * want_slope.abs()[finite] + 1e-6).all()
+    assert got[v == float("inf")].item() == float("inf") and got[v.isnan()].isnan().all()
+
+
 def test_gemm_planner_splits_where_tiles_are_few():
     import ctypes
 
