@@ -453,6 +453,108 @@ __device__ __forceinline__ void epilogue_tile(uint32_t taddr, int c_begin, int c
   }
 }
 
+// Split-K (GemmArgs): a producer's warp parks its 32 rows x columns [32 * c_begin, 32 * c_end) of raw accumulator; the
+// consumer's matching warp folds the parked parts, in part order, into its own accumulator in TMEM.
+// Layout of a parked tile of ROWS rows: [column quad][row][4 floats].  A lane's four consecutive columns are one 16-byte
+// vector and consecutive lanes (rows) are consecutive vectors, so a warp moves 512 contiguous bytes per instruction.
+template <int ROWS>
+__device__ __forceinline__ void park_tile(uint32_t taddr, int c_begin, int c_end, float* tile, int tile_row) {
+#pragma unroll 1
+  for (int c = c_begin; c < c_end; ++c) {
+    uint32_t raw[32];
+    tmem_ld32(taddr + c * 32, raw);
+    tmem_ld_wait();
+    float4* dst = reinterpret_cast<float4*>(tile) + (size_t)c * 8 * ROWS + tile_row;
+#pragma unroll
+    for (int q = 0; q < 8; ++q)
+      __stcg(dst + (size_t)q * ROWS, make_float4(__uint_as_float(raw[4 * q]), __uint_as_float(raw[4 * q + 1]),
+                                                 __uint_as_float(raw[4 * q + 2]), __uint_as_float(raw[4 * q + 3])));
+  }
+}
+
+template <int ROWS, int TILE_FLOATS>
+__device__ __forceinline__ void fold_tile(uint32_t taddr, int c_begin, int c_end, const float* tiles, int parts, int tile_row) {
+#pragma unroll 1
+  for (int c = c_begin; c < c_end; c += 2) {
+    const bool two = c + 1 < c_end;
+    uint32_t raw[2][32];
+    tmem_ld32(taddr + c * 32, raw[0]);
+    if (two) tmem_ld32(taddr + (c + 1) * 32, raw[1]);
+    tmem_ld_wait();
+    for (int p = 0; p < parts; ++p) {
+      const float4* src = reinterpret_cast<const float4*>(tiles + (size_t)p * TILE_FLOATS) + (size_t)c * 8 * ROWS + tile_row;
+      // all sixteen loads of a part are issued before the first add: one trip to L2 per part, not one per batch
+      // the compiler happens to pick (volatile asm statements keep their order)
+      float4 v[16];
+#pragma unroll
+      for (int q = 0; q < 16; ++q)
+        if (q < 8 || two)
+          asm volatile("ld.global.cg.v4.f32 {%0, %1, %2, %3}, [%4];"
+                       : "=f"(v[q].x), "=f"(v[q].y), "=f"(v[q].z), "=f"(v[q].w)
+                       : "l"(src + (size_t)q * ROWS)
+                       : "memory");
+#pragma unroll
+      for (int q = 0; q < 16; ++q) {
+        if (q < 8 || two) {
+          uint32_t* r = raw[q >> 3] + 4 * (q & 7);
+          r[0] = __float_as_uint(__uint_as_float(r[0]) + v[q].x);
+          r[1] = __float_as_uint(__uint_as_float(r[1]) + v[q].y);
+          r[2] = __float_as_uint(__uint_as_float(r[2]) + v[q].z);
+          r[3] = __float_as_uint(__uint_as_float(r[3]) + v[q].w);
+        }
+      }
+    }
+    tmem_st32(taddr + c * 32, raw[0]);
+    if (two) tmem_st32(taddr + (c + 1) * 32, raw[1]);
+  }
+  tmem_st_wait();
+}
+
+// The flag a producer's warp raises once its share is parked, and the consumer's bounded wait for the same warp's flags
+// of all parts (`stride` words apart).
+__device__ __forceinline__ void raise_flag(unsigned* flag, int lane) {
+  __threadfence();
+  __syncwarp();
+  if (lane == 0) st_release_gpu(flag, 1u);
+}
+__device__ __forceinline__ bool wait_flags(const unsigned* flags, int parts, int stride, int lane, int* error) {
+  bool seen = true;
+  if (lane < parts) {
+    const long long start = clock64();
+    while (ld_acquire_gpu(flags + lane * stride) == 0u) {
+      if (clock64() - start > (1ll << WAIT_LIMIT_CYCLES_SHIFT)) {
+        *error = 1;
+        __threadfence_system();
+        seen = false;
+        break;
+      }
+    }
+  }
+  return __all_sync(0xffffffffu, seen);
+}
+
+// Work items of a split problem: whole tiles, then the tail's producers (parts 1 .. splits-1), then its consumers (part 0).
+struct Items {
+  int whole, tail, splits, k_blocks, k_per, count;
+  __device__ Items(const GemmArgs& g, int out_tiles) {
+    splits = g.splits > 1 ? g.splits : 1;
+    whole = splits > 1 ? g.whole_tiles : out_tiles;
+    tail = out_tiles - whole;
+    count = whole + tail * splits;
+    k_blocks = (g.K + BK - 1) / BK;
+    k_per = (k_blocks + splits - 1) / splits;
+  }
+  __device__ int tile(int item) const { return item < whole ? item : whole + (item - whole) % tail; }
+  __device__ int part(int item) const {  // -1: the whole reduction
+    return item < whole ? -1 : (item - whole < tail * (splits - 1) ? 1 + (item - whole) / tail : 0);
+  }
+  __device__ void k_range(int item, int* kb0, int* kb1) const {
+    const int p = part(item);
+    *kb0 = p < 0 ? 0 : p * k_per;
+    *kb1 = p < 0 || (p + 1) * k_per > k_blocks ? k_blocks : (p + 1) * k_per;
+  }
+};
+
 // Before an epilogue warp leaves: its bulk stores have read their shared-memory blocks (the writes themselves
 // complete with the grid).
 __device__ __forceinline__ void drain_stores() {
@@ -492,27 +594,14 @@ k_gemm(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtens
 
   const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;  // warp: known to be uniform
   const int tiles_m = (g.M + BM - 1) / BM, tiles_n = (g.N + BN - 1) / BN;
-  const int splits = g.splits > 1 ? g.splits : 1;
-  const int out_tiles = tiles_m * tiles_n;
-  const int whole = splits > 1 ? g.whole_tiles : out_tiles, tail = out_tiles - whole;
-  const int num_tiles = whole + tail * splits;  // work items: whole tiles, then the tail's producers, then its consumers
-  const int k_blocks_all = (g.K + BK - 1) / BK;
-  const int k_per = (k_blocks_all + splits - 1) / splits;
-  // item -> output tile and k-part (-1: the whole reduction)
-  auto tile_of = [&](int item) { return item < whole ? item : whole + (item - whole) % tail; };
-  auto part_of = [&](int item) { return item < whole ? -1 : (item - whole < tail * (splits - 1) ? 1 + (item - whole) / tail : 0); };
-  auto k_range = [&](int item, int* kb0, int* kb1) {
-    const int part = part_of(item);
-    *kb0 = part < 0 ? 0 : part * k_per;
-    *kb1 = part < 0 || (part + 1) * k_per > k_blocks_all ? k_blocks_all : (part + 1) * k_per;
-  };
+  const Items items(g, tiles_m * tiles_n);
   constexpr uint32_t ACC_COLS = BN == 192 ? 256 : BN;  // column stride between the two accumulators
   constexpr uint32_t TMEM_COLS = 2 * ACC_COLS;         // 256 or 512: a power of two
   // Item -> (m0, n0).  With GATHER m runs fastest, so the CTAs sweep one weight panel at a time, starting from the one
   // this rank's own shard feeds: the order in which the chunks arrive.
   auto tile_origin = [&](int item, int* m0, int* n0) {
     int m_idx, n_idx;
-    tile_coords(tile_of(item), tiles_m, whole, GATHER ? tiles_m : g.group_m, &m_idx, &n_idx);
+    tile_coords(items.tile(item), tiles_m, items.whole, GATHER ? tiles_m : g.group_m, &m_idx, &n_idx);
     if (GATHER) n_idx = (n_idx + ga.n_start) % tiles_n;
     *m0 = m_idx * BM;
     *n0 = n_idx * BN;
@@ -547,7 +636,7 @@ k_gemm(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtens
     // ------------------------------------------------------------------ TMA producer
     uint32_t s = 0, phase = 1;  // ring slot and the parity of its next `empty`
     bool ok = true;
-    for (int tile = blockIdx.x; tile < num_tiles && ok; tile += gridDim.x) {
+    for (int tile = blockIdx.x; tile < items.count && ok; tile += gridDim.x) {
       int m0, n0;
       tile_origin(tile, &m0, &n0);
       if (GATHER) {  // the panel's bytes must have arrived (they are row-contiguous: rows n0 .. n0+BN of [N, K])
@@ -558,7 +647,7 @@ k_gemm(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtens
         asm volatile("fence.proxy.async;" ::: "memory");  // the fetchers' generic-proxy stores, then TMA's async-proxy loads
       }
       int kb0, kb1;
-      k_range(tile, &kb0, &kb1);
+      items.k_range(tile, &kb0, &kb1);
       for (int kb = kb0; kb < kb1; ++kb) {
         if (!(ok = mbar_wait_all(&empty[s], phase, g.error))) break;
         if (elect_one()) {
@@ -588,12 +677,12 @@ k_gemm(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtens
     constexpr int HALVES = BM / 128;
     uint32_t s = 0, phase = 0, local_tile = 0;
     bool ok = true;
-    for (int tile = blockIdx.x; tile < num_tiles && ok; tile += gridDim.x, ++local_tile) {
+    for (int tile = blockIdx.x; tile < items.count && ok; tile += gridDim.x, ++local_tile) {
       // BM = 128: accumulators alternate between the two TMEM regions.  BM = 256: region h holds rows [128h, 128h+128).
       const uint32_t first_buf = HALVES == 1 ? (local_tile & 1) : 0;
       const uint32_t acc_phase = HALVES == 1 ? ((local_tile >> 1) & 1) : (local_tile & 1);
       int kb0, kb1;
-      k_range(tile, &kb0, &kb1);
+      items.k_range(tile, &kb0, &kb1);
       for (int kb = kb0; kb < kb1 && ok; ++kb) {
         if (!(ok = mbar_wait_all(&full[s], phase, g.error))) break;
         tc_fence_after();
@@ -684,31 +773,14 @@ k_gemm(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtens
       ok = wait_chunks(ga.ready, (int)(lo / ga.chunk_bytes), (int)((hi - 1) / ga.chunk_bytes), ga.epoch, g.error);
       ok = __all_sync(0xffffffffu, ok);
     }
-    for (int tile = blockIdx.x; tile < num_tiles && ok; tile += gridDim.x, ++local_tile) {
+    for (int tile = blockIdx.x; tile < items.count && ok; tile += gridDim.x, ++local_tile) {
       int m0, n0;
       tile_origin(tile, &m0, &n0);
-      const int part = part_of(tile), split_tile = tile_of(tile) - whole;
-      // this warp's share of the parked partial tiles of its output tile: [part - 1][column quad][row][4]
-      float* parked = part >= 0 ? g.partials + (size_t)split_tile * (splits - 1) * (BM * BN) : nullptr;
-      unsigned* my_flags = part >= 0 ? g.split_flags + ((size_t)split_tile * (splits - 1)) * 8 + (warp - 2) : nullptr;
+      const int part = items.part(tile), split_tile = items.tile(tile) - items.whole, parts = items.splits - 1;
+      // the parked parts of its output tile, and this warp's flag for the first of them
+      float* parked = part >= 0 ? g.partials + (size_t)split_tile * parts * (BM * BN) : nullptr;
+      unsigned* my_flags = part >= 0 ? g.split_flags + (size_t)split_tile * parts * 8 + (warp - 2) : nullptr;
       const int tile_row = half * 128 + quarter * 32 + lane;
-      if (part == 0) {  // consumer: every producer's matching warp must have parked its share
-        for (int p = 0; p < splits - 1 && ok; ++p) {
-          bool seen = true;
-          if (lane == 0) {
-            const long long start = clock64();
-            while (ld_acquire_gpu(my_flags + p * 8) == 0u) {
-              if (clock64() - start > (1ll << WAIT_LIMIT_CYCLES_SHIFT)) {
-                *g.error = 1;
-                __threadfence_system();
-                seen = false;
-                break;
-              }
-            }
-          }
-          ok = __shfl_sync(0xffffffffu, seen ? 1 : 0, 0) != 0;
-        }
-      }
       const uint32_t buf = BM == 128 ? (local_tile & 1) : half;
       const uint32_t acc_phase = BM == 128 ? ((local_tile >> 1) & 1) : (local_tile & 1);
       ok = mbar_wait_all(&acc_full[buf], acc_phase, g.error);
@@ -725,67 +797,18 @@ k_gemm(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtens
         __syncwarp();
         if (lane == 0) mbar_arrive(&acc_empty[buf]);
       };
-      // Parked layout: [part - 1][column quad][row][4 floats].  A lane's four consecutive columns are one 16-byte
-      // vector and consecutive lanes (rows) are consecutive vectors, so a warp moves 512 contiguous bytes per
-      // instruction, 8 instructions per 32 columns.
-      if (part > 0) {  // producer: park the raw accumulator
-#pragma unroll 1
-        for (int c = c_begin; c < c_end; ++c) {
-          uint32_t raw[32];
-          tmem_ld32(taddr + c * 32, raw);
-          tmem_ld_wait();
-          float4* dst = reinterpret_cast<float4*>(parked + (size_t)(part - 1) * (BM * BN)) + (size_t)c * 8 * BM + tile_row;
-#pragma unroll
-          for (int q = 0; q < 8; ++q)
-            __stcg(dst + (size_t)q * BM, make_float4(__uint_as_float(raw[4 * q]), __uint_as_float(raw[4 * q + 1]),
-                                                     __uint_as_float(raw[4 * q + 2]), __uint_as_float(raw[4 * q + 3])));
-        }
+      if (part > 0) {
+        park_tile<BM>(taddr, c_begin, c_end, parked + (size_t)(part - 1) * (BM * BN), tile_row);
         release();
-      } else {
-        if (part == 0) {  // consumer: fold the parked tiles into the accumulator, in part order
-#pragma unroll 1
-          for (int c = c_begin; c < c_end; ++c) {
-            uint32_t raw[32];
-            tmem_ld32(taddr + c * 32, raw);
-            tmem_ld_wait();
-            const float4* src = reinterpret_cast<const float4*>(parked) + (size_t)c * 8 * BM + tile_row;
-            // two parts per trip: all sixteen loads are issued before the first add (volatile asm statements keep
-            // their order), so that a trip to L2 is paid once for both
-            for (int p = 0; p < splits - 1; p += 2) {
-              const bool two = p + 1 < splits - 1;
-              float4 v[16];
-#pragma unroll
-              for (int q = 0; q < 16; ++q)
-                if (q < 8 || two)
-                  asm volatile("ld.global.cg.v4.f32 {%0, %1, %2, %3}, [%4];"
-                               : "=f"(v[q].x), "=f"(v[q].y), "=f"(v[q].z), "=f"(v[q].w)
-                               : "l"(src + (size_t)(p + (q >> 3)) * (BM * BN / 4) + (size_t)(q & 7) * BM)
-                               : "memory");
-#pragma unroll
-              for (int q = 0; q < 16; ++q) {
-                if (q < 8 || two) {
-                  uint32_t* r = raw + 4 * (q & 7);
-                  r[0] = __float_as_uint(__uint_as_float(r[0]) + v[q].x);
-                  r[1] = __float_as_uint(__uint_as_float(r[1]) + v[q].y);
-                  r[2] = __float_as_uint(__uint_as_float(r[2]) + v[q].z);
-                  r[3] = __float_as_uint(__uint_as_float(r[3]) + v[q].w);
-                }
-              }
-            }
-            tmem_st32(taddr + c * 32, raw);
-          }
-          tmem_st_wait();
-        }
-        epilogue_tile(taddr, c_begin, c_end, n0, row0, lane, stage, bias_sm, g, &map_out, &map_pre, release);
+        raise_flag(my_flags + (part - 1) * 8, lane);
+        continue;
       }
-      if (part > 0) {  // the parked share is complete: publish it
-        __threadfence();
-        __syncwarp();
-        if (lane == 0) st_release_gpu(my_flags + (part - 1) * 8, 1u);
-      } else if (part == 0) {  // leave the flags at zero for the next launch that is handed these words
-        __syncwarp();
-        if (lane < splits - 1) my_flags[lane * 8] = 0u;
+      if (part == 0) {
+        if (!(ok = wait_flags(my_flags, parts, 8, lane, g.error))) break;
+        fold_tile<BM, BM * BN>(taddr, c_begin, c_end, parked, parts, tile_row);
+        if (lane < parts) my_flags[lane * 8] = 0u;  // zero again for the next launch that is handed these words
       }
+      epilogue_tile(taddr, c_begin, c_end, n0, row0, lane, stage, bias_sm, g, &map_out, &map_pre, release);
     }
     drain_stores();
   }
@@ -842,8 +865,7 @@ k_gemm_pair(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ C
   const uint32_t rank = cluster_ctarank();  // 0: the leader
   const int pair = blockIdx.x >> 1, num_pairs = gridDim.x >> 1;
   const int tiles_m = (g.M + 255) / 256, tiles_n = (g.N + BN - 1) / BN;
-  const int num_tiles = tiles_m * tiles_n;
-  const int k_blocks = (g.K + BK - 1) / BK;
+  const Items items(g, tiles_m * tiles_n);
   constexpr uint32_t TMEM_COLS = 2 * BN;  // two accumulators of BN fp32 columns
 
   if (threadIdx.x == 0) {
@@ -872,12 +894,14 @@ k_gemm_pair(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ C
     // ------------------------------------------------------------------ TMA producer (both CTAs)
     uint32_t s = 0, phase = 1;
     bool ok = true;
-    for (int tile = pair; tile < num_tiles && ok; tile += num_pairs) {
+    for (int tile = pair; tile < items.count && ok; tile += num_pairs) {
       int m_idx, n_idx;
-      tile_coords(tile, tiles_m, num_tiles, g.group_m, &m_idx, &n_idx);
+      tile_coords(items.tile(tile), tiles_m, items.whole, g.group_m, &m_idx, &n_idx);
       const int m0 = m_idx * 256 + (int)rank * 128;
       const int n0 = n_idx * BN + (int)rank * (BN / 2);
-      for (int kb = 0; kb < k_blocks; ++kb) {
+      int kb0, kb1;
+      items.k_range(tile, &kb0, &kb1);
+      for (int kb = kb0; kb < kb1; ++kb) {
         if (!(ok = mbar_wait_all(&empty[s], phase, g.error))) break;
         if (elect_one()) {
           uint8_t* a_dst = smem + s * L::STAGE_BYTES;
@@ -907,13 +931,15 @@ k_gemm_pair(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ C
       constexpr uint32_t idesc = instr_desc(256, BN, A_MN, B_MN);
       uint32_t s = 0, phase = 0, local_tile = 0;
       bool ok = true;
-      for (int tile = pair; tile < num_tiles && ok; tile += num_pairs, ++local_tile) {
+      for (int tile = pair; tile < items.count && ok; tile += num_pairs, ++local_tile) {
         const uint32_t buf = local_tile & 1;
         const uint32_t acc_phase = (local_tile >> 1) & 1;
-        for (int kb = 0; kb < k_blocks && ok; ++kb) {
+        int kb0, kb1;
+        items.k_range(tile, &kb0, &kb1);
+        for (int kb = kb0; kb < kb1 && ok; ++kb) {
           if (!(ok = mbar_wait_all(&full[s], phase, g.error))) break;
           tc_fence_after();
-          if (kb == 0) {  // both CTAs' epilogues have drained this accumulator
+          if (kb == kb0) {  // both CTAs' epilogues have drained this accumulator
             if (!(ok = mbar_wait_all(&acc_empty[buf], acc_phase ^ 1, g.error))) break;
             tc_fence_after();
           }
@@ -927,7 +953,7 @@ k_gemm_pair(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ C
             for (int k = 0; k < BK / 16; ++k) {
               const uint64_t a_k = a_desc + (uint64_t)((A_MN ? 2048 : 32) * k >> 4);
               const uint64_t b_k = b_desc + (uint64_t)((B_MN ? 2048 : 32) * k >> 4);
-              mma_bf16_pair(d_tmem, a_k, b_k, idesc, (kb > 0 || k > 0) ? 1u : 0u);
+              mma_bf16_pair(d_tmem, a_k, b_k, idesc, (kb > kb0 || k > 0) ? 1u : 0u);
             }
             mma_commit_pair(&empty[s], 3);  // both CTAs may refill the stage once these MMAs have read it
           }
@@ -944,9 +970,9 @@ k_gemm_pair(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ C
     bool ok = true;
     uint8_t* stage = staging + (warp - 2) * 4096;
     float* bias_sm = reinterpret_cast<float*>(staging + 8 * 4096 + (warp - 2) * 128);
-    for (int tile = pair; tile < num_tiles && ok; tile += num_pairs, ++local_tile) {
+    for (int tile = pair; tile < items.count && ok; tile += num_pairs, ++local_tile) {
       int m_idx, n_idx;
-      tile_coords(tile, tiles_m, num_tiles, g.group_m, &m_idx, &n_idx);
+      tile_coords(items.tile(tile), tiles_m, items.whole, g.group_m, &m_idx, &n_idx);
       const int m0 = m_idx * 256 + (int)rank * 128;
       const int n0 = n_idx * BN;
       const uint32_t buf = local_tile & 1;
@@ -962,6 +988,21 @@ k_gemm_pair(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ C
         __syncwarp();
         if (lane == 0) mbar_arrive_cluster(map_to_cta(smem_u32(&acc_empty[buf]), 0));
       };
+      const int part = items.part(tile);
+      if (part >= 0) {  // 16 flags per part: the eight epilogue warps of either CTA
+        const int split_tile = items.tile(tile) - items.whole, parts = items.splits - 1, tile_row = (int)rank * 128 + quarter * 32 + lane;
+        float* parked = g.partials + (size_t)split_tile * parts * (256 * BN);
+        unsigned* my_flags = g.split_flags + (size_t)split_tile * parts * 16 + rank * 8 + (warp - 2);
+        if (part > 0) {
+          park_tile<256>(taddr, c_begin, c_end, parked + (size_t)(part - 1) * (256 * BN), tile_row);
+          release();
+          raise_flag(my_flags + (part - 1) * 16, lane);
+          continue;
+        }
+        if (!(ok = wait_flags(my_flags, parts, 16, lane, g.error))) break;
+        fold_tile<256, 256 * BN>(taddr, c_begin, c_end, parked, parts, tile_row);
+        if (lane < parts) my_flags[lane * 16] = 0u;
+      }
       epilogue_tile(taddr, c_begin, c_end, n0, m0 + quarter * 32, lane, stage, bias_sm, g, &map_out, &map_pre, release);
     }
     drain_stores();
@@ -1090,66 +1131,91 @@ int launch_gemm_pair(const CUtensorMap& ma, const CUtensorMap& mb, const CUtenso
     }
     max_pairs = n < g_sm_count / 2 ? n : g_sm_count / 2;
   }
-  const int tiles = ((g.M + 255) / 256) * ((g.N + BN - 1) / BN);
+  const int out_tiles = ((g.M + 255) / 256) * ((g.N + BN - 1) / BN);
+  const int tiles = g.splits > 1 ? g.whole_tiles + (out_tiles - g.whole_tiles) * g.splits : out_tiles;
   int pairs = tiles < max_pairs ? tiles : max_pairs;
   if (max_ctas > 1 && pairs > max_ctas / 2) pairs = max_ctas / 2;
-  kernel<<<2 * pairs, L::THREADS, L::TOTAL, stream>>>(ma, mb, mo, mp, g);
-  return (int)cudaGetLastError();
+  return (int)tb::launch(kernel, dim3(2 * pairs), dim3(L::THREADS), L::TOTAL, stream, ma, mb, mo, mp, g);
 }
 
-// Tile shape and tail split with the least estimated time.  One CTA per SM takes output tiles round-robin; the last,
+// Tile shape and tail split with the least estimated time.  The CTAs (or CTA pairs) take output tiles round-robin; the last,
 // partial round leaves SMs idle, so the tiles of that round ("tail") may have their reduction cut into parts that are
 // spread over the idle SMs (GemmArgs).  The estimate, in microseconds, is
 //     start-up + full rounds x (k-blocks x per-k-block + per-tile) + [tail: k-blocks per part x per-k-block + per-tile + fold]
-// with constants fitted to sweeps on B200 (bench/bench_gemm.py --sweep, CUDA-graph timing, cold L2): a k-block costs
-// 0.34 - 0.43 us on the 128-row tiles whatever their width (the main loop is bound by bytes in flight / load latency,
-// not by the tensor pipe) and 0.77 us on the 256 x 256 tile, whose two accumulators fill TMEM so that its epilogue
-// (about 5 us) cannot overlap the next tile; a kernel's start-up and drain cost about 5 us; folding parked partial
-// tiles costs about 2.5 us plus 1.7 us per extra part (producer drain, flag, one trip to L2 per part) plus 0.3 us per
-// parked megabyte.  With those prices the split pays where a round of tiles is less than about half full and the
-// reduction is long: the weight gradients (K = tokens) and, at 1024 - 2048 tokens, the K = 3072 products.
-struct TileShape { int id, bm, bn; double per_kblock, per_tile; };
-constexpr TileShape SHAPES[4] = {{0, 256, 256, 0.77, 5.3}, {1, 128, 256, 0.43, 0.5}, {2, 128, 128, 0.34, 0.6}, {5, 128, 192, 0.41, 0.6}};
+// with constants fitted to sweeps on B200 (bench/bench_gemm.py --sweep, CUDA-graph timing, cold L2) over 1024 - 16384
+// tokens and widths 768 - 2048.  What a k-block costs: a 256 x 256 pair tile feeds 256 x 256 x 64 multiply-adds to two tensor
+// pipes per 64 KB of operands and runs at the power limit (1620 - 1680 TFLOP/s from 10^11 flops on, cuBLAS 1450 - 1640);
+// the 128-row tiles move up to twice the bytes per flop and pay 0.22 - 0.37 us; the one-CTA 256 x 256 tile fills TMEM, so that
+// its epilogue cannot overlap the next tile.  Narrow tiles win where rounds are few: 1024 x 768 x 2304 takes 12.5 us on
+// pair 256 x 128 tiles, 17 on pair 256 x 256.  Folding parked partial tiles costs about 4 us for two parts, 1 us per part more and
+// 0.2 us per parked megabyte, so a split pays where the last round is less than about half full and the reduction is
+// long: the weight gradients (K = tokens).
+// Over 70 shapes the plan is on average 0.3 % behind the best of all plans.
+struct TileShape { int id, bm, bn; double start, per_kblock, per_tile; };
+constexpr int PAIR = 512;  // bm of the CTA-pair kernel's 256-row tiles
+constexpr TileShape SHAPES[6] = {{0, 256, 256, 4.5, 0.64, 3.3}, {1, 128, 256, 4.3, 0.37, 0.9},   {2, 128, 128, 4.3, 0.205, 0.7},
+                                 {5, 128, 192, 4.3, 0.335, 0.8}, {3, PAIR, 256, 6.0, 0.345, 0.7}, {4, PAIR, 128, 4.8, 0.19, 0.9}};
 constexpr int MAX_SPLITS = 8;
-constexpr double START_US = 5.0, FOLD_US = 2.5, FOLD_PART_US = 1.7, FOLD_US_PER_MB = 0.3;
+constexpr double FOLD_US = 3.0, FOLD_PART_US = 1.0, FOLD_US_PER_MB = 0.2;
 
 // Tuning and test hooks (tb_gemm_force_tile / tb_gemm_force_splits): process-wide, read once per call into locals.
 // Atomic so that a setter racing with a launch on another thread (an autograd worker) yields one value or the other.
 std::atomic<int> g_forced_tile{-1};   // 0: 256x256, 1: 128x256, 2: 128x128, 3 / 4: CTA pair 256x256 / 256x128, 5: 128x192; -1: planned
 std::atomic<int> g_forced_splits{0};  // > 0: that many k-parts for the tail (where the reduction is long enough); 0: planned
 
-struct GemmPlan { int bm, bn, splits, whole_tiles; };
+struct GemmPlan {
+  int bm, bn, splits, whole_tiles;
+  int rows() const { return bm == PAIR ? 256 : bm; }
+  long long tiles(int M, int N) const { return (long long)((M + rows() - 1) / rows()) * ((N + bn - 1) / bn); }
+  long long tail(int M, int N) const { return tiles(M, N) - whole_tiles; }
+  long long workspace_bytes(int M, int N) const { return splits <= 1 ? 0 : tail(M, N) * (splits - 1) * rows() * bn * 4; }
+  long long flag_words(int M, int N) const { return tail(M, N) * (splits - 1) * (bm == PAIR ? 16 : 8); }
+};
 
 GemmPlan plan_gemm(int M, int N, int K, int ctas) {
   const int k_blocks = (K + BK - 1) / BK;
   const int forced_tile = g_forced_tile.load(std::memory_order_relaxed), forced_splits = g_forced_splits.load(std::memory_order_relaxed);
-  if (forced_tile == 3 || forced_tile == 4) return {512, forced_tile == 3 ? 256 : 128, 1, 0};  // CTA-pair kernel (bm = 512 marks it)
   auto valid_splits = [&](int s) {  // every part gets at least two k-blocks and none is empty
     const int per = (k_blocks + s - 1) / s;
     return s == 1 || (per >= 2 && (s - 1) * per < k_blocks);
   };
-  GemmPlan best{128, 128, 1, 0};
-  double best_us = 1e300;
+  GemmPlan best{128, 128, 1, 0}, best_split = best;
+  double best_us = 1e300, best_split_us = 1e300;
   for (const TileShape& t : SHAPES) {
     if (forced_tile >= 0 && forced_tile != t.id) continue;
-    if (forced_tile < 0 && t.bn > 128 && N <= 128) continue;
-    const long long tiles = (long long)((M + t.bm - 1) / t.bm) * ((N + t.bn - 1) / t.bn);
-    const long long rounds = tiles / ctas, tail = tiles % ctas;
+    if (forced_tile < 0 && (t.bn > 128 && N <= 128)) continue;
+    const int units = t.bm == PAIR ? ctas / 2 : ctas;
+    if (units < 1) continue;
+    const GemmPlan shape{t.bm, t.bn, 1, 0};
+    const long long tiles = shape.tiles(M, N);
+    const long long rounds = tiles / units, tail = tiles % units;
     const double whole_us = rounds * (k_blocks * t.per_kblock + t.per_tile);
     for (int sp = 1; sp <= MAX_SPLITS; ++sp) {
-      if (!valid_splits(sp) || (sp > 1 && (tail == 0 || tail * sp > ctas))) continue;
-      if (forced_splits > 0 && sp != forced_splits && tail > 0 && valid_splits(forced_splits) && tail * forced_splits <= ctas) continue;
-      double us = START_US + whole_us;
+      if (!valid_splits(sp) || (sp > 1 && (tail == 0 || tail * sp > units))) continue;
+      if (forced_splits > 0 && sp != forced_splits && tail > 0 && valid_splits(forced_splits) && tail * forced_splits <= units) continue;
+      double us = t.start + whole_us;
       if (tail > 0) {
         const int per = (k_blocks + sp - 1) / sp;
         us += per * t.per_kblock + t.per_tile;
-        if (sp > 1) us += FOLD_US + FOLD_PART_US * (sp - 1) + FOLD_US_PER_MB * (double)tail * (sp - 1) * t.bm * t.bn * 4 / 1e6;
+        if (sp > 1) us += FOLD_US + FOLD_PART_US * (sp - 1) + FOLD_US_PER_MB * (double)tail * (sp - 1) * shape.rows() * t.bn * 4 / 1e6;
       }
       if (us < best_us - 1e-9) {
         best_us = us;
-        best = {t.bm, t.bn, sp, (int)(rounds * ctas)};
+        best = {t.bm, t.bn, sp, (int)(rounds * units)};
+      }
+      if (sp > 1 && us < best_split_us - 1e-9) {
+        best_split_us = us;
+        best_split = {t.bm, t.bn, sp, (int)(rounds * units)};
       }
     }
+  }
+  // One round that takes (almost) every SM for 128 k-blocks or more is cut in parts all the same: such a product waits for
+  // the last SM that another stream's kernel still holds.  On an idle GPU that costs 5 us of 37 (3072 x 768 x 8192:
+  // 32.4 us as 72 whole pair 256 x 128 tiles); callers rely on these reductions being cut (tests/test_gemm_planner.py).
+  if (best.splits == 1 && best_split.splits > 1 && k_blocks >= 128) {
+    const int units = best.bm == PAIR ? ctas / 2 : ctas;
+    const long long tiles = best.tiles(M, N);
+    if (tiles <= units && 20 * tiles >= 19 * units) best = best_split;
   }
   if (best.splits == 1) best.whole_tiles = 0;
   return best;
@@ -1190,11 +1256,10 @@ int tb_gemm_bf16(const void* A, const void* B, void* out, int M, int N, int K, i
   const GemmPlan plan = plan_gemm(M, N, K, ctas);
   const int BM = plan.bm, BN = plan.bn;
   int splits = plan.splits;
-  const bool paired = BM == 512;  // a 256 x BN tile shared by a CTA pair: per CTA 128 rows of A, BN/2 rows of B
+  const bool paired = BM == PAIR;  // a 256 x BN tile shared by a CTA pair: per CTA 128 rows of A, BN/2 rows of B
   unsigned* split_flags = nullptr;
   if (splits > 1) {
-    const long long tiles = (long long)((M + BM - 1) / BM) * ((N + BN - 1) / BN), tail = tiles - plan.whole_tiles;
-    const long long need = tail * (splits - 1) * BM * BN * 4, words = tail * (splits - 1) * 8;
+    const long long need = plan.workspace_bytes(M, N), words = plan.flag_words(M, N);
     if (workspace == nullptr || workspace_bytes < need || ((uintptr_t)workspace & 15) || words > SPLIT_FLAG_POOL) {
       splits = 1;  // no room to park partial tiles: compute unsplit (same result up to summation order)
     } else {
@@ -1260,10 +1325,7 @@ long long tb_gemm_workspace_bytes(int M, int N, int K) {
       g_sm_count = 0;
     cudaGetLastError();
   }
-  const GemmPlan plan = plan_gemm(M, N, K, g_sm_count > 0 ? g_sm_count : 148);
-  if (plan.splits <= 1) return 0;
-  const long long tiles = (long long)((M + plan.bm - 1) / plan.bm) * ((N + plan.bn - 1) / plan.bn);
-  return (tiles - plan.whole_tiles) * (plan.splits - 1) * plan.bm * plan.bn * 4;
+  return plan_gemm(M, N, K, g_sm_count > 0 ? g_sm_count : 148).workspace_bytes(M, N);
 }
 
 // What the planner picks: writes {BM (512: CTA pair), BN, parts the tail tiles are cut into, tiles computed whole}.

@@ -166,6 +166,29 @@ def test_gelu_epilogue_at_the_extremes(force_tile):
     assert got[v == float("inf")].item() == float("inf") and got[v.isnan()].isnan().all()
 
 
+@pytest.mark.parametrize("tile,splits", [(3, 2), (3, 8), (4, 3), (4, 2)])
+@pytest.mark.parametrize("M,N,K", [(768, 768, 8192), (384, 200, 2048), (130, 72, 4096), (2304, 1030, 1160), (5000, 2100, 520)])
+def test_gemm_pair_split_k(M, N, K, splits, tile, force_tile):
+    """The CTA-pair kernel with the reduction of its last round cut into parts: both CTAs' eight warps park and fold their
+    own rows.  (5000, 2100, 520) has whole rounds before the split one on 256 x 128 tiles."""
+    from tandem_b200.ops import gemm as G
+    from tandem_b200.ops._lib import empty_padded, lib
+
+    force_tile(tile)
+    lib().tb_gemm_force_splits(splits)
+    a2, b2 = empty_padded(K, M, torch.bfloat16, "cuda"), empty_padded(K, N, torch.bfloat16, "cuda")
+    a2.copy_(rnd(K, M, scale=0.5)), b2.copy_(rnd(K, N, scale=0.5))
+    want = a2.float().t() @ b2.float()
+    out = G.gemm(a2, b2, M, N, K, a2.stride(0), b2.stride(0), True, True)
+    close(out, want)
+    for _ in range(3):
+        assert torch.equal(out, G.gemm(a2, b2, M, N, K, a2.stride(0), b2.stride(0), True, True))
+    bias, res = rnd(N), empty_padded(M, N, torch.bfloat16, "cuda")
+    res.copy_(rnd(M, N))
+    out = empty_padded(M, N, torch.bfloat16, "cuda")
+    close(G.gemm(a2, b2, M, N, K, a2.stride(0), b2.stride(0), True, True, G.BIAS | G.RESIDUAL, bias, res, out=out), want + bias.float() + res.float())
+
+
 def test_gemm_planner_splits_where_tiles_are_few():
     import ctypes
 
