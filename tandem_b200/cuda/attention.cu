@@ -44,12 +44,13 @@ __device__ __forceinline__ void load_tile(uint8_t* dst, const CUtensorMap* map, 
 // D[128, N] (+)= A[128, K=HD] . B[N=128, K=HD]^T with both operands K-major strips.
 template <int HD>
 __device__ __forceinline__ void mma_kmajor(uint32_t d_tmem, const uint8_t* a, const uint8_t* b, uint32_t idesc, bool accumulate) {
+  const uint64_t a_desc = smem_desc(smem_u32(a), 16, 1024), b_desc = smem_desc(smem_u32(b), 16, 1024);
 #pragma unroll
   for (int s = 0; s < HD / 64; ++s)
 #pragma unroll
     for (int k = 0; k < 4; ++k)
-      mma_bf16(d_tmem, smem_desc(smem_u32(a + s * STRIP) + k * 32, 16, 1024), smem_desc(smem_u32(b + s * STRIP) + k * 32, 16, 1024),
-               idesc, (accumulate || s > 0 || k > 0) ? 1u : 0u);
+      mma_bf16(d_tmem, a_desc + ((s * STRIP + k * 32) >> 4), b_desc + ((s * STRIP + k * 32) >> 4), idesc,
+               (accumulate || s > 0 || k > 0) ? 1u : 0u);
 }
 
 // ------------------------------------------------------------------------------------------ forward, warp-specialised
@@ -98,7 +99,7 @@ k_attn_fwd_ws(const __grid_constant__ CUtensorMap map, __nv_bfloat16* __restrict
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem + L::BARS);
   uint64_t *q_full = bars, *s_full = bars + 2, *p_full = bars + 4, *o_full = bars + 6, *kv_full = bars + 8, *kv_empty = bars + 8 + SLOTS;
   uint32_t* holder = reinterpret_cast<uint32_t*>(bars + 8 + 2 * SLOTS);
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;  // warp: known to be uniform
   const int n_qt = T / TILE, n_pairs = (n_qt + 1) / 2;
   // consecutive CTAs share one head's K and V (they stay in L2), longest pair first within the head
   const int pair = n_pairs - 1 - (int)blockIdx.x % n_pairs;
@@ -136,63 +137,66 @@ k_attn_fwd_ws(const __grid_constant__ CUtensorMap map, __nv_bfloat16* __restrict
 
   if (warp == 0) {
     // ------------------------------------------------------------------ TMA producer
-    if (lane == 0) {
+    if (elect_one()) {
       mbar_expect_tx(&q_full[0], TILE_BYTES);
       load_tile<HD>(smem + L::Q, &map, &q_full[0], h * HD, b * T + qt0 * TILE);
       if (n1) {
         mbar_expect_tx(&q_full[1], TILE_BYTES);
         load_tile<HD>(smem + L::Q + TILE_BYTES, &map, &q_full[1], h * HD, b * T + qt1 * TILE);
       }
-      bool ok = true;
-      for (int ld = 0; ld < 2 * n_steps && ok; ++ld) {  // load 2j: K_j, load 2j+1: V_j
-        const int s = ld % SLOTS, j = ld >> 1, part = ld & 1;
-        if (!(ok = mbar_wait(&kv_empty[s], ((ld / SLOTS) & 1) ^ 1, error))) break;
+    }
+    for (int ld = 0; ld < 2 * n_steps; ++ld) {  // load 2j: K_j, load 2j+1: V_j
+      const int s = ld % SLOTS, j = ld >> 1, part = ld & 1;
+      if (!mbar_wait_all(&kv_empty[s], ((ld / SLOTS) & 1) ^ 1, error)) break;
+      if (elect_one()) {
         mbar_expect_tx(&kv_full[s], TILE_BYTES);
         load_tile<HD>(smem + L::RING + s * TILE_BYTES, &map, &kv_full[s], (1 + part) * d + h * HD, b * T + j * TILE);
       }
     }
   } else if (warp == 1) {
     // ------------------------------------------------------------------ MMA issuer
-    if (lane == 0) {
-      constexpr uint32_t idesc_s = instr_desc(128, 128, false, false);
-      constexpr uint32_t idesc_o = instr_desc(128, HD, false, true);
-      auto slot_of = [&](int ld) { return smem + L::RING + (ld % SLOTS) * TILE_BYTES; };
-      auto wait_slot = [&](int ld) { return mbar_wait(&kv_full[ld % SLOTS], (ld / SLOTS) & 1, error); };
-      auto issue_s = [&](int i, int j) {  // S_i = Q_i . K_j^T
-        mma_kmajor<HD>(tmem + i * 128, smem + L::Q + i * TILE_BYTES, slot_of(2 * j), idesc_s, false);
-        mma_commit(&s_full[i]);
-      };
-      auto issue_pv = [&](int i, int j) {  // O_i (+)= P_i . V_j: eight steps of 16 keys; V is MN-major (head dim contiguous)
-        const uint32_t tO = tmem + 256 + i * HD;
-        const uint32_t v_addr = smem_u32(slot_of(2 * j + 1));
+    constexpr uint32_t idesc_s = instr_desc(128, 128, false, false);
+    constexpr uint32_t idesc_o = instr_desc(128, HD, false, true);
+    auto slot_of = [&](int ld) { return smem + L::RING + (ld % SLOTS) * TILE_BYTES; };
+    auto wait_slot = [&](int ld) { return mbar_wait_all(&kv_full[ld % SLOTS], (ld / SLOTS) & 1, error); };
+    auto issue_s = [&](int i, int j) {  // S_i = Q_i . K_j^T
+      mma_kmajor<HD>(tmem + i * 128, smem + L::Q + i * TILE_BYTES, slot_of(2 * j), idesc_s, false);
+      mma_commit(&s_full[i]);
+    };
+    auto issue_pv = [&](int i, int j) {  // O_i (+)= P_i . V_j: eight steps of 16 keys; V is MN-major (head dim contiguous)
+      const uint32_t tO = tmem + 256 + i * HD;
+      const uint64_t v_desc = smem_desc(smem_u32(slot_of(2 * j + 1)), STRIP, 1024);
 #pragma unroll
-        for (int kk = 0; kk < 8; ++kk) {
-          const uint64_t v_desc = smem_desc(v_addr + kk * 2048, STRIP, 1024);
-          mma_bf16_ts(tO, tmem + i * 128 + kk * 8, v_desc, idesc_o, (j > 0 || kk > 0) ? 1u : 0u);  // 16 keys = 8 TMEM columns of P
-        }
-      };
-      bool ok = mbar_wait(&q_full[0], 0, error) && (!n1 || mbar_wait(&q_full[1], 0, error)) && wait_slot(0);
-      if (ok) {
-        tc_fence_after();
+      for (int kk = 0; kk < 8; ++kk)
+        mma_bf16_ts(tO, tmem + i * 128 + kk * 8, v_desc + kk * (2048 >> 4), idesc_o, (j > 0 || kk > 0) ? 1u : 0u);  // 16 keys = 8 TMEM columns of P
+    };
+    bool ok = mbar_wait_all(&q_full[0], 0, error) && (!n1 || mbar_wait_all(&q_full[1], 0, error)) && wait_slot(0);
+    if (ok) {
+      tc_fence_after();
+      if (elect_one()) {
         issue_s(0, 0);
         if (n1) issue_s(1, 0);
         mma_commit(&kv_empty[0]);  // K_0 is free once these have read it
       }
-      for (int j = 0; j < n_steps && ok; ++j) {
-        if (!(ok = wait_slot(2 * j + 1))) break;                       // V_j
-        if (j + 1 < n_steps && !(ok = wait_slot(2 * j + 2))) break;    // K_{j+1}
+    }
+    for (int j = 0; j < n_steps && ok; ++j) {
+      if (!(ok = wait_slot(2 * j + 1))) break;                       // V_j
+      if (j + 1 < n_steps && !(ok = wait_slot(2 * j + 2))) break;    // K_{j+1}
+      tc_fence_after();
+      for (int i = 0; i < 2 && ok; ++i) {
+        const int n_i = i == 0 ? n0 : n1;
+        if (j >= n_i) continue;
+        if (!(ok = mbar_wait_all(&p_full[i], j & 1, error))) break;  // P_i(j) is in place, O_i rescaled if it had to be
         tc_fence_after();
-        for (int i = 0; i < 2 && ok; ++i) {
-          const int n_i = i == 0 ? n0 : n1;
-          if (j >= n_i) continue;
-          if (!(ok = mbar_wait(&p_full[i], j & 1, error))) break;      // P_i(j) is in place, O_i rescaled if it had to be
-          tc_fence_after();
+        if (elect_one()) {
           issue_pv(i, j);
           if (j == n_i - 1) mma_commit(&o_full[i]);
           else issue_s(i, j + 1);
         }
-        if (!ok) break;
-        mma_commit(&kv_empty[(2 * j + 1) % SLOTS]);                    // V_j
+      }
+      if (!ok) break;
+      if (elect_one()) {
+        mma_commit(&kv_empty[(2 * j + 1) % SLOTS]);                      // V_j
         if (j + 1 < n_steps) mma_commit(&kv_empty[(2 * j + 2) % SLOTS]);  // K_{j+1}
       }
     }
@@ -209,7 +213,7 @@ k_attn_fwd_ws(const __grid_constant__ CUtensorMap map, __nv_bfloat16* __restrict
     float m_used = -INFINITY, l = 0.f;  // m_used in raw score units
     bool ok = true;
     for (int j = 0; j < n_i && ok; ++j) {
-      if (!(ok = mbar_wait_warp_spin(&s_full[i], j & 1, error))) break;
+      if (!(ok = mbar_wait_all(&s_full[i], j & 1, error))) break;
       tc_fence_after();
       uint32_t raw[4][32];
 #pragma unroll
@@ -277,7 +281,7 @@ k_attn_fwd_ws(const __grid_constant__ CUtensorMap map, __nv_bfloat16* __restrict
       __syncwarp();
       if (lane == 0) mbar_arrive(&p_full[i]);
     }
-    if (ok && n_i > 0) ok = mbar_wait_warp_spin(&o_full[i], 0, error);
+    if (ok && n_i > 0) ok = mbar_wait_all(&o_full[i], 0, error);
     if (ok && n_i > 0) {
       tc_fence_after();
       const float inv_l = 1.f / l;
@@ -367,7 +371,7 @@ k_attn_bwd_dq(const __grid_constant__ CUtensorMap map_qkv, const __grid_constant
            *kv_full = bars + 6, *kv_empty = bars + 6 + SLOTS;
   uint32_t* holder = reinterpret_cast<uint32_t*>(bars + 6 + 2 * SLOTS);
   float* delta_sm = reinterpret_cast<float*>(smem + L::DELTA);
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;  // warp: known to be uniform
   const int n_qt = T / TILE;
   const int qt = n_qt - 1 - (int)blockIdx.x % n_qt;  // consecutive CTAs share a head (its K, V stay in L2); longest first
   const int rest = (int)blockIdx.x / n_qt;
@@ -403,53 +407,53 @@ k_attn_bwd_dq(const __grid_constant__ CUtensorMap map_qkv, const __grid_constant
   tb::pdl_wait();  // set-up is done; everything below reads what earlier kernels wrote
 
   if (warp == 0) {
-    if (lane == 0) {
+    if (elect_one()) {
       mbar_expect_tx(qdo_full, 2 * TILE_BYTES);
       load_tile<HD>(smem + L::Q, &map_qkv, qdo_full, h * HD, b * T + qt * TILE);
       load_tile<HD>(smem + L::DO, &map_do, qdo_full, h * HD, b * T + qt * TILE);
-      bool ok = true;
-      for (int ld = 0; ld < 2 * n && ok; ++ld) {  // load 2j: K_j, load 2j+1: V_j
-        const int s = ld % SLOTS, j = ld >> 1, part = ld & 1;
-        if (!(ok = mbar_wait(&kv_empty[s], ((ld / SLOTS) & 1) ^ 1, error))) break;
+    }
+    for (int ld = 0; ld < 2 * n; ++ld) {  // load 2j: K_j, load 2j+1: V_j
+      const int s = ld % SLOTS, j = ld >> 1, part = ld & 1;
+      if (!mbar_wait_all(&kv_empty[s], ((ld / SLOTS) & 1) ^ 1, error)) break;
+      if (elect_one()) {
         mbar_expect_tx(&kv_full[s], TILE_BYTES);
         load_tile<HD>(smem + L::RING + s * TILE_BYTES, &map_qkv, &kv_full[s], (1 + part) * d + h * HD, b * T + j * TILE);
       }
     }
   } else if (warp == 1) {
-    if (lane == 0) {
-      constexpr uint32_t idesc_s = instr_desc(128, 128, false, false);
-      constexpr uint32_t idesc_dq = instr_desc(128, HD, false, true);
-      auto slot_of = [&](int ld) { return smem + L::RING + (ld % SLOTS) * TILE_BYTES; };
-      auto wait_slot = [&](int ld) { return mbar_wait(&kv_full[ld % SLOTS], (ld / SLOTS) & 1, error); };
-      auto issue_scores = [&](int j) {
-        mma_kmajor<HD>(tmem + C_S, smem + L::Q, slot_of(2 * j), idesc_s, false);        // S  = Q . K_j^T
-        mma_kmajor<HD>(tmem + C_DP, smem + L::DO, slot_of(2 * j + 1), idesc_s, false);  // dP = dO . V_j^T
-        mma_commit(sdp_full);
-        mma_commit(&kv_empty[(2 * j + 1) % SLOTS]);  // V_j has no other reader
-      };
-      bool ok = mbar_wait(qdo_full, 0, error) && wait_slot(0) && wait_slot(1);
-      if (ok) {
+    constexpr uint32_t idesc_s = instr_desc(128, 128, false, false);
+    constexpr uint32_t idesc_dq = instr_desc(128, HD, false, true);
+    auto slot_of = [&](int ld) { return smem + L::RING + (ld % SLOTS) * TILE_BYTES; };
+    auto wait_slot = [&](int ld) { return mbar_wait_all(&kv_full[ld % SLOTS], (ld / SLOTS) & 1, error); };
+    auto issue_scores = [&](int j) {
+      mma_kmajor<HD>(tmem + C_S, smem + L::Q, slot_of(2 * j), idesc_s, false);        // S  = Q . K_j^T
+      mma_kmajor<HD>(tmem + C_DP, smem + L::DO, slot_of(2 * j + 1), idesc_s, false);  // dP = dO . V_j^T
+      mma_commit(sdp_full);
+      mma_commit(&kv_empty[(2 * j + 1) % SLOTS]);  // V_j has no other reader
+    };
+    bool ok = mbar_wait_all(qdo_full, 0, error) && wait_slot(0) && wait_slot(1);
+    if (ok) {
+      tc_fence_after();
+      if (elect_one()) issue_scores(0);
+    }
+    for (int j = 0; j < n && ok; ++j) {
+      if (j + 1 < n) {
+        if (!(ok = mbar_wait_all(sdp_read, j & 1, error))) break;  // tile j's S and dP are in registers
+        if (!(ok = wait_slot(2 * j + 2) && wait_slot(2 * j + 3))) break;
         tc_fence_after();
-        issue_scores(0);
+        if (elect_one()) issue_scores(j + 1);
       }
-      for (int j = 0; j < n && ok; ++j) {
-        if (j + 1 < n) {
-          if (!(ok = mbar_wait(sdp_read, j & 1, error))) break;  // tile j's S and dP are in registers
-          if (!(ok = wait_slot(2 * j + 2) && wait_slot(2 * j + 3))) break;
-          tc_fence_after();
-          issue_scores(j + 1);
-        }
-        if (!(ok = mbar_wait(&ds_full[j & 1], (j >> 1) & 1, error))) break;
-        tc_fence_after();
-        const uint32_t k_addr = smem_u32(slot_of(2 * j));
+      if (!(ok = mbar_wait_all(&ds_full[j & 1], (j >> 1) & 1, error))) break;
+      tc_fence_after();
+      if (elect_one()) {
+        const uint64_t k_desc = smem_desc(smem_u32(slot_of(2 * j)), STRIP, 1024);
 #pragma unroll
         for (int kk = 0; kk < 8; ++kk)  // dQ += dS . K_j: dS from TMEM (16 keys = 8 columns per step), K_j MN-major over the keys
-          mma_bf16_ts(tmem + C_DQ, tmem + C_DS + (j & 1) * 64 + kk * 8, smem_desc(k_addr + kk * 2048, STRIP, 1024), idesc_dq,
-                      (j > 0 || kk > 0) ? 1u : 0u);
+          mma_bf16_ts(tmem + C_DQ, tmem + C_DS + (j & 1) * 64 + kk * 8, k_desc + kk * (2048 >> 4), idesc_dq, (j > 0 || kk > 0) ? 1u : 0u);
         mma_commit(&kv_empty[(2 * j) % SLOTS]);
       }
-      if (ok) mma_commit(dq_full);
     }
+    if (ok && elect_one()) mma_commit(dq_full);
   } else {
     const int quarter = warp & 3, half = (warp - 2) >> 2;
     const int r = quarter * 32 + lane;
@@ -483,7 +487,7 @@ k_attn_bwd_dq(const __grid_constant__ CUtensorMap map_qkv, const __grid_constant
     const float neg_lse2 = -lse[((size_t)b * H + h) * T + q_idx] * 1.4426950408889634f;
     bool ok = true;
     for (int j = 0; j < n && ok; ++j) {
-      if (!(ok = mbar_wait_warp_spin(sdp_full, j & 1, error))) break;
+      if (!(ok = mbar_wait_all(sdp_full, j & 1, error))) break;
       tc_fence_after();
       uint32_t s[2][32], dp[2][32];
 #pragma unroll
@@ -515,7 +519,7 @@ k_attn_bwd_dq(const __grid_constant__ CUtensorMap map_qkv, const __grid_constant
       __syncwarp();
       if (lane == 0) mbar_arrive(&ds_full[j & 1]);
     }
-    if (ok) ok = mbar_wait_warp_spin(dq_full, 0, error);
+    if (ok) ok = mbar_wait_all(dq_full, 0, error);
     if (ok) {
       tc_fence_after();
       constexpr int COLS = HD / 2;
@@ -581,7 +585,7 @@ k_attn_bwd_dkv(const __grid_constant__ CUtensorMap map_qkv, const __grid_constan
   uint64_t *kv_full = bars, *s_full = bars + 1, *dp_full = bars + 2, *p_full = bars + 3, *ds_full = bars + 4, *acc_full = bars + 5,
            *st_full = bars + 6, *st_empty = bars + 6 + STAGES;
   uint32_t* holder = reinterpret_cast<uint32_t*>(bars + 6 + 2 * STAGES);
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;  // warp: known to be uniform
   const int n_tiles = T / TILE;
   const int kt = (int)blockIdx.x % n_tiles;  // consecutive CTAs share a head; key tile 0 visits every query tile: longest first
   const int rest = (int)blockIdx.x / n_tiles;
@@ -618,14 +622,15 @@ k_attn_bwd_dkv(const __grid_constant__ CUtensorMap map_qkv, const __grid_constan
   auto stage_at = [&](int t) { return smem + L::STAGES_AT + (t % STAGES) * STAGE_BYTES; };
 
   if (warp == 0) {
-    if (lane == 0) {
+    if (elect_one()) {
       mbar_expect_tx(kv_full, 2 * TILE_BYTES);
       load_tile<HD>(smem + L::K, &map_qkv, kv_full, d + h * HD, b * T + kt * TILE);
       load_tile<HD>(smem + L::V, &map_qkv, kv_full, 2 * d + h * HD, b * T + kt * TILE);
-      bool ok = true;
-      for (int t = 0; t < nt && ok; ++t) {
-        const int s = t % STAGES, i = kt + t;
-        if (!(ok = mbar_wait(&st_empty[s], ((t / STAGES) & 1) ^ 1, error))) break;
+    }
+    for (int t = 0; t < nt; ++t) {
+      const int s = t % STAGES, i = kt + t;
+      if (!mbar_wait_all(&st_empty[s], ((t / STAGES) & 1) ^ 1, error)) break;
+      if (elect_one()) {
         uint8_t* st = stage_at(t);
         mbar_expect_tx(&st_full[s], STAGE_BYTES);
         load_tile<HD>(st, &map_qkv, &st_full[s], h * HD, b * T + i * TILE);
@@ -636,46 +641,53 @@ k_attn_bwd_dkv(const __grid_constant__ CUtensorMap map_qkv, const __grid_constan
       }
     }
   } else if (warp == 1) {
-    if (lane == 0) {
-      constexpr uint32_t idesc_s = instr_desc(128, 128, false, false);
-      constexpr uint32_t idesc_acc = instr_desc(128, HD, false, true);
-      auto wait_stage = [&](int t) { return mbar_wait(&st_full[t % STAGES], (t / STAGES) & 1, error); };
-      // bf16 A operand written over an fp32 tile: keys k-step kk sits at columns (kk / 4) * 64 + (kk % 4) * 8
-      auto a_cols = [](int kk) { return (uint32_t)((kk >> 2) * 64 + (kk & 3) * 8); };
-      bool ok = mbar_wait(kv_full, 0, error) && wait_stage(0);
-      if (ok) {
-        tc_fence_after();
+    constexpr uint32_t idesc_s = instr_desc(128, 128, false, false);
+    constexpr uint32_t idesc_acc = instr_desc(128, HD, false, true);
+    auto wait_stage = [&](int t) { return mbar_wait_all(&st_full[t % STAGES], (t / STAGES) & 1, error); };
+    // bf16 A operand written over an fp32 tile: keys k-step kk sits at columns (kk / 4) * 64 + (kk % 4) * 8
+    auto a_cols = [](int kk) { return (uint32_t)((kk >> 2) * 64 + (kk & 3) * 8); };
+    bool ok = mbar_wait_all(kv_full, 0, error) && wait_stage(0);
+    if (ok) {
+      tc_fence_after();
+      if (elect_one()) {
         mma_kmajor<HD>(tmem + C_S, smem + L::K, stage_at(0), idesc_s, false);  // S^T = K . Q_i^T
         mma_commit(s_full);
         mma_kmajor<HD>(tmem + C_DP, smem + L::V, stage_at(0) + TILE_BYTES, idesc_s, false);  // dP^T = V . dO_i^T
         mma_commit(dp_full);
       }
-      for (int t = 0; t < nt && ok; ++t) {
-        const uint32_t q_addr = smem_u32(stage_at(t)), do_addr = q_addr + TILE_BYTES;
-        if (!(ok = mbar_wait(p_full, t & 1, error))) break;
-        tc_fence_after();
+    }
+    for (int t = 0; t < nt && ok; ++t) {
+      const uint64_t q_desc = smem_desc(smem_u32(stage_at(t)), STRIP, 1024);
+      const uint64_t do_desc = smem_desc(smem_u32(stage_at(t)) + TILE_BYTES, STRIP, 1024);
+      if (!(ok = mbar_wait_all(p_full, t & 1, error))) break;
+      tc_fence_after();
+      if (elect_one()) {
 #pragma unroll
         for (int kk = 0; kk < 8; ++kk)  // dV += P^T . dO_i (16 queries per step; dO_i MN-major over the queries)
-          mma_bf16_ts(tmem + C_DV, tmem + C_S + a_cols(kk), smem_desc(do_addr + kk * 2048, STRIP, 1024), idesc_acc, (t > 0 || kk > 0) ? 1u : 0u);
-        if (t + 1 < nt) {
-          if (!(ok = wait_stage(t + 1))) break;
-          tc_fence_after();
+          mma_bf16_ts(tmem + C_DV, tmem + C_S + a_cols(kk), do_desc + kk * (2048 >> 4), idesc_acc, (t > 0 || kk > 0) ? 1u : 0u);
+      }
+      if (t + 1 < nt) {
+        if (!(ok = wait_stage(t + 1))) break;
+        tc_fence_after();
+        if (elect_one()) {
           mma_kmajor<HD>(tmem + C_S, smem + L::K, stage_at(t + 1), idesc_s, false);
           mma_commit(s_full);
         }
-        if (!(ok = mbar_wait(ds_full, t & 1, error))) break;
-        tc_fence_after();
+      }
+      if (!(ok = mbar_wait_all(ds_full, t & 1, error))) break;
+      tc_fence_after();
+      if (elect_one()) {
 #pragma unroll
         for (int kk = 0; kk < 8; ++kk)  // dK += dS^T . Q_i
-          mma_bf16_ts(tmem + C_DK, tmem + C_DP + a_cols(kk), smem_desc(q_addr + kk * 2048, STRIP, 1024), idesc_acc, (t > 0 || kk > 0) ? 1u : 0u);
+          mma_bf16_ts(tmem + C_DK, tmem + C_DP + a_cols(kk), q_desc + kk * (2048 >> 4), idesc_acc, (t > 0 || kk > 0) ? 1u : 0u);
         mma_commit(&st_empty[t % STAGES]);  // Q_i, dO_i (and its lse / delta, read before ds_full) are done with
         if (t + 1 < nt) {
           mma_kmajor<HD>(tmem + C_DP, smem + L::V, stage_at(t + 1) + TILE_BYTES, idesc_s, false);
           mma_commit(dp_full);
         }
       }
-      if (ok) mma_commit(acc_full);
     }
+    if (ok && elect_one()) mma_commit(acc_full);
   } else {
     const int quarter = warp & 3, half = (warp - 2) >> 2;
     const int r = quarter * 32 + lane;  // key row within the tile
@@ -685,8 +697,8 @@ k_attn_bwd_dkv(const __grid_constant__ CUtensorMap map_qkv, const __grid_constan
     for (int t = 0; t < nt && ok; ++t) {
       const int i = kt + t;
       const float* stat = reinterpret_cast<const float*>(stage_at(t) + 2 * TILE_BYTES) + half * 64;  // lse, then (+128) delta
-      if (!(ok = mbar_wait_warp_spin(&st_full[t % STAGES], (t / STAGES) & 1, error))) break;  // lse / delta have landed
-      if (!(ok = mbar_wait_warp_spin(s_full, t & 1, error))) break;
+      if (!(ok = mbar_wait_all(&st_full[t % STAGES], (t / STAGES) & 1, error))) break;  // lse / delta have landed
+      if (!(ok = mbar_wait_all(s_full, t & 1, error))) break;
       tc_fence_after();
       float p[64];
       {
@@ -711,7 +723,7 @@ k_attn_bwd_dkv(const __grid_constant__ CUtensorMap map_qkv, const __grid_constan
       tc_fence_before();
       __syncwarp();
       if (lane == 0) mbar_arrive(p_full);
-      if (!(ok = mbar_wait_warp_spin(dp_full, t & 1, error))) break;
+      if (!(ok = mbar_wait_all(dp_full, t & 1, error))) break;
       tc_fence_after();
       {
         uint32_t dp[2][32], pk[32];
@@ -731,7 +743,7 @@ k_attn_bwd_dkv(const __grid_constant__ CUtensorMap map_qkv, const __grid_constan
       __syncwarp();
       if (lane == 0) mbar_arrive(ds_full);
     }
-    if (ok) ok = mbar_wait_warp_spin(acc_full, 0, error);
+    if (ok) ok = mbar_wait_all(acc_full, 0, error);
     if (ok) {
       tc_fence_after();
       constexpr int COLS = HD / 2;
