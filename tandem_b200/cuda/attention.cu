@@ -22,6 +22,7 @@
 #include <math.h>
 #include <stdint.h>
 
+#include "f32x2.cuh"
 #include "launch.cuh"
 #include "tcgen05.cuh"
 
@@ -228,15 +229,18 @@ k_attn_fwd_ws(const __grid_constant__ CUtensorMap map, __nv_bfloat16* __restrict
             if (c * 32 + e > r) raw[c][e] = 0xff800000u;  // -inf
       }
       {
-        // eight independent running maxima: a single chain of 128 dependent FMNMX would cost ~5 cycles each
+        // eight independent running maxima, two elements at a time: a single chain of dependent maxima would cost ~5 cycles each
         float part[8];
 #pragma unroll
-        for (int e = 0; e < 8; ++e) part[e] = -INFINITY;
+        for (int e = 0; e < 8; ++e) part[e] = __uint_as_float(raw[0][e]);
 #pragma unroll
-        for (int c = 0; c < 4; ++c)
+        for (int e = 8; e < 120; e += 16)
 #pragma unroll
-          for (int e = 0; e < 32; ++e) part[e & 7] = fmaxf(part[e & 7], __uint_as_float(raw[c][e]));
-        mx = fmaxf(fmaxf(fmaxf(part[0], part[1]), fmaxf(part[2], part[3])), fmaxf(fmaxf(part[4], part[5]), fmaxf(part[6], part[7])));
+          for (int u = 0; u < 8; ++u)
+            part[u] = max3(part[u], __uint_as_float(raw[(e + u) >> 5][(e + u) & 31]), __uint_as_float(raw[(e + 8 + u) >> 5][(e + 8 + u) & 31]));
+#pragma unroll
+        for (int u = 0; u < 8; ++u) part[u] = fmaxf(part[u], __uint_as_float(raw[3][24 + u]));
+        mx = max3(max3(part[0], part[1], part[2]), max3(part[3], part[4], part[5]), fmaxf(part[6], part[7]));
       }
       if (j == 0) {
         m_used = mx;
@@ -259,22 +263,26 @@ k_attn_fwd_ws(const __grid_constant__ CUtensorMap map, __nv_bfloat16* __restrict
         }
       }
       const float mc = m_used * scale_log2e;
-      float sums[4] = {0.f, 0.f, 0.f, 0.f};
+      const f32x2 scale2 = pair2(scale_log2e, scale_log2e), shift2 = pair2(-mc, -mc);
+      f32x2 sums01 = pair2(0.f, 0.f), sums23 = sums01;  // four running sums: columns 0, 1, 2, 3 modulo 4
 #pragma unroll
       for (int hh = 0; hh < 2; ++hh) {  // 64 keys at a time: 32 registers of bf16 pairs
         uint32_t pk[32];
 #pragma unroll
         for (int e = 0; e < 32; ++e) {
           const int col = hh * 64 + 2 * e;
-          const float p0 = ex2_approx(fmaf(__uint_as_float(raw[col >> 5][col & 31]), scale_log2e, -mc));
-          const float p1 = ex2_approx(fmaf(__uint_as_float(raw[(col + 1) >> 5][(col + 1) & 31]), scale_log2e, -mc));
-          sums[(2 * e) & 3] += p0;
-          sums[(2 * e + 1) & 3] += p1;
-          const __nv_bfloat162 pp = __floats2bfloat162_rn(p0, p1);
-          pk[e] = *reinterpret_cast<const uint32_t*>(&pp);
+          float p0, p1;
+          split2(fma2(pair2(__uint_as_float(raw[col >> 5][col & 31]), __uint_as_float(raw[col >> 5][(col & 31) + 1])), scale2, shift2), &p0, &p1);
+          const f32x2 p = pair2(ex2_approx(p0), ex2_approx(p1));
+          if (e & 1) sums23 = add2(sums23, p);
+          else sums01 = add2(sums01, p);
+          pk[e] = bf16_pair(p);
         }
         tmem_st32(tS + hh * 32, pk);  // P over the first 64 columns of S: keys 2c, 2c+1 in column c
       }
+      float sums[4];
+      split2(sums01, &sums[0], &sums[1]);
+      split2(sums23, &sums[2], &sums[3]);
       l += (sums[0] + sums[1]) + (sums[2] + sums[3]);
       tmem_st_wait();
       tc_fence_before();
@@ -500,18 +508,19 @@ k_attn_bwd_dq(const __grid_constant__ CUtensorMap map_qkv, const __grid_constant
       __syncwarp();
       if (lane == 0) mbar_arrive(sdp_read);
       uint32_t pk[32];
-      const bool diagonal = j == qt;
+      if (j == qt) {  // the diagonal tile: exp2(-inf) = 0 for keys beyond the query
+#pragma unroll
+        for (int col = 0; col < 64; ++col)
+          if (half * 64 + col > r) s[col >> 5][col & 31] = 0xff800000u;
+      }
+      const f32x2 scale_log2e2 = pair2(c2, c2), shift2 = pair2(neg_lse2, neg_lse2), minus_delta2 = pair2(-delta, -delta), scale2 = pair2(scale, scale);
 #pragma unroll
       for (int e = 0; e < 32; ++e) {
-        float ds2[2];
-#pragma unroll
-        for (int u = 0; u < 2; ++u) {
-          const int col = 2 * e + u;  // within this thread's 64 columns
-          float p = ex2_approx(fmaf(__uint_as_float(s[col >> 5][col & 31]), c2, neg_lse2));
-          if (diagonal && half * 64 + col > r) p = 0.f;
-          ds2[u] = p * (__uint_as_float(dp[col >> 5][col & 31]) - delta) * scale;
-        }
-        pk[e] = pack_bf16(ds2[0], ds2[1]);
+        const int c = (2 * e) >> 5, i = (2 * e) & 31;  // within this thread's 64 columns
+        float p0, p1;
+        split2(fma2(pair2(__uint_as_float(s[c][i]), __uint_as_float(s[c][i + 1])), scale_log2e2, shift2), &p0, &p1);
+        const f32x2 over = add2(pair2(__uint_as_float(dp[c][i]), __uint_as_float(dp[c][i + 1])), minus_delta2);
+        pk[e] = bf16_pair(mul2(mul2(pair2(ex2_approx(p0), ex2_approx(p1)), over), scale2));
       }
       tmem_st32(tmem + C_DS + (j & 1) * 64 + lane_base + half * 32, pk);
       tmem_st_wait();
@@ -700,23 +709,33 @@ k_attn_bwd_dkv(const __grid_constant__ CUtensorMap map_qkv, const __grid_constan
       if (!(ok = mbar_wait_all(&st_full[t % STAGES], (t / STAGES) & 1, error))) break;  // lse / delta have landed
       if (!(ok = mbar_wait_all(s_full, t & 1, error))) break;
       tc_fence_after();
-      float p[64];
+      const float4* lse4 = reinterpret_cast<const float4*>(stat);
+      const float4* delta4 = reinterpret_cast<const float4*>(stat + 128);
+      const f32x2 minus_log2e2 = pair2(-1.4426950408889634f, -1.4426950408889634f), scale_log2e2 = pair2(c2, c2);
+      f32x2 p[32];
       {
-        uint32_t s[2][32];
+        uint32_t s[2][32], pk[32];
         tmem_ld32(tmem + C_S + lane_base + half * 64, s[0]);
         tmem_ld32(tmem + C_S + lane_base + half * 64 + 32, s[1]);
         tmem_ld_wait();
-        const bool diagonal = i == kt;
+        if (i == kt) {  // the diagonal tile: exp2(-inf) = 0 for keys after the query
 #pragma unroll
-        for (int col = 0; col < 64; ++col) {
-          const float x = ex2_approx(fmaf(__uint_as_float(s[col >> 5][col & 31]), c2, -1.4426950408889634f * stat[col]));
-          p[col] = (diagonal && r > half * 64 + col) ? 0.f : x;  // key after the query
+          for (int col = 0; col < 64; ++col)
+            if (r > half * 64 + col) s[col >> 5][col & 31] = 0xff800000u;
         }
-      }
-      {
-        uint32_t pk[32];
 #pragma unroll
-        for (int e = 0; e < 32; ++e) pk[e] = pack_bf16(p[2 * e], p[2 * e + 1]);
+        for (int q = 0; q < 16; ++q) {
+          const float4 l4 = lse4[q];
+#pragma unroll
+          for (int u = 0; u < 2; ++u) {
+            const int e = 2 * q + u, c = (2 * e) >> 5, k = (2 * e) & 31;
+            const f32x2 shift = mul2(minus_log2e2, u == 0 ? pair2(l4.x, l4.y) : pair2(l4.z, l4.w));
+            float x0, x1;
+            split2(fma2(pair2(__uint_as_float(s[c][k]), __uint_as_float(s[c][k + 1])), scale_log2e2, shift), &x0, &x1);
+            p[e] = pair2(ex2_approx(x0), ex2_approx(x1));
+            pk[e] = bf16_pair(p[e]);
+          }
+        }
         tmem_st32(tmem + C_S + lane_base + half * 64, pk);
         tmem_st_wait();
       }
@@ -730,11 +749,17 @@ k_attn_bwd_dkv(const __grid_constant__ CUtensorMap map_qkv, const __grid_constan
         tmem_ld32(tmem + C_DP + lane_base + half * 64, dp[0]);
         tmem_ld32(tmem + C_DP + lane_base + half * 64 + 32, dp[1]);
         tmem_ld_wait();
+        const f32x2 scale2 = pair2(scale, scale), minus_one2 = pair2(-1.f, -1.f);
 #pragma unroll
-        for (int e = 0; e < 32; ++e) {
-          const float a = p[2 * e] * (__uint_as_float(dp[(2 * e) >> 5][(2 * e) & 31]) - stat[128 + 2 * e]) * scale;
-          const float c = p[2 * e + 1] * (__uint_as_float(dp[(2 * e + 1) >> 5][(2 * e + 1) & 31]) - stat[128 + 2 * e + 1]) * scale;
-          pk[e] = pack_bf16(a, c);
+        for (int q = 0; q < 16; ++q) {
+          const float4 d4 = delta4[q];
+#pragma unroll
+          for (int u = 0; u < 2; ++u) {
+            const int e = 2 * q + u, c = (2 * e) >> 5, k = (2 * e) & 31;
+            const f32x2 dp2 = pair2(__uint_as_float(dp[c][k]), __uint_as_float(dp[c][k + 1]));
+            const f32x2 over = fma2(u == 0 ? pair2(d4.x, d4.y) : pair2(d4.z, d4.w), minus_one2, dp2);  // dP - delta
+            pk[e] = bf16_pair(mul2(mul2(p[e], over), scale2));
+          }
         }
         tmem_st32(tmem + C_DP + lane_base + half * 64, pk);
         tmem_st_wait();
