@@ -38,6 +38,16 @@ __device__ __forceinline__ void load8(const __nv_bfloat16* p, float* f) {
   }
 }
 
+__device__ __forceinline__ void unpack8(const uint4& v, float* f) {
+  const __nv_bfloat162* h = reinterpret_cast<const __nv_bfloat162*>(&v);
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    float2 t = __bfloat1622float2(h[i]);
+    f[2 * i] = t.x;
+    f[2 * i + 1] = t.y;
+  }
+}
+
 __device__ __forceinline__ void store8(__nv_bfloat16* p, const float* f) {
   uint4 v;
   __nv_bfloat162* h = reinterpret_cast<__nv_bfloat162*>(&v);
@@ -109,23 +119,13 @@ k_ln_fwd(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ 
 // current row is requested before the row's reductions start.  With one row per warp in flight the kernel ran at
 // the pace of one memory round trip per row (0.42 of the copy bandwidth); two rows per warp and two blocks per SM
 // keep about 100 KB per SM on the way.
-__device__ __forceinline__ void unpack8(const uint4& v, float* f) {
-  const __nv_bfloat162* h = reinterpret_cast<const __nv_bfloat162*>(&v);
-#pragma unroll
-  for (int i = 0; i < 4; ++i) {
-    float2 t = __bfloat1622float2(h[i]);
-    f[2 * i] = t.x;
-    f[2 * i + 1] = t.y;
-  }
-}
-
 template <int MAXV>
 __global__ void __launch_bounds__(256, MAXV <= 4 ? 2 : 1)
 k_ln_bwd(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ w,
          const float* __restrict__ mean_in, const float* __restrict__ rstd_in, const __nv_bfloat16* __restrict__ add,
          __nv_bfloat16* __restrict__ dx, float* __restrict__ part, int M, int D) {
   tb::pdl_enter();
-  extern __shared__ float sh[];  // [warps][2][D]
+  extern __shared__ __align__(16) float sh[];  // [warps][2][D]
   const int warps = blockDim.x >> 5;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int nvec = D >> 3;
@@ -219,9 +219,9 @@ k_ln_bwd(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* __restrict__
     const int vi = lane + 32 * j;
     if (vi < nvec) {
 #pragma unroll
-      for (int e = 0; e < 8; ++e) {
-        sh[(warp * 2 + 0) * D + vi * 8 + e] = dw[j][e];
-        sh[(warp * 2 + 1) * D + vi * 8 + e] = db[j][e];
+      for (int q = 0; q < 2; ++q) {  // 16-byte stores: scalar ones, 32 bytes apart from lane to lane, meet in the same bank eight at a time
+        *reinterpret_cast<float4*>(sh + (warp * 2 + 0) * D + vi * 8 + 4 * q) = *reinterpret_cast<const float4*>(&dw[j][4 * q]);
+        *reinterpret_cast<float4*>(sh + (warp * 2 + 1) * D + vi * 8 + 4 * q) = *reinterpret_cast<const float4*>(&db[j][4 * q]);
       }
     }
   }
@@ -243,8 +243,17 @@ k_reduce_partials(const float* __restrict__ part, int parts, int width, __nv_bfl
   const int cx = threadIdx.x & 31, ry = threadIdx.x >> 5;
   const int c = blockIdx.x * 32 + cx;
   float acc = 0.f;
-  if (c < width)
-    for (int p = ry; p < parts; p += 8) acc += part[(size_t)p * width + c];
+  if (c < width) {
+    int p = ry;
+    for (; p + 56 < parts; p += 64) {  // eight loads in flight, added in order
+      float v[8];
+#pragma unroll
+      for (int u = 0; u < 8; ++u) v[u] = part[(size_t)(p + 8 * u) * width + c];
+#pragma unroll
+      for (int u = 0; u < 8; ++u) acc += v[u];
+    }
+    for (; p < parts; p += 8) acc += part[(size_t)p * width + c];
+  }
   sh[ry][cx] = acc;
   __syncthreads();
   if (ry == 0 && c < width) {
@@ -307,32 +316,36 @@ k_col_sum(const __nv_bfloat16* __restrict__ x, int M, int N, int ld, float* __re
 }
 
 // The same job for matrices whose rows are 16-byte aligned (N, ld multiples of 8): every thread reads 16-byte vectors
-// (8 columns) and keeps four row-strided loads in flight, so the kernel runs at memory speed instead of at the pace of
-// 2-byte loads.  256 threads = 32 column vectors (256 columns) x 8 row lanes; grid.x = column groups of 256, grid.y = row
-// slices.  Same partials, tickets and summation order per column as k_col_sum, hence the same result.
+// (8 columns) and keeps eight row-strided loads in flight.  256 threads = 8 column vectors (64 columns) x 32 row lanes; grid.x =
+// column groups of 64, grid.y = row slices.  What bounds it is loads in flight: groups of 256 columns x 8 row lanes
+// with four loads each left most SMs idle for narrow matrices (96 blocks at N = 768; 8192 x 768: 11.3 us).
+// Same partials, tickets and summation order per column as k_col_sum, hence the same result.
 __global__ void __launch_bounds__(256)
 k_col_sum_vec(const __nv_bfloat16* __restrict__ x, int M, int N, int ld, float* __restrict__ part, unsigned* tickets,
               __nv_bfloat16* __restrict__ out) {
   tb::pdl_enter();
-  __shared__ float sh[8][256 + 8];
+  __shared__ __align__(16) float sh[32][64 + 4];
   __shared__ int is_last;
-  const int cx = threadIdx.x & 31, ry = threadIdx.x >> 5;
-  const int col = blockIdx.x * 256 + cx * 8;
+  const int cx = threadIdx.x & 7, ry = threadIdx.x >> 3;
+  const int col = blockIdx.x * 64 + cx * 8;
   const int rows_per = (M + gridDim.y - 1) / gridDim.y;
   const int r0 = blockIdx.y * rows_per, r1 = min(M, r0 + rows_per);
   float acc[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
   if (col < N) {
     int r = r0 + ry;
-    for (; r + 24 < r1; r += 32) {
-      float v[4][8];
+    for (; r + 224 < r1; r += 256) {
+      uint4 v[8];
 #pragma unroll
-      for (int u = 0; u < 4; ++u) load8(x + (size_t)(r + 8 * u) * ld + col, v[u]);
+      for (int u = 0; u < 8; ++u) v[u] = *reinterpret_cast<const uint4*>(x + (size_t)(r + 32 * u) * ld + col);
 #pragma unroll
-      for (int u = 0; u < 4; ++u)
+      for (int u = 0; u < 8; ++u) {
+        float f[8];
+        unpack8(v[u], f);
 #pragma unroll
-        for (int e = 0; e < 8; ++e) acc[e] += v[u][e];
+        for (int e = 0; e < 8; ++e) acc[e] += f[e];
+      }
     }
-    for (; r < r1; r += 8) {
+    for (; r < r1; r += 32) {
       float v[8];
       load8(x + (size_t)r * ld + col, v);
 #pragma unroll
@@ -340,16 +353,14 @@ k_col_sum_vec(const __nv_bfloat16* __restrict__ x, int M, int N, int ld, float* 
     }
   }
 #pragma unroll
-  for (int e = 0; e < 8; ++e) sh[ry][cx * 8 + e] = acc[e];
+  for (int q = 0; q < 2; ++q) *reinterpret_cast<float4*>(&sh[ry][cx * 8 + 4 * q]) = *reinterpret_cast<const float4*>(&acc[4 * q]);
   __syncthreads();
-  {
-    const int c = blockIdx.x * 256 + threadIdx.x;
-    if (c < N) {
-      float t = 0.f;
+  const int c = blockIdx.x * 64 + threadIdx.x;
+  if (threadIdx.x < 64 && c < N) {
+    float t = 0.f;
 #pragma unroll
-      for (int k = 0; k < 8; ++k) t += sh[k][threadIdx.x];
-      part[(size_t)blockIdx.y * N + c] = t;
-    }
+    for (int k = 0; k < 32; ++k) t += sh[k][threadIdx.x];
+    part[(size_t)blockIdx.y * N + c] = t;
   }
   if (tickets == nullptr) return;
   __threadfence();
@@ -359,14 +370,19 @@ k_col_sum_vec(const __nv_bfloat16* __restrict__ x, int M, int N, int ld, float* 
   if (!is_last) return;
   __threadfence();
   {
-    const int c = blockIdx.x * 256 + threadIdx.x;
-    if (c < N) {
-      // eight lanes of every-eighth slice, combined in lane order: the grouping of k_reduce_partials
-      float lanes[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
-      for (int p = 0; p < (int)gridDim.y; ++p) lanes[p & 7] += __ldcg(part + (size_t)p * N + c);
+    // eight lanes of every-eighth slice, combined in lane order: the grouping of k_reduce_partials
+    const int lx = threadIdx.x & 63;
+    for (int lane8 = threadIdx.x >> 6; lane8 < 8; lane8 += 4) {
+      float t = 0.f;
+      if (blockIdx.x * 64 + lx < N)
+        for (int p = lane8; p < (int)gridDim.y; p += 8) t += __ldcg(part + (size_t)p * N + blockIdx.x * 64 + lx);
+      sh[lane8][lx] = t;
+    }
+    __syncthreads();
+    if (threadIdx.x < 64 && c < N) {
       float t = 0.f;
 #pragma unroll
-      for (int k = 0; k < 8; ++k) t += lanes[k];
+      for (int k = 0; k < 8; ++k) t += sh[k][threadIdx.x];
       out[c] = __float2bfloat16_rn(t);
     }
   }
@@ -383,8 +399,30 @@ k_xent_fwd(const __nv_bfloat16* __restrict__ logits, const long long* __restrict
   const int row = blockIdx.x;
   const __nv_bfloat16* z = logits + (size_t)row * ld;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, warps = blockDim.x >> 5;
+  // Both passes keep eight loads in flight per thread: at a 50304-wide vocabulary one load at a time ran at a tenth of the
+  // memory rate (4096 rows: 666 us).  The order of the sum is one column per thread and step.
   float m = -INFINITY;
-  for (int i = threadIdx.x; i < V; i += blockDim.x) m = fmaxf(m, __bfloat162float(z[i]));
+  {
+    int i = threadIdx.x;
+    const int vectors = ((uintptr_t)z & 15) == 0 ? V / 8 : 0;  // 16-byte loads where the row allows
+    int v = threadIdx.x;
+    for (; v < vectors; v += 4 * blockDim.x) {
+      uint4 x[4];
+#pragma unroll
+      for (int u = 0; u < 4; ++u)
+        if (v + u * (int)blockDim.x < vectors) x[u] = *reinterpret_cast<const uint4*>(z + 8 * (v + u * blockDim.x));
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        if (v + u * (int)blockDim.x < vectors) {
+          float f[8];
+          unpack8(x[u], f);
+#pragma unroll
+          for (int e = 0; e < 8; ++e) m = fmaxf(m, f[e]);
+        }
+      }
+    }
+    for (i += 8 * vectors; i < V; i += blockDim.x) m = fmaxf(m, __bfloat162float(z[i]));
+  }
   m = warp_max(m);
   if (lane == 0) red[warp] = m;
   __syncthreads();
@@ -392,7 +430,17 @@ k_xent_fwd(const __nv_bfloat16* __restrict__ logits, const long long* __restrict
   for (int k = 1; k < warps; ++k) m = fmaxf(m, red[k]);
   __syncthreads();
   float s = 0.f;
-  for (int i = threadIdx.x; i < V; i += blockDim.x) s += __expf(__bfloat162float(z[i]) - m);
+  {
+    int i = threadIdx.x;
+    for (; i + 7 * (int)blockDim.x < V; i += 8 * blockDim.x) {
+      __nv_bfloat16 x[8];
+#pragma unroll
+      for (int u = 0; u < 8; ++u) x[u] = z[i + u * blockDim.x];
+#pragma unroll
+      for (int u = 0; u < 8; ++u) s += __expf(__bfloat162float(x[u]) - m);
+    }
+    for (; i < V; i += blockDim.x) s += __expf(__bfloat162float(z[i]) - m);
+  }
   s = warp_sum(s);
   if (lane == 0) red[warp] = s;
   __syncthreads();
@@ -416,11 +464,27 @@ k_xent_bwd(__nv_bfloat16* __restrict__ logits, const long long* __restrict__ tar
   const float l = lse[row];
   const float scale = grad_scale[0] * inv_rows;
   const int t = (int)targets[row];
-  for (int i = threadIdx.x; i < width; i += blockDim.x) {
-    float g = 0.f;
-    if (i < V) g = (__expf(__bfloat162float(z[i]) - l) - (i == t ? 1.f : 0.f)) * scale;
-    z[i] = __float2bfloat16_rn(g);
+  auto grad = [&](float x, int i) { return i < V ? (__expf(x - l) - (i == t ? 1.f : 0.f)) * scale : 0.f; };
+  // 16-byte vectors, four in flight per thread, where the row allows (element by element: 424 us at 4096 x 50304)
+  const int vectors = ((uintptr_t)z & 15) == 0 ? width / 8 : 0;
+  for (int v = threadIdx.x; v < vectors; v += 4 * blockDim.x) {
+    uint4 x[4];
+#pragma unroll
+    for (int u = 0; u < 4; ++u)
+      if (v + u * (int)blockDim.x < vectors) x[u] = *reinterpret_cast<const uint4*>(z + 8 * (v + u * blockDim.x));
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      const int at = 8 * (v + u * blockDim.x);
+      if (v + u * (int)blockDim.x < vectors) {
+        float f[8];
+        unpack8(x[u], f);
+#pragma unroll
+        for (int e = 0; e < 8; ++e) f[e] = grad(f[e], at + e);
+        store8(z + at, f);
+      }
+    }
   }
+  for (int i = 8 * vectors + threadIdx.x; i < width; i += blockDim.x) z[i] = __float2bfloat16_rn(grad(__bfloat162float(z[i]), i));
 }
 
 // loss = mean(per_row) in a fixed order (one block).
@@ -456,30 +520,57 @@ k_embed_fwd(const long long* __restrict__ idx, const __nv_bfloat16* __restrict__
   }
 }
 
-// dtok32[idx[row]] += dy[row] (fp32 atomics); dpos[t] = sum over batch of dy[b, t] (fixed order).
+// dtok32[idx[row]] += dy[row] (fp32 atomics, four columns each); dpos[t] = sum over batch of dy[b, t] (fixed order).
+__device__ __forceinline__ void add4(float* p, float a, float b, float c, float d) {
+  asm volatile("red.relaxed.gpu.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(p), "f"(a), "f"(b), "f"(c), "f"(d) : "memory");
+}
+
 __global__ void __launch_bounds__(256)
 k_embed_bwd_tok(const long long* __restrict__ idx, const __nv_bfloat16* __restrict__ dy, float* __restrict__ dtok32, int rows, int D) {
   tb::pdl_enter();
-  for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < (long long)rows * D; i += (long long)gridDim.x * blockDim.x) {
-    const int row = (int)(i / D), c = (int)(i % D);
-    atomicAdd(dtok32 + (size_t)idx[row] * D + c, __bfloat162float(dy[i]));
+  const int nvec = D >> 3;
+  for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < (long long)rows * nvec; i += (long long)gridDim.x * blockDim.x) {
+    const int row = (int)(i / nvec), v = (int)(i % nvec);
+    float f[8];
+    load8(dy + (size_t)row * D + v * 8, f);
+    float* dst = dtok32 + (size_t)idx[row] * D + v * 8;
+    add4(dst, f[0], f[1], f[2], f[3]);
+    add4(dst + 4, f[4], f[5], f[6], f[7]);
   }
 }
 
 __global__ void __launch_bounds__(256)
 k_embed_bwd_pos(const __nv_bfloat16* __restrict__ dy, __nv_bfloat16* __restrict__ dpos, int B, int T, int D) {
   tb::pdl_enter();
-  for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < (long long)T * D; i += (long long)gridDim.x * blockDim.x) {
-    float acc = 0.f;
-    for (int b = 0; b < B; ++b) acc += __bfloat162float(dy[(size_t)b * T * D + i]);
-    dpos[i] = __float2bfloat16_rn(acc);
+  const long long vectors = (long long)T * D / 8;
+  for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < vectors; i += (long long)gridDim.x * blockDim.x) {
+    float acc[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+#pragma unroll 4
+    for (int b = 0; b < B; ++b) {
+      float f[8];
+      load8(dy + (size_t)b * T * D + i * 8, f);
+#pragma unroll
+      for (int e = 0; e < 8; ++e) acc[e] += f[e];
+    }
+    store8(dpos + i * 8, acc);
   }
 }
 
+// n is a multiple of 8 (whole embedding rows).
 __global__ void __launch_bounds__(256) k_f32_to_bf16(const float* __restrict__ in, __nv_bfloat16* __restrict__ out, long long n) {
   tb::pdl_enter();
-  for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x)
-    out[i] = __float2bfloat16_rn(in[i]);
+  const long long stride = (long long)gridDim.x * blockDim.x;
+  for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n / 8; i += 2 * stride) {
+    float4 v[4];
+#pragma unroll
+    for (int u = 0; u < 4; ++u)
+      if (i + (u >> 1) * stride < n / 8) v[u] = *reinterpret_cast<const float4*>(in + (i + (u >> 1) * stride) * 8 + 4 * (u & 1));
+#pragma unroll
+    for (int u = 0; u < 2; ++u) {
+      const float f[8] = {v[2 * u].x, v[2 * u].y, v[2 * u].z, v[2 * u].w, v[2 * u + 1].x, v[2 * u + 1].y, v[2 * u + 1].z, v[2 * u + 1].w};
+      if (i + u * stride < n / 8) store8(out + (i + u * stride) * 8, f);
+    }
+  }
 }
 
 int grid_for(long long work, int per_block, int cap) {
@@ -507,8 +598,9 @@ int tb_layernorm_fwd(const void* x, const void* w, const void* b, void* y, float
 
 // scratch: fp32 [blocks * 2 * D] with blocks = tb_layernorm_bwd_blocks(M).
 // Few rows: one row per warp on as many SMs as it takes (at 1024 rows four rows per warp would leave 116 SMs idle);
-// many rows: several rows per warp, so that the row look-ahead has something to fetch.
-int tb_layernorm_bwd_blocks(int M) { return M < 8192 ? grid_for(M, 8, 296) : grid_for(M, 8 * 4, 592); }
+// many rows: several rows per warp, so that the row look-ahead has something to fetch, and no more blocks than run at a time
+// (two per SM), because each one ends with a reduction over its warps and leaves a row of partial sums to add up.
+int tb_layernorm_bwd_blocks(int M) { return M < 8192 ? grid_for(M, 8, 296) : grid_for(M, 8 * 4, 296); }
 
 int tb_layernorm_bwd_add(const void* dy, const void* x, const void* w, const float* mean, const float* rstd, const void* add, void* dx,
                          void* dw, void* db, float* scratch, int M, int D, cudaStream_t s);
@@ -545,7 +637,7 @@ int tb_layernorm_bwd_add(const void* dy, const void* x, const void* w, const flo
 int tb_col_sum(const void* x, int M, int N, int ld, void* out_bf16, float* scratch, cudaStream_t s) {
   const int slices = M >= 2048 ? 32 : (M >= 256 ? 8 : 1);
   const bool vectors = (N & 7) == 0 && (ld & 7) == 0 && ((uintptr_t)x & 15) == 0;
-  dim3 grid(vectors ? (N + 255) / 256 : (N + 31) / 32, slices);
+  dim3 grid(vectors ? (N + 63) / 64 : (N + 31) / 32, slices);
   // One launch: each column group's last block finishes the sum.  The ticket words come from a fixed pool handed
   // out round-robin, so launches in flight at the same time never share one (a pool's worth of launches would
   // have to overlap); matrices wider than the pool take the two-kernel path.
@@ -605,10 +697,11 @@ int tb_embed_fwd(const long long* idx, const void* tok, const void* pos, void* o
 // dtok32: zeroed fp32 [V, D] scratch; dtok / dpos: bf16 outputs.
 int tb_embed_bwd(const long long* idx, const void* dy, float* dtok32, void* dtok, void* dpos, int B, int T, int D, int V,
                  cudaStream_t s) {
+  if (D % 8) return -20;
   tb_note_launch(3);
-  tb::launch(k_embed_bwd_tok, dim3(grid_for((long long)B * T * D, 256, 148 * 8)), dim3(256), 0, s, idx, (const __nv_bfloat16*)dy, dtok32, B * T, D);
-  tb::launch(k_f32_to_bf16, dim3(grid_for((long long)V * D, 256, 148 * 8)), dim3(256), 0, s, (const float*)dtok32, (__nv_bfloat16*)dtok, (long long)V * D);
-  tb::launch(k_embed_bwd_pos, dim3(grid_for((long long)T * D, 256, 148 * 8)), dim3(256), 0, s, (const __nv_bfloat16*)dy, (__nv_bfloat16*)dpos, B, T, D);
+  tb::launch(k_embed_bwd_tok, dim3(grid_for((long long)B * T * (D / 8), 256, 148 * 8)), dim3(256), 0, s, idx, (const __nv_bfloat16*)dy, dtok32, B * T, D);
+  tb::launch(k_f32_to_bf16, dim3(grid_for((long long)V * D / 8, 256, 148 * 8)), dim3(256), 0, s, (const float*)dtok32, (__nv_bfloat16*)dtok, (long long)V * D);
+  tb::launch(k_embed_bwd_pos, dim3(grid_for((long long)T * D / 8, 256, 148 * 8)), dim3(256), 0, s, (const __nv_bfloat16*)dy, (__nv_bfloat16*)dpos, B, T, D);
   return (int)cudaGetLastError();
 }
 

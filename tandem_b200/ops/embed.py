@@ -27,6 +27,8 @@ class _Embedding(torch.autograd.Function):
         (V, D), (S, _) = ctx.shapes
         B, T = idx.shape
         dy = dy.contiguous()
+        if dy.data_ptr() % 16:  # a contiguous slice may start anywhere; the kernels read 16-byte vectors
+            dy = dy.clone()
         dtok32 = torch.zeros(V, D, dtype=torch.float32, device=dy.device)
         dtok = torch.empty(V, D, dtype=torch.bfloat16, device=dy.device)
         dpos = torch.zeros(S, D, dtype=torch.bfloat16, device=dy.device)

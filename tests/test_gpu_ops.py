@@ -527,3 +527,69 @@ def test_optimizer_during_backward_equals_optimizer_after_backward():
     assert after[0] == during[0], (after[0], during[0])
     assert torch.equal(after[1], during[1])  # the same arithmetic on the same gradients: bit for bit
     assert after[0] == replayed[0] and torch.equal(after[1], replayed[1])
+
+
+@pytest.mark.parametrize("V,ld,first", [(65, 72, 0), (1003, 1003, 0), (1003, 1008, 0), (8200, 8200, 3), (50304, 50304, 0), (2049, 2056, 8)])
+def test_cross_entropy_row_layouts(V, ld, first):
+    """Rows that can and cannot be read in 16-byte vectors (odd strides, a first element in mid-vector), vector tails and
+    batches of loads that end early; gradients land in place and nothing outside the columns changes."""
+    from tandem_b200 import ops
+
+    rows = 37
+    store = torch.full((rows * ld + first + 8,), 7.0, dtype=torch.bfloat16, device="cuda")
+    logits = store[first:first + rows * ld].view(rows, ld)[:, :V]
+    logits.copy_(rnd(rows, V) * 3)
+    targets = torch.randint(0, V, (rows,), device="cuda")
+    targets[0], targets[1] = 0, V - 1
+    z = logits.detach().double().requires_grad_()
+    want = torch.nn.functional.cross_entropy(z, targets)
+    (want * 2).backward()
+    x = logits.detach().requires_grad_()
+    loss = ops.cross_entropy(x, targets)
+    (grad,) = torch.autograd.grad(loss * 2, x)
+    assert abs(loss.item() - want.item()) < 1e-5 * want.item()
+    # one bf16 rounding, and exp(z - lse) with lse ~ 10 rounded to fp32
+    assert ((grad.double() - z.grad).abs() <= 2.0**-8 * z.grad.abs() + 2e-6 / rows).all()
+    if first:
+        assert (store[:first] == 7).all()
+    assert (store[first + rows * ld:] == 7).all()
+
+
+@pytest.mark.parametrize("n,offset", [(1, 0), (3, 0), (4097, 0), (4096, 1), (1000003, 0), (1000002, 2)])
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+def test_fused_adamw_alignment_and_tails(n, offset, dtype):
+    """Arrays that start off a 16-byte boundary take the element-wise loop, aligned ones four elements at a time plus a tail:
+    the arithmetic is the same, so both must agree bit for bit."""
+    from tandem_b200.ops import fused_adamw
+
+    scalars = (1 - 3e-5, 0.1, 0.999, 0.001, 0.0316, 1e-8, -3e-3)
+
+    def run(at):
+        gen = torch.Generator(device="cuda").manual_seed(3)
+        arrays = [torch.zeros(n + 8, device="cuda") for _ in range(3)] + [torch.zeros(n + 8, device="cuda", dtype=dtype), torch.zeros(n + 8, device="cuda", dtype=torch.bfloat16)]
+        p, m, v, g, shadow = (a[at:at + n] for a in arrays)
+        p.copy_(torch.randn(n, device="cuda", generator=gen)), m.copy_(torch.randn(n, device="cuda", generator=gen) * 0.1)
+        v.copy_(torch.rand(n, device="cuda", generator=gen)), g.copy_(torch.randn(n, device="cuda", generator=gen))
+        fused_adamw(p, g, m, v, scalars, True, shadow)
+        for a in arrays:
+            assert (a[:at] == 0).all() and (a[at + n:] == 0).all()
+        return p, m, v, shadow
+
+    for a, b in zip(run(offset), run(5)):
+        assert torch.equal(a, b)
+
+
+@pytest.mark.parametrize("M,N,ld", [(1, 64, 64), (300, 72, 72), (2048, 768, 768), (5000, 200, 208), (8191, 4104, 4104)])
+def test_column_sums_in_vectors(M, N, ld):
+    from tandem_b200.ops._lib import lib
+
+    x = rnd(M, ld)
+    scratch = torch.empty(32 * N, dtype=torch.float32, device="cuda")
+    out, again = (torch.empty(N, dtype=torch.bfloat16, device="cuda") for _ in range(2))
+    s = torch.cuda.current_stream().cuda_stream
+    assert lib().tb_col_sum(x.data_ptr(), M, N, ld, out.data_ptr(), scratch.data_ptr(), s) == 0
+    assert lib().tb_col_sum(x.data_ptr(), M, N, ld, again.data_ptr(), scratch.data_ptr(), s) == 0
+    want = x[:, :N].double().sum(0)
+    # fp32 partial sums of M unit normals (error ~ sqrt(M) * 6e-8 * a few), then one bf16 rounding
+    assert ((out.double() - want).abs() <= 2.0**-8 * want.abs() + 1e-5 * M**0.5).all()
+    assert torch.equal(out, again)
