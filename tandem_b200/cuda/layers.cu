@@ -582,6 +582,20 @@ int grid_for(long long work, int per_block, int cap) {
 
 extern "C" {
 
+// Work queued on `waiter` from here on starts after everything now queued on `signaller`.  One event per thread and device:
+// a wait refers to the record before it, so the event is free again as soon as this returns, and no other thread can
+// record it in between.
+int tb_stream_wait(cudaStream_t waiter, cudaStream_t signaller) {
+  static thread_local cudaEvent_t events[64] = {};
+  int dev = 0;
+  cudaError_t e = cudaGetDevice(&dev);
+  if (e == cudaSuccess && dev >= 64) e = cudaErrorInvalidDevice;
+  if (e == cudaSuccess && events[dev] == nullptr) e = cudaEventCreateWithFlags(&events[dev], cudaEventDisableTiming);
+  if (e == cudaSuccess) e = cudaEventRecord(events[dev], signaller);
+  if (e == cudaSuccess) e = cudaStreamWaitEvent(waiter, events[dev], 0);
+  return (int)e;
+}
+
 int tb_layernorm_fwd(const void* x, const void* w, const void* b, void* y, float* mean, float* rstd, int M, int D, float eps,
                      cudaStream_t s) {
   if (D % 8 || D > 32 * 8 * 8) return -20;

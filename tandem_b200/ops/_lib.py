@@ -30,6 +30,7 @@ def lib():
         "tb_col_sum": ([vp, i, i, i, vp, vp, vp], i),
         "tb_xent_fwd": ([vp, vp, vp, vp, vp, i, i, i, vp], i),
         "tb_xent_bwd": ([vp, vp, vp, vp, i, i, i, i, vp], i),
+        "tb_stream_wait": ([vp, vp], i),
         "tb_embed_fwd": ([vp, vp, vp, vp, i, i, i, vp], i),
         "tb_embed_bwd": ([vp, vp, vp, vp, vp, i, i, i, i, vp], i),
     }
@@ -42,7 +43,29 @@ def lib():
 
 
 def stream(t):
-    return torch.cuda.current_stream(t.device).cuda_stream
+    """The raw handle of the current stream of t's device (building a torch.cuda.Stream object for it costs 2 us a launch)."""
+    return torch._C._cuda_getCurrentRawStream(t.get_device())
+
+
+class _Untracked:
+    """Stands in for the context of an autograd function whose backward cannot be asked for."""
+
+    def save_for_backward(self, *tensors):
+        pass
+
+
+def run(function, *args):
+    """function.apply(*args), or its forward alone (5 us less a call) where nothing can want the node: gradients are off, and
+    no functorch transform, forward-mode level or tracer is active, which Function.apply would have to answer or refuse."""
+    if (torch.is_grad_enabled() or torch.autograd.forward_ad._current_level >= 0 or torch._C._functorch.peek_interpreter_stack() is not None
+            or torch._C._get_tracing_state() is not None):
+        return function.apply(*args)
+    return function.forward(_Untracked(), *args)
+
+
+def stream_wait(waiter, signaller):
+    """Work queued on raw stream `waiter` from here on starts after everything now queued on `signaller`."""
+    check_rc(lib().tb_stream_wait(waiter, signaller), "stream wait")
 
 
 def pad8(n):
@@ -52,6 +75,8 @@ def pad8(n):
 def empty_padded(rows, cols, dtype, device):
     """A [rows, cols] view of [rows, pad8(cols)] storage: every row starts 16-byte aligned."""
     ld = pad8(cols)
+    if ld == cols:
+        return torch.empty(rows, cols, dtype=dtype, device=device)
     return torch.empty(rows, ld, dtype=dtype, device=device)[:, :cols]
 
 

@@ -11,7 +11,7 @@ import functools
 
 import torch
 
-from ._lib import check_rc, lib, need_bf16, stream
+from ._lib import check_rc, lib, need_bf16, run, stream
 
 
 @functools.cache
@@ -60,7 +60,7 @@ class _CausalAttention(torch.autograd.Function):
 
 def causal_attention(qkv, heads):
     """Returns [B, T, dim]."""
-    return _CausalAttention.apply(qkv, heads)
+    return run(_CausalAttention, qkv, heads)
 
 
 def attention_error():

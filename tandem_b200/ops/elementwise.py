@@ -8,7 +8,7 @@ from ..parallel.symm import _ll_array, _ptr_array, check_rc, cuda_lib
 
 
 def _stream(t):
-    return torch.cuda.current_stream(t.device).cuda_stream
+    return torch._C._cuda_getCurrentRawStream(t.get_device())
 
 
 def multi_copy(flat, pairs):

@@ -11,7 +11,7 @@ import os
 
 import torch
 
-from ._lib import check_rc, empty_padded, lib, need_bf16, pad8, stream
+from ._lib import check_rc, empty_padded, lib, need_bf16, pad8, run, stream, stream_wait
 
 BIAS, GELU, RESIDUAL, DGELU, ACCUMULATE, OUT_F32 = 1, 2, 4, 8, 16, 32
 
@@ -31,10 +31,10 @@ def _repack(t2):
 
 
 def gemm(a, b, M, N, K, lda, ldb, a_mn, b_mn, flags=0, bias=None, aux_in=None, aux_out=None, out=None, out_dtype=torch.bfloat16,
-         workspace=None):
+         workspace=None, on=None):
     """out[M, N] = op(a) . op(b) (+ epilogue).  Returns a [M, N] view with a 16-byte-aligned row stride.
     workspace: a uint8 tensor of at least lib().tb_gemm_workspace_bytes(M, N, K) bytes, for callers that launch on another stream
-    than the one their memory belongs to (else it is allocated here)."""
+    than the one their memory belongs to (else it is allocated here).  on: the raw stream to launch on (default: the current one)."""
     if out is None:
         out = empty_padded(M, N, out_dtype, a.device)
     ldc = out.stride(0) if M > 1 else pad8(N)
@@ -53,7 +53,7 @@ def gemm(a, b, M, N, K, lda, ldb, a_mn, b_mn, flags=0, bias=None, aux_in=None, a
                             bias.data_ptr() if bias is not None else None,
                             aux_in.data_ptr() if aux_in is not None else None,
                             aux_out.data_ptr() if aux_out is not None else None, 0,
-                            workspace.data_ptr() if workspace is not None else None, need, stream(a))
+                            workspace.data_ptr() if workspace is not None else None, need, stream(a) if on is None else on)
     if rc in (-11, -12):
         raise RuntimeError(f"gemm: operand not addressable by TMA (M={M} N={N} K={K} lda={lda} ldb={ldb} a_mn={a_mn} b_mn={b_mn} "
                            f"a={a.data_ptr():#x} b={b.data_ptr():#x}): {lib().tb_gemm_last_error().decode()}")
@@ -114,7 +114,7 @@ def _parameter_grads_beside(dy2, ldy, x2, ldx, dtype, want_w, want_b):
         db = _grad_bias(dy2, ldy) if want_b else None
         return dw, db, lambda: None
     dev = dy2.device
-    main = torch.cuda.current_stream(dev)
+    main = stream(dy2)
     side = _side_streams.get(dev.index)
     if side is None:
         side = _side_streams[dev.index] = torch.cuda.Stream(dev)
@@ -130,16 +130,16 @@ def _parameter_grads_beside(dy2, ldy, x2, ldx, dtype, want_w, want_b):
     if want_b:
         db = torch.empty(N, dtype=torch.bfloat16, device=dev)
         scratch = torch.empty(32 * N, dtype=torch.float32, device=dev)
-    side.wait_stream(main)
-    with torch.cuda.stream(side):
-        if want_w:
-            gemm(dy2, x2, N, K, M, ldy, ldx, True, True, 0, out=dw, workspace=workspace)
-        if want_b:
-            check_rc(lib().tb_col_sum(dy2.data_ptr(), M, N, ldy, db.data_ptr(), scratch.data_ptr(), side.cuda_stream), "col_sum")
+    beside = side.cuda_stream
+    stream_wait(beside, main)
+    if want_w:
+        gemm(dy2, x2, N, K, M, ldy, ldx, True, True, 0, out=dw, workspace=workspace, on=beside)
+    if want_b:
+        check_rc(lib().tb_col_sum(dy2.data_ptr(), M, N, ldy, db.data_ptr(), scratch.data_ptr(), beside), "col_sum")
     keep = (scratch, workspace)  # released by the caller's frame, after the join
 
     def join():
-        main.wait_stream(side)
+        stream_wait(main, beside)
         return keep
 
     return dw, db, join
@@ -233,11 +233,11 @@ class _MLP(torch.autograd.Function):
 def linear(x, weight, bias=None, gelu=False, residual=None):
     if gelu:
         raise ValueError("use ops.mlp for the GELU MLP (its backward fuses GELU's derivative into a GEMM epilogue)")
-    return _Linear.apply(x, weight, bias, residual)
+    return run(_Linear, x, weight, bias, residual)
 
 
 def mlp(x, w1, b1, w2, b2, residual):
-    return _MLP.apply(x, w1, b1, w2, b2, residual)
+    return run(_MLP, x, w1, b1, w2, b2, residual)
 
 
 def gemm_error():

@@ -4,7 +4,7 @@ partial sums of the weight and bias gradients, reduced in a fixed order."""
 
 import torch
 
-from ._lib import check_rc, lib, need_bf16, stream
+from ._lib import check_rc, lib, need_bf16, run, stream
 
 
 class _LayerNorm(torch.autograd.Function):
@@ -14,16 +14,15 @@ class _LayerNorm(torch.autograd.Function):
         x2 = x.reshape(-1, x.shape[-1]).contiguous()
         M, D = x2.shape
         y = torch.empty_like(x2)
-        mean = torch.empty(M, dtype=torch.float32, device=x.device)
-        rstd = torch.empty(M, dtype=torch.float32, device=x.device)
-        check_rc(lib().tb_layernorm_fwd(x2.data_ptr(), w.data_ptr(), b.data_ptr(), y.data_ptr(), mean.data_ptr(), rstd.data_ptr(),
+        stats = torch.empty(2, M, dtype=torch.float32, device=x.device)  # the rows' mean and 1 / std
+        check_rc(lib().tb_layernorm_fwd(x2.data_ptr(), w.data_ptr(), b.data_ptr(), y.data_ptr(), stats.data_ptr(), stats.data_ptr() + 4 * M,
                                         M, D, eps, stream(x)), "layernorm forward")
-        ctx.save_for_backward(x2, w, mean, rstd)
+        ctx.save_for_backward(x2, w, stats)
         return y.view(x.shape)
 
     @staticmethod
     def backward(ctx, dy):
-        x2, w, mean, rstd = ctx.saved_tensors
+        x2, w, stats = ctx.saved_tensors
         M, D = x2.shape
         dy2 = dy.reshape(-1, D).contiguous()
         dx = torch.empty_like(x2)
@@ -31,13 +30,13 @@ class _LayerNorm(torch.autograd.Function):
         db = torch.empty_like(w)
         blocks = lib().tb_layernorm_bwd_blocks(M)
         scratch = torch.empty(blocks * 2 * D, dtype=torch.float32, device=x2.device)
-        check_rc(lib().tb_layernorm_bwd(dy2.data_ptr(), x2.data_ptr(), w.data_ptr(), mean.data_ptr(), rstd.data_ptr(), dx.data_ptr(),
+        check_rc(lib().tb_layernorm_bwd(dy2.data_ptr(), x2.data_ptr(), w.data_ptr(), stats.data_ptr(), stats.data_ptr() + 4 * M, dx.data_ptr(),
                                         dw.data_ptr(), db.data_ptr(), scratch.data_ptr(), M, D, stream(x2)), "layernorm backward")
         return dx.view(dy.shape), dw, db, None
 
 
 def layer_norm(x, weight, bias, eps=1e-5):
-    return _LayerNorm.apply(x, weight, bias, eps)
+    return run(_LayerNorm, x, weight, bias, eps)
 
 
 class _ResidualLayerNorm(torch.autograd.Function):
@@ -51,16 +50,15 @@ class _ResidualLayerNorm(torch.autograd.Function):
         x2 = x.reshape(-1, x.shape[-1]).contiguous()
         M, D = x2.shape
         y = torch.empty_like(x2)
-        mean = torch.empty(M, dtype=torch.float32, device=x.device)
-        rstd = torch.empty(M, dtype=torch.float32, device=x.device)
-        check_rc(lib().tb_layernorm_fwd(x2.data_ptr(), w.data_ptr(), b.data_ptr(), y.data_ptr(), mean.data_ptr(), rstd.data_ptr(),
+        stats = torch.empty(2, M, dtype=torch.float32, device=x.device)  # the rows' mean and 1 / std
+        check_rc(lib().tb_layernorm_fwd(x2.data_ptr(), w.data_ptr(), b.data_ptr(), y.data_ptr(), stats.data_ptr(), stats.data_ptr() + 4 * M,
                                         M, D, eps, stream(x)), "layernorm forward")
-        ctx.save_for_backward(x2, w, mean, rstd)
+        ctx.save_for_backward(x2, w, stats)
         return x.view_as(x), y.view(x.shape)
 
     @staticmethod
     def backward(ctx, dres, dy):
-        x2, w, mean, rstd = ctx.saved_tensors
+        x2, w, stats = ctx.saved_tensors
         M, D = x2.shape
         if dy is None:
             return dres, None, None, None
@@ -71,7 +69,7 @@ class _ResidualLayerNorm(torch.autograd.Function):
         db = torch.empty_like(w)
         blocks = lib().tb_layernorm_bwd_blocks(M)
         scratch = torch.empty(blocks * 2 * D, dtype=torch.float32, device=x2.device)
-        check_rc(lib().tb_layernorm_bwd_add(dy2.data_ptr(), x2.data_ptr(), w.data_ptr(), mean.data_ptr(), rstd.data_ptr(),
+        check_rc(lib().tb_layernorm_bwd_add(dy2.data_ptr(), x2.data_ptr(), w.data_ptr(), stats.data_ptr(), stats.data_ptr() + 4 * M,
                                             None if add is None else add.data_ptr(), dx.data_ptr(), dw.data_ptr(), db.data_ptr(),
                                             scratch.data_ptr(), M, D, stream(x2)), "layernorm backward")
         return dx.view(dy.shape), dw, db, None
@@ -79,4 +77,4 @@ class _ResidualLayerNorm(torch.autograd.Function):
 
 def residual_layer_norm(x, weight, bias, eps=1e-5):
     """Returns (x, LayerNorm(x)); use the returned x for the residual connection."""
-    return _ResidualLayerNorm.apply(x, weight, bias, eps)
+    return run(_ResidualLayerNorm, x, weight, bias, eps)

@@ -593,3 +593,58 @@ def test_column_sums_in_vectors(M, N, ld):
     # fp32 partial sums of M unit normals (error ~ sqrt(M) * 6e-8 * a few), then one bf16 rounding
     assert ((out.double() - want).abs() <= 2.0**-8 * want.abs() + 1e-5 * M**0.5).all()
     assert torch.equal(out, again)
+
+
+def test_operators_without_gradients_equal_those_with():
+    """Where gradients are off the operators skip the autograd node: same results; transforms that the node refuses or a
+    saved-tensor hook still meet it."""
+    from tandem_b200 import ops
+
+    x, w, b = rnd(256, 128), rnd(384, 128, scale=0.05), rnd(384)
+    ln_w, ln_b, w2, b2 = rnd(128), rnd(128), rnd(128, 384, scale=0.05), rnd(128)
+    qkv = rnd(2, 128, 3 * 128)
+    idx, tok, pos = torch.randint(0, 50, (2, 128), device="cuda"), rnd(50, 128), rnd(128, 128)
+    calls = [lambda: ops.linear(x, w, b), lambda: ops.layer_norm(x, ln_w, ln_b), lambda: ops.residual_layer_norm(x, ln_w, ln_b)[1],
+             lambda: ops.mlp(x, w, b, w2, b2, x), lambda: ops.causal_attention(qkv, 2), lambda: ops.embedding(idx, tok, pos),
+             lambda: ops.cross_entropy(x, torch.zeros(256, dtype=torch.long, device="cuda"))]
+    for call in calls:
+        want = call()
+        with torch.no_grad():
+            got = call()
+        assert torch.equal(got, want) and not got.requires_grad
+    with torch.no_grad(), pytest.raises(RuntimeError):
+        torch.func.vmap(lambda v: ops.linear(v, w, b))(x.unsqueeze(0))
+    with torch.no_grad(), torch.autograd.forward_ad.dual_level(), pytest.raises((RuntimeError, NotImplementedError)):
+        ops.linear(torch.autograd.forward_ad.make_dual(x, torch.ones_like(x)), w, b)
+
+
+def test_stream_wait_from_two_threads():
+    """Each thread orders its own pair of streams through one native call, many times over."""
+    import threading
+
+    from tandem_b200.ops._lib import stream_wait
+
+    bad = []
+
+    def work():
+        torch.cuda.set_device(0)
+        first, second = torch.cuda.Stream(), torch.cuda.Stream()
+        x = torch.zeros(1 << 20, device="cuda")
+        torch.cuda.synchronize()
+        for i in range(50):
+            with torch.cuda.stream(first):
+                x.fill_(float(i))
+            stream_wait(second.cuda_stream, first.cuda_stream)
+            with torch.cuda.stream(second):
+                y = x + 1
+            stream_wait(first.cuda_stream, second.cuda_stream)
+            second.synchronize()
+            if not (y == i + 1).all():
+                bad.append(i)
+
+    threads = [threading.Thread(target=work) for _ in range(2)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not bad
