@@ -350,12 +350,13 @@ template <int HD>
 struct BwdDqSmem {
   static constexpr int TILE_BYTES = (HD / 64) * STRIP;
   static constexpr int Q = 0, DO = TILE_BYTES, RING = 2 * TILE_BYTES;
-  static constexpr int SLOTS_FIT = (225 * 1024 - RING) / TILE_BYTES;
-  static constexpr int SLOTS = SLOTS_FIT > 6 ? 6 : SLOTS_FIT;
+  // K_j is read again by dQ += dS.K_j, V_j only by dP: with rings of their own V_j+2 is on its way as soon as the scores of
+  // tile j are done.  In one ring of five slots (head dim 128) it waited for K_j's slot, 1500 of 3350 cycles per tile.
+  static constexpr int K_SLOTS = HD == 128 ? 3 : 4, V_SLOTS = HD == 128 ? 2 : 3, SLOTS = K_SLOTS + V_SLOTS;
   static constexpr int DELTA = RING + SLOTS * TILE_BYTES;  // [2 halves][128 rows] floats
   static constexpr int BARS = DELTA + 1024;
   static constexpr int TOTAL = BARS + 256;
-  static_assert(SLOTS >= 4, "K_j, V_j, K_j+1 and V_j+1 are in flight together");
+  static_assert(TOTAL <= 227 * 1024, "shared memory of one SM");
 };
 
 template <int HD>
@@ -373,7 +374,7 @@ k_attn_bwd_dq(const __grid_constant__ CUtensorMap map_qkv, const __grid_constant
     return;
   }
   using L = BwdDqSmem<HD>;
-  constexpr int TILE_BYTES = L::TILE_BYTES, SLOTS = L::SLOTS;
+  constexpr int TILE_BYTES = L::TILE_BYTES, SLOTS = L::SLOTS, K_SLOTS = L::K_SLOTS, V_SLOTS = L::V_SLOTS;  // K's slots, then V's
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem + L::BARS);
   uint64_t *qdo_full = bars, *sdp_full = bars + 1, *sdp_read = bars + 2, *ds_full = bars + 3 /* [2] */, *dq_full = bars + 5,
            *kv_full = bars + 6, *kv_empty = bars + 6 + SLOTS;
@@ -420,26 +421,35 @@ k_attn_bwd_dq(const __grid_constant__ CUtensorMap map_qkv, const __grid_constant
       load_tile<HD>(smem + L::Q, &map_qkv, qdo_full, h * HD, b * T + qt * TILE);
       load_tile<HD>(smem + L::DO, &map_do, qdo_full, h * HD, b * T + qt * TILE);
     }
-    for (int ld = 0; ld < 2 * n; ++ld) {  // load 2j: K_j, load 2j+1: V_j
-      const int s = ld % SLOTS, j = ld >> 1, part = ld & 1;
-      if (!mbar_wait_all(&kv_empty[s], ((ld / SLOTS) & 1) ^ 1, error)) break;
+    bool ok = true;
+    auto load = [&](int part, int j, int s, int turn) {  // part 0: K_j, 1: V_j, into slot s for the turn-th time
+      if (j >= n || !ok || !(ok = mbar_wait_all(&kv_empty[s], (turn & 1) ^ 1, error))) return;
       if (elect_one()) {
         mbar_expect_tx(&kv_full[s], TILE_BYTES);
         load_tile<HD>(smem + L::RING + s * TILE_BYTES, &map_qkv, &kv_full[s], (1 + part) * d + h * HD, b * T + j * TILE);
       }
+    };
+    load(0, 0, 0, 0);
+    for (int j = 0; j < n && ok; ++j) {  // in the order in which the slots come free
+      load(1, j, K_SLOTS + j % V_SLOTS, j / V_SLOTS);
+      load(0, j + 1, (j + 1) % K_SLOTS, (j + 1) / K_SLOTS);
     }
   } else if (warp == 1) {
     constexpr uint32_t idesc_s = instr_desc(128, 128, false, false);
     constexpr uint32_t idesc_dq = instr_desc(128, HD, false, true);
-    auto slot_of = [&](int ld) { return smem + L::RING + (ld % SLOTS) * TILE_BYTES; };
-    auto wait_slot = [&](int ld) { return mbar_wait_all(&kv_full[ld % SLOTS], (ld / SLOTS) & 1, error); };
-    auto issue_scores = [&](int j) {
-      mma_kmajor<HD>(tmem + C_S, smem + L::Q, slot_of(2 * j), idesc_s, false);        // S  = Q . K_j^T
-      mma_kmajor<HD>(tmem + C_DP, smem + L::DO, slot_of(2 * j + 1), idesc_s, false);  // dP = dO . V_j^T
-      mma_commit(sdp_full);
-      mma_commit(&kv_empty[(2 * j + 1) % SLOTS]);  // V_j has no other reader
+    auto k_of = [&](int j) { return smem + L::RING + (j % K_SLOTS) * TILE_BYTES; };
+    auto v_of = [&](int j) { return smem + L::RING + (K_SLOTS + j % V_SLOTS) * TILE_BYTES; };
+    auto wait_tiles = [&](int j) {
+      return mbar_wait_all(&kv_full[j % K_SLOTS], (j / K_SLOTS) & 1, error) &&
+             mbar_wait_all(&kv_full[K_SLOTS + j % V_SLOTS], (j / V_SLOTS) & 1, error);
     };
-    bool ok = mbar_wait_all(qdo_full, 0, error) && wait_slot(0) && wait_slot(1);
+    auto issue_scores = [&](int j) {
+      mma_kmajor<HD>(tmem + C_S, smem + L::Q, k_of(j), idesc_s, false);    // S  = Q . K_j^T
+      mma_kmajor<HD>(tmem + C_DP, smem + L::DO, v_of(j), idesc_s, false);  // dP = dO . V_j^T
+      mma_commit(sdp_full);
+      mma_commit(&kv_empty[K_SLOTS + j % V_SLOTS]);  // V_j has no other reader
+    };
+    bool ok = mbar_wait_all(qdo_full, 0, error) && wait_tiles(0);
     if (ok) {
       tc_fence_after();
       if (elect_one()) issue_scores(0);
@@ -447,18 +457,18 @@ k_attn_bwd_dq(const __grid_constant__ CUtensorMap map_qkv, const __grid_constant
     for (int j = 0; j < n && ok; ++j) {
       if (j + 1 < n) {
         if (!(ok = mbar_wait_all(sdp_read, j & 1, error))) break;  // tile j's S and dP are in registers
-        if (!(ok = wait_slot(2 * j + 2) && wait_slot(2 * j + 3))) break;
+        if (!(ok = wait_tiles(j + 1))) break;
         tc_fence_after();
         if (elect_one()) issue_scores(j + 1);
       }
       if (!(ok = mbar_wait_all(&ds_full[j & 1], (j >> 1) & 1, error))) break;
       tc_fence_after();
       if (elect_one()) {
-        const uint64_t k_desc = smem_desc(smem_u32(slot_of(2 * j)), STRIP, 1024);
+        const uint64_t k_desc = smem_desc(smem_u32(k_of(j)), STRIP, 1024);
 #pragma unroll
         for (int kk = 0; kk < 8; ++kk)  // dQ += dS . K_j: dS from TMEM (16 keys = 8 columns per step), K_j MN-major over the keys
           mma_bf16_ts(tmem + C_DQ, tmem + C_DS + (j & 1) * 64 + kk * 8, k_desc + kk * (2048 >> 4), idesc_dq, (j > 0 || kk > 0) ? 1u : 0u);
-        mma_commit(&kv_empty[(2 * j) % SLOTS]);
+        mma_commit(&kv_empty[j % K_SLOTS]);
       }
     }
     if (ok && elect_one()) mma_commit(dq_full);
