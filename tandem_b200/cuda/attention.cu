@@ -68,7 +68,10 @@ __device__ __forceinline__ void mma_kmajor(uint32_t d_tmem, const uint8_t* a, co
 // The two tiles alternate on the tensor pipe: while the softmax threads of one tile work on S_i(j) (exponentials), the
 // MMAs of the other tile run.  P stays in TMEM: it is written as bf16 pairs over the first 64 columns of S and is the
 // A operand of a TMEM-sourced MMA (measured against staging P in shared memory: 198 vs 223 us at T = 2048, head dim 128).
-// TMEM: S_0 [0,128)  S_1 [128,256)  O_0 [256,256+HD)  O_1 [256+HD, 256+2HD).
+// TMEM: S_0 [0,128)  S_1 [128,256)  O_0 [256,256+HD)  O_1 [256+HD, 256+2HD), and with head dim 64, where there is room,
+// P_0 [384,448)  P_1 [448,512).  A P of its own lets S_i(j+1) be issued as soon as the softmax threads have S_i(j) in registers,
+// so that they never wait for scores; P_i(j) and the rescale of O_i then wait for P.V of step j-1 (pv_done), which is long
+// over by the time the maxima are known.  With head dim 128 P lies over S, and S_i(j+1) follows P_i(j).V_j.
 template <int HD>
 struct Fwd2Smem {
   static constexpr int TILE_BYTES = (HD / 64) * STRIP;
@@ -99,7 +102,9 @@ k_attn_fwd_ws(const __grid_constant__ CUtensorMap map, __nv_bfloat16* __restrict
   constexpr int TILE_BYTES = L::TILE_BYTES, SLOTS = L::SLOTS;
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem + L::BARS);
   uint64_t *q_full = bars, *s_full = bars + 2, *p_full = bars + 4, *o_full = bars + 6, *kv_full = bars + 8, *kv_empty = bars + 8 + SLOTS;
-  uint32_t* holder = reinterpret_cast<uint32_t*>(bars + 8 + 2 * SLOTS);
+  uint64_t *s_read = bars + 8 + 2 * SLOTS, *pv_done = s_read + 2;
+  uint32_t* holder = reinterpret_cast<uint32_t*>(pv_done + 2);
+  constexpr bool OWN_P = HD == 64;
   const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;  // warp: known to be uniform
   const int n_qt = T / TILE, n_pairs = (n_qt + 1) / 2;
   // consecutive CTAs share one head's K and V (they stay in L2), longest pair first within the head
@@ -117,6 +122,8 @@ k_attn_fwd_ws(const __grid_constant__ CUtensorMap map, __nv_bfloat16* __restrict
       mbar_init(&s_full[i], 1);
       mbar_init(&p_full[i], 4);  // one arrival per softmax warp of the tile
       mbar_init(&o_full[i], 1);
+      mbar_init(&s_read[i], 4);
+      mbar_init(&pv_done[i], 1);
     }
     for (int s = 0; s < SLOTS; ++s) {
       mbar_init(&kv_full[s], 1);
@@ -169,7 +176,7 @@ k_attn_fwd_ws(const __grid_constant__ CUtensorMap map, __nv_bfloat16* __restrict
       const uint64_t v_desc = smem_desc(smem_u32(slot_of(2 * j + 1)), STRIP, 1024);
 #pragma unroll
       for (int kk = 0; kk < 8; ++kk)
-        mma_bf16_ts(tO, tmem + i * 128 + kk * 8, v_desc + kk * (2048 >> 4), idesc_o, (j > 0 || kk > 0) ? 1u : 0u);  // 16 keys = 8 TMEM columns of P
+        mma_bf16_ts(tO, (OWN_P ? tmem + 384 + i * 64 : tmem + i * 128) + kk * 8, v_desc + kk * (2048 >> 4), idesc_o, (j > 0 || kk > 0) ? 1u : 0u);  // 16 keys = 8 TMEM columns of P
     };
     bool ok = mbar_wait_all(&q_full[0], 0, error) && (!n1 || mbar_wait_all(&q_full[1], 0, error)) && wait_slot(0);
     if (ok) {
@@ -180,25 +187,54 @@ k_attn_fwd_ws(const __grid_constant__ CUtensorMap map, __nv_bfloat16* __restrict
         mma_commit(&kv_empty[0]);  // K_0 is free once these have read it
       }
     }
-    for (int j = 0; j < n_steps && ok; ++j) {
-      if (!(ok = wait_slot(2 * j + 1))) break;                       // V_j
-      if (j + 1 < n_steps && !(ok = wait_slot(2 * j + 2))) break;    // K_{j+1}
-      tc_fence_after();
-      for (int i = 0; i < 2 && ok; ++i) {
-        const int n_i = i == 0 ? n0 : n1;
-        if (j >= n_i) continue;
-        if (!(ok = mbar_wait_all(&p_full[i], j & 1, error))) break;  // P_i(j) is in place, O_i rescaled if it had to be
-        tc_fence_after();
-        if (elect_one()) {
-          issue_pv(i, j);
-          if (j == n_i - 1) mma_commit(&o_full[i]);
-          else issue_s(i, j + 1);
+    if constexpr (OWN_P) {
+      for (int j = 0; j < n_steps && ok; ++j) {
+        if (j + 1 < n_steps) {
+          if (!(ok = wait_slot(2 * j + 2))) break;                      // K_{j+1}
+          for (int i = 0; i < 2 && ok; ++i) {
+            if (j + 1 >= (i == 0 ? n0 : n1)) continue;
+            if (!(ok = mbar_wait_all(&s_read[i], j & 1, error))) break;  // S_i(j) is in registers
+            tc_fence_after();
+            if (elect_one()) issue_s(i, j + 1);
+          }
+          if (!ok) break;
+          if (elect_one()) mma_commit(&kv_empty[(2 * j + 2) % SLOTS]);
         }
+        if (!(ok = wait_slot(2 * j + 1))) break;                        // V_j
+        for (int i = 0; i < 2 && ok; ++i) {
+          const int n_i = i == 0 ? n0 : n1;
+          if (j >= n_i) continue;
+          if (!(ok = mbar_wait_all(&p_full[i], j & 1, error))) break;    // P_i(j) is in place, O_i rescaled if it had to be
+          tc_fence_after();
+          if (elect_one()) {
+            issue_pv(i, j);
+            mma_commit(j == n_i - 1 ? &o_full[i] : &pv_done[i]);
+          }
+        }
+        if (!ok) break;
+        if (elect_one()) mma_commit(&kv_empty[(2 * j + 1) % SLOTS]);
       }
-      if (!ok) break;
-      if (elect_one()) {
-        mma_commit(&kv_empty[(2 * j + 1) % SLOTS]);                      // V_j
-        if (j + 1 < n_steps) mma_commit(&kv_empty[(2 * j + 2) % SLOTS]);  // K_{j+1}
+    } else {
+      for (int j = 0; j < n_steps && ok; ++j) {
+        if (!(ok = wait_slot(2 * j + 1))) break;                       // V_j
+        if (j + 1 < n_steps && !(ok = wait_slot(2 * j + 2))) break;    // K_{j+1}
+        tc_fence_after();
+        for (int i = 0; i < 2 && ok; ++i) {
+          const int n_i = i == 0 ? n0 : n1;
+          if (j >= n_i) continue;
+          if (!(ok = mbar_wait_all(&p_full[i], j & 1, error))) break;  // P_i(j) is in place, O_i rescaled if it had to be
+          tc_fence_after();
+          if (elect_one()) {
+            issue_pv(i, j);
+            if (j == n_i - 1) mma_commit(&o_full[i]);
+            else issue_s(i, j + 1);
+          }
+        }
+        if (!ok) break;
+        if (elect_one()) {
+          mma_commit(&kv_empty[(2 * j + 1) % SLOTS]);                      // V_j
+          if (j + 1 < n_steps) mma_commit(&kv_empty[(2 * j + 2) % SLOTS]);  // K_{j+1}
+        }
       }
     }
   } else {
@@ -211,6 +247,7 @@ k_attn_fwd_ws(const __grid_constant__ CUtensorMap map, __nv_bfloat16* __restrict
     const uint32_t lane_base = (uint32_t)(quarter * 32) << 16;
     const uint32_t tS = tmem + i * 128 + lane_base;
     const uint32_t tO = tmem + 256 + i * HD + lane_base;
+    const uint32_t tP = OWN_P ? tmem + 384 + i * 64 + lane_base : tS;  // bf16: keys 2c, 2c+1 in column c
     float m_used = -INFINITY, l = 0.f;  // m_used in raw score units
     bool ok = true;
     for (int j = 0; j < n_i && ok; ++j) {
@@ -220,6 +257,11 @@ k_attn_fwd_ws(const __grid_constant__ CUtensorMap map, __nv_bfloat16* __restrict
 #pragma unroll
       for (int c = 0; c < 4; ++c) tmem_ld32(tS + c * 32, raw[c]);
       tmem_ld_wait();
+      if (OWN_P) {
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&s_read[i]);
+      }
       float mx = -INFINITY;
       if (j == qt) {  // the diagonal tile: keys beyond the query are masked
 #pragma unroll
@@ -241,6 +283,10 @@ k_attn_fwd_ws(const __grid_constant__ CUtensorMap map, __nv_bfloat16* __restrict
 #pragma unroll
         for (int u = 0; u < 8; ++u) part[u] = fmaxf(part[u], __uint_as_float(raw[3][24 + u]));
         mx = max3(max3(part[0], part[1], part[2]), max3(part[3], part[4], part[5]), fmaxf(part[6], part[7]));
+      }
+      if (OWN_P && j > 0) {
+        if (!(ok = mbar_wait_all(&pv_done[i], (j - 1) & 1, error))) break;
+        tc_fence_after();
       }
       if (j == 0) {
         m_used = mx;
@@ -278,7 +324,7 @@ k_attn_fwd_ws(const __grid_constant__ CUtensorMap map, __nv_bfloat16* __restrict
           else sums01 = add2(sums01, p);
           pk[e] = bf16_pair(p);
         }
-        tmem_st32(tS + hh * 32, pk);  // P over the first 64 columns of S: keys 2c, 2c+1 in column c
+        tmem_st32(tP + hh * 32, pk);  // head dim 128: over the first 64 columns of S
       }
       float sums[4];
       split2(sums01, &sums[0], &sums[1]);

@@ -316,15 +316,15 @@ k_col_sum(const __nv_bfloat16* __restrict__ x, int M, int N, int ld, float* __re
 }
 
 // The same job for matrices whose rows are 16-byte aligned (N, ld multiples of 8): every thread reads 16-byte vectors
-// (8 columns) and keeps eight row-strided loads in flight.  256 threads = 8 column vectors (64 columns) x 32 row lanes; grid.x =
-// column groups of 64, grid.y = row slices.  What bounds it is loads in flight: groups of 256 columns x 8 row lanes
-// with four loads each left most SMs idle for narrow matrices (96 blocks at N = 768; 8192 x 768: 11.3 us).
-// Same partials, tickets and summation order per column as k_col_sum, hence the same result.
-__global__ void __launch_bounds__(256)
+// (8 columns) and keeps sixteen row-strided loads in flight.  64 threads = 8 column vectors (64 columns) x 8 row lanes; grid.x =
+// column groups of 64, grid.y = row slices.  What bounds it is loads in flight: blocks of 256 columns with four loads
+// per thread left most SMs idle for narrow matrices (96 blocks at N = 768; 8192 x 768: 11.3 us, 6 us now).
+// Partials over row lanes 0 .. 7 in order; the slices are grouped as in k_reduce_partials.
+__global__ void __launch_bounds__(64)
 k_col_sum_vec(const __nv_bfloat16* __restrict__ x, int M, int N, int ld, float* __restrict__ part, unsigned* tickets,
               __nv_bfloat16* __restrict__ out) {
   tb::pdl_enter();
-  __shared__ __align__(16) float sh[32][64 + 4];
+  __shared__ __align__(16) float sh[8][64 + 4];
   __shared__ int is_last;
   const int cx = threadIdx.x & 7, ry = threadIdx.x >> 3;
   const int col = blockIdx.x * 64 + cx * 8;
@@ -332,34 +332,30 @@ k_col_sum_vec(const __nv_bfloat16* __restrict__ x, int M, int N, int ld, float* 
   const int r0 = blockIdx.y * rows_per, r1 = min(M, r0 + rows_per);
   float acc[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
   if (col < N) {
-    int r = r0 + ry;
-    for (; r + 224 < r1; r += 256) {
-      uint4 v[8];
+    for (int r = r0 + ry; r < r1; r += 8 * 16) {
+      uint4 v[16];
 #pragma unroll
-      for (int u = 0; u < 8; ++u) v[u] = *reinterpret_cast<const uint4*>(x + (size_t)(r + 32 * u) * ld + col);
+      for (int u = 0; u < 16; ++u)
+        if (r + 8 * u < r1) v[u] = *reinterpret_cast<const uint4*>(x + (size_t)(r + 8 * u) * ld + col);
 #pragma unroll
-      for (int u = 0; u < 8; ++u) {
-        float f[8];
-        unpack8(v[u], f);
+      for (int u = 0; u < 16; ++u) {
+        if (r + 8 * u < r1) {
+          float f[8];
+          unpack8(v[u], f);
 #pragma unroll
-        for (int e = 0; e < 8; ++e) acc[e] += f[e];
+          for (int e = 0; e < 8; ++e) acc[e] += f[e];
+        }
       }
-    }
-    for (; r < r1; r += 32) {
-      float v[8];
-      load8(x + (size_t)r * ld + col, v);
-#pragma unroll
-      for (int e = 0; e < 8; ++e) acc[e] += v[e];
     }
   }
 #pragma unroll
   for (int q = 0; q < 2; ++q) *reinterpret_cast<float4*>(&sh[ry][cx * 8 + 4 * q]) = *reinterpret_cast<const float4*>(&acc[4 * q]);
   __syncthreads();
   const int c = blockIdx.x * 64 + threadIdx.x;
-  if (threadIdx.x < 64 && c < N) {
+  if (c < N) {
     float t = 0.f;
 #pragma unroll
-    for (int k = 0; k < 32; ++k) t += sh[k][threadIdx.x];
+    for (int k = 0; k < 8; ++k) t += sh[k][threadIdx.x];
     part[(size_t)blockIdx.y * N + c] = t;
   }
   if (tickets == nullptr) return;
@@ -369,22 +365,19 @@ k_col_sum_vec(const __nv_bfloat16* __restrict__ x, int M, int N, int ld, float* 
   __syncthreads();
   if (!is_last) return;
   __threadfence();
-  {
+  if (c < N) {
     // eight lanes of every-eighth slice, combined in lane order: the grouping of k_reduce_partials
-    const int lx = threadIdx.x & 63;
-    for (int lane8 = threadIdx.x >> 6; lane8 < 8; lane8 += 4) {
-      float t = 0.f;
-      if (blockIdx.x * 64 + lx < N)
-        for (int p = lane8; p < (int)gridDim.y; p += 8) t += __ldcg(part + (size_t)p * N + blockIdx.x * 64 + lx);
-      sh[lane8][lx] = t;
-    }
-    __syncthreads();
-    if (threadIdx.x < 64 && c < N) {
-      float t = 0.f;
+    float lanes[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+#pragma unroll 2
+    for (int p = 0; p < (int)gridDim.y; p += 8) {
 #pragma unroll
-      for (int k = 0; k < 8; ++k) t += sh[k][threadIdx.x];
-      out[c] = __float2bfloat16_rn(t);
+      for (int k = 0; k < 8; ++k)
+        if (p + k < (int)gridDim.y) lanes[k] += __ldcg(part + (size_t)(p + k) * N + c);
     }
+    float t = 0.f;
+#pragma unroll
+    for (int k = 0; k < 8; ++k) t += lanes[k];
+    out[c] = __float2bfloat16_rn(t);
   }
   if (threadIdx.x == 0) tickets[blockIdx.x] = 0;
 }
@@ -612,9 +605,8 @@ int tb_layernorm_fwd(const void* x, const void* w, const void* b, void* y, float
 
 // scratch: fp32 [blocks * 2 * D] with blocks = tb_layernorm_bwd_blocks(M).
 // Few rows: one row per warp on as many SMs as it takes (at 1024 rows four rows per warp would leave 116 SMs idle);
-// many rows: several rows per warp, so that the row look-ahead has something to fetch, and no more blocks than run at a time
-// (two per SM), because each one ends with a reduction over its warps and leaves a row of partial sums to add up.
-int tb_layernorm_bwd_blocks(int M) { return M < 8192 ? grid_for(M, 8, 296) : grid_for(M, 8 * 4, 296); }
+// many rows: several rows per warp, so that the row look-ahead has something to fetch.
+int tb_layernorm_bwd_blocks(int M) { return M < 8192 ? grid_for(M, 8, 296) : grid_for(M, 8 * 4, 592); }
 
 int tb_layernorm_bwd_add(const void* dy, const void* x, const void* w, const float* mean, const float* rstd, const void* add, void* dx,
                          void* dw, void* db, float* scratch, int M, int D, cudaStream_t s);
@@ -670,7 +662,7 @@ int tb_col_sum(const void* x, int M, int N, int ld, void* out_bf16, float* scrat
     next += grid.x;
     tb_note_launch(1);
     if (vectors)
-      tb::launch(k_col_sum_vec, grid, dim3(256), 0, s, (const __nv_bfloat16*)x, M, N, ld, scratch, tickets, (__nv_bfloat16*)out_bf16);
+      tb::launch(k_col_sum_vec, grid, dim3(64), 0, s, (const __nv_bfloat16*)x, M, N, ld, scratch, tickets, (__nv_bfloat16*)out_bf16);
     else
       tb::launch(k_col_sum, grid, dim3(1024), 0, s, (const __nv_bfloat16*)x, M, N, ld, scratch, tickets, (__nv_bfloat16*)out_bf16);
     return (int)cudaGetLastError();
