@@ -7,7 +7,7 @@
 // an MN-major operand when it runs over the rows (P.V, P^T.dO, dS^T.Q, dS.K).
 //
 // Three warp-specialised kernels (one TMA producer warp, one MMA-issuing thread, eight element-wise warps):
-//   k_attn_fwd_ws    two 128-query tiles per CTA alternate on the tensor pipe; single pass, online softmax with a lazy
+//   k_attn_fwd_ws    two 128-query tiles per SM alternate on the tensor pipe; single pass, online softmax with a lazy
 //                    rescale of the accumulator in TMEM; P stays in TMEM as the A operand of P.V
 //   k_attn_bwd_dq    per query tile: S, dP -> dS (TMEM) -> dQ += dS.K; also produces delta = rowsum(dO * O)
 //   k_attn_bwd_dkv   per key tile, transposed scores: P^T, dS^T (TMEM) -> dV += P^T.dO, dK += dS^T.Q
@@ -55,38 +55,39 @@ __device__ __forceinline__ void mma_kmajor(uint32_t d_tmem, const uint8_t* a, co
 }
 
 // ------------------------------------------------------------------------------------------ forward, warp-specialised
-// One CTA per PAIR of 128-query tiles of one head, 320 threads in four roles:
-//   warp 0       TMA producer: both Q tiles once, then K_0, V_0, K_1, V_1, ... through a ring of tile slots
-//   warp 1       MMA issuer (one thread): S_i = Q_i.K_j^T and O_i += P_i.V_j for the two query tiles i in turn
+// A CTA owns NT 128-query tiles of one head: two with head dim 128; one with head dim 64, where two such CTAs share an SM.
+//   warp 0       TMA producer: the Q tiles once, then K_0, V_0, K_1, V_1, ... through a ring of tile slots
+//   warp 1       MMA issuer (one elected thread): S_i = Q_i.K_j^T and O_i += P_i.V_j for the query tiles i in turn
 //   warps 2-5    softmax of query tile 0: one thread per query row (= TMEM lane)
 //   warps 6-9    softmax of query tile 1
 // Single pass with an online softmax: a row keeps the maximum it is currently scaled by (m_used) and only rescales its
 // accumulator row in TMEM (tcgen05.ld, multiply, tcgen05.st) when a new maximum exceeds it by more than 2^8; otherwise
-// the probabilities simply run up to 256, which fp32 accumulation and bf16 probabilities absorb.  The rescale needs no
-// barrier of its own: S_i(j) is committed after O_i += P.V of step j-1 on the in-order tensor pipe, and the next one is
-// only issued after this row's thread has arrived on p_full.
-// The two tiles alternate on the tensor pipe: while the softmax threads of one tile work on S_i(j) (exponentials), the
-// MMAs of the other tile run.  P stays in TMEM: it is written as bf16 pairs over the first 64 columns of S and is the
-// A operand of a TMEM-sourced MMA (measured against staging P in shared memory: 198 vs 223 us at T = 2048, head dim 128).
-// TMEM: S_0 [0,128)  S_1 [128,256)  O_0 [256,256+HD)  O_1 [256+HD, 256+2HD), and with head dim 64, where there is room,
-// P_0 [384,448)  P_1 [448,512).  A P of its own lets S_i(j+1) be issued as soon as the softmax threads have S_i(j) in registers,
-// so that they never wait for scores; P_i(j) and the rescale of O_i then wait for P.V of step j-1 (pv_done), which is long
-// over by the time the maxima are known.  With head dim 128 P lies over S, and S_i(j+1) follows P_i(j).V_j.
+// the probabilities simply run up to 256, which fp32 accumulation and bf16 probabilities absorb.
+// Two tiles alternate on the tensor pipe: while the softmax threads of one tile work on S_i(j) (exponentials), the
+// MMAs of the other tile run.  P stays in TMEM, as bf16 pairs, and is the A operand of a TMEM-sourced MMA (measured
+// against staging P in shared memory: 198 vs 223 us at T = 2048, head dim 128).
+// Head dim 128.  TMEM: S_0 [0,128)  S_1 [128,256)  O_0 [256,384)  O_1 [384,512); P_i lies over the first 64 columns of S_i.
+//   The rescale needs no barrier of its own: S_i(j) is committed after O_i += P.V of step j-1 on the in-order tensor
+//   pipe, and the next one is only issued after this row's thread has arrived on p_full.
+// Head dim 64.  TMEM: S [0,128)  O [128,192)  P [192,256).  With a P of its own, S(j+1) is issued as soon as the softmax threads
+//   have S(j) in registers, so that they never wait for scores; P(j) and the rescale of O wait for P.V of step j-1 (pv_done),
+//   which is long over by the time the maxima are known.  256 columns and 100 KB let two CTAs share an SM, and
+//   one's start and end overlap the other's work: sequences of 512 have one to four key tiles per query tile.
 template <int HD>
 struct Fwd2Smem {
   static constexpr int TILE_BYTES = (HD / 64) * STRIP;
-  static constexpr int Q = 0;                                       // two query tiles
-  static constexpr int RING = Q + 2 * TILE_BYTES;
-  static constexpr int BUDGET = 224 * 1024;
-  static constexpr int SLOTS_FIT = (BUDGET - RING) / TILE_BYTES;
-  static constexpr int SLOTS = SLOTS_FIT > 6 ? 6 : SLOTS_FIT;       // K and V tiles in flight
+  static constexpr int NT = HD == 64 ? 1 : 2;                        // query tiles
+  static constexpr int THREADS = 64 + 128 * NT;
+  static constexpr int Q = 0;
+  static constexpr int RING = Q + NT * TILE_BYTES;
+  static constexpr int SLOTS = 5;                                   // K and V tiles in flight
   static constexpr int BARS = RING + SLOTS * TILE_BYTES;
   static constexpr int TOTAL = BARS + 256;
-  static_assert(SLOTS >= 3, "the K/V ring needs at least three slots");
+  static_assert(TOTAL <= (HD == 64 ? 113 : 227) * 1024, "shared memory of one SM");
 };
 
 template <int HD>
-__global__ void __launch_bounds__(320, 1)
+__global__ void __launch_bounds__(Fwd2Smem<HD>::THREADS, HD == 64 ? 2 : 1)
 k_attn_fwd_ws(const __grid_constant__ CUtensorMap map, __nv_bfloat16* __restrict__ out, float* __restrict__ lse, int B, int T, int H,
               int d, float scale_log2e, int* error) {
   extern __shared__ __align__(1024) uint8_t fwd2_smem[];
@@ -106,15 +107,17 @@ k_attn_fwd_ws(const __grid_constant__ CUtensorMap map, __nv_bfloat16* __restrict
   uint32_t* holder = reinterpret_cast<uint32_t*>(pv_done + 2);
   constexpr bool OWN_P = HD == 64;
   const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;  // warp: known to be uniform
-  const int n_qt = T / TILE, n_pairs = (n_qt + 1) / 2;
-  // consecutive CTAs share one head's K and V (they stay in L2), longest pair first within the head
-  const int pair = n_pairs - 1 - (int)blockIdx.x % n_pairs;
-  const int rest = (int)blockIdx.x / n_pairs;
+  constexpr int NT = L::NT;
+  const int n_qt = T / TILE, n_groups = (n_qt + NT - 1) / NT;
+  // consecutive CTAs share one head's K and V (they stay in L2), longest first within the head
+  const int group = n_groups - 1 - (int)blockIdx.x % n_groups;
+  const int rest = (int)blockIdx.x / n_groups;
   const int h = rest % H, b = rest / H;
-  const int qt0 = 2 * pair, qt1 = 2 * pair + 1;
-  const int n0 = qt0 + 1, n1 = qt1 < n_qt ? qt1 + 1 : 0;  // key tiles each query tile visits
+  const int qt0 = NT * group, qt1 = qt0 + 1;
+  const int n0 = qt0 + 1, n1 = NT == 2 && qt1 < n_qt ? qt1 + 1 : 0;  // key tiles each query tile visits
   const int n_steps = n1 > n0 ? n1 : n0;
-  constexpr uint32_t TMEM_COLS = 512;
+  constexpr uint32_t TMEM_COLS = HD == 64 ? 256 : 512;
+  constexpr uint32_t C_O = HD == 64 ? 128 : 256, C_P = 192;  // S_i at 128 * i; C_P: with OWN_P
 
   if (tid == 0) {
     for (int i = 0; i < 2; ++i) {
@@ -172,11 +175,11 @@ k_attn_fwd_ws(const __grid_constant__ CUtensorMap map, __nv_bfloat16* __restrict
       mma_commit(&s_full[i]);
     };
     auto issue_pv = [&](int i, int j) {  // O_i (+)= P_i . V_j: eight steps of 16 keys; V is MN-major (head dim contiguous)
-      const uint32_t tO = tmem + 256 + i * HD;
+      const uint32_t tO = tmem + C_O + i * HD;
       const uint64_t v_desc = smem_desc(smem_u32(slot_of(2 * j + 1)), STRIP, 1024);
 #pragma unroll
       for (int kk = 0; kk < 8; ++kk)
-        mma_bf16_ts(tO, (OWN_P ? tmem + 384 + i * 64 : tmem + i * 128) + kk * 8, v_desc + kk * (2048 >> 4), idesc_o, (j > 0 || kk > 0) ? 1u : 0u);  // 16 keys = 8 TMEM columns of P
+        mma_bf16_ts(tO, (OWN_P ? tmem + C_P : tmem + i * 128) + kk * 8, v_desc + kk * (2048 >> 4), idesc_o, (j > 0 || kk > 0) ? 1u : 0u);  // 16 keys = 8 TMEM columns of P
     };
     bool ok = mbar_wait_all(&q_full[0], 0, error) && (!n1 || mbar_wait_all(&q_full[1], 0, error)) && wait_slot(0);
     if (ok) {
@@ -191,7 +194,7 @@ k_attn_fwd_ws(const __grid_constant__ CUtensorMap map, __nv_bfloat16* __restrict
       for (int j = 0; j < n_steps && ok; ++j) {
         if (j + 1 < n_steps) {
           if (!(ok = wait_slot(2 * j + 2))) break;                      // K_{j+1}
-          for (int i = 0; i < 2 && ok; ++i) {
+          for (int i = 0; i < NT && ok; ++i) {
             if (j + 1 >= (i == 0 ? n0 : n1)) continue;
             if (!(ok = mbar_wait_all(&s_read[i], j & 1, error))) break;  // S_i(j) is in registers
             tc_fence_after();
@@ -201,7 +204,7 @@ k_attn_fwd_ws(const __grid_constant__ CUtensorMap map, __nv_bfloat16* __restrict
           if (elect_one()) mma_commit(&kv_empty[(2 * j + 2) % SLOTS]);
         }
         if (!(ok = wait_slot(2 * j + 1))) break;                        // V_j
-        for (int i = 0; i < 2 && ok; ++i) {
+        for (int i = 0; i < NT && ok; ++i) {
           const int n_i = i == 0 ? n0 : n1;
           if (j >= n_i) continue;
           if (!(ok = mbar_wait_all(&p_full[i], j & 1, error))) break;    // P_i(j) is in place, O_i rescaled if it had to be
@@ -219,7 +222,7 @@ k_attn_fwd_ws(const __grid_constant__ CUtensorMap map, __nv_bfloat16* __restrict
         if (!(ok = wait_slot(2 * j + 1))) break;                       // V_j
         if (j + 1 < n_steps && !(ok = wait_slot(2 * j + 2))) break;    // K_{j+1}
         tc_fence_after();
-        for (int i = 0; i < 2 && ok; ++i) {
+        for (int i = 0; i < NT && ok; ++i) {
           const int n_i = i == 0 ? n0 : n1;
           if (j >= n_i) continue;
           if (!(ok = mbar_wait_all(&p_full[i], j & 1, error))) break;  // P_i(j) is in place, O_i rescaled if it had to be
@@ -246,8 +249,8 @@ k_attn_fwd_ws(const __grid_constant__ CUtensorMap map, __nv_bfloat16* __restrict
     const int r = quarter * 32 + lane;                      // query row within the tile = TMEM lane
     const uint32_t lane_base = (uint32_t)(quarter * 32) << 16;
     const uint32_t tS = tmem + i * 128 + lane_base;
-    const uint32_t tO = tmem + 256 + i * HD + lane_base;
-    const uint32_t tP = OWN_P ? tmem + 384 + i * 64 + lane_base : tS;  // bf16: keys 2c, 2c+1 in column c
+    const uint32_t tO = tmem + C_O + i * HD + lane_base;
+    const uint32_t tP = OWN_P ? tmem + C_P + lane_base : tS;  // bf16: keys 2c, 2c+1 in column c
     float m_used = -INFINITY, l = 0.f;  // m_used in raw score units
     bool ok = true;
     for (int j = 0; j < n_i && ok; ++j) {
@@ -910,8 +913,8 @@ int tb_attn_fwd(const void* qkv, void* out, float* lse, int B, int T, int H, int
   int rc = make_map(&map, qkv, 3LL * d, (long long)B * T, 3LL * d);
   if (rc) return rc;
   const float scale_log2e = 1.4426950408889634f / sqrtf((float)HD);
-  const int n_pairs = (T / TILE + 1) / 2;
-  const unsigned ctas = (unsigned)(n_pairs * H * B);
+  const int tiles = HD == 64 ? 1 : 2;
+  const unsigned ctas = (unsigned)((T / TILE + tiles - 1) / tiles * H * B);
   tb_note_launch(1);
 #define LAUNCH_FWD(HD_) \
   do { \
@@ -921,7 +924,7 @@ int tb_attn_fwd(const void* qkv, void* out, float* lse, int B, int T, int H, int
       if (e != cudaSuccess) return (int)e; \
       once = true; \
     } \
-    return (int)tb::launch(k_attn_fwd_ws<HD_>, dim3(ctas), dim3(320), Fwd2Smem<HD_>::TOTAL, stream, map, (__nv_bfloat16*)out, lse, B, T, H, d, \
+    return (int)tb::launch(k_attn_fwd_ws<HD_>, dim3(ctas), dim3(Fwd2Smem<HD_>::THREADS), Fwd2Smem<HD_>::TOTAL, stream, map, (__nv_bfloat16*)out, lse, B, T, H, d, \
                            scale_log2e, g_err_dev); \
   } while (0)
   if (HD == 64) LAUNCH_FWD(64);
