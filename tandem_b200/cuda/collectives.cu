@@ -121,12 +121,18 @@ __device__ __forceinline__ T fold_one(const PeerPtrs& buf, int n, int c, long lo
   return from_f<T>(acc);
 }
 
+struct NoFetch {
+  __device__ __forceinline__ uint4 operator()(long long) const { return make_uint4(0, 0, 0, 0); }
+};
+
 // Vector body shared by the two-shot all-reduce and reduce-scatter: folds `nvec` 16-byte vectors of chunk
-// `rank` starting at byte offset `off0`.  NR is the group size when it is 2, 4 or 8 (loops unroll exactly and
-// eight operand vectors are in flight per thread), 0 otherwise (predicated over TB_MAX_RANKS).
-template <typename T, bool EXACT, int NR, typename Sink>
+// `rank` starting at byte offset `off0`.  NR is the group size when it is 1, 2, 4 or 8 (loops unroll exactly and
+// eight operand vectors are in flight per thread), 0 otherwise (predicated over TB_MAX_RANKS).  `fetch` loads what the
+// sink needs besides (the vector that a gradient shard already holds): its loads go out with the operands', while a load in the
+// sink would wait for the store before it.
+template <typename T, bool EXACT, int NR, typename Fetch, typename Sink>
 __device__ __forceinline__ void fold_vectors(const PeerPtrs& buf, int n_runtime, int rank, long long off0, long long nvec, int smode,
-                                             float sval, long long tid, long long nth, Sink&& sink) {
+                                             float sval, long long tid, long long nth, Fetch&& fetch, Sink&& sink) {
   constexpr int U = NR ? 8 / NR : 1;
   const int n = NR ? NR : n_runtime;
   const char* ord[TB_MAX_RANKS];  // operands in fold order: ranks rank+1, ..., rank
@@ -139,11 +145,12 @@ __device__ __forceinline__ void fold_vectors(const PeerPtrs& buf, int n_runtime,
     }
   }
   for (long long v = tid; v < nvec; v += nth * U) {
-    uint4 x[U][TB_MAX_RANKS];
+    uint4 x[U][TB_MAX_RANKS], more[U];
 #pragma unroll
     for (int u = 0; u < U; ++u) {
       const long long vv = v + u * nth;
       if (vv < nvec) {
+        more[u] = fetch(off0 + vv * 16);
 #pragma unroll
         for (int j = 0; j < TB_MAX_RANKS; ++j)
           if (j < n) x[u][j] = ld_vec_peer(ord[j] + off0 + vv * 16);
@@ -152,7 +159,7 @@ __device__ __forceinline__ void fold_vectors(const PeerPtrs& buf, int n_runtime,
 #pragma unroll
     for (int u = 0; u < U; ++u) {
       const long long vv = v + u * nth;
-      if (vv < nvec) sink(off0 + vv * 16, fold_vec<T, EXACT>(x[u], n, smode, sval));
+      if (vv < nvec) sink(off0 + vv * 16, fold_vec<T, EXACT>(x[u], n, smode, sval), more[u]);
     }
   }
 }
@@ -166,16 +173,25 @@ __device__ __forceinline__ void local_copy(char* dst, const char* src, long long
   const long long nth = (long long)gridDim.x * blockDim.x;
   const bool aligned = (((uintptr_t)dst | (uintptr_t)src) & 15) == 0;
   long long nvec = aligned ? numel / N : 0;
-  for (long long v = tid; v < nvec; v += nth) {
-    uint4 x = ld_vec_peer(src + v * 16);
-    if (smode != SCALE_NONE) {
-      float f[N];
-      unpack<T>(x, f);
+  constexpr int U = 8;  // loads in flight per thread: one at a time copied 100 MB in 0.7 ms
+  for (long long v = tid; v < nvec; v += nth * U) {
+    uint4 x[U];
 #pragma unroll
-      for (int e = 0; e < N; ++e) f[e] = scaled(f[e], smode, sval);
-      x = pack<T>(f);
+    for (int u = 0; u < U; ++u)
+      if (v + u * nth < nvec) x[u] = ld_vec_peer(src + (v + u * nth) * 16);
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      if (v + u * nth < nvec) {
+        if (smode != SCALE_NONE) {
+          float f[N];
+          unpack<T>(x[u], f);
+#pragma unroll
+          for (int e = 0; e < N; ++e) f[e] = scaled(f[e], smode, sval);
+          x[u] = pack<T>(f);
+        }
+        st_vec(dst + (v + u * nth) * 16, x[u]);
+      }
     }
-    st_vec(dst + v * 16, x);
   }
   for (long long i = nvec * N + tid; i < numel; i += nth) {
     float f = to_f<T>(reinterpret_cast<const T*>(src)[i]);
@@ -212,7 +228,7 @@ k_allreduce_twoshot(CommCtx c, PeerPtrs buf, Locals lin, Locals lout, long long 
     if (head > hi - lo) head = hi - lo;
     long long nvec = (hi - lo - head) / N;
     long long body = lo + head;
-    fold_vectors<T, EXACT, NR>(buf, n, rank, body * (long long)sizeof(T), nvec, smode, sval, tid, nth, [&](long long off, const uint4& r) {
+    fold_vectors<T, EXACT, NR>(buf, n, rank, body * (long long)sizeof(T), nvec, smode, sval, tid, nth, NoFetch{}, [&](long long off, const uint4& r, const uint4&) {
 #pragma unroll
       for (int q = 0; q < TB_MAX_RANKS; ++q)
         if (q < (NR ? NR : n)) st_vec(buf.p[q] + off, r);
@@ -375,12 +391,23 @@ k_reduce_scatter(CommCtx c, PeerPtrs buf, Locals lin, long long numel, Bounds bo
     if (head > hi - lo) head = hi - lo;
     const long long nvec = (hi - lo - head) / N;
     const long long body = lo + head;
-    fold_vectors<T, EXACT, NR>(buf, n, rank, body * (long long)sizeof(T), nvec, smode, sval, tid, nth, [&](long long off, const uint4& r) {
+    const bool acc_vectors = EPI == 1 && ((uintptr_t)(acc_out + (body - lo)) & 15) == 0;
+    auto held = [&](long long off) {  // the shard's vector that is added to
+      return acc_vectors ? *reinterpret_cast<const uint4*>(acc_out + (off / (long long)sizeof(T) - lo)) : make_uint4(0, 0, 0, 0);
+    };
+    fold_vectors<T, EXACT, NR>(buf, n, rank, body * (long long)sizeof(T), nvec, smode, sval, tid, nth, held,
+                               [&](long long off, const uint4& r, const uint4& old) {
       st_vec(buf.p[rank] + off, r);
       if (EPI != 0) {
         const long long i0 = off / (long long)sizeof(T);
         const T* e = reinterpret_cast<const T*>(&r);
-        if (EPI == 1) {
+        if (EPI == 1 && acc_vectors) {
+          const T* a = reinterpret_cast<const T*>(&old);
+          uint4 sum;
+#pragma unroll
+          for (int j = 0; j < N; ++j) reinterpret_cast<T*>(&sum)[j] = from_f<T>(__fadd_rn(to_f<T>(a[j]), to_f<T>(e[j])));
+          *reinterpret_cast<uint4*>(acc_out + (i0 - lo)) = sum;
+        } else if (EPI == 1) {
 #pragma unroll
           for (int j = 0; j < N; ++j) acc_out[i0 - lo + j] = from_f<T>(__fadd_rn(to_f<T>(acc_out[i0 - lo + j]), to_f<T>(e[j])));
         }
@@ -922,6 +949,7 @@ int tb_reduce_scatter(TbComm* c, void* const* bufs, void* const* local_in, long 
   }
 #define RS(T, E, EPI)                                                                                                                      \
   do {                                                                                                                                 \
+    if (nr == 1) return (int)launch(c, k_reduce_scatter<T, E, EPI, 1>, blocks, stream, c->ctx, buf, in, numel, bounds, smode, sval, acc, adams); \
     if (nr == 2) return (int)launch(c, k_reduce_scatter<T, E, EPI, 2>, blocks, stream, c->ctx, buf, in, numel, bounds, smode, sval, acc, adams); \
     if (nr == 4) return (int)launch(c, k_reduce_scatter<T, E, EPI, 4>, blocks, stream, c->ctx, buf, in, numel, bounds, smode, sval, acc, adams); \
     if (nr == 8) return (int)launch(c, k_reduce_scatter<T, E, EPI, 8>, blocks, stream, c->ctx, buf, in, numel, bounds, smode, sval, acc, adams); \

@@ -6,15 +6,15 @@
 // Structure of k_gemm (one persistent CTA per SM, 320 threads, no cluster):
 //   warp 0      TMA producer: cp.async.bulk.tensor.2d loads A and B tiles (128B swizzle) into a
 //               3- to 6-stage shared-memory ring, signalling `full[s]` by transaction bytes.
-//   warp 1      MMA issuer: one elected thread issues tcgen05.mma.cta_group::1.kind::f16
+//   warp 1      MMA issuer: one elected lane issues tcgen05.mma.cta_group::1.kind::f16
 //               (128 x BN x 16 per instruction, 4 per stage), releases stages with
 //               tcgen05.commit -> `empty[s]`, and hands a finished accumulator to the epilogue
 //               with tcgen05.commit -> `acc_full[b]`.  TMEM holds two accumulators (2 x BN
 //               columns), so the next tile's MMAs overlap this tile's epilogue.
-//   warps 2-9   epilogue: tcgen05.ld 32 lanes x 64 columns at a time, then bias / GELU / residual /
-//               dGELU / accumulate in registers; a bf16 block is staged in shared memory (128-byte
+//   warps 2-9   epilogue: tcgen05.ld 32 lanes x 32 columns at a time, then bias / GELU / residual /
+//               dGELU / accumulate in registers; a bf16 block is staged in shared memory (64-byte
 //               swizzle) and written by one cp.async.bulk.tensor store, fp32 outputs by 16-byte stores.
-// Tile shapes: 256x256, 128x256, 128x192, 128x128 (choose_tile); split-K for outputs with very few tiles.
+// Tile shapes: 256x256, 128x256, 128x192, 128x128 and pair 256x256, 256x128 (plan_gemm); split-K of the last round.
 //
 // Operand layouts.  Each operand is either K-major (the reduction dimension is contiguous in
 // global memory) or MN-major (the other dimension is).  That covers all three GEMMs of a linear

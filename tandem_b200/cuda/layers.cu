@@ -244,15 +244,16 @@ k_reduce_partials(const float* __restrict__ part, int parts, int width, __nv_bfl
   const int c = blockIdx.x * 32 + cx;
   float acc = 0.f;
   if (c < width) {
-    int p = ry;
-    for (; p + 56 < parts; p += 64) {  // eight loads in flight, added in order
-      float v[8];
+    constexpr int U = 40;  // loads in flight, added in order: one trip to L2 for up to 320 partials
+    for (int p = ry; p < parts; p += 8 * U) {
+      float v[U];
 #pragma unroll
-      for (int u = 0; u < 8; ++u) v[u] = part[(size_t)(p + 8 * u) * width + c];
+      for (int u = 0; u < U; ++u)
+        if (p + 8 * u < parts) v[u] = part[(size_t)(p + 8 * u) * width + c];
 #pragma unroll
-      for (int u = 0; u < 8; ++u) acc += v[u];
+      for (int u = 0; u < U; ++u)
+        if (p + 8 * u < parts) acc += v[u];
     }
-    for (; p < parts; p += 8) acc += part[(size_t)p * width + c];
   }
   sh[ry][cx] = acc;
   __syncthreads();

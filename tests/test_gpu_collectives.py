@@ -115,6 +115,28 @@ def test_reduce_scatter_uneven_with_accumulate(emu, n, dtype):
         assert torch.equal(shards[r], (before[r].float() + got.float()).to(dtype)), r
 
 
+@pytest.mark.parametrize("n", [1, 2, 8])
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("skew", [0, 1])
+def test_reduce_scatter_accumulates_vectors_and_elements(emu, n, dtype, skew):
+    """Chunks and gradient shards that start on 16-byte boundaries are added to a vector at a time, others (skew) element by
+    element; a group of one folds a single operand.  More vectors than one turn of the threads takes, and a tail."""
+    e = emu(n)
+    chunk = 160_000 if n > 1 else 1_300_011
+    sizes = [chunk] * (n - 1) + [chunk + 13]
+    numel = sum(sizes)
+    xs = [torch.randn(numel, device="cuda").to(dtype) for _ in range(n)]
+    bufs = [x.clone() for x in xs]
+    shards = [torch.randn(s + skew, device="cuda").to(dtype)[skew:] for s in sizes]
+    before = [s.clone() for s in shards]
+    offs = e.reduce_scatter(bufs, sizes, average=True, accumulate_into=shards)
+    want, _ = expected_fold(xs, True, sizes)
+    for r in range(n):
+        lo, hi = offs[r], offs[r + 1]
+        assert torch.equal(bufs[r][lo:hi], want[lo:hi].to(dtype)), r
+        assert torch.equal(shards[r], (before[r].float() + bufs[r][lo:hi].float()).to(dtype)), r
+
+
 def adam_scalars(lr, betas, eps, wd, step):
     b1, b2 = betas
     return (1 - lr * wd, 1 - b1, b2, 1 - b2, (1 - b2 ** step) ** 0.5, eps, -(lr / (1 - b1 ** step)))
