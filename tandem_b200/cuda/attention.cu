@@ -6,7 +6,7 @@
 // operand when the reduction runs over the head dimension (Q.K^T, dO.V^T) and, with the same bytes,
 // an MN-major operand when it runs over the rows (P.V, P^T.dO, dS^T.Q, dS.K).
 //
-// Three warp-specialised kernels (one TMA producer warp, one MMA-issuing thread, eight element-wise warps):
+// Three warp-specialised kernels (one TMA producer warp, one MMA-issuing warp, four or eight element-wise warps):
 //   k_attn_fwd_ws    two 128-query tiles per SM alternate on the tensor pipe; single pass, online softmax with a lazy
 //                    rescale of the accumulator in TMEM; P stays in TMEM as the A operand of P.V
 //   k_attn_bwd_dq    per query tile: S, dP -> dS (TMEM) -> dQ += dS.K; also produces delta = rowsum(dO * O)
@@ -373,7 +373,7 @@ k_attn_fwd_ws(const __grid_constant__ CUtensorMap map, __nv_bfloat16* __restrict
 // Two kernels, no atomics: k_attn_bwd_dq owns a tile of 128 queries and walks the key tiles at or below the
 // diagonal (dQ accumulates in TMEM); k_attn_bwd_dkv owns a tile of 128 keys and walks the query tiles at or above it
 // (dK and dV accumulate in TMEM).  Both recompute S and dP; results are deterministic.  Roles per CTA (320 threads):
-// warp 0 TMA producer, warp 1 MMA issuer (one thread), warps 2-9 element-wise work, two threads per TMEM lane (warps
+// warp 0 TMA producer, warp 1 MMA issuer (one elected lane), warps 2-9 element-wise work, two threads per TMEM lane (warps
 // w and w + 4 share a lane quarter and split the 128 columns).  Probabilities and dS never touch shared memory: they
 // are written back to TMEM as bf16 pairs and feed the next MMA as its A operand.
 

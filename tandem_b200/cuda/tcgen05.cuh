@@ -39,20 +39,6 @@ __device__ __forceinline__ bool mbar_try_wait(uint64_t* bar, uint32_t parity) {
   return ok != 0;
 }
 
-// Bounded wait.  Returns false (and raises the error word) if the phase does not complete.
-__device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, int* error) {
-  if (mbar_try_wait(bar, parity)) return true;
-  const long long start = clock64();
-  while (!mbar_try_wait(bar, parity)) {
-    if (clock64() - start > (1ll << WAIT_LIMIT_CYCLES_SHIFT)) {
-      *error = 1;
-      __threadfence_system();
-      return false;
-    }
-  }
-  return true;
-}
-
 // One lane of a converged warp, the same one every time.  Loops that issue TMA loads or MMAs are run by a whole warp and
 // only the instructions themselves sit behind this predicate: their operands are warp-uniform registers, and in a branch
 // taken by `lane == 0` the compiler cannot know them to be uniform and moves each one through a slow path
@@ -69,7 +55,7 @@ __device__ __forceinline__ bool elect_one() {
   return p != 0;
 }
 
-// Bounded wait by a converged warp; all lanes return the same answer (so that a wait that runs out takes the whole warp out
+// Bounded wait by a converged warp: false (and the error word raised) if the phase does not complete.  All lanes return the same answer (so that a wait that runs out takes the whole warp out
 // of its loop and no later warp-wide instruction waits for missing lanes).
 __device__ __forceinline__ bool mbar_wait_all(uint64_t* bar, uint32_t parity, int* error) {
   if (__all_sync(0xffffffffu, mbar_try_wait(bar, parity))) return true;
@@ -82,34 +68,6 @@ __device__ __forceinline__ bool mbar_wait_all(uint64_t* bar, uint32_t parity, in
     }
   }
   return true;
-}
-
-// The same for a whole warp that has nothing else to do (the epilogue waiting for an accumulator): one lane polls,
-// sleeping between polls, so the warp neither competes for issue slots with the producer and MMA threads nor
-// keeps the barrier's shared-memory word busy; the others wait at the warp barrier.  Returns the result to all lanes.
-__device__ __forceinline__ bool mbar_wait_warp(uint64_t* bar, uint32_t parity, int* error) {
-  bool ok = true;
-  if ((threadIdx.x & 31) == 0 && !mbar_try_wait(bar, parity)) {
-    const long long start = clock64();
-    while (!mbar_try_wait(bar, parity)) {
-      __nanosleep(128);
-      if (clock64() - start > (1ll << WAIT_LIMIT_CYCLES_SHIFT)) {
-        *error = 1;
-        __threadfence_system();
-        ok = false;
-        break;
-      }
-    }
-  }
-  return __shfl_sync(0xffffffffu, ok ? 1 : 0, 0) != 0;
-}
-
-// The same without sleeping between polls, for warps on the critical path (softmax warps waiting for their scores):
-// lane 0 polls (try_wait itself parks the thread for a hardware-defined slice), the others wait at the shuffle.
-__device__ __forceinline__ bool mbar_wait_warp_spin(uint64_t* bar, uint32_t parity, int* error) {
-  bool ok = true;
-  if ((threadIdx.x & 31) == 0) ok = mbar_wait(bar, parity, error);
-  return __shfl_sync(0xffffffffu, ok ? 1 : 0, 0) != 0;
 }
 
 // Starts fetching a tensor map (a kernel parameter) so that the first TMA operation does not wait for it.
