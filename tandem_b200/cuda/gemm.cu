@@ -1108,19 +1108,24 @@ int launch_gemm_pair(const CUtensorMap& ma, const CUtensorMap& mb, const CUtenso
   return (int)tb::launch(kernel, dim3(2 * pairs), dim3(L::THREADS), L::TOTAL, stream, ma, mb, mo, mp, g);
 }
 
-// Tile shape and tail split with the least estimated time.  The CTAs (or CTA pairs) take output tiles round-robin; the last,
-// partial round leaves SMs idle, so the tiles of that round ("tail") may have their reduction cut into parts that are
-// spread over the idle SMs (GemmArgs).  The estimate, in microseconds, is
-//     start-up + full rounds x (k-blocks x per-k-block + per-tile) + [tail: k-blocks per part x per-k-block + per-tile + fold]
-// with constants fitted to sweeps on B200 (bench/bench_gemm.py --sweep, CUDA-graph timing, cold L2) over 1024 - 16384
-// tokens and widths 768 - 2048.  What a k-block costs: a 256 x 256 pair tile feeds 256 x 256 x 64 multiply-adds to two tensor
-// pipes per 64 KB of operands and runs at the power limit (1620 - 1680 TFLOP/s from 10^11 flops on, cuBLAS 1450 - 1640);
-// the 128-row tiles move up to twice the bytes per flop and pay 0.22 - 0.37 us; the one-CTA 256 x 256 tile fills TMEM, so that
-// its epilogue cannot overlap the next tile.  Narrow tiles win where rounds are few: 1024 x 768 x 2304 takes 12.5 us on
-// pair 256 x 128 tiles, 17 on pair 256 x 256.  Folding parked partial tiles costs about 4 us for two parts, 1 us per part more and
-// 0.2 us per parked megabyte, so a split pays where the last round is less than about half full and the reduction is
-// long: the weight gradients (K = tokens).
-// Over 70 shapes the plan is on average 0.3 % behind the best of all plans.
+// Plans.  The CTAs (or CTA pairs) take output tiles round-robin; the last, partial round leaves SMs idle, so the tiles of
+// that round ("tail") may have their reduction cut into parts that are spread over the idle SMs (GemmArgs).  A plan is made
+// in two steps.
+//
+// 1. Which sums are cut, and where (plan_cut).  That order of summation is part of a product's result: single bf16 roundings
+//    flip with it, and after 24 layers every gradient differs by about 1 %.  So it depends on the product's sizes and the
+//    number of SMs alone, by a model that stays as it is when kernels get faster: a run gives the same bits before and after.
+//
+// 2. Tile shape (plan_gemm): among all shapes that make those very sums, the one with the least estimated time.  The estimate,
+//    in microseconds, is
+//        start-up + full rounds x (k-blocks x per-k-block + per-tile) + [tail: k-blocks per part x per-k-block + per-tile + fold]
+//    with constants fitted to sweeps on B200 (bench/bench_gemm.py --sweep, CUDA-graph timing, cold L2) over 1024 - 16384
+//    tokens and widths 768 - 2048.  What a k-block costs: a 256 x 256 pair tile feeds 256 x 256 x 64 multiply-adds to two tensor
+//    pipes per 64 KB of operands and runs at the power limit (1620 - 1680 TFLOP/s from 10^11 flops on, cuBLAS 1450 - 1640);
+//    the 128-row tiles move up to twice the bytes per flop and pay 0.22 - 0.37 us; the one-CTA 256 x 256 tile fills TMEM, so that
+//    its epilogue cannot overlap the next tile.  Narrow tiles win where rounds are few: 1024 x 768 x 2304 takes 12.5 us on
+//    pair 256 x 128 tiles, 17 on pair 256 x 256.  Folding parked partial tiles costs about 4 us for two parts, 1 us per part more
+//    and 0.2 us per parked megabyte.
 struct TileShape { int id, bm, bn; double start, per_kblock, per_tile; };
 constexpr int PAIR = 512;  // bm of the CTA-pair kernel's 256-row tiles
 constexpr TileShape SHAPES[6] = {{0, 256, 256, 4.5, 0.64, 3.3}, {1, 128, 256, 4.3, 0.37, 0.9},   {2, 128, 128, 4.3, 0.205, 0.7},
@@ -1142,15 +1147,63 @@ struct GemmPlan {
   long long flag_words(int M, int N) const { return tail(M, N) * (splits - 1) * (bm == PAIR ? 16 : 8); }
 };
 
+// Every part gets at least two k-blocks and none is empty.
+bool valid_splits(int k_blocks, int s) {
+  const int per = (k_blocks + s - 1) / s;
+  return s == 1 || (per >= 2 && (s - 1) * per < k_blocks);
+}
+
+// The plan whose sums every plan of this product makes: the tail of a one-CTA shape's tiles is cut where one round takes much
+// longer than folding its parts.  The prices, fitted to early kernels, no longer say how long anything takes: they fix where
+// the cuts are.
+GemmPlan plan_cut(int M, int N, int K, int ctas) {
+  struct { int bm, bn; double per_kblock, per_tile; } constexpr shapes[] = {{256, 256, 0.77, 5.3}, {128, 256, 0.43, 0.5}, {128, 128, 0.34, 0.6}, {128, 192, 0.41, 0.6}};
+  const int k_blocks = (K + BK - 1) / BK;
+  GemmPlan best{128, 128, 1, 0};
+  double best_us = 1e300;
+  for (const auto& t : shapes) {
+    if (t.bn > 128 && N <= 128) continue;
+    const long long tiles = GemmPlan{t.bm, t.bn, 1, 0}.tiles(M, N);
+    const long long rounds = tiles / ctas, tail = tiles % ctas;
+    for (int sp = 1; sp <= MAX_SPLITS; ++sp) {
+      if (!valid_splits(k_blocks, sp) || (sp > 1 && (tail == 0 || tail * sp > ctas))) continue;
+      double us = 5.0 + rounds * (k_blocks * t.per_kblock + t.per_tile);
+      if (tail > 0) {
+        const int per = (k_blocks + sp - 1) / sp;
+        us += per * t.per_kblock + t.per_tile;
+        if (sp > 1) us += 2.5 + 1.7 * (sp - 1) + 0.3 * (double)tail * (sp - 1) * t.bm * t.bn * 4 / 1e6;
+      }
+      if (us < best_us - 1e-9) {
+        best_us = us;
+        best = {t.bm, t.bn, sp, sp > 1 ? (int)(rounds * ctas) : 0};
+      }
+    }
+  }
+  return best;
+}
+
+// Do two plans add up every output element in the same order?  Whole tiles come first, column by column of tiles, so the uncut
+// region is some full columns of the matrix and the upper rows of the tiles' next column.
+bool same_sums(const GemmPlan& a, const GemmPlan& b, int M, int N) {
+  if (a.splits != b.splits) return false;
+  if (a.splits == 1) return true;
+  struct Region { long long columns, rows, columns_with_rows; };
+  auto region = [&](const GemmPlan& p) {
+    const int tiles_m = (M + p.rows() - 1) / p.rows();
+    const long long columns = (long long)(p.whole_tiles / tiles_m) * p.bn, rows = (long long)(p.whole_tiles % tiles_m) * p.rows();
+    return Region{columns, rows, rows == 0 ? columns : columns + p.bn < N ? columns + p.bn : N};
+  };
+  const Region x = region(a), y = region(b);
+  return x.columns == y.columns && x.rows == y.rows && x.columns_with_rows == y.columns_with_rows;
+}
+
 GemmPlan plan_gemm(int M, int N, int K, int ctas) {
   const int k_blocks = (K + BK - 1) / BK;
   const int forced_tile = g_forced_tile.load(std::memory_order_relaxed), forced_splits = g_forced_splits.load(std::memory_order_relaxed);
-  auto valid_splits = [&](int s) {  // every part gets at least two k-blocks and none is empty
-    const int per = (k_blocks + s - 1) / s;
-    return s == 1 || (per >= 2 && (s - 1) * per < k_blocks);
-  };
-  GemmPlan best{128, 128, 1, 0}, best_split = best;
-  double best_us = 1e300, best_split_us = 1e300;
+  const bool pinned = forced_tile >= 0 || forced_splits > 0;
+  const GemmPlan cut = plan_cut(M, N, K, ctas);
+  GemmPlan best{128, 128, 1, 0};
+  double best_us = 1e300;
   for (const TileShape& t : SHAPES) {
     if (forced_tile >= 0 && forced_tile != t.id) continue;
     if (forced_tile < 0 && (t.bn > 128 && N <= 128)) continue;
@@ -1161,8 +1214,10 @@ GemmPlan plan_gemm(int M, int N, int K, int ctas) {
     const long long rounds = tiles / units, tail = tiles % units;
     const double whole_us = rounds * (k_blocks * t.per_kblock + t.per_tile);
     for (int sp = 1; sp <= MAX_SPLITS; ++sp) {
-      if (!valid_splits(sp) || (sp > 1 && (tail == 0 || tail * sp > units))) continue;
-      if (forced_splits > 0 && sp != forced_splits && tail > 0 && valid_splits(forced_splits) && tail * forced_splits <= units) continue;
+      if (!valid_splits(k_blocks, sp) || (sp > 1 && (tail == 0 || tail * sp > units))) continue;
+      if (forced_splits > 0 && sp != forced_splits && tail > 0 && valid_splits(k_blocks, forced_splits) && tail * forced_splits <= units) continue;
+      const GemmPlan plan{t.bm, t.bn, sp, sp > 1 ? (int)(rounds * units) : 0};
+      if (!pinned && !same_sums(plan, cut, M, N)) continue;
       double us = t.start + whole_us;
       if (tail > 0) {
         const int per = (k_blocks + sp - 1) / sp;
@@ -1171,23 +1226,10 @@ GemmPlan plan_gemm(int M, int N, int K, int ctas) {
       }
       if (us < best_us - 1e-9) {
         best_us = us;
-        best = {t.bm, t.bn, sp, (int)(rounds * units)};
-      }
-      if (sp > 1 && us < best_split_us - 1e-9) {
-        best_split_us = us;
-        best_split = {t.bm, t.bn, sp, (int)(rounds * units)};
+        best = plan;
       }
     }
   }
-  // One round that takes (almost) every SM for 128 k-blocks or more is cut in parts all the same: such a product waits for
-  // the last SM that another stream's kernel still holds.  On an idle GPU that costs 5 us of 37 (3072 x 768 x 8192:
-  // 32.4 us as 72 whole pair 256 x 128 tiles); callers rely on these reductions being cut (tests/test_gemm_planner.py).
-  if (best.splits == 1 && best_split.splits > 1 && k_blocks >= 128) {
-    const int units = best.bm == PAIR ? ctas / 2 : ctas;
-    const long long tiles = best.tiles(M, N);
-    if (tiles <= units && 20 * tiles >= 19 * units) best = best_split;
-  }
-  if (best.splits == 1) best.whole_tiles = 0;
   return best;
 }
 
