@@ -306,7 +306,8 @@ __device__ __forceinline__ void bulk_store_2d(const CUtensorMap* map, const uint
 // One warp's share of a finished tile: 32 rows x columns [32 * c_begin, 32 * c_end), 32 columns at a time.
 // TMEM -> registers -> element-wise work -> a swizzled 2 KB block in shared memory -> one bulk tensor store, which clips
 // rows >= M and columns >= N.  Two blocks per warp: the store of one chunk reads its block while the next chunk is computed
-// (GELU needs both at once, for its output and its derivative).  The stores never pass through the load/store unit, whose
+// (GELU needs both at once, for its output and its derivative).  A tile's first chunk waits for every earlier store: the tile
+// before may have ended in the same block (192-column tiles and clipped ones have an odd number of chunks per warp).  The stores never pass through the load/store unit, whose
 // global stores (measured on B200) slow the MMA/TMA traffic of the main loop several times more than their size
 // would suggest.  What this loop costs is instruction fetch: with every flag tested in one body unrolled over 64
 // columns it took 1100 cycles per 64 columns to convert and store plain results, 3400 with a bias and 12000 with GELU.
@@ -350,7 +351,7 @@ __device__ __forceinline__ void store_tile(uint32_t taddr, int c_begin, int c_en
     if (c + 1 < c_end) fetch(c + 1);
     uint8_t* block = stage + (KIND == KIND_GELU ? 0 : (c & 1) * 2048);
     if (elect_one()) {  // the store that last used this block has read it
-      if (KIND == KIND_GELU) asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
+      if (KIND == KIND_GELU || c == c_begin) asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
       else asm volatile("cp.async.bulk.wait_group.read 1;" ::: "memory");
     }
     __syncwarp();

@@ -142,6 +142,23 @@ def test_gemm_raster_and_edges(M, N, K, tile, force_tile):
     close(slope, gelu_slope(ref))
 
 
+@pytest.mark.parametrize("tile,N", [(5, 384), (2, 96), (1, 160), (4, 352), (3, 416), (0, 288)])
+def test_gemm_store_blocks_with_odd_chunk_counts(tile, N, force_tile):
+    """Six tiles and more per CTA whose epilogue warps write an odd number of 32-column blocks each: a tile's first block is the
+    one that the tile before stored last.  One k-block, so that the epilogue follows on the tile before at once.  Sums of 64
+    products of -1, 0 and 1 are exact in bf16."""
+    from tandem_b200.ops import gemm as G
+
+    force_tile(tile)
+    M, K = 148 * 128 * 6, 64
+    x, w = (torch.randint(-1, 2, (rows, K), device="cuda").bfloat16() for rows in (M, N))
+    res = torch.randint(-1, 2, (M, N), device="cuda").bfloat16()
+    ref = x.float() @ w.float().t()
+    for _ in range(4):
+        assert torch.equal(G.gemm(x, w, M, N, K, K, K, False, False).float(), ref)
+        assert torch.equal(G.gemm(x, w, M, N, K, K, K, False, False, G.RESIDUAL, None, res).float(), ref + res.float())
+
+
 def test_gelu_epilogue_at_the_extremes(force_tile):
     """GELU and its derivative where the reciprocal and the exponential saturate, and for infinities and NaN."""
     from tandem_b200.ops import gemm as G
