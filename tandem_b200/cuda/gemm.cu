@@ -482,13 +482,13 @@ __device__ __forceinline__ void fold_tile(uint32_t taddr, int c_begin, int c_end
 }
 
 // The flag a producer's warp raises once its share is parked, and the consumer's bounded wait for the same warp's flags
-// of all parts (`stride` words apart).
+// of all parts (`stride` words apart).  The flags are zero again afterwards, for the next launch that is handed these words.
 __device__ __forceinline__ void raise_flag(unsigned* flag, int lane) {
   __threadfence();
   __syncwarp();
   if (lane == 0) st_release_gpu(flag, 1u);
 }
-__device__ __forceinline__ bool wait_flags(const unsigned* flags, int parts, int stride, int lane, int* error) {
+__device__ __forceinline__ bool wait_flags(unsigned* flags, int parts, int stride, int lane, int* error) {
   bool seen = true;
   if (lane < parts) {
     const long long start = clock64();
@@ -500,8 +500,11 @@ __device__ __forceinline__ bool wait_flags(const unsigned* flags, int parts, int
         break;
       }
     }
+    flags[lane * stride] = 0u;
   }
-  return __all_sync(0xffffffffu, seen);
+  seen = __all_sync(0xffffffffu, seen);
+  __syncwarp();  // every lane reads the parked parts next: behind what the polling lanes acquired (a vote orders no memory)
+  return seen;
 }
 
 // Work items of a split problem: whole tiles, then the tail's producers (parts 1 .. splits-1), then its consumers (part 0).
@@ -777,7 +780,6 @@ k_gemm(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtens
       if (part == 0) {
         if (!(ok = wait_flags(my_flags, parts, 8, lane, g.error))) break;
         fold_tile<BM, BM * BN>(taddr, c_begin, c_end, parked, parts, tile_row);
-        if (lane < parts) my_flags[lane * 8] = 0u;  // zero again for the next launch that is handed these words
       }
       epilogue_tile(taddr, c_begin, c_end, n0, row0, lane, stage, bias_sm, g, &map_out, &map_pre, release);
     }
@@ -972,7 +974,6 @@ k_gemm_pair(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ C
         }
         if (!(ok = wait_flags(my_flags, parts, 16, lane, g.error))) break;
         fold_tile<256, 256 * BN>(taddr, c_begin, c_end, parked, parts, tile_row);
-        if (lane < parts) my_flags[lane * 16] = 0u;
       }
       epilogue_tile(taddr, c_begin, c_end, n0, m0 + quarter * 32, lane, stage, bias_sm, g, &map_out, &map_pre, release);
     }
