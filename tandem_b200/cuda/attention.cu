@@ -777,11 +777,6 @@ k_attn_bwd_dkv(const __grid_constant__ CUtensorMap map_qkv, const __grid_constan
         tmem_ld32(tmem + C_S + lane_base + half * 64, s[0]);
         tmem_ld32(tmem + C_S + lane_base + half * 64 + 32, s[1]);
         tmem_ld_wait();
-        if (i == kt) {  // the diagonal tile: exp2(-inf) = 0 for keys after the query
-#pragma unroll
-          for (int col = 0; col < 64; ++col)
-            if (r > half * 64 + col) s[col >> 5][col & 31] = 0xff800000u;
-        }
 #pragma unroll
         for (int q = 0; q < 16; ++q) {
           const float4 l4 = lse4[q];
@@ -792,6 +787,15 @@ k_attn_bwd_dkv(const __grid_constant__ CUtensorMap map_qkv, const __grid_constan
             float x0, x1;
             split2(fma2(pair2(__uint_as_float(s[c][k]), __uint_as_float(s[c][k + 1])), scale_log2e2, shift), &x0, &x1);
             p[e] = pair2(ex2_approx(x0), ex2_approx(x1));
+            pk[e] = bf16_pair(p[e]);
+          }
+        }
+        if (i == kt) {  // the diagonal tile: nothing of a query reaches the keys after it, not even the NaN of one whose sum is NaN
+#pragma unroll
+          for (int e = 0; e < 32; ++e) {
+            float x0, x1;
+            split2(p[e], &x0, &x1);
+            p[e] = pair2(r > half * 64 + 2 * e ? 0.f : x0, r > half * 64 + 2 * e + 1 ? 0.f : x1);
             pk[e] = bf16_pair(p[e]);
           }
         }

@@ -458,6 +458,20 @@ def test_causal_attention_matches_fp32(B, T, H, hd, spread):
         close(qkv.grad[..., part * d:(part + 1) * d], ref.grad[..., part * d:(part + 1) * d], rtol=4e-2, atol=2e-2, frobenius=1e-2)
 
 
+@pytest.mark.parametrize("hd", [64, 128])
+def test_causal_attention_keeps_nan_queries_from_later_keys(hd):
+    """The value gradient of a key is a sum over the queries from that key on: a query that is NaN reaches no key after it."""
+    from tandem_b200 import ops
+
+    T, H, row = 256, 2, 133
+    qkv, dy = rnd(1, T, 3 * H * hd), rnd(1, T, H * hd)
+    want = torch.autograd.grad(ops.causal_attention(x := qkv.clone().requires_grad_(), H), x, dy)[0][..., 2 * H * hd:]
+    qkv[0, row, :hd] = float("nan")
+    got = torch.autograd.grad(ops.causal_attention(x := qkv.clone().requires_grad_(), H), x, dy)[0][..., 2 * H * hd:]
+    assert got[0, row, :hd].isnan().all()
+    assert torch.equal(got[0, row + 1:], want[0, row + 1:]) and torch.equal(got[..., hd:], want[..., hd:])
+
+
 def test_causal_attention_is_deterministic():
     """No atomics anywhere: two runs give the same bits."""
     from tandem_b200 import ops
