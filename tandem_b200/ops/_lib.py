@@ -43,7 +43,11 @@ def lib():
 
 
 def stream(t):
-    """The raw handle of the current stream of t's device (building a torch.cuda.Stream object for it costs 2 us a launch)."""
+    """The raw handle of the current stream of t's device (building a torch.cuda.Stream object for it costs 2 us a launch).
+    A CPU tensor is refused, as torch.cuda.current_stream does: its device number, -1, would get the current GPU's stream,
+    and a kernel host pointers."""
+    if not t.is_cuda:
+        raise ValueError(f"Expected a cuda device, but got: {t.device}")
     return torch._C._cuda_getCurrentRawStream(t.get_device())
 
 

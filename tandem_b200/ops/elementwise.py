@@ -5,10 +5,7 @@ import ctypes
 import torch
 
 from ..parallel.symm import _ll_array, _ptr_array, check_rc, cuda_lib
-
-
-def _stream(t):
-    return torch._C._cuda_getCurrentRawStream(t.get_device())
+from ._lib import stream
 
 
 def multi_copy(flat, pairs):
@@ -23,7 +20,7 @@ def multi_copy(flat, pairs):
         dsts.append(dst.data_ptr())
         sizes.append(src.numel() * src.element_size())
     if srcs:
-        check_rc(cuda_lib().tb_multi_copy(_ptr_array(srcs), _ptr_array(dsts), _ll_array(sizes), len(srcs), _stream(flat)),
+        check_rc(cuda_lib().tb_multi_copy(_ptr_array(srcs), _ptr_array(dsts), _ll_array(sizes), len(srcs), stream(flat)),
                  "multi_copy")
 
 
@@ -39,13 +36,13 @@ def adamw_step(param, grad, exp_avg, exp_avg_sq, scalars, decay, shadow=None, gr
     sc = (ctypes.c_float * 7)(*scalars)
     check_rc(cuda_lib().tb_adamw(param.data_ptr(), grad.contiguous().data_ptr(), int(grad.dtype == torch.bfloat16),
                                  exp_avg.data_ptr(), exp_avg_sq.data_ptr(), shadow.data_ptr() if shadow is not None else None,
-                                 param.numel(), sc, int(decay), float(grad_scale), _stream(param)), "adamw")
+                                 param.numel(), sc, int(decay), float(grad_scale), stream(param)), "adamw")
 
 
 def adam_prepare(step_counter, hyper, scalars):
     """step_counter (1 double on the device) += 1; `scalars` (8 floats on the device) <- that step's constants."""
     lr, (b1, b2), eps, wd = hyper
-    check_rc(cuda_lib().tb_adam_prepare(step_counter.data_ptr(), lr, b1, b2, eps, wd, scalars.data_ptr(), _stream(scalars)),
+    check_rc(cuda_lib().tb_adam_prepare(step_counter.data_ptr(), lr, b1, b2, eps, wd, scalars.data_ptr(), stream(scalars)),
              "adam_prepare")
 
 
@@ -53,4 +50,4 @@ def adamw_step_dev(param, grad, exp_avg, exp_avg_sq, scalars, shadow=None):
     """adamw_step with the step's constants read from device memory (safe inside a CUDA graph)."""
     check_rc(cuda_lib().tb_adamw_dev(param.data_ptr(), grad.data_ptr(), int(grad.dtype == torch.bfloat16), exp_avg.data_ptr(),
                                      exp_avg_sq.data_ptr(), shadow.data_ptr() if shadow is not None else None, param.numel(),
-                                     scalars.data_ptr(), _stream(param)), "adamw")
+                                     scalars.data_ptr(), stream(param)), "adamw")
