@@ -48,7 +48,15 @@ def stream(t):
     and a kernel host pointers."""
     if not t.is_cuda:
         raise ValueError(f"Expected a cuda device, but got: {t.device}")
-    return torch._C._cuda_getCurrentRawStream(t.get_device())
+    return _raw_stream(t.get_device())
+
+
+# Two shortcuts of the host path rest on names that torch does not document: the raw stream query, and whether a functorch
+# transform or a tracer is active.  A torch without one of them takes the documented, slower way.
+_raw_stream = getattr(torch._C, "_cuda_getCurrentRawStream", None) or (lambda device: torch.cuda.current_stream(device).cuda_stream)
+_functorch_level = getattr(getattr(torch._C, "_functorch", None), "peek_interpreter_stack", None)
+_tracing_state = getattr(torch._C, "_get_tracing_state", None)
+_can_tell = _functorch_level is not None and _tracing_state is not None and hasattr(torch.autograd.forward_ad, "_current_level")
 
 
 class _Untracked:
@@ -61,8 +69,8 @@ class _Untracked:
 def run(function, *args):
     """function.apply(*args), or its forward alone (5 us less a call) where nothing can want the node: gradients are off, and
     no functorch transform, forward-mode level or tracer is active, which Function.apply would have to answer or refuse."""
-    if (torch.is_grad_enabled() or torch.autograd.forward_ad._current_level >= 0 or torch._C._functorch.peek_interpreter_stack() is not None
-            or torch._C._get_tracing_state() is not None):
+    if (torch.is_grad_enabled() or not _can_tell or torch.autograd.forward_ad._current_level >= 0 or _functorch_level() is not None
+            or _tracing_state() is not None):
         return function.apply(*args)
     return function.forward(_Untracked(), *args)
 
