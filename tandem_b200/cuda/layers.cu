@@ -8,6 +8,9 @@
 #include <stdint.h>
 #include <stdio.h>
 
+#include <atomic>
+#include <mutex>
+
 #include "launch.cuh"
 #include "noalloc.h"
 
@@ -575,6 +578,12 @@ __global__ void __launch_bounds__(256) k_f32_to_bf16(const float* __restrict__ i
   }
 }
 
+constexpr int DEVICES = 64, IDLE_EVENTS = 32;
+std::mutex g_events_lock;
+cudaEvent_t g_idle_events[DEVICES][IDLE_EVENTS];
+int g_idle_count[DEVICES];
+std::atomic<int> g_events_made{0};
+
 int grid_for(long long work, int per_block, int cap) {
   long long b = (work + per_block - 1) / per_block;
   return (int)(b < 1 ? 1 : (b > cap ? cap : b));
@@ -584,19 +593,39 @@ int grid_for(long long work, int per_block, int cap) {
 
 extern "C" {
 
-// Work queued on `waiter` from here on starts after everything now queued on `signaller`.  One event per thread and device:
-// a wait refers to the record before it, so the event is free again as soon as this returns, and no other thread can
-// record it in between.
+// Work queued on `waiter` from here on starts after everything now queued on `signaller`.  A wait refers to the record before
+// it, so an event is free again as soon as this returns: up to IDLE_EVENTS of them wait per device for the next call, on
+// whatever thread, and the rest are given back.
 int tb_stream_wait(cudaStream_t waiter, cudaStream_t signaller) {
-  static thread_local cudaEvent_t events[64] = {};
   int dev = 0;
   cudaError_t e = cudaGetDevice(&dev);
-  if (e == cudaSuccess && dev >= 64) e = cudaErrorInvalidDevice;
-  if (e == cudaSuccess && events[dev] == nullptr) e = cudaEventCreateWithFlags(&events[dev], cudaEventDisableTiming);
-  if (e == cudaSuccess) e = cudaEventRecord(events[dev], signaller);
-  if (e == cudaSuccess) e = cudaStreamWaitEvent(waiter, events[dev], 0);
+  if (e != cudaSuccess) return (int)e;
+  if (dev >= DEVICES) return (int)cudaErrorInvalidDevice;
+  cudaEvent_t event = nullptr;
+  {
+    std::lock_guard<std::mutex> hold(g_events_lock);
+    if (g_idle_count[dev] > 0) event = g_idle_events[dev][--g_idle_count[dev]];
+  }
+  if (event == nullptr) {
+    e = cudaEventCreateWithFlags(&event, cudaEventDisableTiming);
+    if (e != cudaSuccess) return (int)e;
+    ++g_events_made;
+  }
+  e = cudaEventRecord(event, signaller);
+  if (e == cudaSuccess) e = cudaStreamWaitEvent(waiter, event, 0);
+  {
+    std::lock_guard<std::mutex> hold(g_events_lock);
+    if (g_idle_count[dev] < IDLE_EVENTS) {
+      g_idle_events[dev][g_idle_count[dev]++] = event;
+      event = nullptr;
+    }
+  }
+  if (event != nullptr) cudaEventDestroy(event);
   return (int)e;
 }
+
+// Events that tb_stream_wait has made so far in this process.
+int tb_stream_wait_events() { return g_events_made; }
 
 int tb_layernorm_fwd(const void* x, const void* w, const void* b, void* y, float* mean, float* rstd, int M, int D, float eps,
                      cudaStream_t s) {

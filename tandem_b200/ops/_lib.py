@@ -31,6 +31,7 @@ def lib():
         "tb_xent_fwd": ([vp, vp, vp, vp, vp, i, i, i, vp], i),
         "tb_xent_bwd": ([vp, vp, vp, vp, i, i, i, i, vp], i),
         "tb_stream_wait": ([vp, vp], i),
+        "tb_stream_wait_events": ([], i),
         "tb_embed_fwd": ([vp, vp, vp, vp, i, i, i, vp], i),
         "tb_embed_bwd": ([vp, vp, vp, vp, vp, i, i, i, i, vp], i),
     }

@@ -680,3 +680,24 @@ def test_stream_wait_from_two_threads():
     for t in threads:
         t.join()
     assert not bad
+
+
+def test_stream_waits_of_many_threads_share_their_events():
+    """A program that starts a thread per step makes no event per thread."""
+    import threading
+
+    from tandem_b200.ops._lib import lib, stream_wait
+
+    first, second = torch.cuda.Stream(), torch.cuda.Stream()
+
+    def work():
+        torch.cuda.set_device(0)
+        stream_wait(second.cuda_stream, first.cuda_stream)
+
+    work()
+    before = lib().tb_stream_wait_events()
+    for _ in range(20):
+        t = threading.Thread(target=work)
+        t.start()
+        t.join()
+    assert lib().tb_stream_wait_events() == before
