@@ -561,7 +561,8 @@ def test_optimizer_during_backward_equals_optimizer_after_backward():
     assert after[0] == replayed[0] and torch.equal(after[1], replayed[1])
 
 
-@pytest.mark.parametrize("V,ld,first", [(65, 72, 0), (1003, 1003, 0), (1003, 1008, 0), (8200, 8200, 3), (50304, 50304, 0), (2049, 2056, 8)])
+@pytest.mark.parametrize("V,ld,first", [(65, 72, 0), (1003, 1003, 0), (1003, 1008, 0), (8200, 8200, 3), (50304, 50304, 0), (2049, 2056, 8),
+                                         (256, 256, 0), (512, 512, 0), (505, 512, 0), (517, 520, 0), (300, 301, 1)])
 def test_cross_entropy_row_layouts(V, ld, first):
     """Rows that can and cannot be read in 16-byte vectors (odd strides, a first element in mid-vector), vector tails and
     batches of loads that end early; gradients land in place and nothing outside the columns changes."""
