@@ -394,6 +394,71 @@ k_col_sum_vec(const __nv_bfloat16* __restrict__ x, int M, int N, int ld, float* 
   if (threadIdx.x == 0) tickets[blockIdx.x] = 0;
 }
 
+// The same sums with 256 columns per block: 32 column vectors x 8 row lanes, each lane reading four rows at a time by itself.
+// Fewer and longer blocks, whose reads of a row are 512 bytes long: for wide matrices (tb_col_sum).
+__global__ void __launch_bounds__(256)
+k_col_sum_wide(const __nv_bfloat16* __restrict__ x, int M, int N, int ld, float* __restrict__ part, unsigned* tickets,
+              __nv_bfloat16* __restrict__ out) {
+  tb::pdl_enter();
+  __shared__ float sh[8][256 + 8];
+  __shared__ int is_last;
+  const int cx = threadIdx.x & 31, ry = threadIdx.x >> 5;
+  const int col = blockIdx.x * 256 + cx * 8;
+  const int rows_per = (M + gridDim.y - 1) / gridDim.y;
+  const int r0 = blockIdx.y * rows_per, r1 = min(M, r0 + rows_per);
+  float acc[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+  if (col < N) {
+    int r = r0 + ry;
+    for (; r + 24 < r1; r += 32) {
+      float v[4][8];
+#pragma unroll
+      for (int u = 0; u < 4; ++u) load8(x + (size_t)(r + 8 * u) * ld + col, v[u]);
+#pragma unroll
+      for (int u = 0; u < 4; ++u)
+#pragma unroll
+        for (int e = 0; e < 8; ++e) acc[e] += v[u][e];
+    }
+    for (; r < r1; r += 8) {
+      float v[8];
+      load8(x + (size_t)r * ld + col, v);
+#pragma unroll
+      for (int e = 0; e < 8; ++e) acc[e] += v[e];
+    }
+  }
+#pragma unroll
+  for (int e = 0; e < 8; ++e) sh[ry][cx * 8 + e] = acc[e];
+  __syncthreads();
+  {
+    const int c = blockIdx.x * 256 + threadIdx.x;
+    if (c < N) {
+      float t = 0.f;
+#pragma unroll
+      for (int k = 0; k < 8; ++k) t += sh[k][threadIdx.x];
+      part[(size_t)blockIdx.y * N + c] = t;
+    }
+  }
+  if (tickets == nullptr) return;
+  __threadfence();
+  __syncthreads();
+  if (threadIdx.x == 0) is_last = atomicAdd(&tickets[blockIdx.x], 1u) == gridDim.y - 1;
+  __syncthreads();
+  if (!is_last) return;
+  __threadfence();
+  {
+    const int c = blockIdx.x * 256 + threadIdx.x;
+    if (c < N) {
+      // eight lanes of every-eighth slice, combined in lane order: the grouping of k_reduce_partials
+      float lanes[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+      for (int p = 0; p < (int)gridDim.y; ++p) lanes[p & 7] += __ldcg(part + (size_t)p * N + c);
+      float t = 0.f;
+#pragma unroll
+      for (int k = 0; k < 8; ++k) t += lanes[k];
+      out[c] = __float2bfloat16_rn(t);
+    }
+  }
+  if (threadIdx.x == 0) tickets[blockIdx.x] = 0;
+}
+
 // ------------------------------------------------------------------------------------ cross-entropy
 // One block per row.  Forward: lse[row] and loss[row] = lse - logit[target].
 __global__ void __launch_bounds__(256)
@@ -701,7 +766,18 @@ int tb_layernorm_bwd_add(const void* dy, const void* x, const void* w, const flo
 int tb_col_sum(const void* x, int M, int N, int ld, void* out_bf16, float* scratch, cudaStream_t s) {
   const int slices = M >= 2048 ? 32 : (M >= 256 ? 8 : 1);
   const bool vectors = (N & 7) == 0 && (ld & 7) == 0 && ((uintptr_t)x & 15) == 0;
-  dim3 grid(vectors ? (N + 63) / 64 : (N + 31) / 32, slices);
+  // Wide matrices with few rows per slice take the kernel of 256 columns per block: the other one has four times as many
+  // blocks, more than the 592 that fit at a time, and little to fetch in each.  Measured (us, 256 / 64 columns): 2048 x 2304
+  // 11.1 / 10.3, x 3072 11.1 / 12.4, x 50304 52 / 126; 4096 x 3072 14.2 / 13.6, x 4096 15.3 / 16.2, x 8192 23.9 / 27.1;
+  // 1024 x 4096 7.7 / 7.2, x 6144 8.5 / 9.3; 1536 x 6144 10.5 / 10.3, x 8192 10.9 / 11.4; 100 x 8192 5.9 / 4.5, 64 x 50304
+  // 5.8 / 9.2; from 256 rows per slice on within 8 % of one another up to 16384 columns, 16384 x 50304 258 / 279.
+  const int rows_per = (M + slices - 1) / slices;
+  int wide_from = 16385;
+  if (slices == 1 && rows_per <= 64) wide_from = 8192;
+  if (slices == 8) wide_from = rows_per < 192 ? 5120 : 8192;
+  if (slices == 32 && rows_per <= 192) wide_from = rows_per < 128 ? 3072 : 4096;
+  const bool wide = vectors && N >= wide_from;
+  dim3 grid(wide ? (N + 255) / 256 : vectors ? (N + 63) / 64 : (N + 31) / 32, slices);
   // One launch: each column group's last block finishes the sum.  The ticket words come from a fixed pool handed
   // out round-robin, so launches in flight at the same time never share one (a pool's worth of launches would
   // have to overlap); matrices wider than the pool take the two-kernel path.
@@ -719,7 +795,9 @@ int tb_col_sum(const void* x, int M, int N, int ld, void* out_bf16, float* scrat
     unsigned* tickets = pool + next;
     next += grid.x;
     tb_note_launch(1);
-    if (vectors)
+    if (wide)
+      tb::launch(k_col_sum_wide, grid, dim3(256), 0, s, (const __nv_bfloat16*)x, M, N, ld, scratch, tickets, (__nv_bfloat16*)out_bf16);
+    else if (vectors)
       tb::launch(k_col_sum_vec, grid, dim3(256), 0, s, (const __nv_bfloat16*)x, M, N, ld, scratch, tickets, (__nv_bfloat16*)out_bf16);
     else
       tb::launch(k_col_sum, grid, dim3(1024), 0, s, (const __nv_bfloat16*)x, M, N, ld, scratch, tickets, (__nv_bfloat16*)out_bf16);

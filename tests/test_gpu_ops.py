@@ -628,6 +628,24 @@ def test_column_sums_in_vectors(M, N, ld):
     assert torch.equal(out, again)
 
 
+@pytest.mark.parametrize("M,N", [(2048, 3072), (4096, 4096), (6145, 4104), (300, 5128), (1536, 8192), (9000, 16392)])
+def test_wide_column_sums_equal_narrow_ones(M, N):
+    """Wide matrices take a kernel with more columns per block: every sum is the one that a few columns by themselves get."""
+    from tandem_b200.ops._lib import lib
+
+    x = rnd(M, N)
+    scratch = torch.empty(32 * N, dtype=torch.float32, device="cuda")
+    wide, narrow = (torch.empty(N, dtype=torch.bfloat16, device="cuda") for _ in range(2))
+    s = torch.cuda.current_stream().cuda_stream
+    assert lib().tb_col_sum(x.data_ptr(), M, N, N, wide.data_ptr(), scratch.data_ptr(), s) == 0
+    for a in range(0, N, 1024):
+        n = min(1024, N - a)
+        assert lib().tb_col_sum(x[:, a:].data_ptr(), M, n, N, narrow[a:].data_ptr(), scratch.data_ptr(), s) == 0
+    assert torch.equal(wide, narrow)
+    want = x.double().sum(0)
+    assert ((wide.double() - want).abs() <= 2.0**-8 * want.abs() + 1e-5 * M**0.5).all()
+
+
 def test_operators_without_gradients_equal_those_with():
     """Where gradients are off the operators skip the autograd node: same results; transforms that the node refuses or a
     saved-tensor hook still meet it."""
