@@ -28,17 +28,35 @@ __device__ __forceinline__ float4 grad4(const __nv_bfloat16* g) {
   return make_float4(__uint_as_float(v.x << 16), __uint_as_float(v.x & 0xffff0000u), __uint_as_float(v.y << 16), __uint_as_float(v.y & 0xffff0000u));
 }
 
-// One pass over all elements.  28 bytes per element for 15 operations: memory bounds it.  Where every array is aligned for
-// it, a thread moves four elements per access and keeps two such groups in flight (with 4-byte accesses, one element at
-// a time, 42.9 M fp32 elements took 205 us and 50 M with bf16 gradients 291 us); else, and for the last n % 4, one by one.
+// Elements [from, n) one by one.
+template <typename G>
+__device__ __forceinline__ void adam_elements(float* __restrict__ param, const G* __restrict__ grad, float* __restrict__ exp_avg,
+                                              float* __restrict__ exp_avg_sq, __nv_bfloat16* __restrict__ shadow, long long from, long long n,
+                                              const AdamScalars& s, float grad_scale) {
+  const long long stride = (long long)gridDim.x * blockDim.x;
+  for (long long i = from + (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += stride) {
+    float g = grad_of<G>(grad[i]);
+    if (grad_scale != 1.f) g = __fmul_rn(g, grad_scale);
+    float p = param[i], m = exp_avg[i], v = exp_avg_sq[i];
+    adam_update(p, m, v, g, s);
+    param[i] = p;
+    exp_avg[i] = m;
+    exp_avg_sq[i] = v;
+    if (shadow != nullptr) shadow[i] = __float2bfloat16_rn(p);
+  }
+}
+
+// One pass over all elements.  28 bytes per element for 15 operations: memory bounds it.  Where every array is aligned for it
+// (adam_vectors), a thread moves four elements per access and keeps two such groups in flight (with 4-byte accesses, one element at
+// a time, 42.9 M fp32 elements took 205 us and 50 M with bf16 gradients 291 us), and the last n % 4 go one by one; else all do.
+// Separate kernels: the loop over elements lives on resident warps, and the vectors' 64 registers make it a fifth slower
+// (42.9 M: 308 us, 242 by itself with 32).
 template <typename G, bool SCALED>
-__device__ __forceinline__ void adam_pass(float* __restrict__ param, const G* __restrict__ grad, float* __restrict__ exp_avg,
+__device__ __forceinline__ void adam_quads(float* __restrict__ param, const G* __restrict__ grad, float* __restrict__ exp_avg,
                                           float* __restrict__ exp_avg_sq, __nv_bfloat16* __restrict__ shadow, long long n, const AdamScalars& s,
                                           float grad_scale) {
   const long long stride = (long long)gridDim.x * blockDim.x, first = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  const bool aligned = (((uintptr_t)param | (uintptr_t)exp_avg | (uintptr_t)exp_avg_sq) & 15) == 0 && ((uintptr_t)grad & (4 * sizeof(G) - 1)) == 0 &&
-                       ((uintptr_t)shadow & 7) == 0;
-  const long long quads = aligned ? n / 4 : 0;
+  const long long quads = n / 4;
   for (long long i = first; i < quads; i += 2 * stride) {
     float4 g[2], p[2], m[2], v[2];
 #pragma unroll
@@ -70,36 +88,36 @@ __device__ __forceinline__ void adam_pass(float* __restrict__ param, const G* __
       }
     }
   }
-  for (long long i = 4 * quads + first; i < n; i += stride) {
-    float g = grad_of<G>(grad[i]);
-    if (SCALED) g = __fmul_rn(g, grad_scale);
-    float p = param[i], m = exp_avg[i], v = exp_avg_sq[i];
-    adam_update(p, m, v, g, s);
-    param[i] = p;
-    exp_avg[i] = m;
-    exp_avg_sq[i] = v;
-    if (shadow != nullptr) shadow[i] = __float2bfloat16_rn(p);
-  }
+  adam_elements<G>(param, grad, exp_avg, exp_avg_sq, shadow, 4 * quads, n, s, SCALED ? grad_scale : 1.f);
 }
 
+// (A hundred elements take 1.5 us in the larger kernel, 1.3 in the smaller one; from about 1000 on they are equal.)
 template <typename G>
+bool adam_vectors(const void* param, const void* grad, const void* exp_avg, const void* exp_avg_sq, const void* shadow, long long n) {
+  return n >= 512 && (((uintptr_t)param | (uintptr_t)exp_avg | (uintptr_t)exp_avg_sq) & 15) == 0 && ((uintptr_t)grad & (4 * sizeof(G) - 1)) == 0 &&
+         ((uintptr_t)shadow & 7) == 0;
+}
+
+template <typename G, bool VECTORS>
 __global__ void __launch_bounds__(256)
 k_adamw(float* __restrict__ param, const G* __restrict__ grad, float* __restrict__ exp_avg, float* __restrict__ exp_avg_sq,
         __nv_bfloat16* __restrict__ shadow, long long n, AdamScalars s, float grad_scale) {
   tb::pdl_enter();
-  if (grad_scale != 1.f) adam_pass<G, true>(param, grad, exp_avg, exp_avg_sq, shadow, n, s, grad_scale);
-  else adam_pass<G, false>(param, grad, exp_avg, exp_avg_sq, shadow, n, s, 1.f);
+  if (!VECTORS) adam_elements<G>(param, grad, exp_avg, exp_avg_sq, shadow, 0, n, s, grad_scale);
+  else if (grad_scale != 1.f) adam_quads<G, true>(param, grad, exp_avg, exp_avg_sq, shadow, n, s, grad_scale);
+  else adam_quads<G, false>(param, grad, exp_avg, exp_avg_sq, shadow, n, s, 1.f);
 }
 
 // Same update with the step-dependent scalars read from device memory, so the launch can sit in a
 // CUDA graph and still see a new bias correction on every replay.
-template <typename G>
+template <typename G, bool VECTORS>
 __global__ void __launch_bounds__(256)
 k_adamw_dev(float* __restrict__ param, const G* __restrict__ grad, float* __restrict__ exp_avg, float* __restrict__ exp_avg_sq,
             __nv_bfloat16* __restrict__ shadow, long long n, const AdamScalars* __restrict__ scalars) {
   tb::pdl_enter();
   const AdamScalars s = *scalars;
-  adam_pass<G, false>(param, grad, exp_avg, exp_avg_sq, shadow, n, s, 1.f);
+  if (!VECTORS) adam_elements<G>(param, grad, exp_avg, exp_avg_sq, shadow, 0, n, s, 1.f);
+  else adam_quads<G, false>(param, grad, exp_avg, exp_avg_sq, shadow, n, s, 1.f);
 }
 
 // One thread: step += 1, then the scalars of that step, in double precision as the host would.
@@ -169,12 +187,12 @@ int tb_adamw(void* param, const void* grad, int grad_is_bf16, void* exp_avg, voi
   long long want = (n + 256 * 4 - 1) / (256 * 4);
   int blocks = (int)(want > 148 * 8 ? 148 * 8 : want);
   tb_note_launch(1);
-  if (grad_is_bf16)
-    tb::launch(k_adamw<__nv_bfloat16>, dim3(blocks), dim3(256), 0, stream, (float*)param, (const __nv_bfloat16*)grad, (float*)exp_avg,
-               (float*)exp_avg_sq, (__nv_bfloat16*)shadow_bf16, n, s, grad_scale);
-  else
-    tb::launch(k_adamw<float>, dim3(blocks), dim3(256), 0, stream, (float*)param, (const float*)grad, (float*)exp_avg, (float*)exp_avg_sq,
-               (__nv_bfloat16*)shadow_bf16, n, s, grad_scale);
+#define ADAMW(G) \
+  tb::launch(adam_vectors<G>(param, grad, exp_avg, exp_avg_sq, shadow_bf16, n) ? k_adamw<G, true> : k_adamw<G, false>, dim3(blocks), dim3(256), 0, \
+             stream, (float*)param, (const G*)grad, (float*)exp_avg, (float*)exp_avg_sq, (__nv_bfloat16*)shadow_bf16, n, s, grad_scale)
+  if (grad_is_bf16) ADAMW(__nv_bfloat16);
+  else ADAMW(float);
+#undef ADAMW
   return (int)cudaGetLastError();
 }
 
@@ -193,12 +211,13 @@ int tb_adamw_dev(void* param, const void* grad, int grad_is_bf16, void* exp_avg,
   long long want = (n + 256 * 4 - 1) / (256 * 4);
   int blocks = (int)(want > 148 * 8 ? 148 * 8 : want);
   tb_note_launch(1);
-  if (grad_is_bf16)
-    tb::launch(k_adamw_dev<__nv_bfloat16>, dim3(blocks), dim3(256), 0, stream, (float*)param, (const __nv_bfloat16*)grad, (float*)exp_avg,
-               (float*)exp_avg_sq, (__nv_bfloat16*)shadow_bf16, n, (const AdamScalars*)scalars);
-  else
-    tb::launch(k_adamw_dev<float>, dim3(blocks), dim3(256), 0, stream, (float*)param, (const float*)grad, (float*)exp_avg, (float*)exp_avg_sq,
-               (__nv_bfloat16*)shadow_bf16, n, (const AdamScalars*)scalars);
+#define ADAMW(G) \
+  tb::launch(adam_vectors<G>(param, grad, exp_avg, exp_avg_sq, shadow_bf16, n) ? k_adamw_dev<G, true> : k_adamw_dev<G, false>, dim3(blocks), \
+             dim3(256), 0, stream, (float*)param, (const G*)grad, (float*)exp_avg, (float*)exp_avg_sq, (__nv_bfloat16*)shadow_bf16, n, \
+             (const AdamScalars*)scalars)
+  if (grad_is_bf16) ADAMW(__nv_bfloat16);
+  else ADAMW(float);
+#undef ADAMW
   return (int)cudaGetLastError();
 }
 
