@@ -149,9 +149,12 @@ __device__ __forceinline__ bool wait_chunks(const uint32_t* ready, int c_lo, int
   return true;
 }
 
-// 1 / d of two values given as -d, 1 <= d, correctly rounded: the special-function unit's approximation (1 ulp) and one
-// Newton step on the residual that an FMA leaves exact (Markstein, IBM J. Res. Dev. 34, 1990).  Above 1e30 it
-// answers 1e-30, which the caller multiplies by exp(-x^2 / 2) = 0.  __frcp_rn's range checks cost a third of the GELU epilogue.
+// 1 / d of two values given as -d, 1 <= d: the special-function unit's approximation and one Newton step on the residual that an
+// FMA leaves exact.  From an approximation within one unit in the last place that is the correctly rounded result (Markstein,
+// IBM J. Res. Dev. 34, 1990), except that the theorem leaves out the significand of all ones, where the last place may be
+// off by one; compared with a division over every significand, this unit's results were correct for that one too.  Above
+// 1e30 it answers 1e-30, which the caller multiplies by exp(-x^2 / 2) = 0.  __frcp_rn's range checks cost a third of the GELU
+// epilogue.
 __device__ __forceinline__ f32x2 reciprocal2(f32x2 minus_d) {
   float d0, d1, r0, r1;
   split2(minus_d, &d0, &d1);
@@ -1235,6 +1238,16 @@ GemmPlan plan_gemm(int M, int N, int K, int ctas) {
   return best;
 }
 
+// reciprocal2 as the GELU epilogue uses it, for comparisons with a division.
+__global__ void k_reciprocals(const float* d, float* out, long long pairs) {
+  const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= pairs) return;
+  float a, b;
+  split2(reciprocal2(pair2(-d[2 * i], -d[2 * i + 1])), &a, &b);
+  out[2 * i] = a;
+  out[2 * i + 1] = b;
+}
+
 // Flag words for split-K, handed out round-robin to launches (a launch that is handed words still in use by an earlier
 // one would need a pool's worth of launches in flight at once); all zero between launches.
 constexpr int SPLIT_FLAG_POOL = 1 << 16;
@@ -1430,6 +1443,13 @@ void tb_gemm_force_tile(int which) { g_forced_tile.store(which, std::memory_orde
 
 // 1 (default): bf16 outputs leave through TMA stores; 0: the epilogue warps store them.  For measurements.
 void tb_gemm_tma_store(int on) { g_tma_store_enabled = on; }
+
+// out[i] = 1 / d[i], i < n (even), by the GELU epilogue's own reciprocal.  For tests.
+int tb_gemm_reciprocals(const float* d, float* out, long long n, cudaStream_t stream) {
+  if (n < 2) return 0;
+  k_reciprocals<<<(unsigned)((n / 2 + 255) / 256), 256, 0, stream>>>(d, out, n / 2);
+  return (int)cudaGetLastError();
+}
 
 const char* tb_gemm_last_error() { return g_map_error; }
 

@@ -23,6 +23,7 @@ def lib():
         "tb_gemm_workspace_bytes": ([i, i, i], ctypes.c_longlong),
         "tb_gemm_plan": ([i, i, i, ctypes.POINTER(ctypes.c_int)], None),
         "tb_gemm_force_splits": ([i], None),
+        "tb_gemm_reciprocals": ([vp, vp, ctypes.c_longlong, vp], i),
         "tb_layernorm_fwd": ([vp, vp, vp, vp, vp, vp, i, i, f, vp], i),
         "tb_layernorm_bwd_blocks": ([i], i),
         "tb_layernorm_bwd": ([vp, vp, vp, vp, vp, vp, vp, vp, vp, i, i, vp], i),

@@ -142,6 +142,21 @@ def test_gemm_raster_and_edges(M, N, K, tile, force_tile):
     close(slope, gelu_slope(ref))
 
 
+@pytest.mark.parametrize("exponent", [0, 1, 8, 64, 99])
+def test_gelu_reciprocal_against_a_division(exponent):
+    """Every significand at a few powers of two (a power of two scales the whole computation exactly): one Newton step from an
+    approximation within one unit in the last place rounds correctly, but for the significand of all ones."""
+    from tandem_b200.ops._lib import lib
+
+    d = (torch.arange(1 << 23, device="cuda", dtype=torch.int32) + ((127 + exponent) << 23)).view(torch.float32)
+    d = d.clamp(max=1e30)
+    out = torch.empty_like(d)
+    assert lib().tb_gemm_reciprocals(d.data_ptr(), out.data_ptr(), d.numel(), torch.cuda.current_stream().cuda_stream) == 0
+    want = (1 / d.double()).float()  # never near a rounding tie: 1 / d is at least 2^-48 away from one
+    off = (out.view(torch.int32) - want.view(torch.int32)).abs()
+    assert off[:-1].max() == 0 and off[-1] <= 1
+
+
 @pytest.mark.parametrize("tile,N", [(5, 384), (2, 96), (1, 160), (4, 352), (3, 416), (0, 288)])
 def test_gemm_store_blocks_with_odd_chunk_counts(tile, N, force_tile):
     """Six tiles and more per CTA whose epilogue warps write an odd number of 32-column blocks each: a tile's first block is the
@@ -183,16 +198,24 @@ def test_gelu_epilogue_at_the_extremes(force_tile):
     assert got[v == float("inf")].item() == float("inf") and got[v.isnan()].isnan().all()
 
 
-@pytest.mark.parametrize("tile,splits", [(3, 2), (3, 8), (4, 3), (4, 2)])
-@pytest.mark.parametrize("M,N,K", [(768, 768, 8192), (384, 200, 2048), (130, 72, 4096), (2304, 1030, 1160), (5000, 2100, 520)])
-def test_gemm_pair_split_k(M, N, K, splits, tile, force_tile):
+SPLIT = [(3, 2), (3, 8), (4, 3), (4, 2)]  # CTA-pair tile shape, parts
+
+
+@pytest.mark.parametrize("M,N,K,tile,splits", [(*shape, *how) for shape in [(768, 768, 8192), (384, 200, 2048), (130, 72, 4096), (21100, 250, 2048)] for how in SPLIT]
+                         + [(2304, 1030, 1160, 4, 3), (2304, 1030, 1160, 4, 2), (5000, 2100, 520, 3, 2), (4864, 1030, 520, 4, 3)])
+def test_gemm_pair_split_k(M, N, K, tile, splits, force_tile):
     """The CTA-pair kernel with the reduction of its last round cut into parts: both CTAs' eight warps park and fold their
-    own rows.  (5000, 2100, 520) has whole rounds before the split one on 256 x 128 tiles."""
+    own rows.  From 2304 rows on there are whole rounds before the split one."""
+    import ctypes
+
     from tandem_b200.ops import gemm as G
     from tandem_b200.ops._lib import empty_padded, lib
 
     force_tile(tile)
     lib().tb_gemm_force_splits(splits)
+    plan = (ctypes.c_int * 4)()
+    lib().tb_gemm_plan(M, N, K, plan)
+    assert list(plan[:3]) == [512, 256 if tile == 3 else 128, splits] and (plan[3] > 0) == (M >= 2304)
     a2, b2 = empty_padded(K, M, torch.bfloat16, "cuda"), empty_padded(K, N, torch.bfloat16, "cuda")
     a2.copy_(rnd(K, M, scale=0.5)), b2.copy_(rnd(K, N, scale=0.5))
     want = a2.float().t() @ b2.float()
@@ -367,6 +390,41 @@ def test_embedding_matches_fp32():
     close(y, yf)
     close(tok.grad, tf.grad)
     close(pos.grad, pf.grad)
+
+
+@pytest.mark.parametrize("B,T,V,D", [(1, 1, 3, 8), (3, 7, 65, 24), (5, 130, 1003, 136)])
+def test_embedding_backward_vectors_and_a_misaligned_gradient(B, T, V, D):
+    """Vector tails, every batch count of the position sums' unrolled loop, and a gradient that is a contiguous slice starting in
+    mid-vector: the kernels read a copy of it.  Sums of integers up to 8 are exact in fp32, in any order."""
+    from tandem_b200 import ops
+
+    tok, pos = rnd(V, D).requires_grad_(), rnd(T + 2, D).requires_grad_()
+    idx = torch.randint(0, V, (B, T), device="cuda")
+    store = torch.randint(-8, 9, (B * T * D + 8,), device="cuda").bfloat16()
+    for first in (0, 1, 4):
+        dy = store[first:first + B * T * D].view(B, T, D)
+        assert (dy.data_ptr() % 16 == 0) == (first == 0)
+        got_tok, got_pos = torch.autograd.grad(ops.embedding(idx, tok, pos), [tok, pos], dy)
+        want = torch.zeros(V, D, device="cuda").index_add_(0, idx.view(-1), dy.float().view(-1, D))
+        assert torch.equal(got_tok, want.bfloat16())
+        assert torch.equal(got_pos[:T], dy.float().sum(0).bfloat16()) and (got_pos[T:] == 0).all()
+
+
+@pytest.mark.parametrize("sizes,offset", [([1, 15, 16, 17, 4096], 0), ([4 * 16 * 256 + 5] * 3, 0), ([70_000_003], 0), ([33_000_000, 40], 1),
+                                          ([7] * 100 + [1 << 20] * 5, 0)])
+def test_multi_copy_tails_and_large_tensors(sizes, offset):
+    """Byte tails, misaligned tensors, more tensors than one launch takes, and tensors that take the whole GPU several turns."""
+    from tandem_b200.ops.elementwise import multi_copy
+
+    pairs = []
+    for n in sizes:
+        src = torch.randint(0, 256, (n + 32,), dtype=torch.uint8, device="cuda")
+        dst = torch.zeros(n + 32, dtype=torch.uint8, device="cuda")
+        pairs.append((dst, src, n))
+    multi_copy(pairs[0][0], [(d[offset:offset + n], s[offset:offset + n]) for d, s, n in pairs])
+    for d, s, n in pairs:
+        assert torch.equal(d[offset:offset + n], s[offset:offset + n])
+        assert (d[:offset] == 0).all() and (d[offset + n:] == 0).all()
 
 
 def test_gpt_on_b200_kernels_tracks_torch_path():
@@ -588,7 +646,7 @@ def test_cross_entropy_row_layouts(V, ld, first):
     assert (store[first + rows * ld:] == 7).all()
 
 
-@pytest.mark.parametrize("n,offset", [(1, 0), (3, 0), (4097, 0), (4096, 1), (1000003, 0), (1000002, 2)])
+@pytest.mark.parametrize("n,offset", [(1, 0), (3, 0), (511, 0), (513, 0), (4097, 0), (4096, 1), (1000003, 0), (1000002, 2)])
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
 def test_fused_adamw_alignment_and_tails(n, offset, dtype):
     """Arrays that start off a 16-byte boundary take the element-wise loop, aligned ones four elements at a time plus a tail:
@@ -647,8 +705,8 @@ def test_wide_column_sums_equal_narrow_ones(M, N):
 
 
 def test_operators_without_gradients_equal_those_with():
-    """Where gradients are off the operators skip the autograd node: same results; transforms that the node refuses or a
-    saved-tensor hook still meet it."""
+    """Where gradients are off the operators skip the autograd node: same results, and transforms that the node refuses still
+    meet it.  A saved-tensor hook sees what a node saves where gradients are on, and nothing where they are off."""
     from tandem_b200 import ops
 
     x, w, b = rnd(256, 128), rnd(384, 128, scale=0.05), rnd(384)
@@ -663,6 +721,14 @@ def test_operators_without_gradients_equal_those_with():
         with torch.no_grad():
             got = call()
         assert torch.equal(got, want) and not got.requires_grad
+    seen = []
+    with torch.autograd.graph.saved_tensors_hooks(lambda t: seen.append(t.shape) or t, lambda t: t):
+        with torch.no_grad():
+            ops.linear(x, w, b)
+        assert not seen
+        y = ops.linear(x, w.clone().requires_grad_(), b)
+        assert seen == [x.shape, w.shape]
+    assert torch.equal(y, ops.linear(x, w, b))
     with torch.no_grad(), pytest.raises(RuntimeError):
         torch.func.vmap(lambda v: ops.linear(v, w, b))(x.unsqueeze(0))
     with torch.no_grad(), torch.autograd.forward_ad.dual_level(), pytest.raises((RuntimeError, NotImplementedError)):
