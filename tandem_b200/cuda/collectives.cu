@@ -16,6 +16,8 @@
 // every partial sum to the dtype, as an element-wise add chain does.
 //
 // The gradient-averaging divide is applied to each operand as it is loaded.
+#include <type_traits>
+
 #include "adam.cuh"
 #include "common.cuh"
 
@@ -121,19 +123,20 @@ __device__ __forceinline__ T fold_one(const PeerPtrs& buf, int n, int c, long lo
   return from_f<T>(acc);
 }
 
-struct NoFetch {
-  __device__ __forceinline__ uint4 operator()(long long) const { return make_uint4(0, 0, 0, 0); }
-};
+struct NoFetch {};
 
 // Vector body shared by the two-shot all-reduce and reduce-scatter: folds `nvec` 16-byte vectors of chunk
 // `rank` starting at byte offset `off0`.  NR is the group size when it is 1, 2, 4 or 8 (loops unroll exactly and
 // eight operand vectors are in flight per thread), 0 otherwise (predicated over TB_MAX_RANKS).  `fetch` loads what the
 // sink needs besides (the vector that a gradient shard already holds): its loads go out with the operands', while a load in the
-// sink would wait for the store before it.
+// sink would wait for the store before it.  The launch bounds leave 85 registers: with a fetched vector for each of eight
+// operands they spill inside the loop, so a group of one then has four on the way (24 M bf16 elements accumulated on 64 blocks:
+// 176 us, 481 with eight, 426 one by one).
 template <typename T, bool EXACT, int NR, typename Fetch, typename Sink>
 __device__ __forceinline__ void fold_vectors(const PeerPtrs& buf, int n_runtime, int rank, long long off0, long long nvec, int smode,
                                              float sval, long long tid, long long nth, Fetch&& fetch, Sink&& sink) {
-  constexpr int U = NR ? 8 / NR : 1;
+  constexpr bool FETCHES = !std::is_same<typename std::decay<Fetch>::type, NoFetch>::value;
+  constexpr int U = NR == 0 ? 1 : NR == 1 && FETCHES ? 4 : 8 / NR;
   const int n = NR ? NR : n_runtime;
   const char* ord[TB_MAX_RANKS];  // operands in fold order: ranks rank+1, ..., rank
   {
@@ -145,12 +148,12 @@ __device__ __forceinline__ void fold_vectors(const PeerPtrs& buf, int n_runtime,
     }
   }
   for (long long v = tid; v < nvec; v += nth * U) {
-    uint4 x[U][TB_MAX_RANKS], more[U];
+    uint4 x[U][TB_MAX_RANKS], more[FETCHES ? U : 1];
 #pragma unroll
     for (int u = 0; u < U; ++u) {
       const long long vv = v + u * nth;
       if (vv < nvec) {
-        more[u] = fetch(off0 + vv * 16);
+        if constexpr (FETCHES) more[u] = fetch(off0 + vv * 16);
 #pragma unroll
         for (int j = 0; j < TB_MAX_RANKS; ++j)
           if (j < n) x[u][j] = ld_vec_peer(ord[j] + off0 + vv * 16);
@@ -159,7 +162,10 @@ __device__ __forceinline__ void fold_vectors(const PeerPtrs& buf, int n_runtime,
 #pragma unroll
     for (int u = 0; u < U; ++u) {
       const long long vv = v + u * nth;
-      if (vv < nvec) sink(off0 + vv * 16, fold_vec<T, EXACT>(x[u], n, smode, sval), more[u]);
+      if (vv < nvec) {
+        if constexpr (FETCHES) sink(off0 + vv * 16, fold_vec<T, EXACT>(x[u], n, smode, sval), more[u]);
+        else sink(off0 + vv * 16, fold_vec<T, EXACT>(x[u], n, smode, sval));
+      }
     }
   }
 }
@@ -173,7 +179,7 @@ __device__ __forceinline__ void local_copy(char* dst, const char* src, long long
   const long long nth = (long long)gridDim.x * blockDim.x;
   const bool aligned = (((uintptr_t)dst | (uintptr_t)src) & 15) == 0;
   long long nvec = aligned ? numel / N : 0;
-  constexpr int U = 8;  // loads in flight per thread: one at a time copied 100 MB in 0.7 ms
+  constexpr int U = 4;  // loads in flight per thread: one at a time copied 100 MB in 0.7 ms
   for (long long v = tid; v < nvec; v += nth * U) {
     uint4 x[U];
 #pragma unroll
@@ -228,7 +234,7 @@ k_allreduce_twoshot(CommCtx c, PeerPtrs buf, Locals lin, Locals lout, long long 
     if (head > hi - lo) head = hi - lo;
     long long nvec = (hi - lo - head) / N;
     long long body = lo + head;
-    fold_vectors<T, EXACT, NR>(buf, n, rank, body * (long long)sizeof(T), nvec, smode, sval, tid, nth, NoFetch{}, [&](long long off, const uint4& r, const uint4&) {
+    fold_vectors<T, EXACT, NR>(buf, n, rank, body * (long long)sizeof(T), nvec, smode, sval, tid, nth, NoFetch{}, [&](long long off, const uint4& r) {
 #pragma unroll
       for (int q = 0; q < TB_MAX_RANKS; ++q)
         if (q < (NR ? NR : n)) st_vec(buf.p[q] + off, r);
@@ -391,34 +397,43 @@ k_reduce_scatter(CommCtx c, PeerPtrs buf, Locals lin, long long numel, Bounds bo
     if (head > hi - lo) head = hi - lo;
     const long long nvec = (hi - lo - head) / N;
     const long long body = lo + head;
-    const bool acc_vectors = EPI == 1 && ((uintptr_t)(acc_out + (body - lo)) & 15) == 0;
-    auto held = [&](long long off) {  // the shard's vector that is added to
-      return acc_vectors ? *reinterpret_cast<const uint4*>(acc_out + (off / (long long)sizeof(T) - lo)) : make_uint4(0, 0, 0, 0);
-    };
-    fold_vectors<T, EXACT, NR>(buf, n, rank, body * (long long)sizeof(T), nvec, smode, sval, tid, nth, held,
-                               [&](long long off, const uint4& r, const uint4& old) {
-      st_vec(buf.p[rank] + off, r);
-      if (EPI != 0) {
-        const long long i0 = off / (long long)sizeof(T);
-        const T* e = reinterpret_cast<const T*>(&r);
-        if (EPI == 1 && acc_vectors) {
-          const T* a = reinterpret_cast<const T*>(&old);
+    const long long first = body * (long long)sizeof(T);
+    bool done = false;
+    if constexpr (EPI == 1) {
+      // the shard's vectors are fetched with the operands; a shard that starts in mid-vector is added to element by element, in a
+      // loop of its own (sharing one, it took 170 us instead of 135 for 12 M bf16 elements from two ranks on 64 blocks)
+      if (((uintptr_t)(acc_out + (body - lo)) & 15) == 0) {
+        done = true;
+        auto held = [&](long long off) { return *reinterpret_cast<const uint4*>(acc_out + (off / (long long)sizeof(T) - lo)); };
+        fold_vectors<T, EXACT, NR>(buf, n, rank, first, nvec, smode, sval, tid, nth, held, [&](long long off, const uint4& r, const uint4& old) {
+          st_vec(buf.p[rank] + off, r);
+          const T *a = reinterpret_cast<const T*>(&old), *e = reinterpret_cast<const T*>(&r);
           uint4 sum;
 #pragma unroll
           for (int j = 0; j < N; ++j) reinterpret_cast<T*>(&sum)[j] = from_f<T>(__fadd_rn(to_f<T>(a[j]), to_f<T>(e[j])));
-          *reinterpret_cast<uint4*>(acc_out + (i0 - lo)) = sum;
-        } else if (EPI == 1) {
-#pragma unroll
-          for (int j = 0; j < N; ++j) acc_out[i0 - lo + j] = from_f<T>(__fadd_rn(to_f<T>(acc_out[i0 - lo + j]), to_f<T>(e[j])));
-        }
-        if (EPI == 2) {
-          float gv[N];
-#pragma unroll
-          for (int j = 0; j < N; ++j) gv[j] = to_f<T>(e[j]);
-          adam_vec<N>(adam, i0 - lo, gv);
-        }
+          *reinterpret_cast<uint4*>(acc_out + (off / (long long)sizeof(T) - lo)) = sum;
+        });
       }
-    });
+    }
+    if (!done) {
+      fold_vectors<T, EXACT, NR>(buf, n, rank, first, nvec, smode, sval, tid, nth, NoFetch{}, [&](long long off, const uint4& r) {
+        st_vec(buf.p[rank] + off, r);
+        if (EPI != 0) {
+          const long long i0 = off / (long long)sizeof(T);
+          const T* e = reinterpret_cast<const T*>(&r);
+          if (EPI == 1) {
+#pragma unroll
+            for (int j = 0; j < N; ++j) acc_out[i0 - lo + j] = from_f<T>(__fadd_rn(to_f<T>(acc_out[i0 - lo + j]), to_f<T>(e[j])));
+          }
+          if (EPI == 2) {
+            float gv[N];
+#pragma unroll
+            for (int j = 0; j < N; ++j) gv[j] = to_f<T>(e[j]);
+            adam_vec<N>(adam, i0 - lo, gv);
+          }
+        }
+      });
+    }
     const long long ntail = (hi - lo) - nvec * N;
     for (long long t = tid; t < ntail; t += nth) {
       long long i = t < head ? lo + t : body + nvec * N + (t - head);
