@@ -777,28 +777,29 @@ k_attn_bwd_dkv(const __grid_constant__ CUtensorMap map_qkv, const __grid_constan
         tmem_ld32(tmem + C_S + lane_base + half * 64, s[0]);
         tmem_ld32(tmem + C_S + lane_base + half * 64 + 32, s[1]);
         tmem_ld_wait();
+        auto probabilities = [&](bool diagonal) {
 #pragma unroll
-        for (int q = 0; q < 16; ++q) {
-          const float4 l4 = lse4[q];
+          for (int q = 0; q < 16; ++q) {
+            const float4 l4 = lse4[q];
 #pragma unroll
-          for (int u = 0; u < 2; ++u) {
-            const int e = 2 * q + u, c = (2 * e) >> 5, k = (2 * e) & 31;
-            const f32x2 shift = mul2(minus_log2e2, u == 0 ? pair2(l4.x, l4.y) : pair2(l4.z, l4.w));
-            float x0, x1;
-            split2(fma2(pair2(__uint_as_float(s[c][k]), __uint_as_float(s[c][k + 1])), scale_log2e2, shift), &x0, &x1);
-            p[e] = pair2(ex2_approx(x0), ex2_approx(x1));
-            pk[e] = bf16_pair(p[e]);
+            for (int u = 0; u < 2; ++u) {
+              const int e = 2 * q + u, c = (2 * e) >> 5, k = (2 * e) & 31;
+              const f32x2 shift = mul2(minus_log2e2, u == 0 ? pair2(l4.x, l4.y) : pair2(l4.z, l4.w));
+              float x0, x1;
+              split2(fma2(pair2(__uint_as_float(s[c][k]), __uint_as_float(s[c][k + 1])), scale_log2e2, shift), &x0, &x1);
+              x0 = ex2_approx(x0), x1 = ex2_approx(x1);
+              if (diagonal) {
+                x0 = r > half * 64 + 2 * e ? 0.f : x0;
+                x1 = r > half * 64 + 2 * e + 1 ? 0.f : x1;
+              }
+              p[e] = pair2(x0, x1);
+              pk[e] = bf16_pair(p[e]);
+            }
           }
-        }
-        if (i == kt) {  // the diagonal tile: nothing of a query reaches the keys after it, not even the NaN of one whose sum is NaN
-#pragma unroll
-          for (int e = 0; e < 32; ++e) {
-            float x0, x1;
-            split2(p[e], &x0, &x1);
-            p[e] = pair2(r > half * 64 + 2 * e ? 0.f : x0, r > half * 64 + 2 * e + 1 ? 0.f : x1);
-            pk[e] = bf16_pair(p[e]);
-          }
-        }
+        };
+        // In the diagonal tile nothing of a query reaches the keys after it, not even the NaN of one whose sum is NaN.
+        if (i == kt) probabilities(true);
+        else probabilities(false);
         tmem_st32(tmem + C_S + lane_base + half * 64, pk);
         tmem_st_wait();
       }
