@@ -11,6 +11,7 @@
 #include <atomic>
 #include <mutex>
 
+#include "f32x2.cuh"
 #include "launch.cuh"
 #include "noalloc.h"
 
@@ -59,37 +60,65 @@ __device__ __forceinline__ void store8(__nv_bfloat16* p, const float* f) {
   *reinterpret_cast<uint4*>(p) = v;
 }
 
+__device__ __forceinline__ void named_sync(int id, int threads) { asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(threads) : "memory"); }
+__device__ __forceinline__ void named_arrive(int id, int threads) { asm volatile("bar.arrive %0, %1;" ::"r"(id), "r"(threads) : "memory"); }
+
 // ------------------------------------------------------------------------------------ LayerNorm
-// One warp per row; D is a multiple of 8.  MAXV 16-byte vectors per lane cover D <= 32*8*MAXV.
-template <int MAXV>
-__global__ void __launch_bounds__(256)
+// One warp per row; D is a multiple of 8.  MAXV 16-byte vectors per lane cover D <= 32*8*MAXV.  It is bound by the rows on their
+// way to an SM, so a row waits for its reductions as it came, in bf16 pairs (unpacked, 2048 columns took 64 registers a lane
+// and left 16 warps on an SM: 16384 x 2048 in 34.9 us, now 25.1, 21 at the copy rate).  EARLY also fetches the gain and bias before the
+// reductions, for another 8 * MAXV registers: where all rows are resident at once even so (tb_layernorm_fwd), a trip to L2 is
+// what counts (2048 x 2048: 5.3 us, 7.4 without), elsewhere the resident warps (16384 x 1024: 13.9 us without, 15.0 with).
+template <int MAXV, bool EARLY>
+__global__ void __launch_bounds__(256, EARLY && MAXV == 4 ? 4 : 1)
 k_ln_fwd(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ w, const __nv_bfloat16* __restrict__ b,
          __nv_bfloat16* __restrict__ y, float* __restrict__ mean_out, float* __restrict__ rstd_out, int M, int D, float eps) {
   tb::pdl_enter();
+  using namespace tc;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int row = blockIdx.x * (blockDim.x >> 5) + warp;
   if (row >= M) return;
   const int nvec = D >> 3;
-  float v[MAXV][8];
+  uint4 v[MAXV];
+#pragma unroll
+  for (int j = 0; j < MAXV; ++j)
+    if (lane + 32 * j < nvec) v[j] = *reinterpret_cast<const uint4*>(x + (size_t)row * D + (lane + 32 * j) * 8);
+  uint4 wv[MAXV], bv[MAXV];
+  auto gains = [&](int j) {
+    if (lane + 32 * j < nvec) {
+      wv[j] = __ldg(reinterpret_cast<const uint4*>(w + (lane + 32 * j) * 8));
+      bv[j] = __ldg(reinterpret_cast<const uint4*>(b + (lane + 32 * j) * 8));
+    }
+  };
+  if (EARLY) {
+#pragma unroll
+    for (int j = 0; j < MAXV; ++j) gains(j);
+  }
   float sum = 0.f;
 #pragma unroll
   for (int j = 0; j < MAXV; ++j) {
-    const int vi = lane + 32 * j;
-    if (vi < nvec) {
-      load8(x + (size_t)row * D + vi * 8, v[j]);
+    if (lane + 32 * j < nvec) {
+      const uint32_t xp[4] = {v[j].x, v[j].y, v[j].z, v[j].w};
 #pragma unroll
-      for (int e = 0; e < 8; ++e) sum += v[j][e];
+      for (int p = 0; p < 4; ++p) {
+        sum += __uint_as_float(xp[p] << 16);
+        sum += __uint_as_float(xp[p] & 0xffff0000u);
+      }
     }
   }
   const float mean = warp_sum(sum) / D;
+  const f32x2 minus_mean2 = pair2(-mean, -mean);
   float sq = 0.f;
 #pragma unroll
   for (int j = 0; j < MAXV; ++j) {
     if (lane + 32 * j < nvec) {
+      const uint32_t xp[4] = {v[j].x, v[j].y, v[j].z, v[j].w};
 #pragma unroll
-      for (int e = 0; e < 8; ++e) {
-        const float d = v[j][e] - mean;
-        sq += d * d;
+      for (int p = 0; p < 4; ++p) {
+        float d0, d1;
+        split2(add2(from_bf16_pair(xp[p]), minus_mean2), &d0, &d1);
+        sq = fmaf(d0, d0, sq);
+        sq = fmaf(d1, d1, sq);
       }
     }
   }
@@ -98,153 +127,244 @@ k_ln_fwd(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ 
     mean_out[row] = mean;
     rstd_out[row] = rstd;
   }
+  const f32x2 rstd2 = pair2(rstd, rstd);
 #pragma unroll
   for (int j = 0; j < MAXV; ++j) {
     const int vi = lane + 32 * j;
     if (vi < nvec) {
-      float wv[8], bv[8], o[8];
-      load8(w + vi * 8, wv);
-      load8(b + vi * 8, bv);
+      if (!EARLY) gains(j);
+      const uint32_t xp[4] = {v[j].x, v[j].y, v[j].z, v[j].w}, wp[4] = {wv[j].x, wv[j].y, wv[j].z, wv[j].w},
+                     bp[4] = {bv[j].x, bv[j].y, bv[j].z, bv[j].w};
+      uint32_t o[4];
 #pragma unroll
-      for (int e = 0; e < 8; ++e) o[e] = (v[j][e] - mean) * rstd * wv[e] + bv[e];
-      store8(y + (size_t)row * D + vi * 8, o);
+      for (int p = 0; p < 4; ++p)
+        o[p] = bf16_pair(fma2(mul2(add2(from_bf16_pair(xp[p]), minus_mean2), rstd2), from_bf16_pair(wp[p]), from_bf16_pair(bp[p])));
+      *reinterpret_cast<uint4*>(y + (size_t)row * D + vi * 8) = make_uint4(o[0], o[1], o[2], o[3]);
     }
   }
 }
 
-// dx for each row, and per-block partial sums of dw = sum dy*xhat and db = sum dy into
-// part[blockIdx.x][2][D] (fp32).  A second kernel adds the partials in a fixed order.
+__device__ __forceinline__ void cp_async16(void* dst, const void* src) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src) : "memory");
+}
+__device__ __forceinline__ void cp_async4(void* dst, const void* src) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src) : "memory");
+}
+
+// dx for each row, and partial sums of dw = sum dy*xhat and db = sum dy into part[slice][2][D] (fp32).  A second
+// kernel adds the partials in a fixed order.  Rows are dealt to the `slices` eight at a time, round-robin; within a slice
+// warp w sums row w of every eight in order, and the eight warps' sums are added in order, whatever the grid.
 // add (optional): a second gradient of the same input, summed into dx in fp32 before the one rounding
 // -- the residual branch's gradient in a pre-LayerNorm block, which autograd would otherwise add with a
-// separate pass over the activations.
-// Rows are software-pipelined: while a warp works on one row, the 16-byte loads of its next row (dy and x, kept
-// packed as bf16 so that they cost half the registers) are already in flight, and the residual gradient of the
-// current row is requested before the row's reductions start.  With one row per warp in flight the kernel ran at
-// the pace of one memory round trip per row (0.42 of the copy bandwidth); two rows per warp and two blocks per SM
-// keep about 100 KB per SM on the way.
+// separate pass over the activations.  It may alias dx: a row's dx is written only after its `add` has been read.
+//
+// What bounds it is bytes on the way to an SM.  dw and db of a warp's columns take 16 * MAXV registers, which leaves none for
+// rows that have not arrived yet.  So rows travel by cp.async into a ring of `stages` rows per warp in shared memory; each
+// lane fetches the vectors that it alone reads, so the ring needs no barrier.  With the next row held in registers, and
+// spills, 4096 x 1024 took 17.7 us, now 9.1 (5.1 at the copy rate); 8192 x 768 14.2, now 10.2 (7.7); 16384 x 2048 88, now 50 (41);
+// 1024 x 768 5.2, now 3.8.
+// A block with one slice adds its warps' sums side by side, in the shared memory of the ring.  A block with several keeps the ring
+// busy: the sums meet in one [2][D] array, warp after warp (each adds its own and hands the array on through a named
+// barrier), so that the first warps are on their next rows while the last ones add.
 template <int MAXV>
+struct LnBwd {
+  static constexpr int STAGES = MAXV <= 2 ? 4 : 2;
+  static constexpr int VEC_ROW = 32 * MAXV;  // 16-byte vectors of a row, padded to whole warps
+  static constexpr int SUMS = 2 * 2 * VEC_ROW * 16;  // the array: fp32 dw and db
+  static constexpr int STATS = 8 * STAGES * 2 * 4;   // mean and 1/std of every row in the ring
+  static int smem(int stages, bool add, bool one_slice) {
+    const int ring = SUMS + STATS + 8 * stages * (add ? 3 : 2) * VEC_ROW * 16;
+    return one_slice && ring < 8 * SUMS ? 8 * SUMS : ring;
+  }
+};
+
+template <int MAXV, bool ADD>
 __global__ void __launch_bounds__(256, MAXV <= 4 ? 2 : 1)
 k_ln_bwd(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ w,
-         const float* __restrict__ mean_in, const float* __restrict__ rstd_in, const __nv_bfloat16* __restrict__ add,
-         __nv_bfloat16* __restrict__ dx, float* __restrict__ part, int M, int D) {
+         const float* __restrict__ mean_in, const float* __restrict__ rstd_in, const __nv_bfloat16* add,
+         __nv_bfloat16* dx, float* __restrict__ part, int M, int D, int slices, int stages) {
   tb::pdl_enter();
-  extern __shared__ __align__(16) float sh[];  // [warps][2][D]
-  const int warps = blockDim.x >> 5;
+  using namespace tc;
+  using L = LnBwd<MAXV>;
+  extern __shared__ __align__(16) uint8_t ln_smem[];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int nvec = D >> 3;
-  float dw[MAXV][8], db[MAXV][8];
+  float4* sums = reinterpret_cast<float4*>(ln_smem);  // [dw, db][MAXV][two halves of a lane's vector][32 lanes]
+  float* stats = reinterpret_cast<float*>(ln_smem + L::SUMS) + warp * L::STAGES * 2;
+  constexpr int TENSORS = ADD ? 3 : 2;
+  uint4* ring = reinterpret_cast<uint4*>(ln_smem + L::SUMS + L::STATS) + (size_t)warp * stages * TENSORS * L::VEC_ROW + lane;
+
+  uint4 wv[MAXV];
+  f32x2 dw[MAXV][4], db[MAXV][4];
 #pragma unroll
   for (int j = 0; j < MAXV; ++j)
-#pragma unroll
-    for (int e = 0; e < 8; ++e) dw[j][e] = db[j][e] = 0.f;
-  const int stride = gridDim.x * warps;
-  int row = blockIdx.x * warps + warp;
-  constexpr bool AHEAD = MAXV <= 4;  // wider rows have no registers left for a second row
-  uint4 ndy[MAXV], nx[MAXV];  // the next row, packed
-  float nmean = 0.f, nrstd = 0.f;
-  auto fetch = [&](int r) {
-#pragma unroll
-    for (int j = 0; j < MAXV; ++j) {
-      const int vi = lane + 32 * j;
-      if (vi < nvec) {
-        ndy[j] = __ldg(reinterpret_cast<const uint4*>(dy + (size_t)r * D + vi * 8));
-        nx[j] = __ldg(reinterpret_cast<const uint4*>(x + (size_t)r * D + vi * 8));
-      }
-    }
-    nmean = mean_in[r];
-    nrstd = rstd_in[r];
-  };
-  if (AHEAD && row < M) fetch(row);
-  for (; row < M; row += stride) {
-    if (!AHEAD) fetch(row);
-    uint4 cdy[MAXV], cx[MAXV], cadd[MAXV];
-    const float mean = nmean, rstd = nrstd;
-#pragma unroll
-    for (int j = 0; j < MAXV; ++j) {
-      cdy[j] = ndy[j];
-      cx[j] = nx[j];
-    }
-    if (AHEAD && row + stride < M) fetch(row + stride);
-    if (add != nullptr) {  // may alias dx: this row's dx is written only after these loads have been consumed
+    if (lane + 32 * j < nvec) wv[j] = *reinterpret_cast<const uint4*>(w + (lane + 32 * j) * 8);
+
+  // the warp's rows in the order in which it works on them: (slice, turn) -> row
+  auto row_of = [&](int slice, int turn) { return (slice + turn * slices) * 8 + warp; };
+  int f_slice = blockIdx.x, f_turn = 0, f_stage = 0;  // the next row to fetch
+  auto fetch = [&]() {
+    const int row = row_of(f_slice, f_turn);
+    if (f_slice < slices && row < M) {
+      uint4* slot = ring + (size_t)f_stage * TENSORS * L::VEC_ROW;
 #pragma unroll
       for (int j = 0; j < MAXV; ++j) {
         const int vi = lane + 32 * j;
-        if (vi < nvec) cadd[j] = *reinterpret_cast<const uint4*>(add + (size_t)row * D + vi * 8);
+        if (vi < nvec) {
+          const size_t at = (size_t)row * D + vi * 8;
+          cp_async16(slot + 32 * j, dy + at);
+          cp_async16(slot + L::VEC_ROW + 32 * j, x + at);
+          if (ADD) cp_async16(slot + 2 * L::VEC_ROW + 32 * j, add + at);
+        }
+      }
+      if (lane < 2) cp_async4(stats + 2 * f_stage + lane, (lane == 0 ? mean_in : rstd_in) + row);
+      if (++f_stage == stages) f_stage = 0;
+      ++f_turn;
+      if (row_of(f_slice, f_turn) >= M) f_turn = 0, f_slice += gridDim.x;
+    }
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  };
+  int stage = 0;
+  for (int i = 0; i < stages - 1; ++i) fetch();
+
+  for (int slice = blockIdx.x; slice < slices; slice += gridDim.x) {
+#pragma unroll
+    for (int j = 0; j < MAXV; ++j)
+#pragma unroll
+      for (int p = 0; p < 4; ++p) dw[j][p] = db[j][p] = pair2(0.f, 0.f);
+    for (int turn = 0, row; (row = row_of(slice, turn)) < M; ++turn) {
+      __syncwarp();  // the slot that is filled next has been read by every lane
+      fetch();
+      if (stages == 1) asm volatile("cp.async.wait_group 0;" ::: "memory");
+      else if (stages == 2) asm volatile("cp.async.wait_group 1;" ::: "memory");
+      else if (stages == 3) asm volatile("cp.async.wait_group 2;" ::: "memory");
+      else asm volatile("cp.async.wait_group 3;" ::: "memory");
+      __syncwarp();
+      const uint4* slot = ring + (size_t)stage * TENSORS * L::VEC_ROW;
+      const float mean = stats[2 * stage], rstd = stats[2 * stage + 1];
+      if (++stage == stages) stage = 0;
+      const f32x2 minus_mean2 = pair2(-mean, -mean), rstd2 = pair2(rstd, rstd);
+      float s1 = 0.f, s2 = 0.f;
+#pragma unroll
+      for (int j = 0; j < MAXV; ++j) {
+        if (lane + 32 * j < nvec) {
+          const uint4 a = slot[32 * j], b = slot[L::VEC_ROW + 32 * j];
+          const uint32_t dyp[4] = {a.x, a.y, a.z, a.w}, xp[4] = {b.x, b.y, b.z, b.w}, wp[4] = {wv[j].x, wv[j].y, wv[j].z, wv[j].w};
+#pragma unroll
+          for (int p = 0; p < 4; ++p) {
+            const f32x2 dy2 = from_bf16_pair(dyp[p]);
+            const f32x2 xh2 = mul2(add2(from_bf16_pair(xp[p]), minus_mean2), rstd2);
+            const f32x2 g2 = mul2(dy2, from_bf16_pair(wp[p]));
+            float h0, h1, g0, g1;
+            split2(xh2, &h0, &h1);
+            split2(g2, &g0, &g1);
+            s1 += g0;
+            s2 = fmaf(g0, h0, s2);
+            s1 += g1;
+            s2 = fmaf(g1, h1, s2);
+            dw[j][p] = fma2(dy2, xh2, dw[j][p]);
+            db[j][p] = add2(db[j][p], dy2);
+          }
+        }
+      }
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) {  // warp_sum of both, side by side
+        const float t1 = __shfl_xor_sync(0xffffffffu, s1, o), t2 = __shfl_xor_sync(0xffffffffu, s2, o);
+        s1 += t1;
+        s2 += t2;
+      }
+      s1 /= D;
+      s2 /= D;
+      const f32x2 minus_s1 = pair2(-s1, -s1), minus_s2 = pair2(-s2, -s2);
+#pragma unroll
+      for (int j = 0; j < MAXV; ++j) {
+        const int vi = lane + 32 * j;
+        if (vi < nvec) {
+          const uint4 a = slot[32 * j], b = slot[L::VEC_ROW + 32 * j];
+          const uint4 c = ADD ? slot[2 * L::VEC_ROW + 32 * j] : make_uint4(0, 0, 0, 0);
+          const uint32_t dyp[4] = {a.x, a.y, a.z, a.w}, xp[4] = {b.x, b.y, b.z, b.w}, wp[4] = {wv[j].x, wv[j].y, wv[j].z, wv[j].w},
+                         ap[4] = {c.x, c.y, c.z, c.w};
+          uint32_t o[4];
+#pragma unroll
+          for (int p = 0; p < 4; ++p) {
+            const f32x2 xh2 = mul2(add2(from_bf16_pair(xp[p]), minus_mean2), rstd2);  // the same operations as above: the same values
+            f32x2 t = fma2(xh2, minus_s2, fma2(from_bf16_pair(dyp[p]), from_bf16_pair(wp[p]), minus_s1));
+            t = mul2(rstd2, t);
+            float o0, o1;
+            split2(t, &o0, &o1);
+            if (ADD) {  // scalar: the assembler would make one fma of a packed product and sum, and round once less
+              o0 = __fadd_rn(o0, __uint_as_float(ap[p] << 16));
+              o1 = __fadd_rn(o1, __uint_as_float(ap[p] & 0xffff0000u));
+            }
+            o[p] = bf16_pair(pair2(o0, o1));
+          }
+          *reinterpret_cast<uint4*>(dx + (size_t)row * D + vi * 8) = make_uint4(o[0], o[1], o[2], o[3]);
+        }
       }
     }
-    float s1 = 0.f, s2 = 0.f;
+    float* out = part + (size_t)slice * 2 * D;
+    // value q of vector j: dw's or db's (q >> 1) columns 4 * (q & 1) .. + 3 of the lane's eight
+    auto mine = [&](int j, int q) {
+      float4 t;
+      const f32x2* v = (q < 2 ? dw[j] : db[j]) + 2 * (q & 1);
+      split2(v[0], &t.x, &t.y);
+      split2(v[1], &t.z, &t.w);
+      return t;
+    };
+    auto place = [&](int j, int q, int l) { return ((q >> 1) * MAXV + j) * 64 + (q & 1) * 32 + l; };
+    if (gridDim.x == slices) {  // the block's only slice: the ring is free, and all columns are added side by side
+      __syncthreads();
+      float4* all = sums + warp * 128 * MAXV;
+#pragma unroll
+      for (int j = 0; j < MAXV; ++j)
+#pragma unroll
+        for (int q = 0; q < 4; ++q) all[place(j, q, lane)] = mine(j, q);
+      __syncthreads();
+      for (int i = threadIdx.x; i < 128 * MAXV; i += 256) {
+        const int q = (i >> 5) & 1, j = (i >> 6) % MAXV, half = (i >> 6) / MAXV, vi = (i & 31) + 32 * j;
+        if (vi >= nvec) continue;
+        float4 t = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+        for (int k = 0; k < 8; ++k) {
+          const float4 v = sums[k * 128 * MAXV + i];
+          t.x += v.x; t.y += v.y; t.z += v.z; t.w += v.w;
+        }
+        *reinterpret_cast<float4*>(out + half * D + vi * 8 + 4 * q) = t;
+      }
+      return;
+    }
+    // warp 0 waits until the last warp has read the previous slice's sums, every other one for the warp before it
+    if (warp > 0 || slice != (int)blockIdx.x) named_sync(1 + (warp + 7) % 8, 64);
 #pragma unroll
     for (int j = 0; j < MAXV; ++j) {
       const int vi = lane + 32 * j;
       if (vi < nvec) {
-        float dyv[8], xv[8], wv[8];
-        unpack8(cdy[j], dyv);
-        unpack8(cx[j], xv);
-        load8(w + vi * 8, wv);
 #pragma unroll
-        for (int e = 0; e < 8; ++e) {
-          const float xh = (xv[e] - mean) * rstd;
-          const float gv = dyv[e] * wv[e];
-          s1 += gv;
-          s2 += gv * xh;
-          dw[j][e] += dyv[e] * xh;
-          db[j][e] += dyv[e];
+        for (int q = 0; q < 4; ++q) {
+          const float4 m = mine(j, q);
+          float4 t = warp == 0 ? make_float4(0.f, 0.f, 0.f, 0.f) : sums[place(j, q, lane)];
+          t.x += m.x; t.y += m.y; t.z += m.z; t.w += m.w;
+          if (warp < 7) sums[place(j, q, lane)] = t;
+          else *reinterpret_cast<float4*>(out + (q >> 1) * D + vi * 8 + 4 * (q & 1)) = t;
         }
       }
     }
-    s1 = warp_sum(s1) / D;
-    s2 = warp_sum(s2) / D;
-#pragma unroll
-    for (int j = 0; j < MAXV; ++j) {
-      const int vi = lane + 32 * j;
-      if (vi < nvec) {
-        float dyv[8], xv[8], wv[8], o[8];
-        unpack8(cdy[j], dyv);
-        unpack8(cx[j], xv);
-        load8(w + vi * 8, wv);
-#pragma unroll
-        for (int e = 0; e < 8; ++e) {
-          const float xh = (xv[e] - mean) * rstd;  // the same operations as above: the same values
-          o[e] = rstd * (dyv[e] * wv[e] - s1 - xh * s2);
-        }
-        if (add != nullptr) {
-          float a[8];
-          unpack8(cadd[j], a);
-#pragma unroll
-          for (int e = 0; e < 8; ++e) o[e] += a[e];
-        }
-        store8(dx + (size_t)row * D + vi * 8, o);
-      }
-    }
-  }
-#pragma unroll
-  for (int j = 0; j < MAXV; ++j) {
-    const int vi = lane + 32 * j;
-    if (vi < nvec) {
-#pragma unroll
-      for (int q = 0; q < 2; ++q) {  // 16-byte stores: scalar ones, 32 bytes apart from lane to lane, meet in the same bank eight at a time
-        *reinterpret_cast<float4*>(sh + (warp * 2 + 0) * D + vi * 8 + 4 * q) = *reinterpret_cast<const float4*>(&dw[j][4 * q]);
-        *reinterpret_cast<float4*>(sh + (warp * 2 + 1) * D + vi * 8 + 4 * q) = *reinterpret_cast<const float4*>(&db[j][4 * q]);
-      }
-    }
-  }
-  __syncthreads();
-  for (int i = threadIdx.x; i < 2 * D; i += blockDim.x) {
-    float acc = 0.f;
-    for (int wv = 0; wv < warps; ++wv) acc += sh[wv * 2 * D + i];
-    part[(size_t)blockIdx.x * 2 * D + i] = acc;
+    if (warp < 7 || slice + (int)gridDim.x < slices) named_arrive(1 + warp, 64);
   }
 }
 
-// out[c] = sum over p of part[p][c], written as bf16.  32 columns x 8 row lanes per block: each lane adds
-// every 8th partial, then the 8 lanes are combined in a fixed order (deterministic).
-__global__ void __launch_bounds__(256)
+// out[c] = sum over p of part[p][c], written as bf16.  16 columns x 8 row lanes per block: each lane adds
+// every 8th partial, then the 8 lanes are combined in a fixed order (deterministic).  It is bound by the loads that an SM can
+// have under way, so narrow blocks on many SMs: 296 x 2048 partials 3.7 us with 32 columns, 2.65 with 16, 2.7 with 8.
+constexpr int PARTIAL_COLS = 16;
+__global__ void __launch_bounds__(128)
 k_reduce_partials(const float* __restrict__ part, int parts, int width, __nv_bfloat16* __restrict__ out0,
                   __nv_bfloat16* __restrict__ out1, int split) {
   tb::pdl_enter();
-  __shared__ float sh[8][33];
-  const int cx = threadIdx.x & 31, ry = threadIdx.x >> 5;
-  const int c = blockIdx.x * 32 + cx;
+  constexpr int COLS = PARTIAL_COLS;
+  __shared__ float sh[8][COLS + 1];
+  const int cx = threadIdx.x % COLS, ry = threadIdx.x / COLS;
+  const int c = blockIdx.x * COLS + cx;
   float acc = 0.f;
   if (c < width && parts <= 64) {  // up to eight per lane: the long body below costs more than it saves (512 x 256 backward: 4.5 / 4.9 us)
     for (int p = ry; p < parts; p += 8) acc += part[(size_t)p * width + c];
@@ -719,16 +839,24 @@ int tb_layernorm_fwd(const void* x, const void* w, const void* b, void* y, float
   if (D % 8 || D > 32 * 8 * 8) return -20;
   const int blocks = (M + 7) / 8;
   tb_note_launch(1);
-#define LN(V) tb::launch(k_ln_fwd<V>, dim3(blocks), dim3(256), 0, s, (const __nv_bfloat16*)x, (const __nv_bfloat16*)w, (const __nv_bfloat16*)b, (__nv_bfloat16*)y, mean, rstd, M, D, eps)
+#define LN1(V, EARLY) tb::launch(k_ln_fwd<V, EARLY>, dim3(blocks), dim3(256), 0, s, (const __nv_bfloat16*)x, (const __nv_bfloat16*)w, (const __nv_bfloat16*)b, (__nv_bfloat16*)y, mean, rstd, M, D, eps)
+#define LN(V)                              \
+  do {                                     \
+    if (blocks <= 148 * (V <= 4 ? 4 : 2)) LN1(V, true); \
+    else LN1(V, false);                    \
+  } while (0)
   if (D <= 256 * 1) LN(1);
   else if (D <= 256 * 2) LN(2);
+  else if (D <= 256 * 3) LN(3);
   else if (D <= 256 * 4) LN(4);
+  else if (D <= 256 * 6) LN(6);
   else LN(8);
+#undef LN1
 #undef LN
   return (int)cudaGetLastError();
 }
 
-// scratch: fp32 [blocks * 2 * D] with blocks = tb_layernorm_bwd_blocks(M).
+// scratch: fp32 [slices * 2 * D] with slices = tb_layernorm_bwd_blocks(M), 16-byte aligned.
 // Few rows: one row per warp on as many SMs as it takes (at 1024 rows four rows per warp would leave 116 SMs idle);
 // many rows: several rows per warp, so that the row look-ahead has something to fetch.
 int tb_layernorm_bwd_blocks(int M) { return M < 8192 ? grid_for(M, 8, 296) : grid_for(M, 8 * 4, 592); }
@@ -745,22 +873,34 @@ int tb_layernorm_bwd(const void* dy, const void* x, const void* w, const float* 
 int tb_layernorm_bwd_add(const void* dy, const void* x, const void* w, const float* mean, const float* rstd, const void* add, void* dx,
                          void* dw, void* db, float* scratch, int M, int D, cudaStream_t s) {
   if (D % 8 || D > 32 * 8 * 8) return -20;
-  const int blocks = tb_layernorm_bwd_blocks(M);
-  const size_t smem = (size_t)8 * 2 * D * sizeof(float);
+  // as many blocks as are resident (registers allow two on an SM up to 1024 columns); rows: the most that a warp works on
+  const int slices = tb_layernorm_bwd_blocks(M), per_warp = (M + slices * 8 - 1) / (slices * 8);
   tb_note_launch(2);
-#define LN(V)                                                                                                          \
-  do {                                                                                                                 \
-    if (smem > 48 * 1024) cudaFuncSetAttribute(k_ln_bwd<V>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);   \
-    tb::launch(k_ln_bwd<V>, dim3(blocks), dim3(256), smem, s, (const __nv_bfloat16*)dy, (const __nv_bfloat16*)x,          \
-               (const __nv_bfloat16*)w, mean, rstd, (const __nv_bfloat16*)add, (__nv_bfloat16*)dx, scratch, M, D);          \
+#define LN1(V, ADD)                                                                                                              \
+  do {                                                                                                                           \
+    const int resident = 148 * (V <= 4 ? 2 : 1), grid = slices < resident ? slices : resident;                                  \
+    const int rows = per_warp * ((slices + grid - 1) / grid), stages = rows < LnBwd<V>::STAGES ? rows : LnBwd<V>::STAGES;       \
+    const int smem = LnBwd<V>::smem(stages, ADD, grid == slices);                                                                               \
+    static const cudaError_t allowed = cudaFuncSetAttribute(k_ln_bwd<V, ADD>, cudaFuncAttributeMaxDynamicSharedMemorySize,      \
+                                                            LnBwd<V>::smem(LnBwd<V>::STAGES, ADD, true));                       \
+    if (allowed != cudaSuccess) return (int)allowed;                                                                            \
+    tb::launch(k_ln_bwd<V, ADD>, dim3(grid), dim3(256), (size_t)smem, s, (const __nv_bfloat16*)dy, (const __nv_bfloat16*)x,     \
+               (const __nv_bfloat16*)w, mean, rstd, (const __nv_bfloat16*)add, (__nv_bfloat16*)dx, scratch, M, D, slices, stages); \
+  } while (0)
+#define LN(V)                        \
+  do {                               \
+    if (add != nullptr) LN1(V, true); \
+    else LN1(V, false);              \
   } while (0)
   if (D <= 256 * 1) LN(1);
   else if (D <= 256 * 2) LN(2);
   else if (D <= 256 * 3) LN(3);
   else if (D <= 256 * 4) LN(4);
+  else if (D <= 256 * 6) LN(6);
   else LN(8);
 #undef LN
-  tb::launch(k_reduce_partials, dim3((2 * D + 31) / 32), dim3(256), 0, s, (const float*)scratch, blocks, 2 * D, (__nv_bfloat16*)dw, (__nv_bfloat16*)db, D);
+#undef LN1
+  tb::launch(k_reduce_partials, dim3((2 * D + PARTIAL_COLS - 1) / PARTIAL_COLS), dim3(8 * PARTIAL_COLS), 0, s, (const float*)scratch, slices, 2 * D, (__nv_bfloat16*)dw, (__nv_bfloat16*)db, D);
   return (int)cudaGetLastError();
 }
 
@@ -808,7 +948,7 @@ int tb_col_sum(const void* x, int M, int N, int ld, void* out_bf16, float* scrat
   grid = dim3((N + 31) / 32, slices);
   tb_note_launch(2);
   tb::launch(k_col_sum, grid, dim3(1024), 0, s, (const __nv_bfloat16*)x, M, N, ld, scratch, (unsigned*)nullptr, (__nv_bfloat16*)nullptr);
-  tb::launch(k_reduce_partials, dim3((N + 31) / 32), dim3(256), 0, s, (const float*)scratch, slices, N, (__nv_bfloat16*)out_bf16,
+  tb::launch(k_reduce_partials, dim3((N + PARTIAL_COLS - 1) / PARTIAL_COLS), dim3(8 * PARTIAL_COLS), 0, s, (const float*)scratch, slices, N, (__nv_bfloat16*)out_bf16,
              (__nv_bfloat16*)nullptr, N);
   return (int)cudaGetLastError();
 }
@@ -889,6 +1029,6 @@ extern "C" int tb_col_sum_noalloc(const void* x_bf16, int M, int N, int ld, void
   dim3 grid((N + 31) / 32, slices);
   tb_note_launch(2);
   k_col_sum<<<grid, 1024, 0, stream>>>((const __nv_bfloat16*)x_bf16, M, N, ld, scratch, nullptr, nullptr);
-  k_reduce_partials<<<(N + 31) / 32, 256, 0, stream>>>(scratch, slices, N, (__nv_bfloat16*)out_bf16, nullptr, N);
+  k_reduce_partials<<<(N + PARTIAL_COLS - 1) / PARTIAL_COLS, 8 * PARTIAL_COLS, 0, stream>>>(scratch, slices, N, (__nv_bfloat16*)out_bf16, nullptr, N);
   return (int)cudaGetLastError();
 }

@@ -335,6 +335,38 @@ def test_layer_norm_matches_fp32(D):
     close(b.grad, bf.grad)
 
 
+# widths on both sides of every vector count; rows: fewer than a block's, ragged, one and several slices per block (148 or 296
+# blocks are resident), one to more rows per warp than the ring holds, forward with and without early gains
+@pytest.mark.parametrize("D", [8, 256, 264, 768, 776, 1024, 1032, 1536, 2040])
+@pytest.mark.parametrize("M", [1, 13, 1187, 2375, 4801, 21001])
+def test_layer_norm_rings_and_slices(M, D):
+    from tandem_b200.ops._lib import lib, stream
+
+    x, dy, add, w, b = rnd(M, D), rnd(M, D), rnd(M, D), rnd(D), rnd(D)
+    xf, dyf, addf, wf, bf = (t.double() for t in (x, dy, add, w, b))
+    mean, std = xf.mean(1, keepdim=True), (xf.var(1, unbiased=False, keepdim=True) + 1e-5).sqrt()
+    xh, g = (xf - mean) / std, dyf * wf
+    dxf = (g - g.mean(1, keepdim=True) - xh * (g * xh).mean(1, keepdim=True)) / std
+    y, dx, dw, db = torch.empty_like(x), torch.empty_like(x), torch.empty_like(w), torch.empty_like(w)
+    stats = torch.empty(2, M, device="cuda")
+    L, s, scratch = lib(), stream(x), torch.empty(lib().tb_layernorm_bwd_blocks(M) * 2 * D, device="cuda")
+    assert L.tb_layernorm_fwd(x.data_ptr(), w.data_ptr(), b.data_ptr(), y.data_ptr(), stats[0].data_ptr(), stats[1].data_ptr(), M, D, 1e-5, s) == 0
+    # one bf16 rounding (2^-9 of the value) and fp32 sums: 1e-5 of the largest term covers 2048 or 21001 of them
+    def near(got, want, terms):
+        assert ((got.double() - want).abs() <= want.abs() * 2**-8 + 1e-5 * terms).all()
+
+    near(y, xh * wf + bf, (xh * wf).abs().max() + bf.abs().max())
+    for second in (None, add, dx):  # without a second gradient, with one, with one that dx is written over
+        if second is dx:
+            dx.copy_(add)
+        assert L.tb_layernorm_bwd_add(dy.data_ptr(), x.data_ptr(), w.data_ptr(), stats[0].data_ptr(), stats[1].data_ptr(),
+                                      None if second is None else second.data_ptr(), dx.data_ptr(), dw.data_ptr(), db.data_ptr(),
+                                      scratch.data_ptr(), M, D, s) == 0
+        near(dx, dxf if second is None else dxf + addf, dxf.abs().max() + addf.abs().max())
+        near(dw, (dyf * xh).sum(0), (dyf * xh).abs().sum(0))
+        near(db, dyf.sum(0), dyf.abs().sum(0))
+
+
 def test_residual_layer_norm_sums_both_gradients():
     from tandem_b200 import ops
 
