@@ -139,7 +139,6 @@ k_attn_fwd_ws(const __grid_constant__ CUtensorMap map, __nv_bfloat16* __restrict
     tmem_alloc(holder, TMEM_COLS);
     tmem_relinquish();
   }
-  tb::pdl_launch_dependents();
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
@@ -164,6 +163,7 @@ k_attn_fwd_ws(const __grid_constant__ CUtensorMap map, __nv_bfloat16* __restrict
         load_tile<HD>(smem + L::RING + s * TILE_BYTES, &map, &kv_full[s], (1 + part) * d + h * HD, b * T + j * TILE);
       }
     }
+    tb::pdl_launch_dependents();  // all loads are under way
   } else if (warp == 1) {
     // ------------------------------------------------------------------ MMA issuer
     constexpr uint32_t idesc_s = instr_desc(128, 128, false, false);
@@ -457,7 +457,6 @@ k_attn_bwd_dq(const __grid_constant__ CUtensorMap map_qkv, const __grid_constant
     tmem_alloc(holder, TMEM_COLS);
     tmem_relinquish();
   }
-  tb::pdl_launch_dependents();
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
@@ -483,6 +482,7 @@ k_attn_bwd_dq(const __grid_constant__ CUtensorMap map_qkv, const __grid_constant
       load(1, j, K_SLOTS + j % V_SLOTS, j / V_SLOTS);
       load(0, j + 1, (j + 1) % K_SLOTS, (j + 1) / K_SLOTS);
     }
+    tb::pdl_launch_dependents();  // all loads are under way
   } else if (warp == 1) {
     constexpr uint32_t idesc_s = instr_desc(128, 128, false, false);
     constexpr uint32_t idesc_dq = instr_desc(128, HD, false, true);
@@ -681,7 +681,6 @@ k_attn_bwd_dkv(const __grid_constant__ CUtensorMap map_qkv, const __grid_constan
     tmem_alloc(holder, TMEM_COLS);
     tmem_relinquish();
   }
-  tb::pdl_launch_dependents();
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
@@ -708,6 +707,7 @@ k_attn_bwd_dkv(const __grid_constant__ CUtensorMap map_qkv, const __grid_constan
         bulk_load_1d(st + 2 * TILE_BYTES + 512, delta + stat0, 512, &st_full[s]);
       }
     }
+    tb::pdl_launch_dependents();  // all loads are under way
   } else if (warp == 1) {
     constexpr uint32_t idesc_s = instr_desc(128, 128, false, false);
     constexpr uint32_t idesc_acc = instr_desc(128, HD, false, true);

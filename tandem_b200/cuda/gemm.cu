@@ -602,7 +602,6 @@ k_gemm(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtens
     tmem_alloc(tmem_holder, TMEM_COLS);
     tmem_relinquish();
   }
-  tb::pdl_launch_dependents();  // the next kernel may set itself up while this one computes
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
@@ -648,6 +647,7 @@ k_gemm(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtens
         if (++s == STAGES) s = 0, phase ^= 1;
       }
     }
+    tb::pdl_launch_dependents();  // all loads are under way: the next kernel may set itself up while the last tile is finished
   } else if (warp == 1) {
     // ------------------------------------------------------------------ MMA issuer
     constexpr uint32_t idesc = instr_desc(128, BN, A_MN, B_MN);
@@ -859,7 +859,6 @@ k_gemm_pair(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ C
     tmem_alloc_pair(tmem_holder, TMEM_COLS);
     tmem_relinquish_pair();
   }
-  tb::pdl_launch_dependents();
   tc_fence_before();
   cluster_sync_all();  // both CTAs' barriers are initialised before either one signals the other's
   tc_fence_after();
@@ -901,6 +900,7 @@ k_gemm_pair(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ C
         if (++s == STAGES) s = 0, phase ^= 1;
       }
     }
+    tb::pdl_launch_dependents();
   } else if (warp == 1) {
     // ------------------------------------------------------------------ MMA issuer (leader only)
     if (rank == 0) {

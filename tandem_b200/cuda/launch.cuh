@@ -4,9 +4,13 @@
 // kernel N+1 is only scheduled once kernel N has drained, so every boundary costs a launch latency plus the new
 // kernel's prologue (barrier initialisation, TMEM allocation, tensor-map fetch) with the GPU idle.  With the
 // programmatic-stream-serialization attribute the next kernel's blocks are scheduled as soon as every block of the
-// current one has called pdl_launch_dependents() (all kernels of this library do so first thing), run their prologue
+// current one has called pdl_launch_dependents(), run their prologue
 // while the current kernel's last blocks finish, and stop at pdl_wait() until the current kernel has completed and its
-// writes are visible.  Rules kept by every kernel launched through tb::launch:
+// writes are visible.  The short memory-bound kernels call it first thing.  The GEMM and attention kernels, which run for tens
+// or hundreds of microseconds, call it when their last loads are under way: blocks that sit beside them from their
+// first microsecond on take the registers and threads that the communication and optimizer kernels of other streams need
+// (one step of the 1.3B model under ZeRO-3: 148.9 ms with the early call, 144.7 with the late one, 144.4 without the attribute;
+// 85.8M at 1024 tokens 2.54, 2.50 and 2.57 ms).  Rules kept by every kernel launched through tb::launch:
 //   * every thread calls pdl_wait() before its first access to global memory (read or write) -- unconditionally, on
 //     every path, so that completion of a kernel implies completion of everything before it in the stream;
 //   * nothing before pdl_wait() touches global memory.
