@@ -44,8 +44,8 @@
 namespace {
 
 constexpr int BK = 64;
-constexpr int SMEM_BUDGET = 192 * 1024;   // operand ring
-constexpr int EPI_STAGING = 8 * 4096 + 8 * 128;  // per epilogue warp: two 32-row x 64-byte blocks on their way out, 32 bias values
+constexpr int SMEM_BUDGET = 224 * 1024;  // operand ring and staging blocks
+constexpr int BLOCK_BYTES = 2048;        // a staging block: 32 rows x 32 columns of bf16 on their way in (aux_in) or out
 
 enum EpilogueFlags {
   EPI_BIAS = 1,        // + bias[col]
@@ -155,47 +155,70 @@ __device__ __forceinline__ bool wait_chunks(const uint32_t* ready, int c_lo, int
 // off by one; compared with a division over every significand, this unit's results were correct for that one too.  Above
 // 1e30 it answers 1e-30, which the caller multiplies by exp(-x^2 / 2) = 0.  __frcp_rn's range checks cost a third of the GELU
 // epilogue.
-__device__ __forceinline__ f32x2 reciprocal2(f32x2 minus_d) {
-  float d0, d1, r0, r1;
-  split2(minus_d, &d0, &d1);
-  d0 = fmaxf(d0, -1e30f);
-  d1 = fmaxf(d1, -1e30f);
-  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r0) : "f"(-d0));
-  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r1) : "f"(-d1));
-  const f32x2 r = pair2(r0, r1);
-  return fma2(r, fma2(pair2(d0, d1), r, pair2(1.f, 1.f)), r);
+template <int N>
+__device__ __forceinline__ void reciprocal2(const f32x2 (&minus_d)[N], f32x2 (&out)[N]) {
+  float d[2 * N], r[2 * N];
+#pragma unroll
+  for (int i = 0; i < N; ++i) split2(minus_d[i], &d[2 * i], &d[2 * i + 1]);
+#pragma unroll
+  for (int i = 0; i < 2 * N; ++i) {
+    d[i] = fmaxf(d[i], -1e30f);
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r[i]) : "f"(-d[i]));
+  }
+#pragma unroll
+  for (int i = 0; i < N; ++i) {
+    const f32x2 r2 = pair2(r[2 * i], r[2 * i + 1]);
+    out[i] = fma2(r2, fma2(pair2(d[2 * i], d[2 * i + 1]), r2, pair2(1.f, 1.f)), r2);
+  }
 }
 
-// Exact (erf) GELU and its derivative from one evaluation, two values at a time:  erf through Abramowitz & Stegun 7.1.26
+// Exact (erf) GELU, in place, and its derivative from one evaluation of 2 * N values:  erf through Abramowitz & Stegun 7.1.26
 // (absolute error below 1.5e-7, far inside a bf16 rounding), whose exp(-z^2) with z = |x| / sqrt(2) is the very
-// exp(-x^2 / 2) that the density needs.  Element-wise work is what bounds the K = 768 GEMM with GELU, so everything but
-// the special-function unit's part is packed.
+// exp(-x^2 / 2) that the density needs.  Everything but the special-function unit's part is packed, and the N pairs take each step
+// together (one, two, four and eight at a time: 56, 47.4, 48.0 and 52 us for 8192 x 3072 x 768, where eight spill).
 //   gelu(x)  = x * Phi(x)          Phi(x) = (1 + erf(x / sqrt 2)) / 2
 //   gelu'(x) = Phi(x) + x * phi(x)  phi(x) = exp(-x^2 / 2) / sqrt(2 pi)
-__device__ __forceinline__ void gelu_and_grad2(f32x2 x, f32x2* g, f32x2* dg) {
+template <int N>
+__device__ __forceinline__ void gelu_and_grad2(f32x2 (&x)[N], f32x2 (&slope)[N]) {
   auto both = [](float v) { return pair2(v, v); };
-  float x0, x1, a0, a1;
-  split2(x, &x0, &x1);
-  const f32x2 z = mul2(pair2(fabsf(x0), fabsf(x1)), both(0.70710678118654752440f));
-  const f32x2 t = reciprocal2(fma2(both(-0.3275911f), z, both(-1.f)));
-  split2(mul2(mul2(both(-0.72134752044448170368f), x), x), &a0, &a1);  // log2 of exp(-x^2 / 2)
-  const f32x2 e = pair2(ex2_approx(a0), ex2_approx(a1));
-  f32x2 p = fma2(t, both(-1.061405429f), both(1.453152027f));  // the polynomial with its sign turned
-  p = fma2(t, p, both(-1.421413741f));
-  p = fma2(t, p, both(0.284496736f));
-  p = fma2(t, p, both(-0.254829592f));
-  float r0, r1;
-  split2(fma2(mul2(t, p), e, both(1.f)), &r0, &r1);  // erf(|x| / sqrt 2)
-  const f32x2 cdf = mul2(both(0.5f), add2(both(1.f), pair2(copysignf(r0, x0), copysignf(r1, x1))));
-  *g = mul2(x, cdf);
-  *dg = fma2(mul2(x, both(0.39894228040143267794f)), e, cdf);
+  f32x2 t[N], e[N], p[N];
+  float v[2 * N], r[2 * N];
+#pragma unroll
+  for (int i = 0; i < N; ++i) {
+    split2(x[i], &v[2 * i], &v[2 * i + 1]);
+    const f32x2 z = mul2(pair2(fabsf(v[2 * i]), fabsf(v[2 * i + 1])), both(0.70710678118654752440f));
+    p[i] = fma2(both(-0.3275911f), z, both(-1.f));
+  }
+  reciprocal2(p, t);
+#pragma unroll
+  for (int i = 0; i < N; ++i) {
+    float a0, a1;
+    split2(mul2(mul2(both(-0.72134752044448170368f), x[i]), x[i]), &a0, &a1);  // log2 of exp(-x^2 / 2)
+    e[i] = pair2(ex2_approx(a0), ex2_approx(a1));
+  }
+#pragma unroll
+  for (int i = 0; i < N; ++i) p[i] = fma2(t[i], both(-1.061405429f), both(1.453152027f));  // the polynomial with its sign turned
+#pragma unroll
+  for (int i = 0; i < N; ++i) p[i] = fma2(t[i], p[i], both(-1.421413741f));
+#pragma unroll
+  for (int i = 0; i < N; ++i) p[i] = fma2(t[i], p[i], both(0.284496736f));
+#pragma unroll
+  for (int i = 0; i < N; ++i) p[i] = fma2(t[i], p[i], both(-0.254829592f));
+#pragma unroll
+  for (int i = 0; i < N; ++i) split2(fma2(mul2(t[i], p[i]), e[i], both(1.f)), &r[2 * i], &r[2 * i + 1]);  // erf(|x| / sqrt 2)
+#pragma unroll
+  for (int i = 0; i < N; ++i) {
+    const f32x2 cdf = mul2(both(0.5f), add2(both(1.f), pair2(copysignf(r[2 * i], v[2 * i]), copysignf(r[2 * i + 1], v[2 * i + 1]))));
+    slope[i] = fma2(mul2(x[i], both(0.39894228040143267794f)), e[i], cdf);
+    x[i] = mul2(x[i], cdf);
+  }
 }
 __device__ __forceinline__ void gelu_and_grad(float x, float* g, float* dg) {
-  f32x2 g2, d2;
-  gelu_and_grad2(pair2(x, x), &g2, &d2);
+  f32x2 g2[1] = {pair2(x, x)}, d2[1];
+  gelu_and_grad2(g2, d2);
   float unused;
-  split2(g2, g, &unused);
-  split2(d2, dg, &unused);
+  split2(g2[0], g, &unused);
+  split2(d2[0], dg, &unused);
 }
 
 // ------------------------------------------------------------------------------------------ kernel
@@ -306,126 +329,188 @@ __device__ __forceinline__ void bulk_store_2d(const CUtensorMap* map, const uint
                : "memory");
 }
 
-// One warp's share of a finished tile: 32 rows x columns [32 * c_begin, 32 * c_end), 32 columns at a time.
+// One epilogue warp's way out of a tile: 32 rows x columns [32 * c_begin, 32 * c_end), 32 columns at a time.
 // TMEM -> registers -> element-wise work -> a swizzled 2 KB block in shared memory -> one bulk tensor store, which clips
-// rows >= M and columns >= N.  Two blocks per warp: the store of one chunk reads its block while the next chunk is computed
-// (GELU needs both at once, for its output and its derivative).  A tile's first chunk waits for every earlier store: the tile
-// before may have ended in the same block (192-column tiles and clipped ones have an odd number of chunks per warp).  The stores never pass through the load/store unit, whose
+// rows >= M and columns >= N.  The stores never pass through the load/store unit, whose
 // global stores (measured on B200) slow the MMA/TMA traffic of the main loop several times more than their size
-// would suggest.  What this loop costs is instruction fetch: with every flag tested in one body unrolled over 64
-// columns it took 1100 cycles per 64 columns to convert and store plain results, 3400 with a bias and 12000 with GELU.
-// So there is one body per kind, the loop over chunks stays rolled, the bias passes through shared memory (one
-// coalesced load per chunk instead of a load per column), and a chunk's aux_in is fetched one chunk ahead.
-template <int KIND, typename Release>
-__device__ __forceinline__ void store_tile(uint32_t taddr, int c_begin, int c_end, int n0, int row0, int lane, uint8_t* stage, float* bias_sm,
-                                           const GemmArgs& g, const __nv_bfloat16* aux, const CUtensorMap* out_map,
-                                           const CUtensorMap* pre_map, Release release) {
-  const int left = g.N - n0;  // columns of the matrix from here on
-  if (32 * c_end > left) c_end = (left + 31) / 32;
-  if (row0 >= g.M || c_begin >= c_end) {
-    release();
-    return;
-  }
-  const bool has_bias = g.flags & EPI_BIAS, keep_pre = KIND == KIND_GELU && g.aux_out != nullptr;
-  constexpr bool HAS_AUX = KIND == KIND_ADD || KIND == KIND_MUL;
-  const bool row_ok = row0 + lane < g.M;
-  const __nv_bfloat16* aux_row = HAS_AUX ? aux + (size_t)(row_ok ? row0 + lane : row0) * g.ldc + n0 : nullptr;
-  uint4 next_aux[4];
-  float next_bias = 0.f;
-  auto fetch = [&](int c) {
-    if (has_bias) next_bias = c * 32 + lane < left ? __bfloat162float(g.bias[n0 + c * 32 + lane]) : 0.f;
-    if (HAS_AUX) {
-#pragma unroll
-      for (int v = 0; v < 4; ++v)
-        if (c * 32 + v * 8 < left) next_aux[v] = *reinterpret_cast<const uint4*>(aux_row + c * 32 + v * 8);
-    }
-  };
-  fetch(c_begin);
-#pragma unroll 1
-  for (int c = c_begin; c < c_end; ++c) {
-    uint32_t raw[32];
-    tmem_ld32(taddr + c * 32, raw);
-    if (has_bias) bias_sm[lane] = next_bias;
-    uint4 cur_aux[4];
-    if (HAS_AUX) {
-#pragma unroll
-      for (int v = 0; v < 4; ++v) cur_aux[v] = next_aux[v];
-    }
-    if (c + 1 < c_end) fetch(c + 1);
-    uint8_t* block = stage + (KIND == KIND_GELU ? 0 : (c & 1) * 2048);
-    if (elect_one()) {  // the store that last used this block has read it
-      if (KIND == KIND_GELU || c == c_begin) asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
-      else asm volatile("cp.async.bulk.wait_group.read 1;" ::: "memory");
-    }
-    __syncwarp();
-    tmem_ld_wait();
-    if (c + 1 == c_end) release();  // the accumulator is in registers
-    f32x2 x[16];
-#pragma unroll
-    for (int j = 0; j < 16; ++j) x[j] = pair2(__uint_as_float(raw[2 * j]), __uint_as_float(raw[2 * j + 1]));
-    if (has_bias) {
-#pragma unroll
-      for (int v = 0; v < 8; ++v) {
-        const float4 b = *reinterpret_cast<const float4*>(bias_sm + 4 * v);
-        x[2 * v] = add2(x[2 * v], pair2(b.x, b.y));
-        x[2 * v + 1] = add2(x[2 * v + 1], pair2(b.z, b.w));
-      }
-    }
-#pragma unroll
-    for (int v = 0; v < 4; ++v) {
-      uint32_t y[4], dy[4];
-      const uint32_t a[4] = {cur_aux[v].x, cur_aux[v].y, cur_aux[v].z, cur_aux[v].w};
-#pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        f32x2 w = x[4 * v + j];
-        if (KIND == KIND_ADD) w = add2(w, from_bf16_pair(a[j]));
-        if (KIND == KIND_MUL) w = mul2(w, from_bf16_pair(a[j]));
-        if (KIND == KIND_GELU) {
-          f32x2 slope;
-          gelu_and_grad2(w, &w, &slope);
-          dy[j] = bf16_pair(slope);
-        }
-        y[j] = bf16_pair(w);
-      }
-      put8(block, lane, v, make_uint4(y[0], y[1], y[2], y[3]));
-      if (keep_pre) put8(block + 2048, lane, v, make_uint4(dy[0], dy[1], dy[2], dy[3]));
-    }
-    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");  // generic-proxy writes, then the async proxy's read
-    __syncwarp();
-    if (elect_one()) {
-      bulk_store_2d(out_map, block, n0 + c * 32, row0);
-      if (keep_pre) bulk_store_2d(pre_map, block + 2048, n0 + c * 32, row0);
-      asm volatile("cp.async.bulk.commit_group;" ::: "memory");
-    }
-  }
-}
+// would suggest.  There is one body per kind, the loop over chunks stays rolled (with every flag tested in one body
+// unrolled over 64 columns it cost 1100 cycles per 64 columns to fetch the instructions of plain results, 12000 of GELU), and the bias passes
+// through shared memory (one coalesced load per chunk instead of a load per column).
+// What bounded it was waiting: for a chunk's aux_in, fetched by the lanes one chunk ahead and row by row, for the first bias, and
+// for the stores to release the blocks.  So begin(), called before the accumulator is complete, fetches the tile's bias and starts TMA
+// loads of aux_in into the blocks that the results will leave from (a lane replaces the values of its own row), and there are
+// BLOCKS blocks per warp, four where the ring keeps enough stages without their memory.  Before and after, us, cold: bias + residual
+// 3072 x 384 x 384 7.5, 5.4; 1024 x 768 x 768 8.1, 6.2; 4096 x 1024 x 1024 17.0, 12.5; 8192 x 768 x 3072 46.6, 39.0; times gelu'
+// 8192 x 3072 x 768 45.2, 39.0; GELU at that size 56, 47.4.  From there on shared memory's bandwidth bounds it beside a main loop of
+// twelve k-blocks, which leaves a quarter of that bandwidth.
+template <int BLOCKS, int CHUNKS>
+struct Epilogue {
+  uint8_t* staging;    // of all eight warps: blocks [8][BLOCKS][BLOCK_BYTES], bias values [8][32], barriers of the loads [8][BLOCKS]
+  int warp;            // 0 .. 7
+  uint32_t aux_phase;  // bit b: parity of the next completion of block b's barrier
+  uint32_t stored;     // chunks stored so far
+  uint32_t bias[(CHUNKS + 1) / 2];  // a lane's column of each chunk: bf16, two to a register
 
-template <typename Release>
-__device__ __forceinline__ void epilogue_tile(uint32_t taddr, int c_begin, int c_end, int n0, int row0, int lane, uint8_t* stage,
-                                              float* bias_sm, const GemmArgs& g, const CUtensorMap* out_map, const CUtensorMap* pre_map,
-                                              Release release) {
-  switch (g.kind) {
-    case KIND_PLAIN:
-      return store_tile<KIND_PLAIN>(taddr, c_begin, c_end, n0, row0, lane, stage, bias_sm, g, nullptr, out_map, pre_map, release);
-    case KIND_ADD:  // gradient accumulation adds the output's old value
-      return store_tile<KIND_ADD>(taddr, c_begin, c_end, n0, row0, lane, stage, bias_sm, g,
-                                  g.flags & EPI_ACCUMULATE ? reinterpret_cast<const __nv_bfloat16*>(g.out) : g.aux_in, out_map, pre_map, release);
-    case KIND_MUL:
-      return store_tile<KIND_MUL>(taddr, c_begin, c_end, n0, row0, lane, stage, bias_sm, g, g.aux_in, out_map, pre_map, release);
-    case KIND_GELU:
-      return store_tile<KIND_GELU>(taddr, c_begin, c_end, n0, row0, lane, stage, bias_sm, g, nullptr, out_map, pre_map, release);
-    default: {
-#pragma unroll 1
-      for (int c = c_begin; c < c_end; ++c) {
-        uint32_t raw[32];
-        tmem_ld32(taddr + c * 32, raw);
-        tmem_ld_wait();
-        epilogue_chunk_generic(raw, row0 + lane, n0 + c * 32, g, g.out, g.flags & EPI_OUT_F32);
-      }
-      release();
+  static constexpr int BIAS_AT = 8 * BLOCKS * BLOCK_BYTES, BARRIERS_AT = BIAS_AT + 8 * 128, BYTES = BARRIERS_AT + 8 * BLOCKS * 8;
+  // Worked out where they are used: the compiler would keep them through fold_tile, which needs every register.
+  __device__ __forceinline__ int here() const {
+    int w = warp;
+    asm volatile("" : "+r"(w));
+    return w;
+  }
+  __device__ __forceinline__ uint8_t* blocks() const { return staging + here() * BLOCKS * BLOCK_BYTES; }
+  __device__ __forceinline__ float* bias_sm() const { return reinterpret_cast<float*>(staging + BIAS_AT + here() * 128); }
+  __device__ __forceinline__ uint64_t* aux_full() const { return reinterpret_cast<uint64_t*>(staging + BARRIERS_AT) + here() * BLOCKS; }
+
+  __device__ __forceinline__ void init() {
+#pragma unroll
+    for (int b = 0; b < BLOCKS; ++b) mbar_init(&aux_full()[b], 1);
+  }
+
+  static __device__ __forceinline__ void wait_stores_read() { asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory"); }
+
+  // The chunks that lie in the matrix: none if the warp's rows do not.
+  static __device__ __forceinline__ int clip(const GemmArgs& g, int c_end, int n0, int row0) {
+    const int in = (g.N - n0 + 31) / 32;
+    return row0 >= g.M ? 0 : c_end < in ? c_end : in;
+  }
+
+  __device__ __forceinline__ void load_aux(const CUtensorMap* map, int block, int x, int y) {
+    mbar_expect_tx(&aux_full()[block], BLOCK_BYTES);
+    tma_load_2d(blocks() + block * BLOCK_BYTES, map, &aux_full()[block], x, y);
+  }
+
+  __device__ __forceinline__ void begin(const GemmArgs& g, const CUtensorMap* aux_map, int c_begin, int c_end, int n0, int row0, int lane) {
+    c_end = clip(g, c_end, n0, row0);
+    if ((g.kind == KIND_ADD || g.kind == KIND_MUL) && c_begin < c_end && elect_one()) {
+      wait_stores_read();
+#pragma unroll
+      for (int i = 0; i < BLOCKS; ++i)
+        if (c_begin + i < c_end) load_aux(aux_map, i, n0 + (c_begin + i) * 32, row0);
+    }
+    if (g.kind != KIND_DIRECT && (g.flags & EPI_BIAS)) {
+      const unsigned short* b = reinterpret_cast<const unsigned short*>(g.bias);
+      auto value = [&](int i) {
+        const int col = n0 + (c_begin + i) * 32 + lane;
+        return i < CHUNKS && c_begin + i < c_end && col < g.N ? (uint32_t)b[col] : 0u;
+      };
+#pragma unroll
+      for (int i = 0; i < CHUNKS; i += 2) bias[i / 2] = value(i) | value(i + 1) << 16;
     }
   }
-}
+
+  // False (and the error word raised) if a load did not arrive.
+  template <int KIND, typename Release>
+  __device__ __forceinline__ bool store(uint32_t taddr, int c_begin, int c_end, int n0, int row0, int lane, const GemmArgs& g,
+                                        const CUtensorMap* aux_map, const CUtensorMap* out_map, const CUtensorMap* pre_map, Release release) {
+    c_end = clip(g, c_end, n0, row0);
+    if (c_begin >= c_end) {
+      release();
+      return true;
+    }
+    const bool has_bias = g.flags & EPI_BIAS, keep_pre = KIND == KIND_GELU && g.aux_out != nullptr;
+    constexpr bool HAS_AUX = KIND == KIND_ADD || KIND == KIND_MUL;
+    constexpr int PER_CHUNK = KIND == KIND_GELU ? 2 : 1, TURNS = BLOCKS / PER_CHUNK;  // blocks per chunk; chunks in flight
+    uint8_t* const blocks = this->blocks();
+    float* const bias_sm = this->bias_sm();
+    bool ok = true;
+#pragma unroll 1
+    for (int c = c_begin; c < c_end; ++c) {
+      uint32_t raw[32];
+      tmem_ld32(taddr + c * 32, raw);
+      if (has_bias) {
+        __syncwarp();  // the previous chunk's values have been read
+        bias_sm[lane] = __uint_as_float(bias[0] << 16);
+        constexpr int LAST = (CHUNKS + 1) / 2 - 1;
+#pragma unroll
+        for (int i = 0; i < LAST; ++i) bias[i] = __funnelshift_r(bias[i], bias[i + 1], 16);
+        bias[LAST] >>= 16;
+      }
+      const int turn = HAS_AUX ? (c - c_begin) % TURNS : (int)(stored % TURNS);
+      uint8_t* block = blocks + turn * PER_CHUNK * BLOCK_BYTES;
+      uint4 aux[4];
+      if (HAS_AUX) {
+        if (!(ok = mbar_wait_all(&aux_full()[turn], (aux_phase >> turn) & 1, g.error))) break;
+        aux_phase ^= 1u << turn;
+#pragma unroll
+        for (int v = 0; v < 4; ++v) aux[v] = *reinterpret_cast<const uint4*>(block + lane * 64 + ((v ^ ((lane >> 1) & 3)) << 4));
+      } else if (elect_one()) {  // the store that last used this block has read it
+        asm volatile("cp.async.bulk.wait_group.read %0;" ::"n"(TURNS - 1) : "memory");
+      }
+      __syncwarp();
+      tmem_ld_wait();
+      if (c + 1 == c_end) release();  // the accumulator is in registers
+      f32x2 x[16];
+#pragma unroll
+      for (int j = 0; j < 16; ++j) x[j] = pair2(__uint_as_float(raw[2 * j]), __uint_as_float(raw[2 * j + 1]));
+      if (has_bias) {
+#pragma unroll
+        for (int v = 0; v < 8; ++v) {
+          const float4 b = *reinterpret_cast<const float4*>(bias_sm + 4 * v);
+          x[2 * v] = add2(x[2 * v], pair2(b.x, b.y));
+          x[2 * v + 1] = add2(x[2 * v + 1], pair2(b.z, b.w));
+        }
+      }
+#pragma unroll
+      for (int v = 0; v < 4; ++v) {
+        uint32_t y[4], dy[4];
+        const uint32_t a[4] = {aux[v].x, aux[v].y, aux[v].z, aux[v].w};
+        if (KIND == KIND_GELU) {
+          f32x2 slope[4];
+          gelu_and_grad2(*reinterpret_cast<f32x2(*)[2]>(x + 4 * v), *reinterpret_cast<f32x2(*)[2]>(slope));
+          gelu_and_grad2(*reinterpret_cast<f32x2(*)[2]>(x + 4 * v + 2), *reinterpret_cast<f32x2(*)[2]>(slope + 2));
+#pragma unroll
+          for (int j = 0; j < 4; ++j) dy[j] = bf16_pair(slope[j]);
+        }
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          f32x2 w = x[4 * v + j];
+          if (KIND == KIND_ADD) w = add2(w, from_bf16_pair(a[j]));
+          if (KIND == KIND_MUL) w = mul2(w, from_bf16_pair(a[j]));
+          y[j] = bf16_pair(w);
+        }
+        put8(block, lane, v, make_uint4(y[0], y[1], y[2], y[3]));
+        if (keep_pre) put8(block + BLOCK_BYTES, lane, v, make_uint4(dy[0], dy[1], dy[2], dy[3]));
+      }
+      asm volatile("fence.proxy.async.shared::cta;" ::: "memory");  // generic-proxy accesses, then the async proxy's
+      __syncwarp();
+      if (elect_one()) {
+        bulk_store_2d(out_map, block, n0 + c * 32, row0);
+        if (keep_pre) bulk_store_2d(pre_map, block + BLOCK_BYTES, n0 + c * 32, row0);
+        asm volatile("cp.async.bulk.commit_group;" ::: "memory");
+        if (HAS_AUX && c + TURNS < c_end) {  // fewer blocks than chunks: the next load into this one
+          wait_stores_read();
+          load_aux(aux_map, turn, n0 + (c + TURNS) * 32, row0);
+        }
+      }
+      ++stored;
+    }
+    if (!ok) release();
+    return ok;
+  }
+
+  template <typename Release>
+  __device__ __forceinline__ bool finish(uint32_t taddr, int c_begin, int c_end, int n0, int row0, int lane, const GemmArgs& g,
+                                         const CUtensorMap* aux_map, const CUtensorMap* out_map, const CUtensorMap* pre_map, Release release) {
+    switch (g.kind) {
+      case KIND_PLAIN: return store<KIND_PLAIN>(taddr, c_begin, c_end, n0, row0, lane, g, aux_map, out_map, pre_map, release);
+      case KIND_ADD: return store<KIND_ADD>(taddr, c_begin, c_end, n0, row0, lane, g, aux_map, out_map, pre_map, release);
+      case KIND_MUL: return store<KIND_MUL>(taddr, c_begin, c_end, n0, row0, lane, g, aux_map, out_map, pre_map, release);
+      case KIND_GELU: return store<KIND_GELU>(taddr, c_begin, c_end, n0, row0, lane, g, aux_map, out_map, pre_map, release);
+      default: {
+#pragma unroll 1
+        for (int c = c_begin; c < c_end; ++c) {
+          uint32_t raw[32];
+          tmem_ld32(taddr + c * 32, raw);
+          tmem_ld_wait();
+          epilogue_chunk_generic(raw, row0 + lane, n0 + c * 32, g, g.out, g.flags & EPI_OUT_F32);
+        }
+        release();
+        return true;
+      }
+    }
+  }
+};
 
 // Split-K (GemmArgs): a producer's warp parks its 32 rows x columns [32 * c_begin, 32 * c_end) of raw accumulator; the
 // consumer's matching warp folds the parked parts, in part order, into its own accumulator in TMEM.
@@ -548,8 +633,10 @@ struct SmemLayout {
   static constexpr int A_BYTES = BM * BK * 2;
   static constexpr int B_BYTES = BN * BK * 2;
   static constexpr int STAGE_BYTES = A_BYTES + B_BYTES;
-  static constexpr int STAGES = SMEM_BUDGET / STAGE_BYTES > 8 ? 8 : SMEM_BUDGET / STAGE_BYTES;
-  static constexpr int TOTAL = STAGES * STAGE_BYTES + EPI_STAGING + 1024 /* alignment slack */ + 256 /* barriers */;
+  static constexpr int BLOCKS = BM == 128 && BN == 192 ? 4 : 2;  // staging blocks per epilogue warp
+  static constexpr int STAGING = Epilogue<BLOCKS, 1>::BYTES;
+  static constexpr int FIT = (SMEM_BUDGET - 8 * BLOCKS * BLOCK_BYTES) / STAGE_BYTES, STAGES = FIT > 8 ? 8 : FIT;
+  static constexpr int TOTAL = STAGES * STAGE_BYTES + STAGING + 1024 /* alignment slack */ + 256 /* barriers */;
   static_assert(TOTAL <= 227 * 1024, "shared memory of one SM");
   static constexpr int THREADS = 64 + 256;  // producer warp, MMA warp, eight epilogue warps
 };
@@ -557,13 +644,13 @@ struct SmemLayout {
 template <int BM, int BN, bool A_MN, bool B_MN, bool GATHER = false>
 __global__ void __launch_bounds__(GATHER ? 448 : 320, 1)
 k_gemm(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b, const __grid_constant__ CUtensorMap map_out,
-       const __grid_constant__ CUtensorMap map_pre, const GemmArgs g, const GatherArgs ga) {
+       const __grid_constant__ CUtensorMap map_pre, const __grid_constant__ CUtensorMap map_aux, const GemmArgs g, const GatherArgs ga) {
   extern __shared__ uint8_t smem_raw[];
   using L = SmemLayout<BM, BN>;
   constexpr int STAGES = L::STAGES;
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   uint8_t* staging = smem + STAGES * L::STAGE_BYTES;
-  uint64_t* full = reinterpret_cast<uint64_t*>(staging + EPI_STAGING);
+  uint64_t* full = reinterpret_cast<uint64_t*>(staging + L::STAGING);
   uint64_t* empty = full + STAGES;
   uint64_t* acc_full = empty + STAGES;
   uint64_t* acc_empty = acc_full + 2;
@@ -591,7 +678,9 @@ k_gemm(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtens
     } else if (lane < STAGES + 2) {
       mbar_init(&acc_full[lane - STAGES], 1);
       mbar_init(&acc_empty[lane - STAGES], BM == 128 ? 8 : 4);  // one arrival per epilogue warp that drains it
-    } else if (lane == STAGES + 2) {
+    } else if (lane < STAGES + 2 + 8) {
+      Epilogue<L::BLOCKS, 1>{staging, lane - STAGES - 2}.init();
+    } else if (lane == STAGES + 2 + 8) {
       prefetch_tensormap(&map_a);
       prefetch_tensormap(&map_b);
       if (g.kind != KIND_DIRECT) prefetch_tensormap(&map_out);
@@ -742,8 +831,9 @@ k_gemm(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtens
     const int half = BM == 128 ? 0 : group;
     uint32_t local_tile = 0;
     bool ok = true;
-    uint8_t* stage = staging + (warp - 2) * 4096;
-    float* bias_sm = reinterpret_cast<float*>(staging + 8 * 4096 + (warp - 2) * 128);
+    constexpr int CHUNKS = BN / 32, MINE = BM == 128 ? CHUNKS / 2 : CHUNKS;  // BM = 128: the two warp groups split the columns
+    Epilogue<L::BLOCKS, MINE> epilogue{staging, warp - 2, 0, 0, {}};
+    const int c_begin = BM == 128 ? group * MINE : 0, c_end = c_begin + MINE;
     if (GATHER && (g.flags & EPI_BIAS) && ga.tail_bytes > 0) {
       // the bias sits right behind the weight in the flat buffer and is fetched with it: wait for its chunks
       const long long lo = (long long)g.N * g.K * 2, hi = lo + ga.tail_bytes;
@@ -760,15 +850,12 @@ k_gemm(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtens
       const int tile_row = half * 128 + quarter * 32 + lane;
       const uint32_t buf = BM == 128 ? (local_tile & 1) : half;
       const uint32_t acc_phase = BM == 128 ? ((local_tile >> 1) & 1) : (local_tile & 1);
+      const int row0 = m0 + half * 128 + quarter * 32;  // first row of this warp's block
+      if (part <= 0) epilogue.begin(g, &map_aux, c_begin, c_end, n0, row0, lane);
       ok = mbar_wait_all(&acc_full[buf], acc_phase, g.error);
       if (!ok) break;
       tc_fence_after();
       const uint32_t taddr = tmem_base + ((uint32_t)(quarter * 32) << 16) + buf * ACC_COLS;
-      // BM = 128: the two warp groups split the columns; BN / 64 chunks of 32 columns each
-      constexpr int CHUNKS = BN / 32;
-      const int c_begin = BM == 128 ? group * (CHUNKS / 2) : 0;
-      const int c_end = BM == 128 ? c_begin + CHUNKS / 2 : CHUNKS;
-      const int row0 = m0 + half * 128 + quarter * 32;  // first row of this warp's block
       auto release = [&]() {
         tc_fence_before();
         __syncwarp();
@@ -784,7 +871,7 @@ k_gemm(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtens
         if (!(ok = wait_flags(my_flags, parts, 8, lane, g.error))) break;
         fold_tile<BM, BM * BN>(taddr, c_begin, c_end, parked, parts, tile_row);
       }
-      epilogue_tile(taddr, c_begin, c_end, n0, row0, lane, stage, bias_sm, g, &map_out, &map_pre, release);
+      ok = epilogue.finish(taddr, c_begin, c_end, n0, row0, lane, g, &map_aux, &map_out, &map_pre, release);
     }
     drain_stores();
   }
@@ -811,13 +898,17 @@ k_gemm(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtens
 //   acc_full[b]   each CTA's own barrier, signalled in both by one multicast tcgen05.commit
 //   acc_empty[b]  leader's barrier: 16 arrivals, one per epilogue warp of either CTA
 // No TMA load uses multicast: each CTA reads its own tiles from global memory.
-template <int BN>
+// WEIGHTS (both operands MN-major: weight gradients) never add or multiply and are cut over k most: their blocks make room for a sixth stage
+// (3072 x 768 x 8192 in two parts: 34.9 us with five stages, 34.2 with six; with an addition 256 x 256 tiles gain more from the blocks).
+template <int BN, bool WEIGHTS>
 struct PairLayout {
   static constexpr int A_BYTES = 128 * BK * 2;       // this CTA's 128 rows of the 256-row A tile
   static constexpr int B_BYTES = (BN / 2) * BK * 2;  // this CTA's half of the B tile
   static constexpr int STAGE_BYTES = A_BYTES + B_BYTES;
-  static constexpr int STAGES = SMEM_BUDGET / STAGE_BYTES > 8 ? 8 : SMEM_BUDGET / STAGE_BYTES;
-  static constexpr int TOTAL = STAGES * STAGE_BYTES + EPI_STAGING + 1024 /* alignment slack */ + 256 /* barriers */;
+  static constexpr int BLOCKS = WEIGHTS ? 2 : 4;  // staging blocks per epilogue warp
+  static constexpr int STAGING = Epilogue<BLOCKS, 1>::BYTES;
+  static constexpr int FIT = (SMEM_BUDGET - 8 * BLOCKS * BLOCK_BYTES) / STAGE_BYTES, STAGES = FIT > 8 ? 8 : FIT;
+  static constexpr int TOTAL = STAGES * STAGE_BYTES + STAGING + 1024 /* alignment slack */ + 256 /* barriers */;
   static_assert(TOTAL <= 227 * 1024, "shared memory of one SM");
   static constexpr int THREADS = 64 + 256;
 };
@@ -825,13 +916,13 @@ struct PairLayout {
 template <int BN, bool A_MN, bool B_MN>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(320, 1)
 k_gemm_pair(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b, const __grid_constant__ CUtensorMap map_out,
-            const __grid_constant__ CUtensorMap map_pre, const GemmArgs g) {
+            const __grid_constant__ CUtensorMap map_pre, const __grid_constant__ CUtensorMap map_aux, const GemmArgs g) {
   extern __shared__ uint8_t smem_raw[];
-  using L = PairLayout<BN>;
+  using L = PairLayout<BN, A_MN && B_MN>;
   constexpr int STAGES = L::STAGES;
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   uint8_t* staging = smem + STAGES * L::STAGE_BYTES;
-  uint64_t* full = reinterpret_cast<uint64_t*>(staging + EPI_STAGING);
+  uint64_t* full = reinterpret_cast<uint64_t*>(staging + L::STAGING);
   uint64_t* empty = full + STAGES;
   uint64_t* acc_full = empty + STAGES;
   uint64_t* acc_empty = acc_full + 2;
@@ -853,6 +944,7 @@ k_gemm_pair(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ C
       mbar_init(&acc_full[b], 1);
       mbar_init(&acc_empty[b], 16);
     }
+    for (int w = 0; w < 8; ++w) Epilogue<L::BLOCKS, 1>{staging, w}.init();
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   if (warp == 1) {
@@ -944,8 +1036,9 @@ k_gemm_pair(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ C
     const int group = (warp - 2) >> 2;
     uint32_t local_tile = 0;
     bool ok = true;
-    uint8_t* stage = staging + (warp - 2) * 4096;
-    float* bias_sm = reinterpret_cast<float*>(staging + 8 * 4096 + (warp - 2) * 128);
+    constexpr int MINE = BN / 64;  // chunks of 32 columns: the two warp groups split them
+    Epilogue<L::BLOCKS, MINE> epilogue{staging, warp - 2, 0, 0, {}};
+    const int c_begin = group * MINE, c_end = c_begin + MINE;
     for (int tile = pair; tile < items.count && ok; tile += num_pairs, ++local_tile) {
       int m_idx, n_idx;
       tile_coords(items.tile(tile), tiles_m, items.whole, g.group_m, &m_idx, &n_idx);
@@ -953,18 +1046,17 @@ k_gemm_pair(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ C
       const int n0 = n_idx * BN;
       const uint32_t buf = local_tile & 1;
       const uint32_t acc_phase = (local_tile >> 1) & 1;
+      const int part = items.part(tile), row0 = m0 + quarter * 32;
+      if (part <= 0) epilogue.begin(g, &map_aux, c_begin, c_end, n0, row0, lane);
       ok = mbar_wait_all(&acc_full[buf], acc_phase, g.error);
       if (!ok) break;
       tc_fence_after();
       const uint32_t taddr = tmem_base + ((uint32_t)(quarter * 32) << 16) + buf * BN;
-      constexpr int CHUNKS = BN / 32;
-      const int c_begin = group * (CHUNKS / 2), c_end = c_begin + CHUNKS / 2;
       auto release = [&]() {
         tc_fence_before();
         __syncwarp();
         if (lane == 0) mbar_arrive_cluster(map_to_cta(smem_u32(&acc_empty[buf]), 0));
       };
-      const int part = items.part(tile);
       if (part >= 0) {  // 16 flags per part: the eight epilogue warps of either CTA
         const int split_tile = items.tile(tile) - items.whole, parts = items.splits - 1, tile_row = (int)rank * 128 + quarter * 32 + lane;
         float* parked = g.partials + (size_t)split_tile * parts * (256 * BN);
@@ -978,7 +1070,7 @@ k_gemm_pair(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ C
         if (!(ok = wait_flags(my_flags, parts, 16, lane, g.error))) break;
         fold_tile<256, 256 * BN>(taddr, c_begin, c_end, parked, parts, tile_row);
       }
-      epilogue_tile(taddr, c_begin, c_end, n0, m0 + quarter * 32, lane, stage, bias_sm, g, &map_out, &map_pre, release);
+      ok = epilogue.finish(taddr, c_begin, c_end, n0, row0, lane, g, &map_aux, &map_out, &map_pre, release);
     }
     drain_stores();
   }
@@ -1039,12 +1131,13 @@ int make_map(CUtensorMap* map, const void* ptr, long long inner, long long outer
   return r == CUDA_SUCCESS ? 0 : -11;
 }
 
-// The epilogue of this call, with the tensor maps of its TMA stores: 32-row x 32-column bf16 blocks of out (and of the kept
-// gelu' factors).
+// The epilogue of this call, with the tensor maps of its TMA stores and loads: 32-row x 32-column bf16 blocks of out, of the kept
+// gelu' factors and of what is added or multiplied (when gradients are accumulated, the output's old values).
 int g_tma_store_enabled = 1;
-int plan_epilogue(CUtensorMap* mo, CUtensorMap* mp, void* out, void* aux_out, int M, int N, int ldc, int flags) {
+int plan_epilogue(CUtensorMap* mo, CUtensorMap* mp, CUtensorMap* mx, void* out, void* aux_out, const void* aux_in, int M, int N, int ldc, int flags) {
   memset(mo, 0, sizeof(*mo));
   memset(mp, 0, sizeof(*mp));
+  memset(mx, 0, sizeof(*mx));
   const int work = flags & (EPI_GELU | EPI_RESIDUAL | EPI_DGELU | EPI_ACCUMULATE);
   const int kind = work == 0 ? KIND_PLAIN : work == EPI_RESIDUAL || work == EPI_ACCUMULATE ? KIND_ADD : work == EPI_DGELU ? KIND_MUL
                    : work == EPI_GELU ? KIND_GELU : KIND_DIRECT;
@@ -1053,6 +1146,9 @@ int plan_epilogue(CUtensorMap* mo, CUtensorMap* mp, void* out, void* aux_out, in
   if (keep_pre && ((uintptr_t)aux_out & 15)) return KIND_DIRECT;
   if (make_map(mo, out, N, M, ldc, 32, 32, CU_TENSOR_MAP_SWIZZLE_64B)) return KIND_DIRECT;
   if (keep_pre && make_map(mp, aux_out, N, M, ldc, 32, 32, CU_TENSOR_MAP_SWIZZLE_64B)) return KIND_DIRECT;
+  if ((kind == KIND_ADD || kind == KIND_MUL) &&
+      make_map(mx, flags & EPI_ACCUMULATE ? out : aux_in, N, M, ldc, 32, 32, CU_TENSOR_MAP_SWIZZLE_64B))
+    return KIND_DIRECT;
   return kind;
 }
 
@@ -1061,7 +1157,7 @@ int* g_error_dev = nullptr;
 int g_sm_count = 0;
 
 template <int BM, int BN, bool A_MN, bool B_MN>
-int launch_gemm(const CUtensorMap& ma, const CUtensorMap& mb, const CUtensorMap& mo, const CUtensorMap& mp, const GemmArgs& g, int max_ctas,
+int launch_gemm(const CUtensorMap& ma, const CUtensorMap& mb, const CUtensorMap& mo, const CUtensorMap& mp, const CUtensorMap& mx, const GemmArgs& g, int max_ctas,
                 cudaStream_t stream) {
   auto kernel = k_gemm<BM, BN, A_MN, B_MN>;
   using L = SmemLayout<BM, BN>;
@@ -1075,15 +1171,15 @@ int launch_gemm(const CUtensorMap& ma, const CUtensorMap& mb, const CUtensorMap&
   const int tiles = g.splits > 1 ? g.whole_tiles + (out_tiles - g.whole_tiles) * g.splits : out_tiles;
   int ctas = tiles < g_sm_count ? tiles : g_sm_count;
   if (max_ctas > 0 && ctas > max_ctas) ctas = max_ctas;
-  return (int)tb::launch(kernel, dim3(ctas), dim3(L::THREADS), L::TOTAL, stream, ma, mb, mo, mp, g, GatherArgs{});
+  return (int)tb::launch(kernel, dim3(ctas), dim3(L::THREADS), L::TOTAL, stream, ma, mb, mo, mp, mx, g, GatherArgs{});
 }
 
 
 template <int BN, bool A_MN, bool B_MN>
-int launch_gemm_pair(const CUtensorMap& ma, const CUtensorMap& mb, const CUtensorMap& mo, const CUtensorMap& mp, const GemmArgs& g,
+int launch_gemm_pair(const CUtensorMap& ma, const CUtensorMap& mb, const CUtensorMap& mo, const CUtensorMap& mp, const CUtensorMap& mx, const GemmArgs& g,
                      int max_ctas, cudaStream_t stream) {
   auto kernel = k_gemm_pair<BN, A_MN, B_MN>;
-  using L = PairLayout<BN>;
+  using L = PairLayout<BN, A_MN && B_MN>;
   static int max_pairs = 0;
   if (max_pairs == 0) {
     cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, L::TOTAL);
@@ -1110,7 +1206,7 @@ int launch_gemm_pair(const CUtensorMap& ma, const CUtensorMap& mb, const CUtenso
   const int tiles = g.splits > 1 ? g.whole_tiles + (out_tiles - g.whole_tiles) * g.splits : out_tiles;
   int pairs = tiles < max_pairs ? tiles : max_pairs;
   if (max_ctas > 1 && pairs > max_ctas / 2) pairs = max_ctas / 2;
-  return (int)tb::launch(kernel, dim3(2 * pairs), dim3(L::THREADS), L::TOTAL, stream, ma, mb, mo, mp, g);
+  return (int)tb::launch(kernel, dim3(2 * pairs), dim3(L::THREADS), L::TOTAL, stream, ma, mb, mo, mp, mx, g);
 }
 
 // Plans.  The CTAs (or CTA pairs) take output tiles round-robin; the last, partial round leaves SMs idle, so the tiles of
@@ -1242,10 +1338,10 @@ GemmPlan plan_gemm(int M, int N, int K, int ctas) {
 __global__ void k_reciprocals(const float* d, float* out, long long pairs) {
   const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= pairs) return;
-  float a, b;
-  split2(reciprocal2(pair2(-d[2 * i], -d[2 * i + 1])), &a, &b);
-  out[2 * i] = a;
-  out[2 * i + 1] = b;
+  const f32x2 minus_d[1] = {pair2(-d[2 * i], -d[2 * i + 1])};
+  f32x2 r[1];
+  reciprocal2(minus_d, r);
+  split2(r[0], &out[2 * i], &out[2 * i + 1]);
 }
 
 // Flag words for split-K, handed out round-robin to launches (a launch that is handed words still in use by an earlier
@@ -1312,28 +1408,28 @@ int tb_gemm_bf16(const void* A, const void* B, void* out, int M, int N, int K, i
   if (!b_mn) rc = make_map(&mb, B, K, N, ldb, 64, paired ? BN / 2 : BN);
   else rc = make_map(&mb, B, N, K, ldb, 64, 64);
   if (rc) return rc;
-  CUtensorMap mo, mp;
-  const int kind = plan_epilogue(&mo, &mp, out, aux_out, M, N, ldc, flags);
+  CUtensorMap mo, mp, mx;
+  const int kind = plan_epilogue(&mo, &mp, &mx, out, aux_out, aux_in, M, N, ldc, flags);
   const int group_m = BM == 128 ? 8 : 4;  // 1024 rows
   GemmArgs g{M, N, K, ldc, flags, out, (const __nv_bfloat16*)bias, (const __nv_bfloat16*)aux_in, (__nv_bfloat16*)aux_out, g_error_dev,
              splits, splits > 1 ? plan.whole_tiles : 0, (float*)workspace, split_flags, group_m, kind};
   tb_note_launch(1);
 #define GO2(BN_) \
   do { \
-    if (!a_mn && !b_mn) return launch_gemm_pair<BN_, false, false>(ma, mb, mo, mp, g, max_ctas, stream); \
-    if (!a_mn && b_mn) return launch_gemm_pair<BN_, false, true>(ma, mb, mo, mp, g, max_ctas, stream); \
-    if (a_mn && b_mn) return launch_gemm_pair<BN_, true, true>(ma, mb, mo, mp, g, max_ctas, stream); \
-    return launch_gemm_pair<BN_, true, false>(ma, mb, mo, mp, g, max_ctas, stream); \
+    if (!a_mn && !b_mn) return launch_gemm_pair<BN_, false, false>(ma, mb, mo, mp, mx, g, max_ctas, stream); \
+    if (!a_mn && b_mn) return launch_gemm_pair<BN_, false, true>(ma, mb, mo, mp, mx, g, max_ctas, stream); \
+    if (a_mn && b_mn) return launch_gemm_pair<BN_, true, true>(ma, mb, mo, mp, mx, g, max_ctas, stream); \
+    return launch_gemm_pair<BN_, true, false>(ma, mb, mo, mp, mx, g, max_ctas, stream); \
   } while (0)
   if (paired && BN == 256) GO2(256);
   if (paired) GO2(128);
 #undef GO2
 #define GO(BM_, BN_) \
   do { \
-    if (!a_mn && !b_mn) return launch_gemm<BM_, BN_, false, false>(ma, mb, mo, mp, g, max_ctas, stream); \
-    if (!a_mn && b_mn) return launch_gemm<BM_, BN_, false, true>(ma, mb, mo, mp, g, max_ctas, stream); \
-    if (a_mn && b_mn) return launch_gemm<BM_, BN_, true, true>(ma, mb, mo, mp, g, max_ctas, stream); \
-    return launch_gemm<BM_, BN_, true, false>(ma, mb, mo, mp, g, max_ctas, stream); \
+    if (!a_mn && !b_mn) return launch_gemm<BM_, BN_, false, false>(ma, mb, mo, mp, mx, g, max_ctas, stream); \
+    if (!a_mn && b_mn) return launch_gemm<BM_, BN_, false, true>(ma, mb, mo, mp, mx, g, max_ctas, stream); \
+    if (a_mn && b_mn) return launch_gemm<BM_, BN_, true, true>(ma, mb, mo, mp, mx, g, max_ctas, stream); \
+    return launch_gemm<BM_, BN_, true, false>(ma, mb, mo, mp, mx, g, max_ctas, stream); \
   } while (0)
   if (BM == 256) GO(256, 256);
   if (BN == 256) GO(128, 256);
@@ -1405,8 +1501,8 @@ int tb_gemm_gathered(const void* A, void* out, int M, int N, int K, int lda, int
   if (rc) return rc;
   rc = make_map(&mb, (const char*)full + w_off, K, N, K, 64, BN);
   if (rc) return rc;
-  CUtensorMap mo, mp;
-  const int kind = plan_epilogue(&mo, &mp, out, aux_out, M, N, ldc, flags);
+  CUtensorMap mo, mp, mx;
+  const int kind = plan_epilogue(&mo, &mp, &mx, out, aux_out, aux_in, M, N, ldc, flags);
   GemmArgs g{M, N, K, ldc, flags, out, (const __nv_bfloat16*)bias, (const __nv_bfloat16*)aux_in, (__nv_bfloat16*)aux_out, g_error_dev,
              1, 0, nullptr, nullptr, 1, kind};
   GatherArgs ga{};
@@ -1434,7 +1530,7 @@ int tb_gemm_gathered(const void* A, void* out, int M, int N, int K, int lda, int
   }
   const int tiles = ((M + BM - 1) / BM) * tiles_n;
   int ctas = tiles < g_sm_count ? tiles : g_sm_count;
-  void* params[] = {(void*)&ma, (void*)&mb, (void*)&mo, (void*)&mp, (void*)&g, (void*)&ga};
+  void* params[] = {(void*)&ma, (void*)&mb, (void*)&mo, (void*)&mp, (void*)&mx, (void*)&g, (void*)&ga};
   tb_note_launch(1);
   return (int)cudaLaunchCooperativeKernel(kernel, dim3(ctas), dim3(448), params, smem, stream);
 }

@@ -142,6 +142,26 @@ def test_gemm_raster_and_edges(M, N, K, tile, force_tile):
     close(slope, gelu_slope(ref))
 
 
+@pytest.mark.parametrize("tile", [0, 1, 2, 3, 4, 5])
+@pytest.mark.parametrize("M,N", [(33, 72), (700, 1090), (3900, 4168)])
+def test_gemm_accumulates_in_place(M, N, tile, force_tile):
+    """The output's old values come in through the blocks that the sums leave from: fewer blocks than chunks, clipped chunks and
+    rows, several tiles per CTA.  Sums of 64 products of -1, 0 and 1 and a small integer are exact in bf16."""
+    from tandem_b200.ops import gemm as G
+    from tandem_b200.ops._lib import empty_padded
+
+    force_tile(tile)
+    x, w = (torch.randint(-1, 2, (rows, 64), device="cuda").bfloat16() for rows in (M, N))
+    out = empty_padded(M, N, torch.bfloat16, "cuda")
+    old = torch.randint(-8, 9, (M, N), device="cuda").bfloat16()
+    out.copy_(old)
+    want = old.float()
+    for _ in range(3):
+        G.gemm(x, w, M, N, 64, 64, 64, False, False, G.ACCUMULATE, out=out)
+        want = want + x.float() @ w.float().t()
+        assert torch.equal(out.float(), want)
+
+
 @pytest.mark.parametrize("exponent", [0, 1, 8, 64, 99])
 def test_gelu_reciprocal_against_a_division(exponent):
     """Every significand at a few powers of two (a power of two scales the whole computation exactly): one Newton step from an
