@@ -343,7 +343,7 @@ __device__ __forceinline__ void bulk_store_2d(const CUtensorMap* map, const uint
 // 3072 x 384 x 384 7.5, 5.4; 1024 x 768 x 768 8.1, 6.2; 4096 x 1024 x 1024 17.0, 12.5; 8192 x 768 x 3072 46.6, 39.0; times gelu'
 // 8192 x 3072 x 768 45.2, 39.0; GELU at that size 56, 47.4.  From there on shared memory's bandwidth bounds it beside a main loop of
 // twelve k-blocks, which leaves a quarter of that bandwidth.
-template <int BLOCKS, int CHUNKS>
+template <int BLOCKS, int CHUNKS, int GELU_PAIRS = 2>
 struct Epilogue {
   uint8_t* staging;    // of all eight warps: blocks [8][BLOCKS][BLOCK_BYTES], bias values [8][32], barriers of the loads [8][BLOCKS]
   int warp;            // 0 .. 7
@@ -457,8 +457,9 @@ struct Epilogue {
         const uint32_t a[4] = {aux[v].x, aux[v].y, aux[v].z, aux[v].w};
         if (KIND == KIND_GELU) {
           f32x2 slope[4];
-          gelu_and_grad2(*reinterpret_cast<f32x2(*)[2]>(x + 4 * v), *reinterpret_cast<f32x2(*)[2]>(slope));
-          gelu_and_grad2(*reinterpret_cast<f32x2(*)[2]>(x + 4 * v + 2), *reinterpret_cast<f32x2(*)[2]>(slope + 2));
+#pragma unroll
+          for (int j = 0; j < 4; j += GELU_PAIRS)
+            gelu_and_grad2(*reinterpret_cast<f32x2(*)[GELU_PAIRS]>(x + 4 * v + j), *reinterpret_cast<f32x2(*)[GELU_PAIRS]>(slope + j));
 #pragma unroll
           for (int j = 0; j < 4; ++j) dy[j] = bf16_pair(slope[j]);
         }
@@ -898,14 +899,15 @@ k_gemm(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtens
 //   acc_full[b]   each CTA's own barrier, signalled in both by one multicast tcgen05.commit
 //   acc_empty[b]  leader's barrier: 16 arrivals, one per epilogue warp of either CTA
 // No TMA load uses multicast: each CTA reads its own tiles from global memory.
-// WEIGHTS (both operands MN-major: weight gradients) never add or multiply and are cut over k most: their blocks make room for a sixth stage
-// (3072 x 768 x 8192 in two parts: 34.9 us with five stages, 34.2 with six; with an addition 256 x 256 tiles gain more from the blocks).
-template <int BN, bool WEIGHTS>
+// DEEP: a ring of six stages (BN = 256) and two staging blocks per warp, instead of five and four.  With few k-blocks per tile the epilogue and
+// its blocks count, with many the ring (us, deep / not: 16384 x 4096 x 1024 times gelu' 128 / 119, with GELU 144 / 136;
+// 16384 x 8192 x 2048 444 / 453 and 475 / 496; 3072 x 768 x 8192 in two parts 34.2 / 34.9).
+template <int BN, bool DEEP>
 struct PairLayout {
   static constexpr int A_BYTES = 128 * BK * 2;       // this CTA's 128 rows of the 256-row A tile
   static constexpr int B_BYTES = (BN / 2) * BK * 2;  // this CTA's half of the B tile
   static constexpr int STAGE_BYTES = A_BYTES + B_BYTES;
-  static constexpr int BLOCKS = WEIGHTS ? 2 : 4;  // staging blocks per epilogue warp
+  static constexpr int BLOCKS = DEEP ? 2 : 4;  // staging blocks per epilogue warp
   static constexpr int STAGING = Epilogue<BLOCKS, 1>::BYTES;
   static constexpr int FIT = (SMEM_BUDGET - 8 * BLOCKS * BLOCK_BYTES) / STAGE_BYTES, STAGES = FIT > 8 ? 8 : FIT;
   static constexpr int TOTAL = STAGES * STAGE_BYTES + STAGING + 1024 /* alignment slack */ + 256 /* barriers */;
@@ -913,12 +915,12 @@ struct PairLayout {
   static constexpr int THREADS = 64 + 256;
 };
 
-template <int BN, bool A_MN, bool B_MN>
+template <int BN, bool A_MN, bool B_MN, bool DEEP>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(320, 1)
 k_gemm_pair(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b, const __grid_constant__ CUtensorMap map_out,
             const __grid_constant__ CUtensorMap map_pre, const __grid_constant__ CUtensorMap map_aux, const GemmArgs g) {
   extern __shared__ uint8_t smem_raw[];
-  using L = PairLayout<BN, A_MN && B_MN>;
+  using L = PairLayout<BN, DEEP>;
   constexpr int STAGES = L::STAGES;
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   uint8_t* staging = smem + STAGES * L::STAGE_BYTES;
@@ -1037,7 +1039,7 @@ k_gemm_pair(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ C
     uint32_t local_tile = 0;
     bool ok = true;
     constexpr int MINE = BN / 64;  // chunks of 32 columns: the two warp groups split them
-    Epilogue<L::BLOCKS, MINE> epilogue{staging, warp - 2, 0, 0, {}};
+    Epilogue<L::BLOCKS, MINE, 4> epilogue{staging, warp - 2, 0, 0, {}};
     const int c_begin = group * MINE, c_end = c_begin + MINE;
     for (int tile = pair; tile < items.count && ok; tile += num_pairs, ++local_tile) {
       int m_idx, n_idx;
@@ -1175,11 +1177,11 @@ int launch_gemm(const CUtensorMap& ma, const CUtensorMap& mb, const CUtensorMap&
 }
 
 
-template <int BN, bool A_MN, bool B_MN>
+template <int BN, bool A_MN, bool B_MN, bool DEEP>
 int launch_gemm_pair(const CUtensorMap& ma, const CUtensorMap& mb, const CUtensorMap& mo, const CUtensorMap& mp, const CUtensorMap& mx, const GemmArgs& g,
                      int max_ctas, cudaStream_t stream) {
-  auto kernel = k_gemm_pair<BN, A_MN, B_MN>;
-  using L = PairLayout<BN, A_MN && B_MN>;
+  auto kernel = k_gemm_pair<BN, A_MN, B_MN, DEEP>;
+  using L = PairLayout<BN, DEEP>;
   static int max_pairs = 0;
   if (max_pairs == 0) {
     cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, L::TOTAL);
@@ -1414,12 +1416,15 @@ int tb_gemm_bf16(const void* A, const void* B, void* out, int M, int N, int K, i
   GemmArgs g{M, N, K, ldc, flags, out, (const __nv_bfloat16*)bias, (const __nv_bfloat16*)aux_in, (__nv_bfloat16*)aux_out, g_error_dev,
              splits, splits > 1 ? plan.whole_tiles : 0, (float*)workspace, split_flags, group_m, kind};
   tb_note_launch(1);
+  const bool deep = K >= 32 * BK;
 #define GO2(BN_) \
   do { \
-    if (!a_mn && !b_mn) return launch_gemm_pair<BN_, false, false>(ma, mb, mo, mp, mx, g, max_ctas, stream); \
-    if (!a_mn && b_mn) return launch_gemm_pair<BN_, false, true>(ma, mb, mo, mp, mx, g, max_ctas, stream); \
-    if (a_mn && b_mn) return launch_gemm_pair<BN_, true, true>(ma, mb, mo, mp, mx, g, max_ctas, stream); \
-    return launch_gemm_pair<BN_, true, false>(ma, mb, mo, mp, mx, g, max_ctas, stream); \
+    if (a_mn && b_mn) return launch_gemm_pair<BN_, true, true, true>(ma, mb, mo, mp, mx, g, max_ctas, stream); \
+    if (a_mn) return launch_gemm_pair<BN_, true, false, true>(ma, mb, mo, mp, mx, g, max_ctas, stream); \
+    if (!b_mn && deep) return launch_gemm_pair<BN_, false, false, true>(ma, mb, mo, mp, mx, g, max_ctas, stream); \
+    if (!b_mn) return launch_gemm_pair<BN_, false, false, false>(ma, mb, mo, mp, mx, g, max_ctas, stream); \
+    if (deep) return launch_gemm_pair<BN_, false, true, true>(ma, mb, mo, mp, mx, g, max_ctas, stream); \
+    return launch_gemm_pair<BN_, false, true, false>(ma, mb, mo, mp, mx, g, max_ctas, stream); \
   } while (0)
   if (paired && BN == 256) GO2(256);
   if (paired) GO2(128);
