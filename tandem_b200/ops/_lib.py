@@ -2,6 +2,7 @@
 
 import ctypes
 import functools
+import warnings
 
 import torch
 
@@ -59,6 +60,32 @@ _raw_stream = getattr(torch._C, "_cuda_getCurrentRawStream", None) or (lambda de
 _functorch_level = getattr(getattr(torch._C, "_functorch", None), "peek_interpreter_stack", None)
 _tracing_state = getattr(torch._C, "_get_tracing_state", None)
 _can_tell = _functorch_level is not None and _tracing_state is not None and hasattr(torch.autograd.forward_ad, "_current_level")
+
+
+@functools.cache
+def native():
+    """The natively issued operators (csrc/ops.cpp) bound to the kernel library; None, with a warning, where they are not built
+    for this torch: the Python functions then do the same more slowly."""
+    try:
+        from .. import _ops
+    except ImportError as e:
+        warnings.warn(f"tandem_b200._ops cannot be imported ({e}); eager operators are issued from Python. Build it with "
+                      "python -m tandem_b200.utils.build", stacklevel=3)
+        return None
+    from ..utils.build import CUDA_LIB
+
+    cuda_lib()  # with its message if the library is missing
+    _ops.bind(CUDA_LIB)
+    return _ops
+
+
+def direct(*tensors):
+    """The native operators if they may answer this call, else None: a functorch transform, a forward-mode level, a tracer or a
+    tensor with a __torch_function__ of its own (or a mode with one) has to meet the Python function."""
+    if (not _can_tell or torch.autograd.forward_ad._current_level >= 0 or _functorch_level() is not None or _tracing_state() is not None
+            or torch.overrides.has_torch_function(tensors)):
+        return None
+    return native()
 
 
 class _Untracked:

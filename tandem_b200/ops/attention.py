@@ -11,7 +11,7 @@ import functools
 
 import torch
 
-from ._lib import check_rc, lib, need_bf16, run, stream
+from ._lib import check_rc, direct, lib, need_bf16, run, stream
 
 
 @functools.cache
@@ -60,6 +60,9 @@ class _CausalAttention(torch.autograd.Function):
 
 def causal_attention(qkv, heads):
     """Returns [B, T, dim]."""
+    native = direct(qkv) if heads > 0 else None
+    if native is not None:
+        return native.causal_attention(qkv, heads)
     return run(_CausalAttention, qkv, heads)
 
 

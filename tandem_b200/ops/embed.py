@@ -4,7 +4,7 @@ fixed order (tandem_b200/cuda/layers.cu)."""
 
 import torch
 
-from ._lib import check_rc, lib, need_bf16, run, stream
+from ._lib import check_rc, direct, lib, need_bf16, run, stream
 
 
 class _Embedding(torch.autograd.Function):
@@ -38,4 +38,7 @@ class _Embedding(torch.autograd.Function):
 
 
 def embedding(idx, tok, pos):
+    native = direct(idx, tok, pos)
+    if native is not None:
+        return native.embedding(idx, tok, pos)
     return run(_Embedding, idx, tok, pos)

@@ -11,7 +11,7 @@ import os
 
 import torch
 
-from ._lib import check_rc, empty_padded, lib, need_bf16, pad8, run, stream, stream_wait
+from ._lib import check_rc, direct, empty_padded, lib, need_bf16, pad8, run, stream, stream_wait
 
 BIAS, GELU, RESIDUAL, DGELU, ACCUMULATE, OUT_F32 = 1, 2, 4, 8, 16, 32
 
@@ -233,10 +233,16 @@ class _MLP(torch.autograd.Function):
 def linear(x, weight, bias=None, gelu=False, residual=None):
     if gelu:
         raise ValueError("use ops.mlp for the GELU MLP (its backward fuses GELU's derivative into a GEMM epilogue)")
+    native = None if GATHERED else direct(x, weight, bias, residual)  # a weight that is gathered by its product: below
+    if native is not None:
+        return native.linear(x, weight, bias, residual, SIDE_BELOW_TOKENS)
     return run(_Linear, x, weight, bias, residual)
 
 
 def mlp(x, w1, b1, w2, b2, residual):
+    native = None if residual is None else direct(x, w1, b1, w2, b2, residual)
+    if native is not None:
+        return native.mlp(x, w1, b1, w2, b2, residual, SIDE_BELOW_TOKENS)
     return run(_MLP, x, w1, b1, w2, b2, residual)
 
 

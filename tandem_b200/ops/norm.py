@@ -4,7 +4,7 @@ partial sums of the weight and bias gradients, reduced in a fixed order."""
 
 import torch
 
-from ._lib import check_rc, lib, need_bf16, run, stream
+from ._lib import check_rc, direct, lib, need_bf16, run, stream
 
 
 class _LayerNorm(torch.autograd.Function):
@@ -36,6 +36,9 @@ class _LayerNorm(torch.autograd.Function):
 
 
 def layer_norm(x, weight, bias, eps=1e-5):
+    native = direct(x, weight, bias)
+    if native is not None:
+        return native.layer_norm(x, weight, bias, eps)
     return run(_LayerNorm, x, weight, bias, eps)
 
 
@@ -77,4 +80,7 @@ class _ResidualLayerNorm(torch.autograd.Function):
 
 def residual_layer_norm(x, weight, bias, eps=1e-5):
     """Returns (x, LayerNorm(x)); use the returned x for the residual connection."""
+    native = direct(x, weight, bias)
+    if native is not None:
+        return native.residual_layer_norm(x, weight, bias, eps)
     return run(_ResidualLayerNorm, x, weight, bias, eps)

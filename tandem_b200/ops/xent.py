@@ -5,7 +5,7 @@ tensor is ever allocated (tandem_b200/cuda/layers.cu)."""
 
 import torch
 
-from ._lib import check_rc, lib, need_bf16, run, stream
+from ._lib import check_rc, direct, lib, need_bf16, run, stream
 
 
 class _CrossEntropy(torch.autograd.Function):
@@ -46,4 +46,7 @@ def _owns_padding(logits, width):
 
 
 def cross_entropy(logits, targets):
+    native = direct(logits, targets)
+    if native is not None:
+        return native.cross_entropy(logits, targets)
     return run(_CrossEntropy, logits, targets)

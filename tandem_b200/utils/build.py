@@ -1,11 +1,13 @@
-"""Ahead-of-time, in-tree builds of the two native libraries.
+"""Ahead-of-time, in-tree builds of the native libraries.
 
   _host<ext>.so       C++17 host runtime (shared memory, channels, progress
                       thread, CPU collectives), a pybind11 module.
   libtb200_cuda.so    every sm_100a kernel plus the symmetric-memory helpers,
                       exported as plain C symbols and called through ctypes.
+  _ops<ext>.so        the operators' autograd functions, issued natively
+                      (needs a torch with CUDA; it calls the kernels above).
 
-Both land beside the package so a source checkout with its built libraries can
+All land beside the package so a source checkout with its built libraries can
 be copied to a GPU machine as is.  The reference instead JIT-builds into
 ~/.cache/torch_extensions on first use and passes no -arch flag
 (tandem/engine.py:22-37); here the only target is sm_100a.
@@ -21,6 +23,8 @@ PKG = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
 CSRC = os.path.join(PKG, "csrc")
 CUDA = os.path.join(PKG, "cuda")
 HOST_SOURCES = ["shm.cpp", "channel.cpp", "engine.cpp", "bind.cpp"]
+OPS_SOURCE = os.path.join(CSRC, "ops.cpp")
+OPS_LIB = os.path.join(PKG, "_ops" + sysconfig.get_config_var("EXT_SUFFIX"))
 HOST_LIB = os.path.join(PKG, "_host" + sysconfig.get_config_var("EXT_SUFFIX"))
 CUDA_LIB = os.path.join(PKG, "libtb200_cuda.so")
 NVCC_ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
@@ -52,7 +56,7 @@ def build_host(force=False, verbose=False):
     import pybind11
 
     srcs = [os.path.join(CSRC, s) for s in HOST_SOURCES]
-    deps = _sources(CSRC, (".cpp", ".h"))
+    deps = [s for s in _sources(CSRC, (".cpp", ".h")) if s != OPS_SOURCE]
     if not force and not _newer(HOST_LIB, deps):
         return HOST_LIB
     tmp = HOST_LIB + f".{os.getpid()}.tmp"
@@ -107,8 +111,32 @@ def build_cuda(force=False, verbose=False):
     return CUDA_LIB
 
 
+def build_ops(force=False, verbose=False):
+    """Compiles the native autograd functions against the installed torch, or returns None where that is a CPU build."""
+    import torch
+    from torch.utils.cpp_extension import include_paths
+
+    nvcc = nvcc_path()
+    if torch.version.cuda is None or nvcc is None:
+        return None
+    if not force and not _newer(OPS_LIB, [OPS_SOURCE]):
+        return OPS_LIB
+    cuda_include = os.path.join(os.path.dirname(os.path.dirname(os.path.realpath(nvcc))), "include")
+    includes = [*include_paths(), cuda_include, sysconfig.get_paths()["include"]]
+    libs = os.path.join(os.path.dirname(torch.__file__), "lib")
+    tmp = OPS_LIB + f".{os.getpid()}.tmp"
+    cmd = ["g++", "-O2", "-std=c++17", "-fPIC", "-shared", "-fvisibility=hidden", "-DTORCH_EXTENSION_NAME=_ops",
+           f"-D_GLIBCXX_USE_CXX11_ABI={int(torch.compiled_with_cxx11_abi())}", *(f"-isystem{i}" for i in includes), OPS_SOURCE, "-o", tmp,
+           f"-L{libs}", "-lc10", "-lc10_cuda", "-ltorch_cpu", "-ltorch", "-ltorch_python", "-ldl"]
+    _run(cmd, verbose)
+    os.replace(tmp, OPS_LIB)
+    return OPS_LIB
+
+
 def build_all(force=False, verbose=False):
-    return build_host(force, verbose), build_cuda(force, verbose)
+    host, cuda = build_host(force, verbose), build_cuda(force, verbose)
+    build_ops(force, verbose)
+    return host, cuda
 
 
 if __name__ == "__main__":

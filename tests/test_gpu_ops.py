@@ -787,6 +787,123 @@ def test_operators_without_gradients_equal_those_with():
         ops.linear(torch.autograd.forward_ad.make_dual(x, torch.ones_like(x)), w, b)
 
 
+def _operator_forms():
+    """Every operator with the forms of input that it accepts: leading dimensions, strides, offsets, odd widths, missing and
+    frozen operands, few and many rows (below and above the second stream's limit).  Name -> (function, inputs, which need gradients)."""
+    from tandem_b200 import ops
+
+    def leaf(*shape):
+        return rnd(*shape, scale=0.5)
+
+    forms = {}
+    for rows, inner, outer in [((1,), 64, 64), ((33,), 72, 65), ((3, 40), 100, 96), ((2, 3, 7), 8, 1003), ((4200,), 136, 128), ((), 64, 24), ((2, 130), 65, 40)]:
+        x, w, b = leaf(*rows, inner), leaf(outer, pad8(inner))[:, :inner], leaf(outer)
+        forms[f"linear {rows} {inner} {outer}"] = (ops.linear, [x, w, b], [1, 1, 1])
+        forms[f"linear {rows} {inner} {outer} no bias"] = (ops.linear, [x, w, None], [1, 1, 0])
+        forms[f"linear {rows} {inner} {outer} frozen"] = (ops.linear, [x, w, b], [1, 0, 0])
+        forms[f"linear {rows} {inner} {outer} first layer"] = (ops.linear, [x, w, b], [0, 1, 1])
+        if outer % 8 == 0:
+            forms[f"linear {rows} {inner} {outer} residual"] = (lambda x, w, b, r: ops.linear(x, w, b, residual=r), [x, w, b, leaf(*rows, outer)], [1, 1, 1, 1])
+    wide = leaf(40, 3 * 64)
+    for name, x in {"columns": wide[:, 64:128], "odd columns": wide[:, 3:67], "transposed": leaf(64, 40).t(), "every other row": leaf(80, 64)[::2],
+                    "swapped": leaf(5, 6, 64).transpose(0, 1), "expanded": leaf(1, 64).expand(40, 64), "offset": leaf(40 * 64 + 1)[1:].view(40, 64)}.items():
+        forms[f"linear of {name}"] = (ops.linear, [x, leaf(96, 64), leaf(96)], [1, 1, 1])
+        if name not in ("odd columns", "offset"):  # the LayerNorm kernels read 16-byte vectors of a contiguous input where it lies
+            forms[f"layer_norm of {name}"] = (ops.layer_norm, [x, leaf(64), leaf(64)], [1, 1, 1])
+    for rows in [(1,), (2, 77), (4100,)]:
+        x, r = leaf(*rows, 72), leaf(*rows, 40)
+        forms[f"mlp {rows}"] = (ops.mlp, [x, leaf(96, 72), leaf(96), leaf(40, 96), leaf(40), r], [1] * 6)
+        forms[f"mlp {rows} frozen"] = (ops.mlp, [x, leaf(96, 72), None, leaf(40, 96), None, r], [1, 0, 0, 1, 0, 0])
+        forms[f"residual_layer_norm {rows}"] = (ops.residual_layer_norm, [x, leaf(72), leaf(72)], [1, 1, 1])
+        forms[f"normalized alone {rows}"] = (lambda *a: ops.residual_layer_norm(*a)[1], [x, leaf(72), leaf(72)], [1, 1, 1])
+    for heads, hd in [(1, 64), (3, 64), (2, 128)]:
+        forms[f"attention {heads} {hd}"] = (lambda q, h=heads: ops.causal_attention(q, h), [leaf(2, 256, 3 * heads * hd)], [1])
+    forms["attention of a slice"] = (lambda q: ops.causal_attention(q, 2), [leaf(2, 128, 2 * 384)[:, :, :384]], [1])
+    idx = torch.randperm(60, device="cuda")[:2 * 20].view(2, 20)
+    forms["embedding"] = (lambda t, p: ops.embedding(idx, t, p), [leaf(60, 40), leaf(32, 40)], [1, 1])
+    forms["embedding of transposed ids"] = (lambda t, p: ops.embedding(idx.t(), t, p), [leaf(60, 40), leaf(32, 40)], [1, 1])
+    for V, ld in [(65, 72), (65, 65), (1003, 1008), (64, 200)]:
+        forms[f"cross_entropy {V} {ld}"] = (lambda z: ops.cross_entropy(z * 1.0 if z.stride(0) == z.shape[1] else z, torch.arange(30, device="cuda") % V),
+                                            [leaf(30, ld)[:, :V]], [1])
+    return forms
+
+
+def pad8(n):
+    return (n + 7) // 8 * 8
+
+
+def test_native_operators_equal_the_python_ones(monkeypatch):
+    """Outputs, gradients, saved tensors and second uses, bit for bit, over all forms; and what is refused is refused alike."""
+    from tandem_b200 import ops
+    from tandem_b200.ops import _lib
+
+    assert _lib.native() is not None
+    torch.manual_seed(0)
+    forms = _operator_forms()
+
+    def outcome(function, inputs, needs):
+        inputs = [t if t is None or not n else t.detach().requires_grad_() for t, n in zip(inputs, needs)]
+        saved = []
+        with torch.autograd.graph.saved_tensors_hooks(lambda t: saved.append((t.dtype, t.shape)) or t, lambda t: t):
+            out = function(*inputs)
+        outs = out if isinstance(out, tuple) else (out,)
+        torch.manual_seed(1)
+        grads = [torch.randn_like(o) for o in outs]
+        kept = [o.detach().clone() for o in outs]
+        wanted = [t for t, n in zip(inputs, needs) if n]
+        got = torch.autograd.grad(outs, wanted, grads)
+        with pytest.raises(RuntimeError, match="second time"):
+            torch.autograd.grad(outs, wanted, grads)
+        return saved, [(o.shape, o.stride(), o.is_contiguous()) for o in outs], kept + [g.clone() for g in got]
+
+    for name, (function, inputs, needs) in forms.items():
+        fresh = [None if t is None else t.detach().clone(memory_format=torch.preserve_format) if "cross" in name else t for t in inputs]
+        native = outcome(function, fresh, needs)
+        with monkeypatch.context() as m:
+            m.setattr(_lib, "native", lambda: None)
+            python = outcome(function, inputs, needs)
+        assert native[:2] == python[:2], name
+        for a, b in zip(native[2], python[2]):
+            assert a.shape == b.shape and a.stride() == b.stride() and torch.equal(a, b), name
+
+    x, w, b = rnd(40, 64), rnd(96, 64), rnd(96)
+    refused = [lambda: ops.linear(x.float(), w, b), lambda: ops.linear(x, w.cpu(), b), lambda: ops.linear(x, rnd(65, 64), None, residual=rnd(40, 65)),
+               lambda: ops.linear(x, w, b, residual=rnd(96, 40).t()), lambda: ops.mlp(x, w, b, rnd(40, 96), b, None),
+               lambda: ops.mlp(x, rnd(65, 64), None, rnd(40, 65), None, rnd(40, 40)), lambda: ops.layer_norm(rnd(4, 12), rnd(12), rnd(12)),
+               lambda: ops.causal_attention(rnd(1, 100, 192), 1), lambda: ops.causal_attention(rnd(1, 128, 96), 1), lambda: ops.causal_attention(rnd(128, 192), 1),
+               lambda: ops.causal_attention(rnd(1, 128, 192), 0), lambda: ops.embedding(torch.zeros(3, dtype=torch.long, device="cuda"), w, w),
+               lambda: ops.cross_entropy(rnd(2, 3, 8), torch.zeros(2, dtype=torch.long, device="cuda"))]
+
+    def refusal(call):
+        try:
+            call()
+        except Exception as e:
+            return type(e)
+        return None
+
+    native = [refusal(call) for call in refused]
+    monkeypatch.setattr(_lib, "native", lambda: None)
+    assert native == [refusal(call) for call in refused] and None not in native
+
+
+@pytest.mark.parametrize("python", [False, True])
+def test_operators_notice_a_changed_input(python, monkeypatch):
+    """What backward reads again must not have changed in between; a gradient has no gradient of its own."""
+    from tandem_b200 import ops
+    from tandem_b200.ops import _lib
+
+    if python:
+        monkeypatch.setattr(_lib, "native", lambda: None)
+    x, w = rnd(40, 64), rnd(96, 64).requires_grad_()
+    y = ops.linear(x, w)
+    x.add_(1)
+    with pytest.raises(RuntimeError, match="modified by an inplace operation"):
+        y.sum().backward()
+    x.requires_grad_()
+    (g,) = torch.autograd.grad(ops.linear(x, w).float().square().sum(), x, create_graph=True)
+    assert not g.requires_grad  # as of a constant
+
+
 def test_stream_wait_from_two_threads():
     """Each thread orders its own pair of streams through one native call, many times over."""
     import threading
