@@ -59,7 +59,8 @@ __device__ __forceinline__ void mma_kmajor(uint32_t d_tmem, const uint8_t* a, co
 // ------------------------------------------------------------------------------------------ work lists
 // Head dim 64 leaves shared memory and TMEM for the next tile's operands and accumulators, so its kernels run one CTA per place on the
 // GPU, which takes item after item: the loads of the next item, its barriers' turns and its first scores are under way while the last one is
-// finished.  (A CTA per item spent 2 to 3.5 us of its 5 to 6 outside the loop over tiles.)  Head dim 128 fills an SM with one item; its
+// finished.  (A CTA per item spent 2 to 3.5 us of its 5 to 6 outside the loop over tiles; dQ and dK/dV, us: 16 x 512, 12 heads
+// 40.4 -> 29.5 and 47.1 -> 38.9; 32 x 1024, 16 heads 251 -> 176 and 296 -> 243.)  Head dim 128 fills an SM with one item; its
 // grid has a CTA for each.
 // An item is a tile of a head.  Items come in groups of `heads` heads whose tiles together are worth several rounds: the longest tiles of
 // all heads of a group first, so that the rounds end together, and few enough heads that what they share stays in L2.  CTA c takes
@@ -90,7 +91,7 @@ struct WorkList {
     w.h = w.head - w.b * H;
     return w;
   }
-  __device__ __forceinline__ WorkList(int T, int B, int H_, int heads_per_group) : tiles(T / TILE), all(B * H_), per_group(heads_per_group), H(H_), round(0) {
+  __device__ __forceinline__ WorkList(int tiles_, int heads, int H_, int heads_per_group) : tiles(tiles_), all(heads), per_group(heads_per_group), H(H_), round(0) {
     now = find(blockIdx.x);
   }
   __device__ __forceinline__ void prefetch() {
@@ -122,25 +123,27 @@ struct WorkList {
 //   pipe, and the next one is only issued after this row's thread has arrived on p_full.
 // Head dim 64.  TMEM: S [0,128)  O [128,192)  P [192,256).  With a P of its own, S(j+1) is issued as soon as the softmax threads
 //   have S(j) in registers, so that they never wait for scores; P(j) and the rescale of O wait for P.V of step j-1 (pv_done),
-//   which is long over by the time the maxima are known.  256 columns and 100 KB let two CTAs share an SM, and
-//   one's start and end overlap the other's work: sequences of 512 have one to four key tiles per query tile.
-template <int HD>
+//   which is long over by the time the maxima are known.  256 columns and 113 KB let two CTAs share an SM.
+//   Items follow one another in a CTA (WorkList): Q of the next one is on its way and its first scores are issued ahead of this one's
+//   last P.V (us: 16 x 512, 12 heads 27.6 -> 23.5; 4 x 1024, 16 heads 28.5 -> 21.5; 1 x 8192, 16 heads 240 -> 195).
+template <int HD, bool MANY>
 struct Fwd2Smem {
   static constexpr int TILE_BYTES = (HD / 64) * STRIP;
   static constexpr int NT = HD == 64 ? 1 : 2;                        // query tiles
   static constexpr int THREADS = 64 + 128 * NT;
+  static constexpr int BUFS = MANY ? 2 : 1;                         // sets of Q tiles
   static constexpr int Q = 0;
-  static constexpr int RING = Q + NT * TILE_BYTES;
+  static constexpr int RING = Q + BUFS * NT * TILE_BYTES;
   static constexpr int SLOTS = 5;                                   // K and V tiles in flight
   static constexpr int BARS = RING + SLOTS * TILE_BYTES;
   static constexpr int TOTAL = BARS + 256;
   static_assert(TOTAL <= (HD == 64 ? 113 : 227) * 1024, "shared memory of one SM");
 };
 
-template <int HD>
-__global__ void __launch_bounds__(Fwd2Smem<HD>::THREADS, HD == 64 ? 2 : 1)
+template <int HD, bool MANY>
+__global__ void __launch_bounds__(Fwd2Smem<HD, MANY>::THREADS, HD == 64 ? 2 : 1)
 k_attn_fwd_ws(const __grid_constant__ CUtensorMap map, __nv_bfloat16* __restrict__ out, float* __restrict__ lse, int B, int T, int H,
-              int d, float scale_log2e, int* error) {
+              int d, float scale_log2e, int group_heads, int* error) {
   extern __shared__ __align__(1024) uint8_t fwd2_smem[];
   uint8_t* smem = fwd2_smem;
   if (smem_u32(smem) & 1023) {  // the swizzled tiles need 1024-byte alignment; nothing is allocated yet
@@ -150,22 +153,21 @@ k_attn_fwd_ws(const __grid_constant__ CUtensorMap map, __nv_bfloat16* __restrict
     }
     return;
   }
-  using L = Fwd2Smem<HD>;
-  constexpr int TILE_BYTES = L::TILE_BYTES, SLOTS = L::SLOTS;
+  using L = Fwd2Smem<HD, MANY>;
+  static_assert(!MANY || HD == 64, "two query tiles of head dim 128 leave no room for the next item");
+  constexpr int TILE_BYTES = L::TILE_BYTES, SLOTS = L::SLOTS, BUFS = L::BUFS;
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem + L::BARS);
   uint64_t *q_full = bars, *s_full = bars + 2, *p_full = bars + 4, *o_full = bars + 6, *kv_full = bars + 8, *kv_empty = bars + 8 + SLOTS;
-  uint64_t *s_read = bars + 8 + 2 * SLOTS, *pv_done = s_read + 2;
-  uint32_t* holder = reinterpret_cast<uint32_t*>(pv_done + 2);
+  uint64_t *s_read = bars + 8 + 2 * SLOTS, *pv_done = s_read + 2, *q_empty = pv_done + 2, *o_empty = q_empty + 2;
+  uint32_t* holder = reinterpret_cast<uint32_t*>(o_empty + 1);
   constexpr bool OWN_P = HD == 64;
   const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;  // warp: known to be uniform
   constexpr int NT = L::NT;
+  // An item: NT query tiles of one head (NT = 2: always a CTA's only one).  Query tile i visits n_i key tiles.
   const int n_qt = T / TILE, n_groups = (n_qt + NT - 1) / NT;
-  // consecutive CTAs share one head's K and V (they stay in L2), longest first within the head
-  const int group = n_groups - 1 - (int)blockIdx.x % n_groups;
-  const int rest = (int)blockIdx.x / n_groups;
-  const int h = rest % H, b = rest / H;
-  const int qt0 = NT * group, qt1 = qt0 + 1;
-  const int n0 = qt0 + 1, n1 = NT == 2 && qt1 < n_qt ? qt1 + 1 : 0;  // key tiles each query tile visits
+  WorkList<MANY> work(n_groups, B * H, H, group_heads);
+  const int qt0 = NT * (n_groups - 1 - work.now.rank), qt1 = qt0 + 1;
+  const int n0 = qt0 + 1, n1 = NT == 2 && qt1 < n_qt ? qt1 + 1 : 0;
   const int n_steps = n1 > n0 ? n1 : n0;
   constexpr uint32_t TMEM_COLS = HD == 64 ? 256 : 512;
   constexpr uint32_t C_O = HD == 64 ? 128 : 256, C_P = 192;  // S_i at 128 * i; C_P: with OWN_P
@@ -178,7 +180,9 @@ k_attn_fwd_ws(const __grid_constant__ CUtensorMap map, __nv_bfloat16* __restrict
       mbar_init(&o_full[i], 1);
       mbar_init(&s_read[i], 4);
       mbar_init(&pv_done[i], 1);
+      mbar_init(&q_empty[i], 1);
     }
+    mbar_init(o_empty, 4);
     for (int s = 0; s < SLOTS; ++s) {
       mbar_init(&kv_full[s], 1);
       mbar_init(&kv_empty[s], 1);
@@ -196,24 +200,34 @@ k_attn_fwd_ws(const __grid_constant__ CUtensorMap map, __nv_bfloat16* __restrict
   const uint32_t tmem = *holder;
   tb::pdl_wait();  // set-up is done; everything below reads what earlier kernels wrote
 
+  // Item number `it` of this CTA uses Q buffer it % BUFS for the (it / BUFS)-th time; steps (key tiles) are counted through all items.
   if (warp == 0) {
     // ------------------------------------------------------------------ TMA producer
-    if (elect_one()) {
-      mbar_expect_tx(&q_full[0], TILE_BYTES);
-      load_tile<HD>(smem + L::Q, &map, &q_full[0], h * HD, b * T + qt0 * TILE);
-      if (n1) {
-        mbar_expect_tx(&q_full[1], TILE_BYTES);
-        load_tile<HD>(smem + L::Q + TILE_BYTES, &map, &q_full[1], h * HD, b * T + qt1 * TILE);
-      }
-    }
-    for (int ld = 0; ld < 2 * n_steps; ++ld) {  // load 2j: K_j, load 2j+1: V_j
-      const int s = ld % SLOTS, j = ld >> 1, part = ld & 1;
-      if (!mbar_wait_all(&kv_empty[s], ((ld / SLOTS) & 1) ^ 1, error)) break;
+    bool ok = true;
+    int it = 0, ld = 0;
+    do {
+      const int b = work.now.b, h = work.now.h, q0 = NT * (n_groups - 1 - work.now.rank), buf = it % BUFS;
+      const int steps = MANY ? q0 + 1 : n_steps;
+      if (MANY && !(ok = mbar_wait_all(&q_empty[buf], ((it / BUFS) & 1) ^ 1, error))) break;
       if (elect_one()) {
-        mbar_expect_tx(&kv_full[s], TILE_BYTES);
-        load_tile<HD>(smem + L::RING + s * TILE_BYTES, &map, &kv_full[s], (1 + part) * d + h * HD, b * T + j * TILE);
+        mbar_expect_tx(&q_full[buf], TILE_BYTES);
+        load_tile<HD>(smem + L::Q + buf * TILE_BYTES, &map, &q_full[buf], h * HD, b * T + q0 * TILE);
+        if (n1) {
+          mbar_expect_tx(&q_full[1], TILE_BYTES);
+          load_tile<HD>(smem + L::Q + TILE_BYTES, &map, &q_full[1], h * HD, b * T + qt1 * TILE);
+        }
       }
-    }
+      work.prefetch();
+      for (int end = ld + 2 * steps, first = ld; ld < end; ++ld) {  // load 2j: K_j, load 2j+1: V_j
+        const int s = ld % SLOTS, j = (ld - first) >> 1, part = ld & 1;
+        if (!(ok = mbar_wait_all(&kv_empty[s], ((ld / SLOTS) & 1) ^ 1, error))) break;
+        if (elect_one()) {
+          mbar_expect_tx(&kv_full[s], TILE_BYTES);
+          load_tile<HD>(smem + L::RING + s * TILE_BYTES, &map, &kv_full[s], (1 + part) * d + h * HD, b * T + j * TILE);
+        }
+      }
+      ++it;
+    } while (ok && work.advance());
     tb::pdl_launch_dependents();  // all loads are under way
   } else if (warp == 1) {
     // ------------------------------------------------------------------ MMA issuer
@@ -221,52 +235,75 @@ k_attn_fwd_ws(const __grid_constant__ CUtensorMap map, __nv_bfloat16* __restrict
     constexpr uint32_t idesc_o = instr_desc(128, HD, false, true);
     auto slot_of = [&](int ld) { return smem + L::RING + (ld % SLOTS) * TILE_BYTES; };
     auto wait_slot = [&](int ld) { return mbar_wait_all(&kv_full[ld % SLOTS], (ld / SLOTS) & 1, error); };
-    auto issue_s = [&](int i, int j) {  // S_i = Q_i . K_j^T
-      mma_kmajor<HD>(tmem + i * 128, smem + L::Q + i * TILE_BYTES, slot_of(2 * j), idesc_s, false);
+    auto issue_s = [&](int i, int j, int q) {  // S_i = Q_i . K_j^T, Q_i in place q
+      mma_kmajor<HD>(tmem + i * 128, smem + L::Q + q * TILE_BYTES, slot_of(2 * j), idesc_s, false);
       mma_commit(&s_full[i]);
     };
-    auto issue_pv = [&](int i, int j) {  // O_i (+)= P_i . V_j: eight steps of 16 keys; V is MN-major (head dim contiguous)
+    auto issue_pv = [&](int i, int j, bool first) {  // O_i (+)= P_i . V_j: eight steps of 16 keys; V is MN-major (head dim contiguous)
       const uint32_t tO = tmem + C_O + i * HD;
       const uint64_t v_desc = smem_desc(smem_u32(slot_of(2 * j + 1)), STRIP, 1024);
 #pragma unroll
       for (int kk = 0; kk < 8; ++kk)
-        mma_bf16_ts(tO, (OWN_P ? tmem + C_P : tmem + i * 128) + kk * 8, v_desc + kk * (2048 >> 4), idesc_o, (j > 0 || kk > 0) ? 1u : 0u);  // 16 keys = 8 TMEM columns of P
+        mma_bf16_ts(tO, (OWN_P ? tmem + C_P : tmem + i * 128) + kk * 8, v_desc + kk * (2048 >> 4), idesc_o, (!first || kk > 0) ? 1u : 0u);  // 16 keys = 8 TMEM columns of P
     };
     bool ok = mbar_wait_all(&q_full[0], 0, error) && (!n1 || mbar_wait_all(&q_full[1], 0, error)) && wait_slot(0);
     if (ok) {
       tc_fence_after();
       if (elect_one()) {
-        issue_s(0, 0);
-        if (n1) issue_s(1, 0);
+        issue_s(0, 0, 0);
+        if (n1) issue_s(1, 0, 1);
         mma_commit(&kv_empty[0]);  // K_0 is free once these have read it
+        if (MANY && n0 == 1) mma_commit(&q_empty[0]);
       }
     }
     if constexpr (OWN_P) {
-      for (int j = 0; j < n_steps && ok; ++j) {
-        if (j + 1 < n_steps) {
-          if (!(ok = wait_slot(2 * j + 2))) break;                      // K_{j+1}
-          for (int i = 0; i < NT && ok; ++i) {
-            if (j + 1 >= (i == 0 ? n0 : n1)) continue;
-            if (!(ok = mbar_wait_all(&s_read[i], j & 1, error))) break;  // S_i(j) is in registers
+      int it = 0, step = 0, n = n0;
+      while (ok) {
+        const int buf = it % BUFS;
+        work.prefetch();
+        for (int j = 0; j < (MANY ? n - 1 : n); ++j, ++step) {
+          if (MANY || j + 1 < n) {
+            if (!(ok = wait_slot(2 * step + 2) && mbar_wait_all(&s_read[0], step & 1, error))) break;  // K_{j+1}; S(j) is in registers
             tc_fence_after();
-            if (elect_one()) issue_s(i, j + 1);
+            if (elect_one()) {
+              issue_s(0, step + 1, buf);
+              mma_commit(&kv_empty[(2 * step + 2) % SLOTS]);
+              if (MANY && j + 2 == n) mma_commit(&q_empty[buf]);
+            }
           }
-          if (!ok) break;
-          if (elect_one()) mma_commit(&kv_empty[(2 * j + 2) % SLOTS]);
-        }
-        if (!(ok = wait_slot(2 * j + 1))) break;                        // V_j
-        for (int i = 0; i < NT && ok; ++i) {
-          const int n_i = i == 0 ? n0 : n1;
-          if (j >= n_i) continue;
-          if (!(ok = mbar_wait_all(&p_full[i], j & 1, error))) break;    // P_i(j) is in place, O_i rescaled if it had to be
+          if (!(ok = wait_slot(2 * step + 1) && mbar_wait_all(&p_full[0], step & 1, error))) break;  // V_j; P(j) is in place, O rescaled if it had to be
+          if (MANY && j == 0 && !(ok = mbar_wait_all(o_empty, (it & 1) ^ 1, error))) break;          // the last item's O has been read
           tc_fence_after();
           if (elect_one()) {
-            issue_pv(i, j);
-            mma_commit(j == n_i - 1 ? &o_full[i] : &pv_done[i]);
+            issue_pv(0, step, j == 0);
+            mma_commit(!MANY && j + 1 == n ? &o_full[0] : &pv_done[0]);
+            mma_commit(&kv_empty[(2 * step + 1) % SLOTS]);
           }
         }
-        if (!ok) break;
-        if (elect_one()) mma_commit(&kv_empty[(2 * j + 1) % SLOTS]);
+        if (!MANY || !ok) break;
+        // the item's last step: ahead of its P.V the first scores of the next item
+        const bool more = work.advance(), only = n == 1;
+        if (more) {
+          n = n_groups - work.now.rank;
+          const int next = (it + 1) % BUFS;
+          if (!(ok = mbar_wait_all(&q_full[next], ((it + 1) / BUFS) & 1, error) && wait_slot(2 * step + 2) && mbar_wait_all(&s_read[0], step & 1, error))) break;
+          tc_fence_after();
+          if (elect_one()) {
+            issue_s(0, step + 1, next);
+            mma_commit(&kv_empty[(2 * step + 2) % SLOTS]);
+            if (n == 1) mma_commit(&q_empty[next]);
+          }
+        }
+        if (!(ok = wait_slot(2 * step + 1) && mbar_wait_all(&p_full[0], step & 1, error))) break;
+        if (only && !(ok = mbar_wait_all(o_empty, (it & 1) ^ 1, error))) break;
+        tc_fence_after();
+        if (elect_one()) {
+          issue_pv(0, step, only);
+          mma_commit(&o_full[0]);
+          mma_commit(&kv_empty[(2 * step + 1) % SLOTS]);
+        }
+        if (!more) break;
+        ++it, ++step;
       }
     } else {
       for (int j = 0; j < n_steps && ok; ++j) {
@@ -279,9 +316,9 @@ k_attn_fwd_ws(const __grid_constant__ CUtensorMap map, __nv_bfloat16* __restrict
           if (!(ok = mbar_wait_all(&p_full[i], j & 1, error))) break;  // P_i(j) is in place, O_i rescaled if it had to be
           tc_fence_after();
           if (elect_one()) {
-            issue_pv(i, j);
+            issue_pv(i, j, j == 0);
             if (j == n_i - 1) mma_commit(&o_full[i]);
-            else issue_s(i, j + 1);
+            else issue_s(i, j + 1, i);
           }
         }
         if (!ok) break;
@@ -294,123 +331,135 @@ k_attn_fwd_ws(const __grid_constant__ CUtensorMap map, __nv_bfloat16* __restrict
   } else {
     // ------------------------------------------------------------------ softmax (warps 2-5: tile 0, warps 6-9: tile 1)
     const int i = (warp - 2) >> 2;
-    const int n_i = i == 0 ? n0 : n1;
-    const int qt = i == 0 ? qt0 : qt1;
     const int quarter = warp & 3;
     const int r = quarter * 32 + lane;                      // query row within the tile = TMEM lane
     const uint32_t lane_base = (uint32_t)(quarter * 32) << 16;
     const uint32_t tS = tmem + i * 128 + lane_base;
     const uint32_t tO = tmem + C_O + i * HD + lane_base;
     const uint32_t tP = OWN_P ? tmem + C_P + lane_base : tS;  // bf16: keys 2c, 2c+1 in column c
-    float m_used = -INFINITY, l = 0.f;  // m_used in raw score units
     bool ok = true;
-    for (int j = 0; j < n_i && ok; ++j) {
-      if (!(ok = mbar_wait_all(&s_full[i], j & 1, error))) break;
-      tc_fence_after();
-      uint32_t raw[4][32];
+    int it = 0, step = 0, pv = 0;  // pv: P.V products waited for
+    do {
+      const int n_i = MANY ? n_groups - work.now.rank : i == 0 ? n0 : n1;
+      const int qt = MANY ? n_i - 1 : i == 0 ? qt0 : qt1;
+      const int b = work.now.b, h = work.now.h;
+      float m_used = -INFINITY, l = 0.f;  // m_used in raw score units
+      for (int j = 0; j < n_i && ok; ++j, ++step) {
+        if (!(ok = mbar_wait_all(&s_full[i], step & 1, error))) break;
+        tc_fence_after();
+        uint32_t raw[4][32];
 #pragma unroll
-      for (int c = 0; c < 4; ++c) tmem_ld32(tS + c * 32, raw[c]);
-      tmem_ld_wait();
-      if (OWN_P) {
+        for (int c = 0; c < 4; ++c) tmem_ld32(tS + c * 32, raw[c]);
+        tmem_ld_wait();
+        if (OWN_P) {
+          tc_fence_before();
+          __syncwarp();
+          if (lane == 0) mbar_arrive(&s_read[i]);
+        }
+        float mx = -INFINITY;
+        if (j == qt) {  // the diagonal tile: keys beyond the query are masked
+#pragma unroll
+          for (int c = 0; c < 4; ++c)
+#pragma unroll
+            for (int e = 0; e < 32; ++e)
+              if (c * 32 + e > r) raw[c][e] = 0xff800000u;  // -inf
+        }
+        {
+          // eight independent running maxima, two elements at a time: a single chain of dependent maxima would cost ~5 cycles each
+          float part[8];
+#pragma unroll
+          for (int e = 0; e < 8; ++e) part[e] = __uint_as_float(raw[0][e]);
+#pragma unroll
+          for (int e = 8; e < 120; e += 16)
+#pragma unroll
+            for (int u = 0; u < 8; ++u)
+              part[u] = max3(part[u], __uint_as_float(raw[(e + u) >> 5][(e + u) & 31]), __uint_as_float(raw[(e + 8 + u) >> 5][(e + 8 + u) & 31]));
+#pragma unroll
+          for (int u = 0; u < 8; ++u) part[u] = fmaxf(part[u], __uint_as_float(raw[3][24 + u]));
+          mx = max3(max3(part[0], part[1], part[2]), max3(part[3], part[4], part[5]), fmaxf(part[6], part[7]));
+        }
+        if (OWN_P && j > 0) {
+          if (!(ok = mbar_wait_all(&pv_done[i], pv & 1, error))) break;
+          ++pv;
+          tc_fence_after();
+        }
+        if (j == 0) {
+          m_used = mx;
+        } else {
+          const bool need = (mx - m_used) * scale_log2e > 8.f;
+          if (__any_sync(0xffffffffu, need)) {  // rare after the first tiles: rescale this warp's accumulator rows
+            const float f = need ? ex2_approx((m_used - mx) * scale_log2e) : 1.f;
+            if (need) m_used = mx;
+            l *= f;
+#pragma unroll 1
+            for (int c = 0; c < HD / 32; ++c) {
+              uint32_t o[32];
+              tmem_ld32(tO + c * 32, o);
+              tmem_ld_wait();
+#pragma unroll
+              for (int e = 0; e < 32; ++e) o[e] = __float_as_uint(__uint_as_float(o[e]) * f);
+              tmem_st32(tO + c * 32, o);
+            }
+            tmem_st_wait();
+          }
+        }
+        const float mc = m_used * scale_log2e;
+        const f32x2 scale2 = pair2(scale_log2e, scale_log2e), shift2 = pair2(-mc, -mc);
+        f32x2 sums01 = pair2(0.f, 0.f), sums23 = sums01;  // four running sums: columns 0, 1, 2, 3 modulo 4
+#pragma unroll
+        for (int hh = 0; hh < 2; ++hh) {  // 64 keys at a time: 32 registers of bf16 pairs
+          uint32_t pk[32];
+#pragma unroll
+          for (int e = 0; e < 32; ++e) {
+            const int col = hh * 64 + 2 * e;
+            float p0, p1;
+            split2(fma2(pair2(__uint_as_float(raw[col >> 5][col & 31]), __uint_as_float(raw[col >> 5][(col & 31) + 1])), scale2, shift2), &p0, &p1);
+            const f32x2 p = pair2(ex2_approx(p0), ex2_approx(p1));
+            if (e & 1) sums23 = add2(sums23, p);
+            else sums01 = add2(sums01, p);
+            pk[e] = bf16_pair(p);
+          }
+          tmem_st32(tP + hh * 32, pk);  // head dim 128: over the first 64 columns of S
+        }
+        float sums[4];
+        split2(sums01, &sums[0], &sums[1]);
+        split2(sums23, &sums[2], &sums[3]);
+        l += (sums[0] + sums[1]) + (sums[2] + sums[3]);
+        tmem_st_wait();
         tc_fence_before();
         __syncwarp();
-        if (lane == 0) mbar_arrive(&s_read[i]);
+        if (lane == 0) mbar_arrive(&p_full[i]);
+        if (j == 0) work.prefetch();
       }
-      float mx = -INFINITY;
-      if (j == qt) {  // the diagonal tile: keys beyond the query are masked
-#pragma unroll
-        for (int c = 0; c < 4; ++c)
-#pragma unroll
-          for (int e = 0; e < 32; ++e)
-            if (c * 32 + e > r) raw[c][e] = 0xff800000u;  // -inf
-      }
-      {
-        // eight independent running maxima, two elements at a time: a single chain of dependent maxima would cost ~5 cycles each
-        float part[8];
-#pragma unroll
-        for (int e = 0; e < 8; ++e) part[e] = __uint_as_float(raw[0][e]);
-#pragma unroll
-        for (int e = 8; e < 120; e += 16)
-#pragma unroll
-          for (int u = 0; u < 8; ++u)
-            part[u] = max3(part[u], __uint_as_float(raw[(e + u) >> 5][(e + u) & 31]), __uint_as_float(raw[(e + 8 + u) >> 5][(e + 8 + u) & 31]));
-#pragma unroll
-        for (int u = 0; u < 8; ++u) part[u] = fmaxf(part[u], __uint_as_float(raw[3][24 + u]));
-        mx = max3(max3(part[0], part[1], part[2]), max3(part[3], part[4], part[5]), fmaxf(part[6], part[7]));
-      }
-      if (OWN_P && j > 0) {
-        if (!(ok = mbar_wait_all(&pv_done[i], (j - 1) & 1, error))) break;
+      if (ok && n_i > 0) ok = mbar_wait_all(&o_full[i], it & 1, error);
+      if (ok && n_i > 0) {
         tc_fence_after();
-      }
-      if (j == 0) {
-        m_used = mx;
-      } else {
-        const bool need = (mx - m_used) * scale_log2e > 8.f;
-        if (__any_sync(0xffffffffu, need)) {  // rare after the first tiles: rescale this warp's accumulator rows
-          const float f = need ? ex2_approx((m_used - mx) * scale_log2e) : 1.f;
-          if (need) m_used = mx;
-          l *= f;
+        const float inv_l = 1.f / l;
+        const int q_idx = qt * TILE + r;
+        __nv_bfloat16* o_row = out + (size_t)(b * T + q_idx) * d + h * HD;
 #pragma unroll 1
-          for (int c = 0; c < HD / 32; ++c) {
-            uint32_t o[32];
-            tmem_ld32(tO + c * 32, o);
-            tmem_ld_wait();
-#pragma unroll
-            for (int e = 0; e < 32; ++e) o[e] = __float_as_uint(__uint_as_float(o[e]) * f);
-            tmem_st32(tO + c * 32, o);
+        for (int c = 0; c < HD / 32; ++c) {
+          uint32_t o[32];
+          tmem_ld32(tO + c * 32, o);
+          tmem_ld_wait();
+          if (MANY && c + 1 == HD / 32) {
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(o_empty);
           }
-          tmem_st_wait();
+#pragma unroll
+          for (int v = 0; v < 4; ++v) {
+            __nv_bfloat162 y[4];
+#pragma unroll
+            for (int e = 0; e < 4; ++e)
+              y[e] = __floats2bfloat162_rn(__uint_as_float(o[v * 8 + 2 * e]) * inv_l, __uint_as_float(o[v * 8 + 2 * e + 1]) * inv_l);
+            *reinterpret_cast<uint4*>(o_row + c * 32 + v * 8) = *reinterpret_cast<const uint4*>(y);
+          }
         }
+        lse[((size_t)b * H + h) * T + q_idx] = (m_used * scale_log2e + log2f(l)) * 0.69314718055994530942f;  // natural log
       }
-      const float mc = m_used * scale_log2e;
-      const f32x2 scale2 = pair2(scale_log2e, scale_log2e), shift2 = pair2(-mc, -mc);
-      f32x2 sums01 = pair2(0.f, 0.f), sums23 = sums01;  // four running sums: columns 0, 1, 2, 3 modulo 4
-#pragma unroll
-      for (int hh = 0; hh < 2; ++hh) {  // 64 keys at a time: 32 registers of bf16 pairs
-        uint32_t pk[32];
-#pragma unroll
-        for (int e = 0; e < 32; ++e) {
-          const int col = hh * 64 + 2 * e;
-          float p0, p1;
-          split2(fma2(pair2(__uint_as_float(raw[col >> 5][col & 31]), __uint_as_float(raw[col >> 5][(col & 31) + 1])), scale2, shift2), &p0, &p1);
-          const f32x2 p = pair2(ex2_approx(p0), ex2_approx(p1));
-          if (e & 1) sums23 = add2(sums23, p);
-          else sums01 = add2(sums01, p);
-          pk[e] = bf16_pair(p);
-        }
-        tmem_st32(tP + hh * 32, pk);  // head dim 128: over the first 64 columns of S
-      }
-      float sums[4];
-      split2(sums01, &sums[0], &sums[1]);
-      split2(sums23, &sums[2], &sums[3]);
-      l += (sums[0] + sums[1]) + (sums[2] + sums[3]);
-      tmem_st_wait();
-      tc_fence_before();
-      __syncwarp();
-      if (lane == 0) mbar_arrive(&p_full[i]);
-    }
-    if (ok && n_i > 0) ok = mbar_wait_all(&o_full[i], 0, error);
-    if (ok && n_i > 0) {
-      tc_fence_after();
-      const float inv_l = 1.f / l;
-      const int q_idx = qt * TILE + r;
-      __nv_bfloat16* o_row = out + (size_t)(b * T + q_idx) * d + h * HD;
-#pragma unroll 1
-      for (int c = 0; c < HD / 32; ++c) {
-        uint32_t o[32];
-        tmem_ld32(tO + c * 32, o);
-        tmem_ld_wait();
-#pragma unroll
-        for (int v = 0; v < 4; ++v) {
-          __nv_bfloat162 y[4];
-#pragma unroll
-          for (int e = 0; e < 4; ++e)
-            y[e] = __floats2bfloat162_rn(__uint_as_float(o[v * 8 + 2 * e]) * inv_l, __uint_as_float(o[v * 8 + 2 * e + 1]) * inv_l);
-          *reinterpret_cast<uint4*>(o_row + c * 32 + v * 8) = *reinterpret_cast<const uint4*>(y);
-        }
-      }
-      lse[((size_t)b * H + h) * T + q_idx] = (m_used * scale_log2e + log2f(l)) * 0.69314718055994530942f;  // natural log
-    }
+      ++it;
+    } while (ok && work.advance());
   }
   tc_fence_before();
   __syncthreads();
@@ -489,7 +538,7 @@ k_attn_bwd_dq(const __grid_constant__ CUtensorMap map_qkv, const __grid_constant
   const int n_qt = T / TILE;
   constexpr uint32_t TMEM_COLS = 512;
   constexpr uint32_t C_S = 0, C_DP = 128, C_DQ = 256, C_DS = 256 + BUFS * HD;
-  WorkList<MANY> work(T, B, H, group_heads);
+  WorkList<MANY> work(T / TILE, B * H, H, group_heads);
 
   if (tid == 0) {
     for (int i = 0; i < 2; ++i) {
@@ -795,7 +844,7 @@ k_attn_bwd_dkv(const __grid_constant__ CUtensorMap map_qkv, const __grid_constan
   const int n_tiles = T / TILE;
   constexpr uint32_t TMEM_COLS = 512;
   constexpr uint32_t C_S = 0, C_DP = 128, C_ACC = 256;  // dV of buffer i at C_ACC + i * 2 * HD, dK behind it
-  WorkList<MANY> work(T, B, H, group_heads);
+  WorkList<MANY> work(T / TILE, B * H, H, group_heads);
 
   if (tid == 0) {
     for (int i = 0; i < 2; ++i) {
@@ -1136,21 +1185,26 @@ int tb_attn_fwd(const void* qkv, void* out, float* lse, int B, int T, int H, int
   if (rc) return rc;
   const float scale_log2e = 1.4426950408889634f / sqrtf((float)HD);
   const int tiles = HD == 64 ? 1 : 2;
-  const unsigned ctas = (unsigned)((T / TILE + tiles - 1) / tiles * H * B);
+  const long long items = (long long)((T / TILE + tiles - 1) / tiles) * H * B;
+  const bool many = HD == 64 && items > 2 * sm_count();  // two CTAs share an SM
+  const int group = many ? group_heads(T, H * B) : 1;
+  const unsigned ctas = (unsigned)(many ? 2 * sm_count() : items);
   tb_note_launch(1);
-#define LAUNCH_FWD(HD_) \
+#define LAUNCH_FWD(HD_, MANY_) \
   do { \
+    using L = Fwd2Smem<HD_, MANY_>; \
     static bool once = false; \
     if (!once) { \
-      cudaError_t e = cudaFuncSetAttribute(k_attn_fwd_ws<HD_>, cudaFuncAttributeMaxDynamicSharedMemorySize, Fwd2Smem<HD_>::TOTAL); \
+      cudaError_t e = cudaFuncSetAttribute(k_attn_fwd_ws<HD_, MANY_>, cudaFuncAttributeMaxDynamicSharedMemorySize, L::TOTAL); \
       if (e != cudaSuccess) return (int)e; \
       once = true; \
     } \
-    return (int)tb::launch(k_attn_fwd_ws<HD_>, dim3(ctas), dim3(Fwd2Smem<HD_>::THREADS), Fwd2Smem<HD_>::TOTAL, stream, map, (__nv_bfloat16*)out, lse, B, T, H, d, \
-                           scale_log2e, g_err_dev); \
+    return (int)tb::launch(k_attn_fwd_ws<HD_, MANY_>, dim3(ctas), dim3(L::THREADS), L::TOTAL, stream, map, (__nv_bfloat16*)out, lse, B, T, H, d, scale_log2e, \
+                           group, g_err_dev); \
   } while (0)
-  if (HD == 64) LAUNCH_FWD(64);
-  LAUNCH_FWD(128);
+  if (HD == 128) LAUNCH_FWD(128, false);
+  if (many) LAUNCH_FWD(64, true);
+  LAUNCH_FWD(64, false);
 #undef LAUNCH_FWD
 }
 

@@ -568,6 +568,27 @@ def test_causal_attention_matches_fp32(B, T, H, hd, spread):
         close(qkv.grad[..., part * d:(part + 1) * d], ref.grad[..., part * d:(part + 1) * d], rtol=4e-2, atol=2e-2, frobenius=1e-2)
 
 
+# more tiles than SMs (backward) and than two per SM (forward), by one and by several rounds; one to eight tiles per head; heads that
+# fill no whole group of the work list
+@pytest.mark.parametrize("B,T,H", [(149, 128, 1), (297, 128, 1), (25, 256, 13), (10, 640, 8), (13, 1024, 12), (40, 1024, 5)])
+def test_causal_attention_work_lists(B, T, H):
+    """CTAs that take item after item against a CTA for every item: a sequence by itself has fewer tiles than the GPU has SMs."""
+    from tandem_b200 import ops
+    from tandem_b200.ops.attention import attention_error
+
+    qkv, dy = rnd(B, T, 3 * H * 64), rnd(B, T, H * 64)
+    x = qkv.clone().requires_grad_()
+    y = ops.causal_attention(x, H)
+    (g,) = torch.autograd.grad(y, x, dy)
+    for b in range(B):
+        one = qkv[b:b + 1].clone().requires_grad_()
+        alone = ops.causal_attention(one, H)
+        assert torch.equal(y[b:b + 1], alone)
+        assert torch.equal(g[b:b + 1], torch.autograd.grad(alone, one, dy[b:b + 1])[0])
+    torch.cuda.synchronize()
+    assert not attention_error(), "an attention wait ran out"
+
+
 @pytest.mark.parametrize("hd", [64, 128])
 def test_causal_attention_keeps_nan_queries_from_later_keys(hd):
     """The value gradient of a key is a sum over the queries from that key on: a query that is NaN reaches no key after it."""
