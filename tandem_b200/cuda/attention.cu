@@ -62,9 +62,13 @@ __device__ __forceinline__ void mma_kmajor(uint32_t d_tmem, const uint8_t* a, co
 // finished.  (A CTA per item spent 2 to 3.5 us of its 5 to 6 outside the loop over tiles; dQ and dK/dV, us: 16 x 512, 12 heads
 // 40.4 -> 29.5 and 47.1 -> 38.9; 32 x 1024, 16 heads 251 -> 176 and 296 -> 243.)  Head dim 128 fills an SM with one item; its
 // grid has a CTA for each.
-// An item is a tile of a head.  Items come in groups of `heads` heads whose tiles together are worth several rounds: the longest tiles of
-// all heads of a group first, so that the rounds end together, and few enough heads that what they share stays in L2.  CTA c takes
-// the c-th item of even rounds and the c-th from the end of odd ones.
+// An item is a tile of a head (NT = 2: two query tiles).  The tiles of a head take from one step to as many as it has tiles, so their order decides how evenly the
+// GPU ends.  MANY: items come in groups of `per_group` heads, the longest tiles of all heads of a group first, so that the rounds end together, and few enough
+// heads that what they share stays in L2; CTA c takes the c-th item of even rounds and the c-th from the end of odd ones.
+// Otherwise CTA c has the c-th item: head by head, so that a head's K and V are read once from memory, but for the last group of
+// heads, whose longest tiles come first (head by head to the end, the last CTAs ran alone for as long as a whole
+// head takes: forward, dQ, dK/dV of 2 x 4096, 16 heads of 128 157, 212 and 252 us, now 131, 200 and 232; 3 x 2048 82, 118 and 130, now 68, 112
+// and 120).
 // Finding an item takes a few hundred cycles of divisions: the first is found while the CTA sets itself up, the next one by prefetch(), which
 // every role calls where it would wait anyway.
 struct WorkItem {
@@ -77,15 +81,19 @@ struct WorkList {
 
   __device__ __forceinline__ WorkItem find(int at) const {
     WorkItem w;
-    if (!MANY) {  // consecutive CTAs share a head
-      w.rank = at % tiles;
-      w.head = at / tiles;
-    } else {
+    int first = all - per_group, size = per_group;  // the group's heads
+    if (MANY) {
       if (at >= tiles * all) return {0, -1, 0, 0};
-      const int group = at / (per_group * tiles), in = at - group * per_group * tiles;
-      const int size = all - group * per_group < per_group ? all - group * per_group : per_group;
+      first = at / (per_group * tiles) * per_group;
+      size = all - first < per_group ? all - first : per_group;
+    }
+    if (MANY || at >= first * tiles) {
+      const int in = at - first * tiles;
       w.rank = in / size;
-      w.head = group * per_group + in - w.rank * size;
+      w.head = first + in - w.rank * size;
+    } else {
+      w.head = at / tiles;
+      w.rank = at - w.head * tiles;
     }
     w.b = w.head / H;
     w.h = w.head - w.b * H;
@@ -1163,9 +1171,12 @@ int sm_count() {
   return n;
 }
 
-// WorkList: eight rounds' worth of tiles per group of heads.
-int group_heads(int T, int heads) {
-  const int tiles = T / TILE, want = (8 * sm_count() + tiles - 1) / tiles;
+// WorkList: heads per group.  CTAs that take many items take the same number each, so the groups are as long as L2 allows (eight
+// rounds; 1 x 8192, 16 heads, dK/dV: four rounds 355 us, eight 329).  Of CTAs with one item the GPU starts another whenever one ends, so
+// only the last items have to be sorted: three rounds' worth (one: 2 x 8192, 16 heads of 128, dK/dV 880 us, two 850, three 837, four 863).
+int group_heads(int tiles, int heads, bool many) {
+  if (!many && tiles * heads <= sm_count()) return 1;  // all start at once; neighbours that share a head read it once
+  const int want = ((many ? 8 : 3) * sm_count() + tiles - 1) / tiles;
   return want < heads ? want : heads;
 }
 
@@ -1187,7 +1198,7 @@ int tb_attn_fwd(const void* qkv, void* out, float* lse, int B, int T, int H, int
   const int tiles = HD == 64 ? 1 : 2;
   const long long items = (long long)((T / TILE + tiles - 1) / tiles) * H * B;
   const bool many = HD == 64 && items > 2 * sm_count();  // two CTAs share an SM
-  const int group = many ? group_heads(T, H * B) : 1;
+  const int group = group_heads((T / TILE + tiles - 1) / tiles, H * B, many);
   const unsigned ctas = (unsigned)(many ? 2 * sm_count() : items);
   tb_note_launch(1);
 #define LAUNCH_FWD(HD_, MANY_) \
@@ -1226,7 +1237,7 @@ int tb_attn_bwd(const void* qkv, const void* out, const void* d_out, const float
   const long long items = (long long)(T / TILE) * H * B;
   // Where every item has an SM to itself the kernel for one item is 0.3 to 0.8 us faster (2 x 512, 12 heads: dK/dV 10.7 / 11.5 us).
   const bool many = HD == 64 && items > sm_count();
-  const int group = many ? group_heads(T, H * B) : 1;
+  const int group = group_heads(T / TILE, H * B, many);
   const unsigned ctas = (unsigned)(many ? sm_count() : items);
   tb_note_launch(2);
 #define LAUNCH_BWD(HD_, MANY_) \
