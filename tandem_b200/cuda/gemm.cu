@@ -573,8 +573,7 @@ __device__ __forceinline__ void fold_tile(uint32_t taddr, int c_begin, int c_end
 // The flag a producer's warp raises once its share is parked, and the consumer's bounded wait for the same warp's flags
 // of all parts (`stride` words apart).  The flags are zero again afterwards, for the next launch that is handed these words.
 __device__ __forceinline__ void raise_flag(unsigned* flag, int lane) {
-  __threadfence();
-  __syncwarp();
+  __syncwarp();  // every lane's stores come before lane 0's release, which is cumulative: it covers them all
   if (lane == 0) st_release_gpu(flag, 1u);
 }
 __device__ __forceinline__ bool wait_flags(unsigned* flags, int parts, int stride, int lane, int* error) {
