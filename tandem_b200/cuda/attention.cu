@@ -25,6 +25,7 @@
 #include <atomic>
 
 #include "f32x2.cuh"
+#include "host_state.h"
 #include "launch.cuh"
 #include "tcgen05.cuh"
 
@@ -1132,13 +1133,14 @@ int make_map(CUtensorMap* map, const void* ptr, long long cols, long long rows, 
     cudaFree(nullptr);
     context_ready = true;
   }
-  static EncodeTiled enc = nullptr;
+  static std::atomic<EncodeTiled> known{nullptr};
+  EncodeTiled enc = known.load(std::memory_order_relaxed);
   if (enc == nullptr) {
     void* p = nullptr;
     cudaDriverEntryPointQueryResult q;
     if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &p, cudaEnableDefault, &q) != cudaSuccess || q != cudaDriverEntryPointSuccess)
       return -10;
-    enc = (EncodeTiled)p;
+    known.store(enc = (EncodeTiled)p, std::memory_order_relaxed);
   }
   cuuint64_t dims[2] = {(cuuint64_t)cols, (cuuint64_t)rows};
   cuuint64_t strides[1] = {(cuuint64_t)row_stride * 2};
@@ -1149,26 +1151,12 @@ int make_map(CUtensorMap* map, const void* ptr, long long cols, long long rows, 
              ? 0 : -11;
 }
 
-int* g_err_host = nullptr;
-int* g_err_dev = nullptr;
-
-int ensure_error_word() {
-  if (g_err_host != nullptr) return 0;
-  if (cudaHostAlloc((void**)&g_err_host, 64, cudaHostAllocMapped) != cudaSuccess) return -13;
-  *g_err_host = 0;
-  return cudaHostGetDevicePointer((void**)&g_err_dev, g_err_host, 0) == cudaSuccess ? 0 : -13;
-}
+tb::ErrorWord g_error;
 
 // Places for one CTA per SM.
 int sm_count() {
-  static std::atomic<int> known{0};
-  int n = known.load(std::memory_order_relaxed);
-  if (n == 0) {
-    int dev = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || n <= 0) n = 148;
-    known.store(n, std::memory_order_relaxed);
-  }
-  return n;
+  const int n = tb::sm_count();
+  return n > 0 ? n : 148;
 }
 
 // WorkList: heads per group.  CTAs that take many items take the same number each, so the groups are as long as L2 allows (eight
@@ -1184,12 +1172,13 @@ int group_heads(int tiles, int heads, bool many) {
 
 extern "C" {
 
-int tb_attn_error() { return g_err_host != nullptr ? *g_err_host : 0; }
+int tb_attn_error() { return g_error.raised(); }
 
 // out[B*T, d] = causal softmax(q k^T / sqrt(HD)) v per head; lse[B, H, T] (fp32) kept for backward.
 int tb_attn_fwd(const void* qkv, void* out, float* lse, int B, int T, int H, int HD, cudaStream_t stream) {
   if (T % TILE || (HD != 64 && HD != 128)) return -21;
-  if (ensure_error_word()) return -13;
+  int* const error = g_error.device();
+  if (error == nullptr) return -13;
   const int d = H * HD;
   CUtensorMap map;
   int rc = make_map(&map, qkv, 3LL * d, (long long)B * T, 3LL * d);
@@ -1211,7 +1200,7 @@ int tb_attn_fwd(const void* qkv, void* out, float* lse, int B, int T, int H, int
       once = true; \
     } \
     return (int)tb::launch(k_attn_fwd_ws<HD_, MANY_>, dim3(ctas), dim3(L::THREADS), L::TOTAL, stream, map, (__nv_bfloat16*)out, lse, B, T, H, d, scale_log2e, \
-                           group, g_err_dev); \
+                           group, error); \
   } while (0)
   if (HD == 128) LAUNCH_FWD(128, false);
   if (many) LAUNCH_FWD(64, true);
@@ -1223,7 +1212,8 @@ int tb_attn_fwd(const void* qkv, void* out, float* lse, int B, int T, int H, int
 int tb_attn_bwd(const void* qkv, const void* out, const void* d_out, const float* lse, void* dqkv, float* delta, int B, int T, int H, int HD,
                 cudaStream_t stream) {
   if (T % TILE || (HD != 64 && HD != 128)) return -21;
-  if (ensure_error_word()) return -13;
+  int* const error = g_error.device();
+  if (error == nullptr) return -13;
   const int d = H * HD;
   const long long rows = (long long)B * T;
   CUtensorMap map_qkv, map_do, map_o;
@@ -1250,10 +1240,10 @@ int tb_attn_bwd(const void* qkv, const void* out, const void* d_out, const float
       once = true; \
     } \
     cudaError_t e = tb::launch(k_attn_bwd_dq<HD_, MANY_>, dim3(ctas), dim3(320), BwdDqSmem<HD_, MANY_>::TOTAL, stream, map_qkv, map_do, map_o, \
-                               (const __nv_bfloat16*)out, (const __nv_bfloat16*)d_out, lse, delta, (__nv_bfloat16*)dqkv, B, T, H, d, scale, group, g_err_dev); \
+                               (const __nv_bfloat16*)out, (const __nv_bfloat16*)d_out, lse, delta, (__nv_bfloat16*)dqkv, B, T, H, d, scale, group, error); \
     if (e != cudaSuccess) return (int)e; \
     return (int)tb::launch(k_attn_bwd_dkv<HD_, MANY_>, dim3(ctas), dim3(320), BwdDkvSmem<HD_, MANY_>::TOTAL, stream, map_qkv, map_do, lse, (const float*)delta, \
-                           (__nv_bfloat16*)dqkv, B, T, H, d, scale, group, g_err_dev); \
+                           (__nv_bfloat16*)dqkv, B, T, H, d, scale, group, error); \
   } while (0)
   if (HD == 128) LAUNCH_BWD(128, false);
   if (many) LAUNCH_BWD(64, true);

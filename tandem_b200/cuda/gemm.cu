@@ -38,6 +38,7 @@
 #include <string.h>
 
 #include "f32x2.cuh"
+#include "host_state.h"
 #include "launch.cuh"
 #include "tcgen05.cuh"
 
@@ -1094,18 +1095,19 @@ typedef CUresult (*EncodeTiled)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, v
                                 CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
 
 EncodeTiled encoder() {
-  static EncodeTiled fn = nullptr;
+  static std::atomic<EncodeTiled> known{nullptr};
+  EncodeTiled fn = known.load(std::memory_order_relaxed);
   if (fn == nullptr) {
     void* p = nullptr;
     cudaDriverEntryPointQueryResult q;
     if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &p, cudaEnableDefault, &q) == cudaSuccess &&
         q == cudaDriverEntryPointSuccess)
-      fn = (EncodeTiled)p;
+      known.store(fn = (EncodeTiled)p, std::memory_order_relaxed);
   }
   return fn;
 }
 
-char g_map_error[256] = "";
+thread_local char g_map_error[256] = "";
 
 // A 2-D bf16 tensor map: `inner` contiguous elements per row, `outer` rows of `row_stride` elements.
 int make_map(CUtensorMap* map, const void* ptr, long long inner, long long outer, long long row_stride, int box_inner, int box_outer,
@@ -1153,9 +1155,7 @@ int plan_epilogue(CUtensorMap* mo, CUtensorMap* mp, CUtensorMap* mx, void* out, 
   return kind;
 }
 
-int* g_error_host = nullptr;
-int* g_error_dev = nullptr;
-int g_sm_count = 0;
+tb::ErrorWord g_error;
 
 template <int BM, int BN, bool A_MN, bool B_MN>
 int launch_gemm(const CUtensorMap& ma, const CUtensorMap& mb, const CUtensorMap& mo, const CUtensorMap& mp, const CUtensorMap& mx, const GemmArgs& g, int max_ctas,
@@ -1170,7 +1170,8 @@ int launch_gemm(const CUtensorMap& ma, const CUtensorMap& mb, const CUtensorMap&
   }
   const int out_tiles = ((g.M + BM - 1) / BM) * ((g.N + BN - 1) / BN);
   const int tiles = g.splits > 1 ? g.whole_tiles + (out_tiles - g.whole_tiles) * g.splits : out_tiles;
-  int ctas = tiles < g_sm_count ? tiles : g_sm_count;
+  const int sms = tb::sm_count();
+  int ctas = tiles < sms ? tiles : sms;
   if (max_ctas > 0 && ctas > max_ctas) ctas = max_ctas;
   return (int)tb::launch(kernel, dim3(ctas), dim3(L::THREADS), L::TOTAL, stream, ma, mb, mo, mp, mx, g, GatherArgs{});
 }
@@ -1186,7 +1187,7 @@ int launch_gemm_pair(const CUtensorMap& ma, const CUtensorMap& mb, const CUtenso
     cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, L::TOTAL);
     if (e != cudaSuccess) return (int)e;
     cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(g_sm_count & ~1);
+    cfg.gridDim = dim3(tb::sm_count() & ~1);
     cfg.blockDim = dim3(L::THREADS);
     cfg.dynamicSmemBytes = L::TOTAL;
     cudaLaunchAttribute attr;
@@ -1199,9 +1200,9 @@ int launch_gemm_pair(const CUtensorMap& ma, const CUtensorMap& mb, const CUtenso
     int n = 0;
     if (cudaOccupancyMaxActiveClusters(&n, kernel, &cfg) != cudaSuccess || n <= 0) {
       cudaGetLastError();
-      n = g_sm_count / 2;
+      n = tb::sm_count() / 2;
     }
-    max_pairs = n < g_sm_count / 2 ? n : g_sm_count / 2;
+    max_pairs = n < tb::sm_count() / 2 ? n : tb::sm_count() / 2;
   }
   const int out_tiles = ((g.M + 255) / 256) * ((g.N + BN - 1) / BN);
   const int tiles = g.splits > 1 ? g.whole_tiles + (out_tiles - g.whole_tiles) * g.splits : out_tiles;
@@ -1335,6 +1336,9 @@ GemmPlan plan_gemm(int M, int N, int K, int ctas) {
   return best;
 }
 
+// Without a device (a build machine) the plan is the one a B200's 148 SMs would get.
+int planned_sms() { return tb::sm_count() > 0 ? tb::sm_count() : 148; }
+
 // reciprocal2 as the GELU epilogue uses it, for comparisons with a division.
 __global__ void k_reciprocals(const float* d, float* out, long long pairs) {
   const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
@@ -1345,10 +1349,10 @@ __global__ void k_reciprocals(const float* d, float* out, long long pairs) {
   split2(r[0], &out[2 * i], &out[2 * i + 1]);
 }
 
-// Flag words for split-K, handed out round-robin to launches (a launch that is handed words still in use by an earlier
-// one would need a pool's worth of launches in flight at once); all zero between launches.
+// Flag words for split-K.
 constexpr int SPLIT_FLAG_POOL = 1 << 16;
 __device__ unsigned g_split_flags[SPLIT_FLAG_POOL];
+tb::WordPool g_flag_pool(SPLIT_FLAG_POOL);
 
 }  // namespace
 
@@ -1357,7 +1361,7 @@ extern "C" void tb_note_launch(int n);
 extern "C" {
 
 // 0 while every GEMM wait so far has completed; 1 after one ran out.
-int tb_gemm_error() { return g_error_host != nullptr ? *g_error_host : 0; }
+int tb_gemm_error() { return g_error.raised(); }
 
 // D[M,N] = op(A) . op(B) with bf16 operands, then the epilogue selected by `flags` (EpilogueFlags).
 //   a_mn == 0: A is [M, K] with leading dimension lda (K contiguous); a_mn == 1: A is [K, M], lda (M contiguous).
@@ -1368,15 +1372,10 @@ int tb_gemm_bf16(const void* A, const void* B, void* out, int M, int N, int K, i
                  cudaStream_t stream) {
   if (M <= 0 || N <= 0 || K <= 0) return 0;
   if ((lda & 7) || (ldb & 7) || (((uintptr_t)A | (uintptr_t)B) & 15)) return -12;
-  if (g_error_host == nullptr) {
-    if (cudaHostAlloc((void**)&g_error_host, 64, cudaHostAllocMapped) != cudaSuccess) return -13;
-    *g_error_host = 0;
-    if (cudaHostGetDevicePointer((void**)&g_error_dev, g_error_host, 0) != cudaSuccess) return -13;
-    int dev = 0;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&g_sm_count, cudaDevAttrMultiProcessorCount, dev);
-  }
-  const int ctas = max_ctas > 0 && max_ctas < g_sm_count ? max_ctas : g_sm_count;
+  int* const error = g_error.device();
+  if (error == nullptr) return -13;
+  const int sms = tb::sm_count();
+  const int ctas = max_ctas > 0 && max_ctas < sms ? max_ctas : sms;
   const GemmPlan plan = plan_gemm(M, N, K, ctas);
   const int BM = plan.bm, BN = plan.bn;
   int splits = plan.splits;
@@ -1387,18 +1386,8 @@ int tb_gemm_bf16(const void* A, const void* B, void* out, int M, int N, int K, i
     if (workspace == nullptr || workspace_bytes < need || ((uintptr_t)workspace & 15) || words > SPLIT_FLAG_POOL) {
       splits = 1;  // no room to park partial tiles: compute unsplit (same result up to summation order)
     } else {
-      static unsigned* pool = nullptr;
-      static int pool_device = -1;
-      static long long next = 0;
-      int dev = 0;
-      cudaGetDevice(&dev);
-      if (pool == nullptr || pool_device != dev) {
-        if (cudaGetSymbolAddress((void**)&pool, g_split_flags) != cudaSuccess) return (int)cudaGetLastError();
-        pool_device = dev;
-      }
-      if (next + words > SPLIT_FLAG_POOL) next = 0;
-      split_flags = pool + next;
-      next += words;
+      const cudaError_t e = g_flag_pool.take(words, &split_flags, [](void** at) { return cudaGetSymbolAddress(at, g_split_flags); });
+      if (e != cudaSuccess) return (int)e;
     }
   }
   CUtensorMap ma, mb;
@@ -1412,7 +1401,7 @@ int tb_gemm_bf16(const void* A, const void* B, void* out, int M, int N, int K, i
   CUtensorMap mo, mp, mx;
   const int kind = plan_epilogue(&mo, &mp, &mx, out, aux_out, aux_in, M, N, ldc, flags);
   const int group_m = BM == 128 ? 8 : 4;  // 1024 rows
-  GemmArgs g{M, N, K, ldc, flags, out, (const __nv_bfloat16*)bias, (const __nv_bfloat16*)aux_in, (__nv_bfloat16*)aux_out, g_error_dev,
+  GemmArgs g{M, N, K, ldc, flags, out, (const __nv_bfloat16*)bias, (const __nv_bfloat16*)aux_in, (__nv_bfloat16*)aux_out, error,
              splits, splits > 1 ? plan.whole_tiles : 0, (float*)workspace, split_flags, group_m, kind};
   tb_note_launch(1);
   const bool deep = K >= 32 * BK;
@@ -1446,25 +1435,12 @@ int tb_gemm_bf16(const void* A, const void* B, void* out, int M, int N, int K, i
 // at least that much (any stream-ordered allocator will do: the kernel is done with it when it completes) and passes it.
 long long tb_gemm_workspace_bytes(int M, int N, int K) {
   if (M <= 0 || N <= 0 || K <= 0) return 0;
-  if (g_sm_count == 0) {
-    int dev = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&g_sm_count, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
-      g_sm_count = 0;
-    cudaGetLastError();
-  }
-  return plan_gemm(M, N, K, g_sm_count > 0 ? g_sm_count : 148).workspace_bytes(M, N);
+  return plan_gemm(M, N, K, planned_sms()).workspace_bytes(M, N);
 }
 
 // What the planner picks: writes {BM (512: CTA pair), BN, parts the tail tiles are cut into, tiles computed whole}.
 void tb_gemm_plan(int M, int N, int K, int* out4) {
-  if (g_sm_count == 0) {
-    int dev = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&g_sm_count, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
-      g_sm_count = 0;
-    cudaGetLastError();
-  }
-  // without a device (a build machine) the plan is the one a B200's 148 SMs would get
-  const GemmPlan plan = plan_gemm(M, N, K, g_sm_count > 0 ? g_sm_count : 148);
+  const GemmPlan plan = plan_gemm(M, N, K, planned_sms());
   out4[0] = plan.bm;
   out4[1] = plan.bn;
   out4[2] = plan.splits;
@@ -1486,19 +1462,14 @@ int tb_gemm_gathered(const void* A, void* out, int M, int N, int K, int lda, int
                      cudaStream_t stream) {
   if (M <= 0 || N <= 0 || K <= 0) return 0;
   if ((lda & 7) || (K & 7) || (w_off & 15) || (((uintptr_t)A | (uintptr_t)full) & 15) || n_ranks < 1 || n_ranks > 8) return -12;
-  if (g_error_host == nullptr) {
-    if (cudaHostAlloc((void**)&g_error_host, 64, cudaHostAllocMapped) != cudaSuccess) return -13;
-    *g_error_host = 0;
-    if (cudaHostGetDevicePointer((void**)&g_error_dev, g_error_host, 0) != cudaSuccess) return -13;
-    int dev = 0;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&g_sm_count, cudaDevAttrMultiProcessorCount, dev);
-  }
+  int* const error = g_error.device();
+  if (error == nullptr) return -13;
+  const int sms = tb::sm_count();
   // 256-row tiles (two MMAs per weight panel in shared memory: a third less operand traffic per flop) once the problem
   // has enough of them for every SM; 128-row tiles otherwise.  The weight panel is 256 columns wide in both.
   constexpr int BN = 256;
   const int tiles_n = (N + BN - 1) / BN;
-  const bool tall = (long long)((M + 255) / 256) * tiles_n >= g_sm_count;
+  const bool tall = (long long)((M + 255) / 256) * tiles_n >= sms;
   const int BM = tall ? 256 : 128;
   CUtensorMap ma, mb;
   int rc = make_map(&ma, A, K, M, lda, 64, BM);
@@ -1507,7 +1478,7 @@ int tb_gemm_gathered(const void* A, void* out, int M, int N, int K, int lda, int
   if (rc) return rc;
   CUtensorMap mo, mp, mx;
   const int kind = plan_epilogue(&mo, &mp, &mx, out, aux_out, aux_in, M, N, ldc, flags);
-  GemmArgs g{M, N, K, ldc, flags, out, (const __nv_bfloat16*)bias, (const __nv_bfloat16*)aux_in, (__nv_bfloat16*)aux_out, g_error_dev,
+  GemmArgs g{M, N, K, ldc, flags, out, (const __nv_bfloat16*)bias, (const __nv_bfloat16*)aux_in, (__nv_bfloat16*)aux_out, error,
              1, 0, nullptr, nullptr, 1, kind};
   GatherArgs ga{};
   for (int q = 0; q < n_ranks; ++q) {
@@ -1533,7 +1504,7 @@ int tb_gemm_gathered(const void* A, void* out, int M, int N, int K, int lda, int
     configured[tall] = true;
   }
   const int tiles = ((M + BM - 1) / BM) * tiles_n;
-  int ctas = tiles < g_sm_count ? tiles : g_sm_count;
+  int ctas = tiles < sms ? tiles : sms;
   void* params[] = {(void*)&ma, (void*)&mb, (void*)&mo, (void*)&mp, (void*)&mx, (void*)&g, (void*)&ga};
   tb_note_launch(1);
   return (int)cudaLaunchCooperativeKernel(kernel, dim3(ctas), dim3(448), params, smem, stream);

@@ -1,0 +1,86 @@
+// What launches on one GPU share on the host.  Several threads launch at once (autograd's workers, an evaluation beside a
+// training step), so whatever is made by the first call or handed out from call to call sits behind a lock or is atomic.
+#pragma once
+#include <cuda_runtime.h>
+
+#include <atomic>
+#include <mutex>
+
+namespace tb {
+
+// SMs of the GPU; 0 where there is none.
+inline int sm_count() {
+  static std::atomic<int> known{0};
+  int n = known.load(std::memory_order_relaxed);
+  if (n == 0) {
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || n < 0) n = 0;
+    cudaGetLastError();
+    known.store(n, std::memory_order_relaxed);
+  }
+  return n;
+}
+
+// A word of host memory that kernels raise when a wait runs out.
+class ErrorWord {
+ public:
+  bool raised() const {
+    const int* word = host_.load(std::memory_order_acquire);
+    return word != nullptr && *reinterpret_cast<const volatile int*>(word) != 0;
+  }
+  // Its device address; null if it cannot be made.
+  int* device() {
+    if (host_.load(std::memory_order_acquire) != nullptr) return dev_;
+    std::lock_guard<std::mutex> hold(lock_);
+    if (host_.load(std::memory_order_relaxed) != nullptr) return dev_;
+    int *host = nullptr, *dev = nullptr;
+    if (cudaHostAlloc((void**)&host, 64, cudaHostAllocMapped) != cudaSuccess) return nullptr;
+    *host = 0;
+    if (cudaHostGetDevicePointer((void**)&dev, host, 0) != cudaSuccess) {
+      cudaFreeHost(host);
+      return nullptr;
+    }
+    dev_ = dev;
+    host_.store(host, std::memory_order_release);  // last: whoever sees it sees dev_
+    return dev;
+  }
+
+ private:
+  std::mutex lock_;
+  std::atomic<int*> host_{nullptr};
+  int* dev_ = nullptr;
+};
+
+// Words of a __device__ array of `size` zeros, lent round-robin to launches that leave them zero again.  Launches in flight at
+// the same time never share one (a pool's worth of them would have to overlap).
+class WordPool {
+ public:
+  explicit WordPool(long long size) : size_(size) {}
+  // `words` <= size of them on the current device; `find(void**)` looks the array up there.
+  template <typename Find>
+  cudaError_t take(long long words, unsigned** out, Find find) {
+    int dev = 0;
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e != cudaSuccess) return e;
+    std::lock_guard<std::mutex> hold(lock_);
+    if (device_ != dev) {
+      void* at = nullptr;
+      if ((e = find(&at)) != cudaSuccess) return e;
+      pool_ = static_cast<unsigned*>(at);
+      device_ = dev;
+    }
+    if (next_ + words > size_) next_ = 0;
+    *out = pool_ + next_;
+    next_ += words;
+    return cudaSuccess;
+  }
+
+ private:
+  std::mutex lock_;
+  const long long size_;
+  unsigned* pool_ = nullptr;
+  int device_ = -1;
+  long long next_ = 0;
+};
+
+}  // namespace tb

@@ -12,6 +12,7 @@
 #include <mutex>
 
 #include "f32x2.cuh"
+#include "host_state.h"
 #include "launch.cuh"
 #include "noalloc.h"
 
@@ -392,8 +393,10 @@ k_reduce_partials(const float* __restrict__ part, int parts, int width, __nv_bfl
 }
 
 // ------------------------------------------------------------------------------------ column sums
-// Ticket words for k_col_sum's single-launch mode: all zero between launches.
-__device__ unsigned g_col_sum_tickets[8192];
+// Ticket words for k_col_sum's single-launch mode.
+constexpr int TICKET_POOL = 8192;
+__device__ unsigned g_col_sum_tickets[TICKET_POOL];
+tb::WordPool g_ticket_pool(TICKET_POOL);
 
 // part[blockIdx.y][c] = sum of x[r, c] over the block's row slice; 32 columns x 32 row lanes.
 // With `tickets` (one zero word per column group) the kernel also finishes the job: the last row slice of a
@@ -920,22 +923,12 @@ int tb_col_sum(const void* x, int M, int N, int ld, void* out_bf16, float* scrat
   if (slices == 32 && rows_per <= 192) wide_from = rows_per < 128 ? 3072 : 4096;
   const bool wide = vectors && N >= wide_from;
   dim3 grid(wide ? (N + 255) / 256 : vectors ? (N + 63) / 64 : (N + 31) / 32, slices);
-  // One launch: each column group's last block finishes the sum.  The ticket words come from a fixed pool handed
-  // out round-robin, so launches in flight at the same time never share one (a pool's worth of launches would
-  // have to overlap); matrices wider than the pool take the two-kernel path.
-  constexpr int POOL = 8192;
-  static unsigned* pool = nullptr;
-  static int pool_device = -1, next = 0;
-  int dev = 0;
-  cudaGetDevice(&dev);
-  if (pool == nullptr || pool_device != dev) {
-    if (cudaGetSymbolAddress((void**)&pool, g_col_sum_tickets) != cudaSuccess) return (int)cudaGetLastError();
-    pool_device = dev;
-  }
-  if ((int)grid.x <= POOL) {
-    if (next + (int)grid.x > POOL) next = 0;
-    unsigned* tickets = pool + next;
-    next += grid.x;
+  // One launch: each column group's last block finishes the sum.  Matrices wider than the pool of ticket words take the
+  // two-kernel path.
+  if ((int)grid.x <= TICKET_POOL) {
+    unsigned* tickets = nullptr;
+    const cudaError_t e = g_ticket_pool.take(grid.x, &tickets, [](void** at) { return cudaGetSymbolAddress(at, g_col_sum_tickets); });
+    if (e != cudaSuccess) return (int)e;
     tb_note_launch(1);
     if (wide)
       tb::launch(k_col_sum_wide, grid, dim3(256), 0, s, (const __nv_bfloat16*)x, M, N, ld, scratch, tickets, (__nv_bfloat16*)out_bf16);

@@ -8,6 +8,8 @@
 #include <stdio.h>
 #include <string.h>
 
+#include <atomic>
+
 static thread_local char g_last_error[256] = "";
 
 static int fail(cudaError_t e, const char* what) {
@@ -16,19 +18,15 @@ static int fail(cudaError_t e, const char* what) {
   return (int)e;
 }
 
-static long long g_launches = 0;
+static std::atomic<long long> g_launches{0};
 
 extern "C" {
 
 // Every kernel launcher in this library reports its launches here, so a caller
 // can count how many of these kernels ran in a region of its program.
-void tb_note_launch(int n) { g_launches += n; }
+void tb_note_launch(int n) { g_launches.fetch_add(n, std::memory_order_relaxed); }
 
-long long tb_launch_count(int reset) {
-  long long v = g_launches;
-  if (reset) g_launches = 0;
-  return v;
-}
+long long tb_launch_count(int reset) { return reset ? g_launches.exchange(0) : g_launches.load(); }
 
 const char* tb_last_error() { return g_last_error; }
 

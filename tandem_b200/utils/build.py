@@ -74,17 +74,9 @@ def nvcc_path():
     return None
 
 
-def build_cuda(force=False, verbose=False):
-    """Compiles every .cu under cuda/ into one shared library for sm_100a."""
-    srcs = [s for s in _sources(CUDA, (".cu",))]
-    deps = _sources(CUDA, (".cu", ".cuh", ".h"))
-    if not srcs:
-        return None
-    if not force and not _newer(CUDA_LIB, deps):
-        return CUDA_LIB
-    nvcc = nvcc_path()
-    if nvcc is None:
-        raise RuntimeError("nvcc not found; cannot build the sm_100a kernels")
+def cuda_objects(force=False, verbose=False):
+    """Compiles the .cu files under cuda/ whose objects are older than they are; returns all objects."""
+    srcs, deps = _sources(CUDA, (".cu",)), _sources(CUDA, (".cuh", ".h"))
     objdir = os.path.join(PKG, "build")
     os.makedirs(objdir, exist_ok=True)
     objs, procs = [], []
@@ -92,7 +84,10 @@ def build_cuda(force=False, verbose=False):
     for s in srcs:
         o = os.path.join(objdir, os.path.basename(s)[:-3] + ".o")
         objs.append(o)
-        if force or _newer(o, [s] + [d for d in deps if not d.endswith(".cu")]):
+        if force or _newer(o, [s, *deps]):
+            nvcc = nvcc_path()
+            if nvcc is None:
+                raise RuntimeError("nvcc not found; cannot build the sm_100a kernels")
             cmd = [nvcc, *flags, "-c", s, "-o", o]
             if verbose:
                 print(" ".join(cmd), flush=True)
@@ -103,8 +98,21 @@ def build_cuda(force=False, verbose=False):
         log.append(out)
         if p.returncode != 0:
             raise RuntimeError(f"build failed: {' '.join(cmd)}\n{out}")
-    with open(os.path.join(objdir, "ptxas.log"), "a" if not force else "w") as f:
-        f.write("\n".join(log))
+    if log:
+        with open(os.path.join(objdir, "ptxas.log"), "a" if not force else "w") as f:
+            f.write("\n".join(log))
+    return objs
+
+
+def build_cuda(force=False, verbose=False):
+    """Links every .cu under cuda/ into one shared library for sm_100a."""
+    deps = _sources(CUDA, (".cu", ".cuh", ".h"))
+    if not force and not _newer(CUDA_LIB, deps):
+        return CUDA_LIB
+    nvcc = nvcc_path()
+    if nvcc is None:
+        raise RuntimeError("nvcc not found; cannot build the sm_100a kernels")
+    objs = cuda_objects(force, verbose)
     tmp = CUDA_LIB + f".{os.getpid()}.tmp"
     _run([nvcc, *NVCC_ARCH, "-shared", "-o", tmp, *objs], verbose)
     os.replace(tmp, CUDA_LIB)

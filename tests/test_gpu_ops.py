@@ -976,3 +976,31 @@ def test_stream_waits_of_many_threads_share_their_events():
         t.start()
         t.join()
     assert lib().tb_stream_wait_events() == before
+
+
+def test_products_and_sums_of_two_threads():
+    """Split products and column sums that two host threads launch on streams of their own equal those of one thread."""
+    import threading
+
+    from tandem_b200.ops import gemm as G
+
+    dy, x = rnd(2048, 768), rnd(2048, 384)
+    results = [[], []]
+
+    def work(mine, rounds):
+        torch.cuda.set_device(0)
+        s = torch.cuda.Stream()
+        s.wait_stream(torch.cuda.default_stream())
+        with torch.cuda.stream(s):
+            for _ in range(rounds):
+                mine.append((G._grad_weight(dy, 768, x, 384, torch.bfloat16), G._grad_bias(dy, 768)))
+        s.synchronize()
+
+    work(results[0], 1)
+    (want,) = results[0]
+    threads = [threading.Thread(target=work, args=(mine, 200)) for mine in results]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert all(torch.equal(a, b) for mine in results for got in mine for a, b in zip(got, want))

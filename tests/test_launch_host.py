@@ -1,0 +1,52 @@
+"""The host code of the kernel library without a GPU: its objects are linked against a CUDA runtime that takes launches down
+instead of executing them (native/fake_cuda.cpp)."""
+
+import ctypes
+import os
+import shutil
+import subprocess
+
+import pytest
+
+from tandem_b200.utils import build
+
+HERE = os.path.dirname(os.path.abspath(__file__))
+I, P, LL = ctypes.c_int, ctypes.c_void_p, ctypes.c_longlong
+WORK = P(1 << 20)  # an address that nothing follows, aligned
+
+
+def signatures(lib):
+    lib.tb_gemm_bf16.argtypes = [P, P, P, I, I, I, I, I, I, I, I, I, P, P, P, I, P, LL, P]
+    lib.tb_gemm_workspace_bytes.argtypes, lib.tb_gemm_workspace_bytes.restype = [I, I, I], LL
+    lib.tb_col_sum.argtypes = [P, I, I, I, P, P, P]
+    lib.tb_layernorm_bwd_add.argtypes = [P] * 10 + [I, I, P]
+    lib.tb_attn_fwd.argtypes = [P, P, P, I, I, I, I, P]
+    lib.tb_attn_bwd.argtypes = [P] * 6 + [I, I, I, I, P]
+    return lib
+
+
+@pytest.fixture(scope="module")
+def fake(tmp_path_factory):
+    if shutil.which("g++") is None or build.nvcc_path() is None:
+        pytest.skip("no compiler")
+    objs = [o for o in build.cuda_objects() if os.path.basename(o) in ("gemm.o", "layers.o", "attention.o")]
+    out = str(tmp_path_factory.mktemp("fake") / "libfake.so")
+    include = os.path.join(os.path.dirname(os.path.dirname(os.path.realpath(build.nvcc_path()))), "include")
+    # -Bsymbolic: its own runtime, not one that torch may have brought into the process
+    r = subprocess.run(["g++", "-O1", "-std=c++17", "-fPIC", "-shared", "-Wl,-Bsymbolic", "-Wl,--no-undefined", f"-I{include}",
+                        os.path.join(HERE, "native", "fake_cuda.cpp"), *objs, "-o", out, "-lpthread"], capture_output=True, text=True)
+    assert r.returncode == 0, r.stderr[-2000:]
+    return signatures(ctypes.CDLL(out))
+
+
+@pytest.mark.parametrize("products", [0, 1])
+def test_threads_never_share_words(fake, products):
+    """Tickets of column sums and flags of split products are handed out in turn, so every place of the pool is lent equally often,
+    whatever the threads' timing.  A place lent twice in a round (two launches in flight would use the same words) is missing elsewhere."""
+    out = (ctypes.c_ulonglong * 3)()  # places, lent at least, lent at most
+    fake.fake_borrowed(out)
+    threads, each = 8, 20000
+    assert fake.fake_threads(threads, each, products) == 0
+    fake.fake_borrowed(out)
+    assert out[0] > 50 and out[0] * out[1] <= threads * each <= out[0] * out[2]
+    assert out[2] - out[1] <= 1, f"{out[0]} places, lent {out[1]} to {out[2]} times"
