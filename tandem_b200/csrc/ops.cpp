@@ -96,13 +96,38 @@ Tensor empty_padded(int64_t rows, int64_t cols, const at::TensorOptions& options
   return ld == cols ? t : t.slice(1, 0, cols);
 }
 
+// The kernels take addresses and sizes: what would read beyond an operand is refused here, before a launch.
+void need(bool ok, const char* what) {
+  if (!ok) throw py::value_error(what);
+}
 void need_bf16(std::initializer_list<Tensor> tensors) {
-  for (const Tensor& t : tensors)
-    if (t.defined() && (!t.is_cuda() || t.scalar_type() != at::kBFloat16))
+  const Tensor* first = nullptr;
+  for (const Tensor& t : tensors) {
+    if (!t.defined()) continue;
+    if (!t.is_cuda() || t.scalar_type() != at::kBFloat16)
       throw py::type_error("the sm_100a operators take bf16 CUDA tensors (cast the model with .bfloat16())");
+    if (first == nullptr) first = &t;
+    need(t.device() == first->device(), "the operands lie on different devices");
+  }
+}
+void need_ids(const Tensor& ids, const Tensor& beside) {
+  if (!ids.is_cuda() || ids.scalar_type() != at::kLong) throw py::type_error("token ids and targets are int64 CUDA tensors");
+  need(ids.device() == beside.device(), "the operands lie on different devices");
+}
+// x . w^T + bias: of w's rows only their distance is free.
+void need_product(const Tensor& x, const Tensor& w, const Tensor& bias) {
+  need(x.dim() > 0 && w.dim() == 2, "a product takes an input of rows and a 2-D weight");
+  need(x.size(-1) == w.size(1), "the input's width is not the weight's");
+  need(w.stride(1) == 1 || w.size(1) == 1, "the weight's rows have to be contiguous");
+  need(!bias.defined() || bias.numel() == w.size(0), "the bias has not one value per output");
 }
 
 bool misaligned(const Tensor& t) { return reinterpret_cast<uintptr_t>(t.data_ptr()) % 16 != 0; }
+// t, or a copy of it, for kernels that read it as a run of 16-byte vectors
+Tensor vectors_of(const Tensor& t) {
+  const Tensor c = t.contiguous();
+  return misaligned(c) ? c.clone() : c;
+}
 void* data(const Tensor& t) { return t.defined() ? t.data_ptr() : nullptr; }
 
 struct Rows {
@@ -133,9 +158,11 @@ Tensor with_rows_of(const Tensor& t2, at::IntArrayRef shape, int64_t width) {
 // ---------------------------------------------------------------- products
 // out[M, N] = op(a) . op(b) (+ epilogue); out and workspace are allocated here unless given, `on` overrides the stream.
 Tensor gemm(const Tensor& a, const Tensor& b, int64_t M, int64_t N, int64_t k, int64_t lda, int64_t ldb, bool a_mn, bool b_mn, int flags,
-            const Tensor& bias, const Tensor& aux_in, const Tensor& aux_out, Tensor out = {}, Tensor workspace = {}, Stream on = nullptr) {
+            const Tensor& bias_in, Tensor aux_in, const Tensor& aux_out, Tensor out = {}, Tensor workspace = {}, Stream on = nullptr) {
   if (!out.defined()) out = empty_padded(M, N, a.options());
   const int64_t ldc = M > 1 ? out.stride(0) : pad8(N);
+  const Tensor bias = bias_in.defined() ? bias_in.contiguous() : bias_in;
+  if (aux_in.defined() && misaligned(aux_in)) aux_in = aux_in.clone();  // it is read in 16-byte vectors
   if (aux_in.defined() && M > 1 && aux_in.stride(0) != ldc) throw std::invalid_argument("aux_in must share the output's row stride");
   const long long need = K.gemm_workspace((int)M, (int)N, (int)k);
   if (need && !workspace.defined()) workspace = at::empty({need}, a.options().dtype(at::kByte));
@@ -231,12 +258,14 @@ enum { NEEDS = 0, LD = 1, SIDE = 2, SHAPE = 3 };
 struct Linear : torch::autograd::Function<Linear> {
   static Tensor run(AutogradContext* ctx, const Tensor& x, const Tensor& w, const Tensor& bias, const Tensor& residual, int64_t side_below) {
     need_bf16({x, w, bias, residual});
+    need_product(x, w, bias);
     const Rows x2 = rows_of(x);
     Tensor res2;
     if (residual.defined()) {
       res2 = residual.reshape({-1, residual.size(-1)});
       if (pad8(w.size(0)) != w.size(0) || !res2.is_contiguous())
         throw py::value_error("a fused residual needs a contiguous tensor whose width is a multiple of 8");
+      need(res2.size(0) == x2.t.size(0) && res2.size(1) == w.size(0), "the residual has not the output's shape");
     }
     const Tensor y = forward_product(x2, w, bias, residual.defined() ? RESIDUAL : 0, res2, {});
     if (ctx != nullptr) {
@@ -272,10 +301,16 @@ struct MLP : torch::autograd::Function<MLP> {
     need_bf16({x, w1, b1, w2, b2, residual});
     if (!residual.defined()) throw py::value_error("ops.mlp adds its input stream: pass the residual tensor");
     if (w1.size(0) % 8 || w2.size(0) % 8) throw py::value_error("ops.mlp needs hidden and output widths that are multiples of 8 (16-byte rows)");
+    need_product(x, w1, b1);
+    need(w2.dim() == 2 && w2.size(1) == w1.size(0), "the second weight's width is not the hidden one");
+    need(w2.stride(1) == 1 || w2.size(1) == 1, "the weight's rows have to be contiguous");
+    need(!b2.defined() || b2.numel() == w2.size(0), "the bias has not one value per output");
     const Rows x2 = rows_of(x);
+    const Tensor res2 = residual.reshape({-1, residual.size(-1)});
+    need(res2.size(0) == x2.t.size(0) && res2.size(1) == w2.size(0) && res2.stride(1) == 1, "the residual has not the output's shape");
     const Tensor slope = empty_padded(x2.t.size(0), w1.size(0), x.options());  // gelu'(W1 . x + b1), written by the same epilogue
     const Tensor h = forward_product(x2, w1, b1, GELU, {}, slope);
-    const Tensor y = forward_product({h, h.stride(0)}, w2, b2, RESIDUAL, residual.reshape({-1, residual.size(-1)}), {});
+    const Tensor y = forward_product({h, h.stride(0)}, w2, b2, RESIDUAL, res2, {});
     if (ctx != nullptr) {
       ctx->save_for_backward({x2.t, w1, w2, slope, h});
       const auto wants = [](const Tensor& t) { return t.defined() && t.requires_grad(); };
@@ -313,24 +348,26 @@ struct Normed {
 };
 Normed normalize(const Tensor& x, const Tensor& w, const Tensor& b, double eps) {
   need_bf16({x, w, b});
+  need(x.dim() > 0 && w.numel() == x.size(-1) && b.numel() == x.size(-1), "layer_norm takes a weight and a bias with one value per column");
   Normed n;
-  n.x2 = x.reshape({-1, x.size(-1)}).contiguous();
+  n.x2 = vectors_of(x.reshape({-1, x.size(-1)}));
   const int64_t M = n.x2.size(0);
   n.y = at::empty_like(n.x2);
   n.stats = at::empty({2, M}, x.options().dtype(at::kFloat));
   float* stats = (float*)data(n.stats);
-  check(K.ln_fwd(data(n.x2), data(w), data(b), data(n.y), stats, stats + M, (int)M, (int)n.x2.size(1), (float)eps, stream_of(x)),
+  const Tensor gain = vectors_of(w), shift = vectors_of(b);
+  check(K.ln_fwd(data(n.x2), data(gain), data(shift), data(n.y), stats, stats + M, (int)M, (int)n.x2.size(1), (float)eps, stream_of(x)),
         "layernorm forward");
   return n;
 }
 variable_list normalize_backward(const variable_list& saved, const Tensor& dy, const Tensor& second) {
   const Tensor &x2 = saved[0], &w = saved[1], &stats = saved[2];
   const int64_t M = x2.size(0), D = x2.size(1);
-  const Tensor dy2 = dy.reshape({-1, D}).contiguous(), add = second.defined() ? second.reshape({-1, D}).contiguous() : Tensor();
-  const Tensor dx = at::empty_like(x2), dw = at::empty_like(w), db = at::empty_like(w);
+  const Tensor dy2 = vectors_of(dy.reshape({-1, D})), add = second.defined() ? vectors_of(second.reshape({-1, D})) : Tensor(), gain = vectors_of(w);
+  const Tensor dx = at::empty_like(x2), dw = at::empty_like(w, at::MemoryFormat::Contiguous), db = at::empty_like(dw);
   const Tensor scratch = at::empty({(int64_t)K.ln_bwd_slices((int)M) * 2 * D}, x2.options().dtype(at::kFloat));
   const float* mean = (const float*)data(stats);
-  check(K.ln_bwd(data(dy2), data(x2), data(w), mean, mean + M, data(add), data(dx), data(dw), data(db), (float*)data(scratch), (int)M, (int)D,
+  check(K.ln_bwd(data(dy2), data(x2), data(gain), mean, mean + M, data(add), data(dx), data(dw), data(db), (float*)data(scratch), (int)M, (int)D,
                  stream_of(x2)),
         "layernorm backward");
   return {dx.view(dy.sizes()), dw, db, Tensor()};
@@ -367,6 +404,7 @@ struct CausalAttention : torch::autograd::Function<CausalAttention> {
     if (T % 128 || (hd != 64 && hd != 128))
       throw py::value_error("causal_attention kernels need T % 128 == 0 and head dim 64 or 128 (got T=" + std::to_string(T) + ", head dim " +
                             std::to_string(hd) + ")");
+    need(qkv_in.size(2) == 3 * heads * hd, "causal_attention takes queries, keys and values of heads * head dim columns each");
     const Tensor qkv = qkv_in.contiguous();
     const Tensor out = at::empty({B, T, d}, qkv.options()), lse = at::empty({B, heads, T}, qkv.options().dtype(at::kFloat));
     check(K.attn_fwd(data(qkv), data(out), (float*)data(lse), (int)B, (int)T, (int)heads, (int)hd, stream_of(qkv)), "attention forward");
@@ -392,10 +430,13 @@ struct Embedding : torch::autograd::Function<Embedding> {
   static Tensor forward(AutogradContext* ctx, const Tensor& idx_in, const Tensor& tok, const Tensor& pos) {
     need_bf16({tok, pos});
     if (idx_in.dim() != 2) throw py::value_error("embedding takes [batch, time] token ids");
+    need_ids(idx_in, tok);
+    need(tok.dim() == 2 && pos.dim() == 2 && tok.size(1) == pos.size(1), "embedding takes two 2-D tables of one width");
+    need(idx_in.size(1) <= pos.size(0), "more positions than the table has rows");
     const int64_t B = idx_in.size(0), T = idx_in.size(1), D = tok.size(1);
-    const Tensor idx = idx_in.contiguous();
+    const Tensor idx = idx_in.contiguous(), tokens = vectors_of(tok), positions = vectors_of(pos);
     const Tensor out = at::empty({B, T, D}, tok.options());
-    check(K.embed_fwd((const long long*)data(idx), data(tok), data(pos), data(out), (int)(B * T), (int)T, (int)D, stream_of(tok)), "embedding forward");
+    check(K.embed_fwd((const long long*)data(idx), data(tokens), data(positions), data(out), (int)(B * T), (int)T, (int)D, stream_of(tok)), "embedding forward");
     if (ctx != nullptr) {
       ctx->save_for_backward({idx});
       ctx->saved_data["sizes"] = std::vector<int64_t>{tok.size(0), D, pos.size(0)};
@@ -406,8 +447,7 @@ struct Embedding : torch::autograd::Function<Embedding> {
     const Tensor idx = ctx->get_saved_variables()[0];
     const std::vector<int64_t> sizes = ctx->saved_data["sizes"].toIntVector();
     const int64_t B = idx.size(0), T = idx.size(1), V = sizes[0], D = sizes[1], S = sizes[2];
-    Tensor dy = grads[0].contiguous();
-    if (misaligned(dy)) dy = dy.clone();  // a contiguous slice may start anywhere; the kernels read 16-byte vectors
+    const Tensor dy = vectors_of(grads[0]);
     const auto bf16 = dy.options().dtype(at::kBFloat16);
     const Tensor dtok32 = at::zeros({V, D}, dy.options().dtype(at::kFloat)), dtok = at::empty({V, D}, bf16), dpos = at::zeros({S, D}, bf16);
     check(K.embed_bwd((const long long*)data(idx), data(dy), (float*)data(dtok32), data(dtok), data(dpos), (int)B, (int)T, (int)D, (int)V,
@@ -421,8 +461,11 @@ struct CrossEntropy : torch::autograd::Function<CrossEntropy> {
   static Tensor forward(AutogradContext* ctx, const Tensor& logits_in, const Tensor& targets_in) {
     need_bf16({logits_in});
     if (logits_in.dim() != 2) throw py::value_error("cross_entropy takes [rows, vocab] logits");
+    need_ids(targets_in, logits_in);
     const int64_t rows = logits_in.size(0), V = logits_in.size(1);
-    const Tensor logits = logits_in.stride(1) != 1 ? logits_in.contiguous() : logits_in;
+    need(targets_in.numel() == rows, "cross_entropy takes one target per row");
+    // backward writes the rows where they lie: none may share memory with another
+    const Tensor logits = logits_in.stride(1) != 1 || (rows > 1 && logits_in.stride(0) < V) ? logits_in.contiguous() : logits_in;
     const int64_t ld = rows > 1 ? logits.stride(0) : V;
     const Tensor targets = targets_in.contiguous();
     const auto f32 = logits.options().dtype(at::kFloat);

@@ -121,7 +121,38 @@ def empty_padded(rows, cols, dtype, device):
     return torch.empty(rows, ld, dtype=dtype, device=device)[:, :cols]
 
 
+# The kernels take addresses and sizes: what would read beyond an operand is refused here, before a launch.
+def need(ok, what):
+    if not ok:
+        raise ValueError(what)
+
+
 def need_bf16(*tensors):
+    first = None
     for t in tensors:
-        if t is not None and (not t.is_cuda or t.dtype != torch.bfloat16):
+        if t is None:
+            continue
+        if not t.is_cuda or t.dtype != torch.bfloat16:
             raise TypeError("the sm_100a operators take bf16 CUDA tensors (cast the model with .bfloat16())")
+        first = t if first is None else first
+        need(t.device == first.device, "the operands lie on different devices")
+
+
+def need_ids(ids, beside):
+    if not ids.is_cuda or ids.dtype != torch.int64:
+        raise TypeError("token ids and targets are int64 CUDA tensors")
+    need(ids.device == beside.device, "the operands lie on different devices")
+
+
+def need_product(x, w, bias):
+    """x . w^T + bias: of w's rows only their distance is free."""
+    need(x.dim() > 0 and w.dim() == 2, "a product takes an input of rows and a 2-D weight")
+    need(x.shape[-1] == w.shape[1], "the input's width is not the weight's")
+    need(w.stride(1) == 1 or w.shape[1] == 1, "the weight's rows have to be contiguous")
+    need(bias is None or bias.numel() == w.shape[0], "the bias has not one value per output")
+
+
+def vectors_of(t):
+    """t, or a copy of it, for kernels that read it as a run of 16-byte vectors."""
+    t = t.contiguous()
+    return t.clone() if t.data_ptr() % 16 else t

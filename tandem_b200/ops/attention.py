@@ -11,7 +11,7 @@ import functools
 
 import torch
 
-from ._lib import check_rc, direct, lib, need_bf16, run, stream
+from ._lib import check_rc, direct, lib, need, need_bf16, run, stream
 
 
 @functools.cache
@@ -36,6 +36,7 @@ class _CausalAttention(torch.autograd.Function):
         hd = d // heads
         if T % 128 or hd not in (64, 128):
             raise ValueError(f"causal_attention kernels need T % 128 == 0 and head dim 64 or 128 (got T={T}, head dim {hd})")
+        need(d3 == 3 * heads * hd, "causal_attention takes queries, keys and values of heads * head dim columns each")
         qkv = qkv.contiguous()
         out = torch.empty(B, T, d, dtype=torch.bfloat16, device=qkv.device)
         lse = torch.empty(B, heads, T, dtype=torch.float32, device=qkv.device)

@@ -4,7 +4,7 @@ fixed order (tandem_b200/cuda/layers.cu)."""
 
 import torch
 
-from ._lib import check_rc, direct, lib, need_bf16, run, stream
+from ._lib import check_rc, direct, lib, need, need_bf16, need_ids, run, stream, vectors_of
 
 
 class _Embedding(torch.autograd.Function):
@@ -12,10 +12,13 @@ class _Embedding(torch.autograd.Function):
     def forward(ctx, idx, tok, pos):
         need_bf16(tok, pos)
         B, T = idx.shape
+        need_ids(idx, tok)
+        need(tok.dim() == 2 and pos.dim() == 2 and tok.shape[1] == pos.shape[1], "embedding takes two 2-D tables of one width")
+        need(T <= pos.shape[0], "more positions than the table has rows")
         D = tok.shape[1]
-        idx = idx.contiguous()
+        idx, tokens, positions = idx.contiguous(), vectors_of(tok), vectors_of(pos)
         out = torch.empty(B, T, D, dtype=torch.bfloat16, device=tok.device)
-        check_rc(lib().tb_embed_fwd(idx.data_ptr(), tok.data_ptr(), pos.data_ptr(), out.data_ptr(), B * T, T, D, stream(tok)),
+        check_rc(lib().tb_embed_fwd(idx.data_ptr(), tokens.data_ptr(), positions.data_ptr(), out.data_ptr(), B * T, T, D, stream(tok)),
                  "embedding forward")
         ctx.save_for_backward(idx)
         ctx.shapes = (tok.shape, pos.shape)
@@ -26,9 +29,7 @@ class _Embedding(torch.autograd.Function):
         (idx,) = ctx.saved_tensors
         (V, D), (S, _) = ctx.shapes
         B, T = idx.shape
-        dy = dy.contiguous()
-        if dy.data_ptr() % 16:  # a contiguous slice may start anywhere; the kernels read 16-byte vectors
-            dy = dy.clone()
+        dy = vectors_of(dy)
         dtok32 = torch.zeros(V, D, dtype=torch.float32, device=dy.device)
         dtok = torch.empty(V, D, dtype=torch.bfloat16, device=dy.device)
         dpos = torch.zeros(S, D, dtype=torch.bfloat16, device=dy.device)

@@ -11,7 +11,7 @@ import os
 
 import torch
 
-from ._lib import check_rc, direct, empty_padded, lib, need_bf16, pad8, run, stream, stream_wait
+from ._lib import check_rc, direct, empty_padded, lib, need, need_bf16, need_product, pad8, run, stream, stream_wait
 
 BIAS, GELU, RESIDUAL, DGELU, ACCUMULATE, OUT_F32 = 1, 2, 4, 8, 16, 32
 
@@ -38,6 +38,10 @@ def gemm(a, b, M, N, K, lda, ldb, a_mn, b_mn, flags=0, bias=None, aux_in=None, a
     if out is None:
         out = empty_padded(M, N, out_dtype, a.device)
     ldc = out.stride(0) if M > 1 else pad8(N)
+    if bias is not None:
+        bias = bias.contiguous()
+    if aux_in is not None and aux_in.data_ptr() % 16:  # it is read in 16-byte vectors
+        aux_in = aux_in.clone()
     if aux_in is not None and (aux_in.stride(0) if M > 1 else ldc) != ldc:
         raise ValueError("aux_in must share the output's row stride")
     if out.dtype == torch.float32:
@@ -154,6 +158,7 @@ class _Linear(torch.autograd.Function):
     @staticmethod
     def forward(ctx, x, w, bias, residual):
         need_bf16(x, w, bias, residual)
+        need_product(x, w, bias)
         x2, ldx = _rows(x)
         fused = GATHERED.pop(w.data_ptr(), None) if GATHERED and residual is None else None
         if fused is not None:
@@ -170,6 +175,7 @@ class _Linear(torch.autograd.Function):
             res2 = residual.reshape(-1, residual.shape[-1])
             if pad8(w.shape[0]) != w.shape[0] or not res2.is_contiguous():
                 raise ValueError("a fused residual needs a contiguous tensor whose width is a multiple of 8")
+            need(res2.shape == (x2.shape[0], w.shape[0]), "the residual has not the output's shape")
         y = _forward(x2, ldx, w, bias, RESIDUAL if res2 is not None else 0, res2)
         ctx.save_for_backward(x2, w)
         ctx.ldx, ctx.has_bias, ctx.has_res = ldx, bias is not None, residual is not None
@@ -202,11 +208,16 @@ class _MLP(torch.autograd.Function):
             raise ValueError("ops.mlp adds its input stream: pass the residual tensor")
         if w1.shape[0] % 8 or w2.shape[0] % 8:
             raise ValueError("ops.mlp needs hidden and output widths that are multiples of 8 (16-byte rows)")
+        need_product(x, w1, b1)
+        need(w2.dim() == 2 and w2.shape[1] == w1.shape[0], "the second weight's width is not the hidden one")
+        need(w2.stride(1) == 1 or w2.shape[1] == 1, "the weight's rows have to be contiguous")
+        need(b2 is None or b2.numel() == w2.shape[0], "the bias has not one value per output")
         x2, ldx = _rows(x)
         M = x2.shape[0]
+        res2 = residual.reshape(-1, residual.shape[-1])
+        need(res2.shape == (M, w2.shape[0]) and res2.stride(1) == 1, "the residual has not the output's shape")
         slope = empty_padded(M, w1.shape[0], torch.bfloat16, x.device)  # gelu'(W1 . x + b1), written by the same epilogue
         h = _forward(x2, ldx, w1, b1, GELU, None, slope)
-        res2 = residual.reshape(-1, residual.shape[-1])
         y = _forward(h, h.stride(0), w2, b2, RESIDUAL, res2)
         ctx.save_for_backward(x2, w1, w2, slope, h)
         ctx.ldx, ctx.in_shape = ldx, x.shape

@@ -5,7 +5,7 @@ tensor is ever allocated (tandem_b200/cuda/layers.cu)."""
 
 import torch
 
-from ._lib import check_rc, direct, lib, need_bf16, run, stream
+from ._lib import check_rc, direct, lib, need, need_bf16, need_ids, run, stream
 
 
 class _CrossEntropy(torch.autograd.Function):
@@ -13,7 +13,10 @@ class _CrossEntropy(torch.autograd.Function):
     def forward(ctx, logits, targets):
         need_bf16(logits)
         rows, V = logits.shape
-        if logits.stride(1) != 1:
+        need_ids(targets, logits)
+        need(targets.numel() == rows, "cross_entropy takes one target per row")
+        # backward writes the rows where they lie: none may share memory with another
+        if logits.stride(1) != 1 or (rows > 1 and logits.stride(0) < V):
             logits = logits.contiguous()
         ld = logits.stride(0) if rows > 1 else V
         targets = targets.contiguous()

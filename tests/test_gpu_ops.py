@@ -2,6 +2,8 @@
 computed from the same bf16 inputs.  Tolerances are those of one bf16 rounding of
 the output (2^-8 relative) plus fp32 accumulation-order noise."""
 
+import math
+
 import pytest
 import torch
 
@@ -829,8 +831,18 @@ def _operator_forms():
     for name, x in {"columns": wide[:, 64:128], "odd columns": wide[:, 3:67], "transposed": leaf(64, 40).t(), "every other row": leaf(80, 64)[::2],
                     "swapped": leaf(5, 6, 64).transpose(0, 1), "expanded": leaf(1, 64).expand(40, 64), "offset": leaf(40 * 64 + 1)[1:].view(40, 64)}.items():
         forms[f"linear of {name}"] = (ops.linear, [x, leaf(96, 64), leaf(96)], [1, 1, 1])
-        if name not in ("odd columns", "offset"):  # the LayerNorm kernels read 16-byte vectors of a contiguous input where it lies
-            forms[f"layer_norm of {name}"] = (ops.layer_norm, [x, leaf(64), leaf(64)], [1, 1, 1])
+        forms[f"layer_norm of {name}"] = (ops.layer_norm, [x, leaf(64), leaf(64)], [1, 1, 1])
+    def offset(*shape):  # contiguous, and not on a 16-byte boundary
+        return leaf(math.prod(shape) + 1)[1:].view(*shape)
+
+    x, w, r, every_other, expanded = leaf(40, 64), leaf(96, 64), offset(40, 96), leaf(192)[::2], leaf(1).expand(96)
+    for name, b in {"every other": every_other, "expanded": expanded, "offset": offset(96)}.items():
+        forms[f"linear with {name} bias"] = (ops.linear, [x, w, b], [1, 1, 1])
+        forms[f"layer_norm with {name} weight"] = (ops.layer_norm, [leaf(40, 96), b, leaf(96)], [1, 1, 1])
+        forms[f"layer_norm with {name} bias"] = (ops.layer_norm, [leaf(40, 96), leaf(96), b], [1, 1, 1])
+    forms["linear with offset residual"] = (lambda x, w, b, r: ops.linear(x, w, b, residual=r), [x, w, leaf(96), r], [1, 1, 1, 1])
+    forms["mlp with offset residual"] = (ops.mlp, [x, leaf(128, 64), leaf(128), leaf(96, 128), leaf(96), r], [1] * 6)
+    forms["residual_layer_norm of offset"] = (ops.residual_layer_norm, [r, leaf(96), leaf(96)], [1, 1, 1])
     for rows in [(1,), (2, 77), (4100,)]:
         x, r = leaf(*rows, 72), leaf(*rows, 40)
         forms[f"mlp {rows}"] = (ops.mlp, [x, leaf(96, 72), leaf(96), leaf(40, 96), leaf(40), r], [1] * 6)
@@ -842,10 +854,12 @@ def _operator_forms():
     forms["attention of a slice"] = (lambda q: ops.causal_attention(q, 2), [leaf(2, 128, 2 * 384)[:, :, :384]], [1])
     idx = torch.randperm(60, device="cuda")[:2 * 20].view(2, 20)
     forms["embedding"] = (lambda t, p: ops.embedding(idx, t, p), [leaf(60, 40), leaf(32, 40)], [1, 1])
+    forms["embedding in views"] = (lambda t, p: ops.embedding(idx, t, p), [leaf(60, 48)[:, 8:48], offset(32, 40)], [1, 1])
     forms["embedding of transposed ids"] = (lambda t, p: ops.embedding(idx.t(), t, p), [leaf(60, 40), leaf(32, 40)], [1, 1])
     for V, ld in [(65, 72), (65, 65), (1003, 1008), (64, 200)]:
         forms[f"cross_entropy {V} {ld}"] = (lambda z: ops.cross_entropy(z * 1.0 if z.stride(0) == z.shape[1] else z, torch.arange(30, device="cuda") % V),
                                             [leaf(30, ld)[:, :V]], [1])
+    forms["cross_entropy of one row for all"] = (lambda z: ops.cross_entropy(z, torch.arange(30, device="cuda")), [leaf(1, 64).expand(30, 64)], [1])
     return forms
 
 
@@ -905,6 +919,30 @@ def test_native_operators_equal_the_python_ones(monkeypatch):
     native = [refusal(call) for call in refused]
     monkeypatch.setattr(_lib, "native", lambda: None)
     assert native == [refusal(call) for call in refused] and None not in native
+
+
+@pytest.mark.parametrize("python", [False, True])
+def test_operators_of_views_equal_those_of_copies(python, monkeypatch):
+    """What the kernels cannot read where it lies is copied: strides, offsets and expanded operands change no bit."""
+    from tandem_b200.ops import _lib
+
+    if python:
+        monkeypatch.setattr(_lib, "native", lambda: None)
+    torch.manual_seed(0)
+
+    def outcome(function, inputs, needs):
+        inputs = [t if t is None or not n else t.detach().requires_grad_() for t, n in zip(inputs, needs)]
+        out = function(*inputs)
+        outs = out if isinstance(out, tuple) else (out,)
+        torch.manual_seed(1)
+        return [o.detach().clone() for o in outs] + list(torch.autograd.grad(outs, [t for t, n in zip(inputs, needs) if n], [torch.randn_like(o) for o in outs]))
+
+    for name, (function, inputs, needs) in _operator_forms().items():
+        copies = [None if t is None else t.clone(memory_format=torch.contiguous_format) for t in inputs]
+        if name.startswith("linear"):
+            copies[1] = inputs[1]  # a weight has to have 16-byte rows, which an odd width takes padding for
+        for a, b in zip(outcome(function, inputs, needs), outcome(function, copies, needs)):
+            assert torch.equal(a, b), name
 
 
 @pytest.mark.parametrize("python", [False, True])

@@ -68,3 +68,59 @@ def test_torch_without_an_undocumented_name(missing, monkeypatch):
             assert not Probe.bare
     again.run(Probe, x)
     assert not Probe.bare
+
+
+def refused_calls(make, ids):
+    """Calls whose operands do not fit together, or are not what the kernels read.  make(*shape) -> a bf16 tensor, ids(*shape) -> int64 zeros."""
+    from tandem_b200 import ops
+
+    x, w, b, r = make(40, 64), make(96, 64), make(96), make(40, 96)
+    table, positions, text = make(50, 64), make(32, 64), ids(2, 16)
+    return {
+        "linear: wider input": (ValueError, lambda: ops.linear(make(40, 72), w, b)),
+        "linear: narrower input": (ValueError, lambda: ops.linear(make(40, 56), w, b)),
+        "linear: transposed weight": (ValueError, lambda: ops.linear(x, make(64, 96).t(), b)),
+        "linear: 1-D weight": (ValueError, lambda: ops.linear(x, make(64), b)),
+        "linear: short bias": (ValueError, lambda: ops.linear(x, w, make(88))),
+        "linear: long bias": (ValueError, lambda: ops.linear(x, w, make(104))),
+        "linear: residual of one row": (ValueError, lambda: ops.linear(x, w, b, residual=make(1, 96))),
+        "linear: narrow residual": (ValueError, lambda: ops.linear(x, w, b, residual=make(40, 88))),
+        "mlp: wider input": (ValueError, lambda: ops.mlp(make(40, 72), w, b, make(64, 96), make(64), x)),
+        "mlp: second weight": (ValueError, lambda: ops.mlp(x, w, b, make(64, 88), make(64), x)),
+        "mlp: first bias": (ValueError, lambda: ops.mlp(x, w, make(88), make(64, 96), make(64), x)),
+        "mlp: second bias": (ValueError, lambda: ops.mlp(x, w, b, make(64, 96), make(56), x)),
+        "mlp: residual of one row": (ValueError, lambda: ops.mlp(x, w, b, make(64, 96), make(64), make(1, 64))),
+        "mlp: wide residual": (ValueError, lambda: ops.mlp(x, w, b, make(64, 96), make(64), r)),
+        "layer_norm: short weight": (ValueError, lambda: ops.layer_norm(x, make(56), make(64))),
+        "layer_norm: short bias": (ValueError, lambda: ops.layer_norm(x, make(64), make(56))),
+        "residual_layer_norm: short weight": (ValueError, lambda: ops.residual_layer_norm(x, make(56), make(64))),
+        "attention: columns left over": (ValueError, lambda: ops.causal_attention(make(1, 128, 385), 2)),
+        "embedding: 32-bit ids": (TypeError, lambda: ops.embedding(text.int(), table, positions)),
+        "embedding: host ids": (TypeError, lambda: ops.embedding(torch.zeros(2, 16, dtype=torch.int64), table, positions)),
+        "embedding: positions": (ValueError, lambda: ops.embedding(ids(2, 33), table, positions)),
+        "embedding: widths": (ValueError, lambda: ops.embedding(text, table, make(32, 56))),
+        "embedding: 1-D table": (ValueError, lambda: ops.embedding(text, table, make(64))),
+        "cross_entropy: 32-bit targets": (TypeError, lambda: ops.cross_entropy(r, ids(40).int())),
+        "cross_entropy: host targets": (TypeError, lambda: ops.cross_entropy(r, torch.zeros(40, dtype=torch.int64))),
+        "cross_entropy: too few targets": (ValueError, lambda: ops.cross_entropy(r, ids(39))),
+        "cross_entropy: too many targets": (ValueError, lambda: ops.cross_entropy(r, ids(41))),
+    }
+
+
+@pytest.mark.parametrize("native", [True, False])
+def test_operands_that_do_not_fit_are_refused(native, monkeypatch):
+    """On tensors that only have the shape of CUDA tensors, so that nothing could be launched."""
+    from torch._subclasses.fake_tensor import FakeTensorMode
+
+    if native and _lib.native() is None:
+        pytest.skip("the native operators are not built")
+    if not native:
+        monkeypatch.setattr(_lib, "native", lambda: None)
+    with FakeTensorMode(allow_non_fake_inputs=True):
+        assert (_lib.direct(torch.empty(2, device="cuda")) is not None) == native
+        calls = refused_calls(lambda *shape: torch.empty(*shape, dtype=torch.bfloat16, device="cuda"),
+                              lambda *shape: torch.zeros(*shape, dtype=torch.int64, device="cuda"))
+        for name, (kind, call) in calls.items():
+            with pytest.raises(kind) as e:
+                call()
+            assert type(e.value) is kind, name
