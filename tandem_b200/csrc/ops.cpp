@@ -181,8 +181,8 @@ Tensor forward_product(const Rows& x, const Tensor& w, const Tensor& bias, int f
 }
 
 // dX[M, K] = dY[M, N] . W[N, K]
-Tensor grad_input(const Rows& dy, const Tensor& w, int flags = 0, const Tensor& aux_in = {}) {
-  return gemm(dy.t, w, dy.t.size(0), w.size(1), dy.t.size(1), dy.ld, w.stride(0), false, true, flags, {}, aux_in, {});
+Tensor grad_input(const Rows& dy, const Rows& w, int flags = 0, const Tensor& aux_in = {}) {
+  return gemm(dy.t, w.t, dy.t.size(0), w.t.size(1), dy.t.size(1), dy.ld, w.ld, false, true, flags, {}, aux_in, {});
 }
 
 // dW[N, K] = dY[M, N]^T . X[M, K]
@@ -252,8 +252,8 @@ struct ParameterGrads {
 Tensor undefined_if_none(const std::optional<Tensor>& t) { return t.has_value() ? *t : Tensor(); }
 
 // ---------------------------------------------------------------- functions
-// What backward needs beside the saved tensors.
-enum { NEEDS = 0, LD = 1, SIDE = 2, SHAPE = 3 };
+// What backward needs beside the saved tensors.  Not their strides: a saved-tensor hook may answer with others (save_on_cpu does).
+enum { NEEDS = 0, SIDE = 1, SHAPE = 2 };
 
 struct Linear : torch::autograd::Function<Linear> {
   static Tensor run(AutogradContext* ctx, const Tensor& x, const Tensor& w, const Tensor& bias, const Tensor& residual, int64_t side_below) {
@@ -271,7 +271,7 @@ struct Linear : torch::autograd::Function<Linear> {
     if (ctx != nullptr) {
       ctx->save_for_backward({x2.t, w});
       const auto wants = [](const Tensor& t) { return t.defined() && t.requires_grad(); };
-      std::vector<int64_t> keep{wants(x) | wants(w) << 1 | wants(bias) << 2 | wants(residual) << 3, x2.ld, side_below};
+      std::vector<int64_t> keep{wants(x) | wants(w) << 1 | wants(bias) << 2 | wants(residual) << 3, side_below};
       keep.insert(keep.end(), x.sizes().begin(), x.sizes().end());
       ctx->saved_data["keep"] = std::move(keep);
     }
@@ -284,12 +284,10 @@ struct Linear : torch::autograd::Function<Linear> {
   static variable_list backward(AutogradContext* ctx, variable_list grads) {
     const auto saved = ctx->get_saved_variables();
     const std::vector<int64_t> keep = ctx->saved_data["keep"].toIntVector();
-    const Rows x{saved[0], keep[LD]};
-    const Tensor& w = saved[1];
-    const Rows dy = rows_of(grads[0]);
+    const Rows x = rows_of(saved[0]), w = rows_of(saved[1]), dy = rows_of(grads[0]);
     ParameterGrads parameters(dy, x, keep[NEEDS] & 2, keep[NEEDS] & 4, keep[SIDE]);
     Tensor dx;
-    if (keep[NEEDS] & 1) dx = with_rows_of(grad_input(dy, w), at::IntArrayRef(keep).slice(SHAPE), w.size(1));
+    if (keep[NEEDS] & 1) dx = with_rows_of(grad_input(dy, w), at::IntArrayRef(keep).slice(SHAPE), w.t.size(1));
     parameters.join();
     return {dx, parameters.dw, parameters.db, keep[NEEDS] & 8 ? grads[0] : Tensor(), Tensor()};
   }
@@ -314,7 +312,7 @@ struct MLP : torch::autograd::Function<MLP> {
     if (ctx != nullptr) {
       ctx->save_for_backward({x2.t, w1, w2, slope, h});
       const auto wants = [](const Tensor& t) { return t.defined() && t.requires_grad(); };
-      std::vector<int64_t> keep{wants(x) | wants(w1) << 1 | wants(b1) << 2 | wants(w2) << 3 | wants(b2) << 4 | wants(residual) << 5, x2.ld, side_below};
+      std::vector<int64_t> keep{wants(x) | wants(w1) << 1 | wants(b1) << 2 | wants(w2) << 3 | wants(b2) << 4 | wants(residual) << 5, side_below};
       keep.insert(keep.end(), x.sizes().begin(), x.sizes().end());
       ctx->saved_data["keep"] = std::move(keep);
     }
@@ -328,15 +326,15 @@ struct MLP : torch::autograd::Function<MLP> {
     const auto saved = ctx->get_saved_variables();
     const std::vector<int64_t> keep = ctx->saved_data["keep"].toIntVector();
     const int64_t needs = keep[NEEDS];
-    const Tensor &w1 = saved[1], &w2 = saved[2], &slope = saved[3], &h = saved[4];
-    const Rows x{saved[0], keep[LD]}, hidden{h, h.stride(0)}, dy = rows_of(grads[0]);
+    const Rows x = rows_of(saved[0]), w1 = rows_of(saved[1]), w2 = rows_of(saved[2]), hidden = rows_of(saved[4]), dy = rows_of(grads[0]);
+    const Tensor slope = saved[3].contiguous();
     ParameterGrads second(dy, hidden, needs & 8, needs & 16, keep[SIDE]);
     const Tensor dpre = grad_input(dy, w2, DGELU, slope);  // (dY . W2) * gelu'(pre)
     second.join();
     const Rows pre{dpre, dpre.stride(0)};
     ParameterGrads first(pre, x, needs & 2, needs & 4, keep[SIDE]);
     Tensor dx;
-    if (needs & 1) dx = with_rows_of(grad_input(pre, w1), at::IntArrayRef(keep).slice(SHAPE), w1.size(1));
+    if (needs & 1) dx = with_rows_of(grad_input(pre, w1), at::IntArrayRef(keep).slice(SHAPE), w1.t.size(1));
     first.join();
     return {dx, first.dw, first.db, second.dw, second.db, needs & 32 ? grads[0] : Tensor(), Tensor()};
   }
@@ -361,7 +359,7 @@ Normed normalize(const Tensor& x, const Tensor& w, const Tensor& b, double eps) 
   return n;
 }
 variable_list normalize_backward(const variable_list& saved, const Tensor& dy, const Tensor& second) {
-  const Tensor &x2 = saved[0], &w = saved[1], &stats = saved[2];
+  const Tensor x2 = vectors_of(saved[0]), w = saved[1], stats = saved[2].contiguous();
   const int64_t M = x2.size(0), D = x2.size(1);
   const Tensor dy2 = vectors_of(dy.reshape({-1, D})), add = second.defined() ? vectors_of(second.reshape({-1, D})) : Tensor(), gain = vectors_of(w);
   const Tensor dx = at::empty_like(x2), dw = at::empty_like(w, at::MemoryFormat::Contiguous), db = at::empty_like(dw);
@@ -416,9 +414,9 @@ struct CausalAttention : torch::autograd::Function<CausalAttention> {
   }
   static variable_list backward(AutogradContext* ctx, variable_list grads) {
     const auto saved = ctx->get_saved_variables();
-    const Tensor &qkv = saved[0], &out = saved[1], &lse = saved[2];
+    const Tensor qkv = vectors_of(saved[0]), out = vectors_of(saved[1]), lse = vectors_of(saved[2]);
     const int64_t B = qkv.size(0), T = qkv.size(1), d = qkv.size(2) / 3, heads = ctx->saved_data["heads"].toInt();
-    const Tensor d_out = grads[0].contiguous(), dqkv = at::empty_like(qkv), delta = at::empty({B * heads * T}, qkv.options().dtype(at::kFloat));
+    const Tensor d_out = vectors_of(grads[0]), dqkv = at::empty_like(qkv), delta = at::empty({B * heads * T}, qkv.options().dtype(at::kFloat));
     check(K.attn_bwd(data(qkv), data(out), data(d_out), (const float*)data(lse), data(dqkv), (float*)data(delta), (int)B, (int)T, (int)heads,
                      (int)(d / heads), stream_of(qkv)),
           "attention backward");
@@ -444,7 +442,7 @@ struct Embedding : torch::autograd::Function<Embedding> {
     return out;
   }
   static variable_list backward(AutogradContext* ctx, variable_list grads) {
-    const Tensor idx = ctx->get_saved_variables()[0];
+    const Tensor idx = ctx->get_saved_variables()[0].contiguous();
     const std::vector<int64_t> sizes = ctx->saved_data["sizes"].toIntVector();
     const int64_t B = idx.size(0), T = idx.size(1), V = sizes[0], D = sizes[1], S = sizes[2];
     const Tensor dy = vectors_of(grads[0]);
@@ -457,6 +455,9 @@ struct Embedding : torch::autograd::Function<Embedding> {
   }
 };
 
+// Backward writes rows of logits where they lie: none may share memory with another.
+Tensor rows_apart(const Tensor& t) { return t.stride(1) != 1 || (t.size(0) > 1 && t.stride(0) < t.size(1)) ? t.contiguous() : t; }
+
 struct CrossEntropy : torch::autograd::Function<CrossEntropy> {
   static Tensor forward(AutogradContext* ctx, const Tensor& logits_in, const Tensor& targets_in) {
     need_bf16({logits_in});
@@ -464,8 +465,7 @@ struct CrossEntropy : torch::autograd::Function<CrossEntropy> {
     need_ids(targets_in, logits_in);
     const int64_t rows = logits_in.size(0), V = logits_in.size(1);
     need(targets_in.numel() == rows, "cross_entropy takes one target per row");
-    // backward writes the rows where they lie: none may share memory with another
-    const Tensor logits = logits_in.stride(1) != 1 || (rows > 1 && logits_in.stride(0) < V) ? logits_in.contiguous() : logits_in;
+    const Tensor logits = rows_apart(logits_in);
     const int64_t ld = rows > 1 ? logits.stride(0) : V;
     const Tensor targets = targets_in.contiguous();
     const auto f32 = logits.options().dtype(at::kFloat);
@@ -473,16 +473,13 @@ struct CrossEntropy : torch::autograd::Function<CrossEntropy> {
     check(K.xent_fwd(data(logits), (const long long*)data(targets), (float*)data(lse), (float*)data(row_loss), (float*)data(loss), (int)rows, (int)V,
                      (int)ld, stream_of(logits)),
           "cross-entropy forward");
-    if (ctx != nullptr) {
-      ctx->save_for_backward({logits, targets, lse});
-      ctx->saved_data["ld"] = ld;
-    }
+    if (ctx != nullptr) ctx->save_for_backward({logits, targets, lse});
     return loss;
   }
   static variable_list backward(AutogradContext* ctx, variable_list grads) {
     const auto saved = ctx->get_saved_variables();
-    const Tensor &logits = saved[0], &targets = saved[1], &lse = saved[2];
-    const int64_t rows = logits.size(0), V = logits.size(1), ld = ctx->saved_data["ld"].toInt();
+    const Tensor logits = rows_apart(saved[0]), targets = saved[1].contiguous(), lse = saved[2].contiguous();
+    const int64_t rows = logits.size(0), V = logits.size(1), ld = rows > 1 ? logits.stride(0) : V;
     const Tensor scale = grads[0].detach().reshape({1}).to(at::kFloat).contiguous();
     // In place: the saved logits become their own gradient (they are not needed again).  The columns [V, ld) of a row are cleared
     // too when they belong to this tensor's storage (a padded allocation).

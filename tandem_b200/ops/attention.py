@@ -11,7 +11,7 @@ import functools
 
 import torch
 
-from ._lib import check_rc, direct, lib, need, need_bf16, run, stream
+from ._lib import check_rc, direct, lib, need, need_bf16, run, stream, vectors_of
 
 
 @functools.cache
@@ -47,11 +47,11 @@ class _CausalAttention(torch.autograd.Function):
 
     @staticmethod
     def backward(ctx, d_out):
-        qkv, out, lse = ctx.saved_tensors
+        qkv, out, lse = map(vectors_of, ctx.saved_tensors)  # a saved-tensor hook may answer with other strides
         B, T, d3 = qkv.shape
         d = d3 // 3
         heads = ctx.heads
-        d_out = d_out.contiguous()
+        d_out = vectors_of(d_out)
         dqkv = torch.empty_like(qkv)
         delta = torch.empty(B * heads * T, dtype=torch.float32, device=qkv.device)
         check_rc(_fns().tb_attn_bwd(qkv.data_ptr(), out.data_ptr(), d_out.data_ptr(), lse.data_ptr(), dqkv.data_ptr(), delta.data_ptr(),

@@ -26,7 +26,7 @@ class _Embedding(torch.autograd.Function):
 
     @staticmethod
     def backward(ctx, dy):
-        (idx,) = ctx.saved_tensors
+        idx = ctx.saved_tensors[0].contiguous()
         (V, D), (S, _) = ctx.shapes
         B, T = idx.shape
         dy = vectors_of(dy)

@@ -73,11 +73,11 @@ def _forward(x2, ldx, w, bias, flags, aux_in=None, aux_out=None):
     return gemm(x2, w, M, N, K, ldx, w.stride(0), False, False, flags, bias, aux_in, aux_out)
 
 
-def _grad_input(dy2, ldy, w, flags=0, aux_in=None):
+def _grad_input(dy2, ldy, w, ldw, flags=0, aux_in=None):
     """dX[M, K] = dY[M, N] . W[N, K]   (reduction over N; W read as an MN-major operand)"""
     M, N = dy2.shape
     K = w.shape[1]
-    return gemm(dy2, w, M, K, N, ldy, w.stride(0), False, True, flags, None, aux_in)
+    return gemm(dy2, w, M, K, N, ldy, ldw, False, True, flags, None, aux_in)
 
 
 def _grad_weight(dy2, ldy, x2, ldx, dtype):
@@ -167,7 +167,7 @@ class _Linear(torch.autograd.Function):
             if after is not None:  # the rest of the unit's parameters, pulled meanwhile on the communication stream
                 torch.cuda.current_stream(x.device).wait_event(after)
             ctx.save_for_backward(x2, w)
-            ctx.ldx, ctx.has_bias, ctx.has_res = ldx, bias is not None, False
+            ctx.has_bias, ctx.has_res = bias is not None, False
             ctx.in_shape = x.shape
             return y.view(*x.shape[:-1], w.shape[0])
         res2 = None
@@ -178,19 +178,19 @@ class _Linear(torch.autograd.Function):
             need(res2.shape == (x2.shape[0], w.shape[0]), "the residual has not the output's shape")
         y = _forward(x2, ldx, w, bias, RESIDUAL if res2 is not None else 0, res2)
         ctx.save_for_backward(x2, w)
-        ctx.ldx, ctx.has_bias, ctx.has_res = ldx, bias is not None, residual is not None
+        ctx.has_bias, ctx.has_res = bias is not None, residual is not None
         ctx.in_shape = x.shape
         return y.view(*x.shape[:-1], w.shape[0]) if y.is_contiguous() else y.unflatten(0, x.shape[:-1])
 
     @staticmethod
     def backward(ctx, dy):
-        x2, w = ctx.saved_tensors
-        dy2, ldy = _rows(dy)
+        # their rows are looked at again: a saved-tensor hook may answer with other strides (save_on_cpu does)
+        (x2, ldx), (w, ldw), (dy2, ldy) = map(_rows, (*ctx.saved_tensors, dy))
         dx = dres = None
-        dw, db, join = _parameter_grads_beside(dy2, ldy, x2, ctx.ldx, w.dtype, ctx.needs_input_grad[1],
+        dw, db, join = _parameter_grads_beside(dy2, ldy, x2, ldx, w.dtype, ctx.needs_input_grad[1],
                                                 ctx.has_bias and ctx.needs_input_grad[2])
         if ctx.needs_input_grad[0]:
-            dx = _grad_input(dy2, ldy, w)
+            dx = _grad_input(dy2, ldy, w, ldw)
             dx = dx.view(ctx.in_shape) if dx.is_contiguous() else dx.unflatten(0, ctx.in_shape[:-1])
         join()
         if ctx.has_res and ctx.needs_input_grad[3]:
@@ -220,22 +220,23 @@ class _MLP(torch.autograd.Function):
         h = _forward(x2, ldx, w1, b1, GELU, None, slope)
         y = _forward(h, h.stride(0), w2, b2, RESIDUAL, res2)
         ctx.save_for_backward(x2, w1, w2, slope, h)
-        ctx.ldx, ctx.in_shape = ldx, x.shape
+        ctx.in_shape = x.shape
         return y.view(*x.shape[:-1], w2.shape[0]) if y.is_contiguous() else y.unflatten(0, x.shape[:-1])
 
     @staticmethod
     def backward(ctx, dy):
         x2, w1, w2, slope, h = ctx.saved_tensors
+        (x2, ldx), (w1, ldw1), (w2, ldw2), (h, ldh), (dy2, ldy) = map(_rows, (x2, w1, w2, h, dy))
+        slope = slope.contiguous()
         need = ctx.needs_input_grad
-        dy2, ldy = _rows(dy)
-        dw2, db2, join2 = _parameter_grads_beside(dy2, ldy, h, h.stride(0), w2.dtype, need[3], need[4])
-        dpre = _grad_input(dy2, ldy, w2, DGELU, slope)  # (dY . W2) * gelu'(pre)
+        dw2, db2, join2 = _parameter_grads_beside(dy2, ldy, h, ldh, w2.dtype, need[3], need[4])
+        dpre = _grad_input(dy2, ldy, w2, ldw2, DGELU, slope)  # (dY . W2) * gelu'(pre)
         join2()
         ldp = dpre.stride(0)
-        dw1, db1, join1 = _parameter_grads_beside(dpre, ldp, x2, ctx.ldx, w1.dtype, need[1], need[2])
+        dw1, db1, join1 = _parameter_grads_beside(dpre, ldp, x2, ldx, w1.dtype, need[1], need[2])
         dx = None
         if need[0]:
-            dx = _grad_input(dpre, ldp, w1)
+            dx = _grad_input(dpre, ldp, w1, ldw1)
             dx = dx.view(ctx.in_shape) if dx.is_contiguous() else dx.unflatten(0, ctx.in_shape[:-1])
         join1()
         return dx, dw1, db1, dw2, db2, (dy if need[5] else None)

@@ -25,6 +25,7 @@ class _LayerNorm(torch.autograd.Function):
     @staticmethod
     def backward(ctx, dy):
         x2, w, stats = ctx.saved_tensors
+        x2, stats = vectors_of(x2), stats.contiguous()  # a saved-tensor hook may answer with other strides
         M, D = x2.shape
         dy2, gain = vectors_of(dy.reshape(-1, D)), vectors_of(w)
         dx = torch.empty_like(x2)
@@ -66,6 +67,7 @@ class _ResidualLayerNorm(torch.autograd.Function):
     @staticmethod
     def backward(ctx, dres, dy):
         x2, w, stats = ctx.saved_tensors
+        x2, stats = vectors_of(x2), stats.contiguous()  # a saved-tensor hook may answer with other strides
         M, D = x2.shape
         if dy is None:
             return dres, None, None, None

@@ -15,9 +15,7 @@ class _CrossEntropy(torch.autograd.Function):
         rows, V = logits.shape
         need_ids(targets, logits)
         need(targets.numel() == rows, "cross_entropy takes one target per row")
-        # backward writes the rows where they lie: none may share memory with another
-        if logits.stride(1) != 1 or (rows > 1 and logits.stride(0) < V):
-            logits = logits.contiguous()
+        logits = _rows_apart(logits)
         ld = logits.stride(0) if rows > 1 else V
         targets = targets.contiguous()
         lse = torch.empty(rows, dtype=torch.float32, device=logits.device)
@@ -26,20 +24,27 @@ class _CrossEntropy(torch.autograd.Function):
         check_rc(lib().tb_xent_fwd(logits.data_ptr(), targets.data_ptr(), lse.data_ptr(), row_loss.data_ptr(), loss.data_ptr(),
                                    rows, V, ld, stream(logits)), "cross-entropy forward")
         ctx.save_for_backward(logits, targets, lse)
-        ctx.ld = ld
         return loss
 
     @staticmethod
     def backward(ctx, grad):
         logits, targets, lse = ctx.saved_tensors
+        # a saved-tensor hook may answer with other strides
+        logits, targets, lse = _rows_apart(logits), targets.contiguous(), lse.contiguous()
         rows, V = logits.shape
         scale = grad.detach().reshape(1).float().contiguous()
         # In place: the saved logits become their own gradient (they are not needed again).
-        ld = ctx.ld
+        ld = logits.stride(0) if rows > 1 else V
         width = ld if ld - V < 8 and _owns_padding(logits, ld) else V
         check_rc(lib().tb_xent_bwd(logits.data_ptr(), targets.data_ptr(), lse.data_ptr(), scale.data_ptr(), rows, V, ld, width,
                                    stream(logits)), "cross-entropy backward")
         return logits, None
+
+
+def _rows_apart(logits):
+    """Backward writes rows where they lie: none may share memory with another."""
+    rows, V = logits.shape
+    return logits.contiguous() if logits.stride(1) != 1 or (rows > 1 and logits.stride(0) < V) else logits
 
 
 def _owns_padding(logits, width):

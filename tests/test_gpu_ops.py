@@ -2,6 +2,7 @@
 computed from the same bf16 inputs.  Tolerances are those of one bf16 rounding of
 the output (2^-8 relative) plus fp32 accumulation-order noise."""
 
+import contextlib
 import math
 
 import pytest
@@ -942,6 +943,40 @@ def test_operators_of_views_equal_those_of_copies(python, monkeypatch):
         if name.startswith("linear"):
             copies[1] = inputs[1]  # a weight has to have 16-byte rows, which an odd width takes padding for
         for a, b in zip(outcome(function, inputs, needs), outcome(function, copies, needs)):
+            assert torch.equal(a, b), name
+
+
+@pytest.mark.parametrize("python", [False, True])
+@pytest.mark.parametrize("hook", ["save_on_cpu", "offset copies", "transposed copies"])
+def test_saved_tensors_may_come_back_elsewhere(hook, python, monkeypatch):
+    """A saved-tensor hook may hand backward a tensor with other strides, or one that starts off a 16-byte boundary."""
+    from tandem_b200.ops import _lib
+
+    if python:
+        monkeypatch.setattr(_lib, "native", lambda: None)
+    torch.manual_seed(0)
+
+    def offset(t):
+        room = torch.empty(t.numel() + 1, dtype=t.dtype, device=t.device)
+        return room[1:].view(t.shape).copy_(t)
+
+    def transposed(t):
+        return t.t().contiguous().t() if t.dim() == 2 else t.clone()
+
+    hooks = {"save_on_cpu": torch.autograd.graph.save_on_cpu(), "offset copies": torch.autograd.graph.saved_tensors_hooks(lambda t: t.clone(), offset),
+             "transposed copies": torch.autograd.graph.saved_tensors_hooks(lambda t: t.clone(), transposed)}
+
+    def gradients(function, inputs, needs, around):
+        inputs = [t if t is None or not n else t.detach().requires_grad_() for t, n in zip(inputs, needs)]
+        with around:
+            out = function(*inputs)
+        outs = out if isinstance(out, tuple) else (out,)
+        torch.manual_seed(1)
+        return torch.autograd.grad(outs, [t for t, n in zip(inputs, needs) if n], [torch.randn_like(o) for o in outs])
+
+    for name, (function, inputs, needs) in _operator_forms().items():
+        hooked = gradients(function, inputs, needs, hooks[hook])  # first: cross_entropy writes its gradient over what it saved
+        for a, b in zip(hooked, gradients(function, inputs, needs, contextlib.nullcontext())):
             assert torch.equal(a, b), name
 
 
