@@ -207,12 +207,13 @@ Stream side_stream(int device) {
 // dW = dY^T . X and dB = column sums of dY, beside the input gradient on a second stream where a layer has few rows (neither
 // fills the GPU by itself).  Everything that the second stream touches is allocated on the caller's stream beforehand and is
 // released after join(), which makes that stream wait: the caching allocator never sees a block used by a stream that it does not know about.
+// The fork is made by start(), not by a constructor: one that throws leaves no object to join.
 struct ParameterGrads {
   Tensor dw, db;
   Tensor scratch, workspace;
   Stream main = nullptr, beside = nullptr;
 
-  ParameterGrads(const Rows& dy, const Rows& x, bool want_w, bool want_b, int64_t side_below) {
+  void start(const Rows& dy, const Rows& x, bool want_w, bool want_b, int64_t side_below) {
     const int64_t M = dy.t.size(0), N = dy.t.size(1), k = x.t.size(1);
     if (!want_w && !want_b) return;
     const auto options = dy.t.options();
@@ -285,7 +286,8 @@ struct Linear : torch::autograd::Function<Linear> {
     const auto saved = ctx->get_saved_variables();
     const std::vector<int64_t> keep = ctx->saved_data["keep"].toIntVector();
     const Rows x = rows_of(saved[0]), w = rows_of(saved[1]), dy = rows_of(grads[0]);
-    ParameterGrads parameters(dy, x, keep[NEEDS] & 2, keep[NEEDS] & 4, keep[SIDE]);
+    ParameterGrads parameters;
+    parameters.start(dy, x, keep[NEEDS] & 2, keep[NEEDS] & 4, keep[SIDE]);
     Tensor dx;
     if (keep[NEEDS] & 1) dx = with_rows_of(grad_input(dy, w), at::IntArrayRef(keep).slice(SHAPE), w.t.size(1));
     parameters.join();
@@ -328,11 +330,13 @@ struct MLP : torch::autograd::Function<MLP> {
     const int64_t needs = keep[NEEDS];
     const Rows x = rows_of(saved[0]), w1 = rows_of(saved[1]), w2 = rows_of(saved[2]), hidden = rows_of(saved[4]), dy = rows_of(grads[0]);
     const Tensor slope = saved[3].contiguous();
-    ParameterGrads second(dy, hidden, needs & 8, needs & 16, keep[SIDE]);
+    ParameterGrads second;
+    second.start(dy, hidden, needs & 8, needs & 16, keep[SIDE]);
     const Tensor dpre = grad_input(dy, w2, DGELU, slope);  // (dY . W2) * gelu'(pre)
     second.join();
     const Rows pre{dpre, dpre.stride(0)};
-    ParameterGrads first(pre, x, needs & 2, needs & 4, keep[SIDE]);
+    ParameterGrads first;
+    first.start(pre, x, needs & 2, needs & 4, keep[SIDE]);
     Tensor dx;
     if (needs & 1) dx = with_rows_of(grad_input(pre, w1), at::IntArrayRef(keep).slice(SHAPE), w1.t.size(1));
     first.join();

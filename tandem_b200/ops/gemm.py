@@ -108,7 +108,7 @@ _side_streams = {}
 
 def _parameter_grads_beside(dy2, ldy, x2, ldx, dtype, want_w, want_b):
     """(dW, dB, join): starts dW = dY^T . X and dB = column sums of dY on the side stream when the problem is small;
-    join() makes the caller's stream wait for them (call it after queuing the input gradient)."""
+    join() makes the caller's stream wait for them (call it after queuing the input gradient, and where that fails, too)."""
     M, N = dy2.shape
     K = x2.shape[1]
     if not (want_w or want_b):
@@ -135,17 +135,21 @@ def _parameter_grads_beside(dy2, ldy, x2, ldx, dtype, want_w, want_b):
         db = torch.empty(N, dtype=torch.bfloat16, device=dev)
         scratch = torch.empty(32 * N, dtype=torch.float32, device=dev)
     beside = side.cuda_stream
-    stream_wait(beside, main)
-    if want_w:
-        gemm(dy2, x2, N, K, M, ldy, ldx, True, True, 0, out=dw, workspace=workspace, on=beside)
-    if want_b:
-        check_rc(lib().tb_col_sum(dy2.data_ptr(), M, N, ldy, db.data_ptr(), scratch.data_ptr(), beside), "col_sum")
     keep = (scratch, workspace)  # released by the caller's frame, after the join
 
     def join():
         stream_wait(main, beside)
         return keep
 
+    stream_wait(beside, main)
+    try:
+        if want_w:
+            gemm(dy2, x2, N, K, M, ldy, ldx, True, True, 0, out=dw, workspace=workspace, on=beside)
+        if want_b:
+            check_rc(lib().tb_col_sum(dy2.data_ptr(), M, N, ldy, db.data_ptr(), scratch.data_ptr(), beside), "col_sum")
+    except BaseException:
+        join()
+        raise
     return dw, db, join
 
 
@@ -189,10 +193,12 @@ class _Linear(torch.autograd.Function):
         dx = dres = None
         dw, db, join = _parameter_grads_beside(dy2, ldy, x2, ldx, w.dtype, ctx.needs_input_grad[1],
                                                 ctx.has_bias and ctx.needs_input_grad[2])
-        if ctx.needs_input_grad[0]:
-            dx = _grad_input(dy2, ldy, w, ldw)
-            dx = dx.view(ctx.in_shape) if dx.is_contiguous() else dx.unflatten(0, ctx.in_shape[:-1])
-        join()
+        try:
+            if ctx.needs_input_grad[0]:
+                dx = _grad_input(dy2, ldy, w, ldw)
+                dx = dx.view(ctx.in_shape) if dx.is_contiguous() else dx.unflatten(0, ctx.in_shape[:-1])
+        finally:
+            join()
         if ctx.has_res and ctx.needs_input_grad[3]:
             dres = dy
         return dx, dw, db, dres
@@ -230,15 +236,19 @@ class _MLP(torch.autograd.Function):
         slope = slope.contiguous()
         need = ctx.needs_input_grad
         dw2, db2, join2 = _parameter_grads_beside(dy2, ldy, h, ldh, w2.dtype, need[3], need[4])
-        dpre = _grad_input(dy2, ldy, w2, ldw2, DGELU, slope)  # (dY . W2) * gelu'(pre)
-        join2()
+        try:
+            dpre = _grad_input(dy2, ldy, w2, ldw2, DGELU, slope)  # (dY . W2) * gelu'(pre)
+        finally:
+            join2()
         ldp = dpre.stride(0)
         dw1, db1, join1 = _parameter_grads_beside(dpre, ldp, x2, ldx, w1.dtype, need[1], need[2])
         dx = None
-        if need[0]:
-            dx = _grad_input(dpre, ldp, w1, ldw1)
-            dx = dx.view(ctx.in_shape) if dx.is_contiguous() else dx.unflatten(0, ctx.in_shape[:-1])
-        join1()
+        try:
+            if need[0]:
+                dx = _grad_input(dpre, ldp, w1, ldw1)
+                dx = dx.view(ctx.in_shape) if dx.is_contiguous() else dx.unflatten(0, ctx.in_shape[:-1])
+        finally:
+            join1()
         return dx, dw1, db1, dw2, db2, (dy if need[5] else None)
 
 

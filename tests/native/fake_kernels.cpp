@@ -1,0 +1,34 @@
+// Stands in for libtb200_cuda.so under the native operators: every launcher succeeds without launching anything, the n-th call
+// of one of them can be made to fail, and the waits of streams on one another are taken down.
+typedef void* S;
+
+extern "C" {
+
+int fake_fail_at = 0;  // this product or column sum (1: the first one from here on) is refused
+int fake_waits = 0;
+S fake_log[64][2];
+
+static int launch() { return fake_fail_at > 0 && --fake_fail_at == 0 ? -77 : 0; }
+
+int tb_gemm_bf16(const void*, const void*, void*, int, int, int, int, int, int, int, int, int, const void*, const void*, void*, int, void*,
+                 long long, S) { return launch(); }
+int tb_col_sum(const void*, int, int, int, void*, float*, S) { return launch(); }
+long long tb_gemm_workspace_bytes(int, int, int) { return 0; }
+int tb_stream_wait(S waiter, S signaller) {
+  fake_log[fake_waits % 64][0] = waiter;
+  fake_log[fake_waits++ % 64][1] = signaller;
+  return 0;
+}
+const char* tb_gemm_last_error() { return ""; }
+const char* tb_error_string(int) { return ""; }
+const char* tb_last_error() { return ""; }
+int tb_layernorm_fwd(const void*, const void*, const void*, void*, float*, float*, int, int, float, S) { return 0; }
+int tb_layernorm_bwd_blocks(int) { return 1; }
+int tb_layernorm_bwd_add(const void*, const void*, const void*, const float*, const float*, const void*, void*, void*, void*, float*, int, int, S) { return 0; }
+int tb_attn_fwd(const void*, void*, float*, int, int, int, int, S) { return 0; }
+int tb_attn_bwd(const void*, const void*, const void*, const float*, void*, float*, int, int, int, int, S) { return 0; }
+int tb_embed_fwd(const long long*, const void*, const void*, void*, int, int, int, S) { return 0; }
+int tb_embed_bwd(const long long*, const void*, float*, void*, void*, int, int, int, int, S) { return 0; }
+int tb_xent_fwd(const void*, const long long*, float*, float*, float*, int, int, int, S) { return 0; }
+int tb_xent_bwd(void*, const long long*, const float*, const float*, int, int, int, int, S) { return 0; }
+}
