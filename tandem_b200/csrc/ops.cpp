@@ -496,9 +496,11 @@ struct CrossEntropy : torch::autograd::Function<CrossEntropy> {
   }
 };
 
-// Where gradients are off nothing can ask for the node: the forward alone.
+// Where gradients are off nothing can ask for the node: the forward alone.  Without the interpreter lock: an allocation or a launch
+// may have to wait for the GPU, and other threads go on meanwhile, as they do beside ctypes (saved-tensor hooks take the lock themselves).
 template <typename F, typename... Args>
 auto call(const Args&... args) {
+  py::gil_scoped_release unlocked;
   return at::GradMode::is_enabled() ? F::apply(args...) : F::forward(nullptr, args...);
 }
 

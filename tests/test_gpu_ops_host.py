@@ -86,3 +86,40 @@ def test_a_refused_launch_leaves_no_branch(name, launches, kernels):
         assert log and len(log) % 2 == 0
         for fork, join in zip(log[::2], log[1::2]):
             assert fork[::-1] == join, (at, log)
+
+
+CALLS = {
+    "linear": lambda ops: ops.linear(leaf(40, 64), leaf(96, 64), leaf(96)),
+    "mlp": lambda ops: ops.mlp(leaf(40, 64), leaf(96, 64), leaf(96), leaf(64, 96), leaf(64), leaf(40, 64)),
+    "layer_norm": lambda ops: ops.layer_norm(leaf(40, 64), leaf(64), leaf(64)),
+    "residual_layer_norm": lambda ops: ops.residual_layer_norm(leaf(40, 64), leaf(64), leaf(64)),
+    "causal_attention": lambda ops: ops.causal_attention(leaf(1, 128, 192), 1),
+    "embedding": lambda ops: ops.embedding(torch.zeros(2, 8, dtype=torch.int64, device="cuda"), leaf(50, 64), leaf(32, 64)),
+    "cross_entropy": lambda ops: ops.cross_entropy(leaf(40, 64), torch.zeros(40, dtype=torch.int64, device="cuda")),
+}
+
+
+@pytest.mark.parametrize("gradients", [True, False])
+@pytest.mark.parametrize("name", CALLS)
+def test_a_launch_that_waits_stops_no_other_thread(name, gradients, kernels):
+    """A launch waits where the queue is full: the interpreter goes on meanwhile, here the thread that ends the wait."""
+    import threading
+    import time
+
+    from tandem_b200 import ops
+
+    closed = ctypes.c_int.in_dll(kernels, "fake_closed")
+    started = threading.Event()
+
+    def open_up():
+        started.wait()
+        time.sleep(0.05)
+        closed.value = 0
+
+    other = threading.Thread(target=open_up)
+    other.start()
+    with torch.set_grad_enabled(gradients):
+        closed.value = 1
+        started.set()
+        CALLS[name](ops)  # ends with an error (-78) if nobody opens up
+    other.join()
