@@ -1193,12 +1193,9 @@ int tb_attn_fwd(const void* qkv, void* out, float* lse, int B, int T, int H, int
 #define LAUNCH_FWD(HD_, MANY_) \
   do { \
     using L = Fwd2Smem<HD_, MANY_>; \
-    static bool once = false; \
-    if (!once) { \
-      cudaError_t e = cudaFuncSetAttribute(k_attn_fwd_ws<HD_, MANY_>, cudaFuncAttributeMaxDynamicSharedMemorySize, L::TOTAL); \
-      if (e != cudaSuccess) return (int)e; \
-      once = true; \
-    } \
+    static tb::SharedMemoryLimit limit; \
+    const cudaError_t e = limit.raise(k_attn_fwd_ws<HD_, MANY_>, L::TOTAL); \
+    if (e != cudaSuccess) return (int)e; \
     return (int)tb::launch(k_attn_fwd_ws<HD_, MANY_>, dim3(ctas), dim3(L::THREADS), L::TOTAL, stream, map, (__nv_bfloat16*)out, lse, B, T, H, d, scale_log2e, \
                            group, error); \
   } while (0)
@@ -1232,14 +1229,11 @@ int tb_attn_bwd(const void* qkv, const void* out, const void* d_out, const float
   tb_note_launch(2);
 #define LAUNCH_BWD(HD_, MANY_) \
   do { \
-    static bool once = false; \
-    if (!once) { \
-      cudaError_t e = cudaFuncSetAttribute(k_attn_bwd_dq<HD_, MANY_>, cudaFuncAttributeMaxDynamicSharedMemorySize, BwdDqSmem<HD_, MANY_>::TOTAL); \
-      if (e == cudaSuccess) e = cudaFuncSetAttribute(k_attn_bwd_dkv<HD_, MANY_>, cudaFuncAttributeMaxDynamicSharedMemorySize, BwdDkvSmem<HD_, MANY_>::TOTAL); \
-      if (e != cudaSuccess) return (int)e; \
-      once = true; \
-    } \
-    cudaError_t e = tb::launch(k_attn_bwd_dq<HD_, MANY_>, dim3(ctas), dim3(320), BwdDqSmem<HD_, MANY_>::TOTAL, stream, map_qkv, map_do, map_o, \
+    static tb::SharedMemoryLimit dq_limit, dkv_limit; \
+    cudaError_t e = dq_limit.raise(k_attn_bwd_dq<HD_, MANY_>, BwdDqSmem<HD_, MANY_>::TOTAL); \
+    if (e == cudaSuccess) e = dkv_limit.raise(k_attn_bwd_dkv<HD_, MANY_>, BwdDkvSmem<HD_, MANY_>::TOTAL); \
+    if (e != cudaSuccess) return (int)e; \
+    e = tb::launch(k_attn_bwd_dq<HD_, MANY_>, dim3(ctas), dim3(320), BwdDqSmem<HD_, MANY_>::TOTAL, stream, map_qkv, map_do, map_o, \
                                (const __nv_bfloat16*)out, (const __nv_bfloat16*)d_out, lse, delta, (__nv_bfloat16*)dqkv, B, T, H, d, scale, group, error); \
     if (e != cudaSuccess) return (int)e; \
     return (int)tb::launch(k_attn_bwd_dkv<HD_, MANY_>, dim3(ctas), dim3(320), BwdDkvSmem<HD_, MANY_>::TOTAL, stream, map_qkv, map_do, lse, (const float*)delta, \

@@ -1162,12 +1162,9 @@ int launch_gemm(const CUtensorMap& ma, const CUtensorMap& mb, const CUtensorMap&
                 cudaStream_t stream) {
   auto kernel = k_gemm<BM, BN, A_MN, B_MN>;
   using L = SmemLayout<BM, BN>;
-  static bool configured = false;
-  if (!configured) {
-    cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, L::TOTAL);
-    if (e != cudaSuccess) return (int)e;
-    configured = true;
-  }
+  static tb::SharedMemoryLimit limit;
+  const cudaError_t e = limit.raise(kernel, L::TOTAL);
+  if (e != cudaSuccess) return (int)e;
   const int out_tiles = ((g.M + BM - 1) / BM) * ((g.N + BN - 1) / BN);
   const int tiles = g.splits > 1 ? g.whole_tiles + (out_tiles - g.whole_tiles) * g.splits : out_tiles;
   const int sms = tb::sm_count();
@@ -1182,10 +1179,12 @@ int launch_gemm_pair(const CUtensorMap& ma, const CUtensorMap& mb, const CUtenso
                      int max_ctas, cudaStream_t stream) {
   auto kernel = k_gemm_pair<BN, A_MN, B_MN, DEEP>;
   using L = PairLayout<BN, DEEP>;
-  static int max_pairs = 0;
+  static tb::SharedMemoryLimit limit;
+  const cudaError_t e = limit.raise(kernel, L::TOTAL);
+  if (e != cudaSuccess) return (int)e;
+  static std::atomic<int> known_pairs{0};
+  int max_pairs = known_pairs.load(std::memory_order_relaxed);
   if (max_pairs == 0) {
-    cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, L::TOTAL);
-    if (e != cudaSuccess) return (int)e;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(tb::sm_count() & ~1);
     cfg.blockDim = dim3(L::THREADS);
@@ -1203,6 +1202,7 @@ int launch_gemm_pair(const CUtensorMap& ma, const CUtensorMap& mb, const CUtenso
       n = tb::sm_count() / 2;
     }
     max_pairs = n < tb::sm_count() / 2 ? n : tb::sm_count() / 2;
+    known_pairs.store(max_pairs, std::memory_order_relaxed);
   }
   const int out_tiles = ((g.M + 255) / 256) * ((g.N + BN - 1) / BN);
   const int tiles = g.splits > 1 ? g.whole_tiles + (out_tiles - g.whole_tiles) * g.splits : out_tiles;
@@ -1495,19 +1495,16 @@ int tb_gemm_gathered(const void* A, void* out, int M, int N, int K, int lda, int
   ga.n = n_ranks;
   ga.chunk_bytes = chunk_bytes;
   ga.n_start = ((n_start % tiles_n) + tiles_n) % tiles_n;
-  const void* kernel = tall ? (const void*)k_gemm<256, BN, false, false, true> : (const void*)k_gemm<128, BN, false, false, true>;
+  const auto kernel = tall ? k_gemm<256, BN, false, false, true> : k_gemm<128, BN, false, false, true>;
   const int smem = tall ? SmemLayout<256, BN>::TOTAL : SmemLayout<128, BN>::TOTAL;
-  static bool configured[2] = {false, false};
-  if (!configured[tall]) {
-    cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-    if (e != cudaSuccess) return (int)e;
-    configured[tall] = true;
-  }
+  static tb::SharedMemoryLimit limits[2];
+  const cudaError_t e = limits[tall].raise(kernel, smem);
+  if (e != cudaSuccess) return (int)e;
   const int tiles = ((M + BM - 1) / BM) * tiles_n;
   int ctas = tiles < sms ? tiles : sms;
   void* params[] = {(void*)&ma, (void*)&mb, (void*)&mo, (void*)&mp, (void*)&mx, (void*)&g, (void*)&ga};
   tb_note_launch(1);
-  return (int)cudaLaunchCooperativeKernel(kernel, dim3(ctas), dim3(448), params, smem, stream);
+  return (int)cudaLaunchCooperativeKernel((const void*)kernel, dim3(ctas), dim3(448), params, smem, stream);
 }
 
 void tb_gemm_force_tile(int which) { g_forced_tile.store(which, std::memory_order_relaxed); }

@@ -21,6 +21,27 @@ inline int sm_count() {
   return n;
 }
 
+// The dynamic shared memory that a kernel may ask for, raised before its first launch on each device: the limit belongs to the
+// device.  Only a success is remembered.
+class SharedMemoryLimit {
+ public:
+  template <typename... Args>
+  cudaError_t raise(void (*kernel)(Args...), int bytes) {
+    int dev = 0;
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e != cudaSuccess) return e;
+    const unsigned long long bit = dev < 64 ? 1ull << dev : 0;
+    if (raised_.load(std::memory_order_relaxed) & bit) return cudaSuccess;
+    e = cudaFuncSetAttribute(reinterpret_cast<const void*>(kernel), cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+    if (e == cudaSuccess) raised_.fetch_or(bit, std::memory_order_relaxed);
+    else cudaGetLastError();  // it is returned: the next launch does not find it again
+    return e;
+  }
+
+ private:
+  std::atomic<unsigned long long> raised_{0};
+};
+
 // A word of host memory that kernels raise when a wait runs out.
 class ErrorWord {
  public:

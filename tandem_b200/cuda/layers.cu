@@ -884,8 +884,8 @@ int tb_layernorm_bwd_add(const void* dy, const void* x, const void* w, const flo
     const int resident = 148 * (V <= 4 ? 2 : 1), grid = slices < resident ? slices : resident;                                  \
     const int rows = per_warp * ((slices + grid - 1) / grid), stages = rows < LnBwd<V>::STAGES ? rows : LnBwd<V>::STAGES;       \
     const int smem = LnBwd<V>::smem(stages, ADD, grid == slices);                                                                               \
-    static const cudaError_t allowed = cudaFuncSetAttribute(k_ln_bwd<V, ADD>, cudaFuncAttributeMaxDynamicSharedMemorySize,      \
-                                                            LnBwd<V>::smem(LnBwd<V>::STAGES, ADD, true));                       \
+    static tb::SharedMemoryLimit limit;                                                                                         \
+    const cudaError_t allowed = limit.raise(k_ln_bwd<V, ADD>, LnBwd<V>::smem(LnBwd<V>::STAGES, ADD, true));                     \
     if (allowed != cudaSuccess) return (int)allowed;                                                                            \
     tb::launch(k_ln_bwd<V, ADD>, dim3(grid), dim3(256), (size_t)smem, s, (const __nv_bfloat16*)dy, (const __nv_bfloat16*)x,     \
                (const __nv_bfloat16*)w, mean, rstd, (const __nv_bfloat16*)add, (__nv_bfloat16*)dx, scratch, M, D, slices, stages); \

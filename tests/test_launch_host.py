@@ -50,3 +50,39 @@ def test_threads_never_share_words(fake, products):
     fake.fake_borrowed(out)
     assert out[0] > 50 and out[0] * out[1] <= threads * each <= out[0] * out[2]
     assert out[2] - out[1] <= 1, f"{out[0]} places, lent {out[1]} to {out[2]} times"
+
+
+def launches(lib):
+    """A call of each kind that needs more than 48 KB of shared memory: (name, function)."""
+    def product(M, N, K):
+        need = lib.tb_gemm_workspace_bytes(M, N, K)
+        return lib.tb_gemm_bf16(WORK, WORK, WORK, M, N, K, M, N, N, 1, 1, 0, None, None, None, 0, WORK if need else None, need, None)
+
+    yield "product of few tiles", lambda: product(256, 256, 256)
+    yield "product of pair tiles", lambda: product(8192, 4096, 512)
+    for D in (256, 768, 1024, 1536, 2048):
+        for add in (None, WORK):
+            yield f"layer norm {D} {add}", lambda D=D, add=add: lib.tb_layernorm_bwd_add(*[WORK] * 5, add, *[WORK] * 4, 30000, D, None)
+    for hd in (64, 128):
+        for batch in (1, 64):
+            yield f"attention {hd} {batch}", lambda hd=hd, batch=batch: (lib.tb_attn_fwd(WORK, WORK, WORK, batch, 1024, 8, hd, None)
+                                                                      or lib.tb_attn_bwd(*[WORK] * 6, batch, 1024, 8, hd, None))
+
+
+def test_shared_memory_is_allowed_on_every_device(fake):
+    """The limit belongs to a device: a process that turns to a second one raises it there, too."""
+    for device in (0, 1, 63, 64, 0):
+        fake.fake_set_device(device)
+        for name, call in launches(fake):
+            assert call() == 0, (name, device)
+    fake.fake_set_device(0)
+
+
+def test_a_refused_limit_is_asked_for_again(fake):
+    for device, (name, call) in enumerate(launches(fake), start=8):  # some share a kernel: each has a device of its own
+        fake.fake_set_device(device)
+        fake.fake_refuse_allowing(1)
+        assert call() != 0, name
+        fake.fake_refuse_allowing(0)
+        assert call() == 0, name
+    fake.fake_set_device(0)
