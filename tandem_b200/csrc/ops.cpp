@@ -160,6 +160,10 @@ Tensor with_rows_of(const Tensor& t2, at::IntArrayRef shape, int64_t width) {
 Tensor gemm(const Tensor& a, const Tensor& b, int64_t M, int64_t N, int64_t k, int64_t lda, int64_t ldb, bool a_mn, bool b_mn, int flags,
             const Tensor& bias_in, Tensor aux_in, const Tensor& aux_out, Tensor out = {}, Tensor workspace = {}, Stream on = nullptr) {
   if (!out.defined()) out = empty_padded(M, N, a.options());
+  if (k == 0) {  // a sum over nothing, as the weight gradient of an empty batch is: the kernel writes nothing
+    need(flags == 0, "a product over no columns takes no bias and no other operand");
+    return out.zero_();
+  }
   const int64_t ldc = M > 1 ? out.stride(0) : pad8(N);
   const Tensor bias = bias_in.defined() ? bias_in.contiguous() : bias_in;
   if (aux_in.defined() && misaligned(aux_in)) aux_in = aux_in.clone();  // it is read in 16-byte vectors

@@ -37,6 +37,9 @@ def gemm(a, b, M, N, K, lda, ldb, a_mn, b_mn, flags=0, bias=None, aux_in=None, a
     than the one their memory belongs to (else it is allocated here).  on: the raw stream to launch on (default: the current one)."""
     if out is None:
         out = empty_padded(M, N, out_dtype, a.device)
+    if K == 0 and not flags & ACCUMULATE:  # a sum over nothing, as the weight gradient of an empty batch is: the kernel writes nothing
+        need(flags == 0, "a product over no columns takes no bias and no other operand")
+        return out.zero_()
     ldc = out.stride(0) if M > 1 else pad8(N)
     if bias is not None:
         bias = bias.contiguous()
@@ -48,16 +51,16 @@ def gemm(a, b, M, N, K, lda, ldb, a_mn, b_mn, flags=0, bias=None, aux_in=None, a
         flags |= OUT_F32
     # Problems with too few output tiles for the SMs (weight gradients, small per-rank batches) are computed with the
     # reduction cut into parts inside the one kernel; it parks partial tiles in this workspace.
-    need = lib().tb_gemm_workspace_bytes(M, N, K)
-    if need and (workspace is None or workspace.numel() < need):
-        workspace = torch.empty(need, dtype=torch.uint8, device=a.device)
-    if not need:
+    parts = lib().tb_gemm_workspace_bytes(M, N, K)
+    if parts and (workspace is None or workspace.numel() < parts):
+        workspace = torch.empty(parts, dtype=torch.uint8, device=a.device)
+    if not parts:
         workspace = None
     rc = lib().tb_gemm_bf16(a.data_ptr(), b.data_ptr(), out.data_ptr(), M, N, K, lda, ldb, ldc, int(a_mn), int(b_mn), flags,
                             bias.data_ptr() if bias is not None else None,
                             aux_in.data_ptr() if aux_in is not None else None,
                             aux_out.data_ptr() if aux_out is not None else None, 0,
-                            workspace.data_ptr() if workspace is not None else None, need, stream(a) if on is None else on)
+                            workspace.data_ptr() if workspace is not None else None, parts, stream(a) if on is None else on)
     if rc in (-11, -12):
         raise RuntimeError(f"gemm: operand not addressable by TMA (M={M} N={N} K={K} lda={lda} ldb={ldb} a_mn={a_mn} b_mn={b_mn} "
                            f"a={a.data_ptr():#x} b={b.data_ptr():#x}): {lib().tb_gemm_last_error().decode()}")

@@ -981,6 +981,30 @@ def test_saved_tensors_may_come_back_elsewhere(hook, python, monkeypatch):
 
 
 @pytest.mark.parametrize("python", [False, True])
+def test_linear_of_an_empty_batch(python, monkeypatch):
+    """Its weight gradient is a sum over no rows: zeros, not what the memory held before."""
+    from tandem_b200 import ops
+    from tandem_b200.ops import _lib
+
+    if python:
+        monkeypatch.setattr(_lib, "native", lambda: None)
+    for inner, outer in [(64, 96), (68, 96), (64, 0)]:
+        x, w, b = rnd(0, inner).requires_grad_(), rnd(outer, pad8(inner))[:, :inner].detach().requires_grad_(), rnd(outer).requires_grad_()
+        del_me = [torch.full((96, pad8(inner)), float("nan"), device="cuda", dtype=torch.bfloat16) for _ in range(8)]
+        del del_me
+        y = ops.linear(x, w, b if outer else None)
+        y.sum().backward()
+        assert y.shape == (0, outer) and x.grad.shape == x.shape and torch.equal(w.grad, torch.zeros_like(w))
+        assert not outer or torch.equal(b.grad, torch.zeros_like(b))
+    x = rnd(40, 64).requires_grad_()
+    (g,) = torch.autograd.grad(ops.linear(x, rnd(0, 64)), x, rnd(40, 0))
+    assert torch.equal(g, torch.zeros_like(x))
+    assert torch.equal(ops.linear(rnd(40, 0), rnd(96, 0)), torch.zeros(40, 96, device="cuda"))
+    with pytest.raises(ValueError, match="no columns"):
+        ops.linear(rnd(40, 0), rnd(96, 0), rnd(96))
+
+
+@pytest.mark.parametrize("python", [False, True])
 def test_operators_notice_a_changed_input(python, monkeypatch):
     """What backward reads again must not have changed in between; a gradient has no gradient of its own."""
     from tandem_b200 import ops
