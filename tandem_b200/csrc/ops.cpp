@@ -508,6 +508,9 @@ auto call(const Args&... args) {
   return at::GradMode::is_enabled() ? F::apply(args...) : F::forward(nullptr, args...);
 }
 
+// Looked for in the file by the build, which cannot import a library of another torch.
+__attribute__((used)) const char built_for[] = BUILT_FOR;
+
 }  // namespace
 
 PYBIND11_MODULE(_ops, m) {

@@ -119,6 +119,20 @@ def build_cuda(force=False, verbose=False):
     return CUDA_LIB
 
 
+def ops_built_for():
+    """What a library of the native autograd functions is bound to, in the words that it carries itself (csrc/ops.cpp)."""
+    import torch
+
+    return f"tandem_b200._ops for torch {torch.__version__} {torch.version.git_version}, CUDA {torch.version.cuda}, {sysconfig.get_config_var('SOABI')};"
+
+
+def _ops_is_stale(deps):
+    if _newer(OPS_LIB, deps):
+        return True
+    with open(OPS_LIB, "rb") as f:
+        return ops_built_for().encode() not in f.read()
+
+
 def build_ops(force=False, verbose=False):
     """Compiles the native autograd functions against the installed torch, or returns None where that is a CPU build."""
     import torch
@@ -127,13 +141,13 @@ def build_ops(force=False, verbose=False):
     nvcc = nvcc_path()
     if torch.version.cuda is None or nvcc is None:
         return None
-    if not force and not _newer(OPS_LIB, [OPS_SOURCE]):
+    if not force and not _ops_is_stale([OPS_SOURCE]):
         return OPS_LIB
     cuda_include = os.path.join(os.path.dirname(os.path.dirname(os.path.realpath(nvcc))), "include")
     includes = [*include_paths(), cuda_include, sysconfig.get_paths()["include"]]
     libs = os.path.join(os.path.dirname(torch.__file__), "lib")
     tmp = OPS_LIB + f".{os.getpid()}.tmp"
-    cmd = ["g++", "-O2", "-std=c++17", "-fPIC", "-shared", "-fvisibility=hidden", "-DTORCH_EXTENSION_NAME=_ops",
+    cmd = ["g++", "-O2", "-std=c++17", "-fPIC", "-shared", "-fvisibility=hidden", "-DTORCH_EXTENSION_NAME=_ops", f'-DBUILT_FOR="{ops_built_for()}"',
            f"-D_GLIBCXX_USE_CXX11_ABI={int(torch.compiled_with_cxx11_abi())}", *(f"-isystem{i}" for i in includes), OPS_SOURCE, "-o", tmp,
            f"-L{libs}", "-lc10", "-lc10_cuda", "-ltorch_cpu", "-ltorch", "-ltorch_python", "-ldl"]
     _run(cmd, verbose)
