@@ -18,6 +18,8 @@
 #include <string>
 #include <vector>
 
+#include "../cuda/operators.h"
+
 namespace {
 
 using at::Tensor;
@@ -25,25 +27,20 @@ using torch::autograd::AutogradContext;
 using torch::autograd::variable_list;
 
 // ---------------------------------------------------------------- the kernel library
-typedef void* Stream;
+// Types from the declarations that the kernels' own sources include, names from the same words.
+#define TB_KERNELS(X)                                                                                                      \
+  X(gemm, tb_gemm_bf16) X(gemm_workspace, tb_gemm_workspace_bytes) X(gemm_error_text, tb_gemm_last_error)                  \
+  X(col_sum, tb_col_sum) X(ln_fwd, tb_layernorm_fwd) X(ln_bwd_slices, tb_layernorm_bwd_blocks)                             \
+  X(ln_bwd, tb_layernorm_bwd_add) X(attn_fwd, tb_attn_fwd) X(attn_bwd, tb_attn_bwd)                                        \
+  X(embed_fwd, tb_embed_fwd) X(embed_bwd, tb_embed_bwd) X(xent_fwd, tb_xent_fwd)                                           \
+  X(xent_bwd, tb_xent_bwd) X(stream_wait, tb_stream_wait) X(error_string, tb_error_string)                                 \
+  X(last_error, tb_last_error)
+
+typedef cudaStream_t Stream;
 struct Kernels {
-  int (*gemm)(const void*, const void*, void*, int, int, int, int, int, int, int, int, int, const void*, const void*, void*, int, void*,
-              long long, Stream);
-  long long (*gemm_workspace)(int, int, int);
-  const char* (*gemm_error_text)();
-  int (*col_sum)(const void*, int, int, int, void*, float*, Stream);
-  int (*ln_fwd)(const void*, const void*, const void*, void*, float*, float*, int, int, float, Stream);
-  int (*ln_bwd_slices)(int);
-  int (*ln_bwd)(const void*, const void*, const void*, const float*, const float*, const void*, void*, void*, void*, float*, int, int, Stream);
-  int (*attn_fwd)(const void*, void*, float*, int, int, int, int, Stream);
-  int (*attn_bwd)(const void*, const void*, const void*, const float*, void*, float*, int, int, int, int, Stream);
-  int (*embed_fwd)(const long long*, const void*, const void*, void*, int, int, int, Stream);
-  int (*embed_bwd)(const long long*, const void*, float*, void*, void*, int, int, int, int, Stream);
-  int (*xent_fwd)(const void*, const long long*, float*, float*, float*, int, int, int, Stream);
-  int (*xent_bwd)(void*, const long long*, const float*, const float*, int, int, int, int, Stream);
-  int (*stream_wait)(Stream, Stream);
-  const char* (*error_string)(int);
-  const char* (*last_error)();
+#define MEMBER(member, name) decltype(&name) member;
+  TB_KERNELS(MEMBER)
+#undef MEMBER
 };
 Kernels K;
 
@@ -54,22 +51,9 @@ void bind(const std::string& path) {
     fn = reinterpret_cast<std::decay_t<decltype(fn)>>(dlsym(lib, name));
     if (fn == nullptr) throw std::runtime_error(std::string("libtb200_cuda.so lacks ") + name);
   };
-  find(K.gemm, "tb_gemm_bf16");
-  find(K.gemm_workspace, "tb_gemm_workspace_bytes");
-  find(K.gemm_error_text, "tb_gemm_last_error");
-  find(K.col_sum, "tb_col_sum");
-  find(K.ln_fwd, "tb_layernorm_fwd");
-  find(K.ln_bwd_slices, "tb_layernorm_bwd_blocks");
-  find(K.ln_bwd, "tb_layernorm_bwd_add");
-  find(K.attn_fwd, "tb_attn_fwd");
-  find(K.attn_bwd, "tb_attn_bwd");
-  find(K.embed_fwd, "tb_embed_fwd");
-  find(K.embed_bwd, "tb_embed_bwd");
-  find(K.xent_fwd, "tb_xent_fwd");
-  find(K.xent_bwd, "tb_xent_bwd");
-  find(K.stream_wait, "tb_stream_wait");
-  find(K.error_string, "tb_error_string");
-  find(K.last_error, "tb_last_error");
+#define FIND(member, name) find(K.member, #name);
+  TB_KERNELS(FIND)
+#undef FIND
 }
 
 void check(int rc, const char* what) {

@@ -27,6 +27,7 @@
 #include "f32x2.cuh"
 #include "host_state.h"
 #include "launch.cuh"
+#include "operators.h"
 #include "tcgen05.cuh"
 
 extern "C" void tb_note_launch(int n);

@@ -15,6 +15,7 @@
 #include "host_state.h"
 #include "launch.cuh"
 #include "noalloc.h"
+#include "operators.h"
 
 extern "C" void tb_note_launch(int n);
 
@@ -863,9 +864,6 @@ int tb_layernorm_fwd(const void* x, const void* w, const void* b, void* y, float
 // Few rows: one row per warp on as many SMs as it takes (at 1024 rows four rows per warp would leave 116 SMs idle);
 // many rows: several rows per warp, so that the row look-ahead has something to fetch.
 int tb_layernorm_bwd_blocks(int M) { return M < 8192 ? grid_for(M, 8, 296) : grid_for(M, 8 * 4, 592); }
-
-int tb_layernorm_bwd_add(const void* dy, const void* x, const void* w, const float* mean, const float* rstd, const void* add, void* dx,
-                         void* dw, void* db, float* scratch, int M, int D, cudaStream_t s);
 
 int tb_layernorm_bwd(const void* dy, const void* x, const void* w, const float* mean, const float* rstd, void* dx, void* dw,
                      void* db, float* scratch, int M, int D, cudaStream_t s) {

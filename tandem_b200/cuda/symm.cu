@@ -10,6 +10,8 @@
 
 #include <atomic>
 
+#include "operators.h"
+
 static thread_local char g_last_error[256] = "";
 
 static int fail(cudaError_t e, const char* what) {

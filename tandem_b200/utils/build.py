@@ -24,6 +24,7 @@ CSRC = os.path.join(PKG, "csrc")
 CUDA = os.path.join(PKG, "cuda")
 HOST_SOURCES = ["shm.cpp", "channel.cpp", "engine.cpp", "bind.cpp"]
 OPS_SOURCE = os.path.join(CSRC, "ops.cpp")
+OPS_HEADER = os.path.join(CUDA, "operators.h")
 OPS_LIB = os.path.join(PKG, "_ops" + sysconfig.get_config_var("EXT_SUFFIX"))
 HOST_LIB = os.path.join(PKG, "_host" + sysconfig.get_config_var("EXT_SUFFIX"))
 CUDA_LIB = os.path.join(PKG, "libtb200_cuda.so")
@@ -72,6 +73,10 @@ def nvcc_path():
         if cand and os.path.exists(cand):
             return cand
     return None
+
+
+def cuda_include():
+    return os.path.join(os.path.dirname(os.path.dirname(os.path.realpath(nvcc_path()))), "include")
 
 
 def cuda_objects(force=False, verbose=False):
@@ -138,13 +143,11 @@ def build_ops(force=False, verbose=False):
     import torch
     from torch.utils.cpp_extension import include_paths
 
-    nvcc = nvcc_path()
-    if torch.version.cuda is None or nvcc is None:
+    if torch.version.cuda is None or nvcc_path() is None:
         return None
-    if not force and not _ops_is_stale([OPS_SOURCE]):
+    if not force and not _ops_is_stale([OPS_SOURCE, OPS_HEADER]):
         return OPS_LIB
-    cuda_include = os.path.join(os.path.dirname(os.path.dirname(os.path.realpath(nvcc))), "include")
-    includes = [*include_paths(), cuda_include, sysconfig.get_paths()["include"]]
+    includes = [*include_paths(), cuda_include(), sysconfig.get_paths()["include"]]
     libs = os.path.join(os.path.dirname(torch.__file__), "lib")
     tmp = OPS_LIB + f".{os.getpid()}.tmp"
     cmd = ["g++", "-O2", "-std=c++17", "-fPIC", "-shared", "-fvisibility=hidden", "-DTORCH_EXTENSION_NAME=_ops", f'-DBUILT_FOR="{ops_built_for()}"',

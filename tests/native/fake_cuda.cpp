@@ -14,9 +14,7 @@
 #include <thread>
 #include <vector>
 
-extern "C" int tb_gemm_bf16(const void*, const void*, void*, int, int, int, int, int, int, int, int, int, const void*, const void*, void*, int, void*, long long, cudaStream_t);
-extern "C" long long tb_gemm_workspace_bytes(int, int, int);
-extern "C" int tb_col_sum(const void*, int, int, int, void*, float*, cudaStream_t);
+#include "operators.h"
 
 namespace {
 

@@ -1,10 +1,12 @@
 // Stands in for libtb200_cuda.so under the native operators: every launcher succeeds without launching anything, the n-th
 // product or column sum can be made to fail, all can be made to wait for a word from another thread, and the waits of streams on one another are taken down.
+#include "operators.h"
+
 #include <atomic>
 #include <chrono>
 #include <thread>
 
-typedef void* S;
+typedef cudaStream_t S;
 
 extern "C" {
 

@@ -52,3 +52,34 @@ def test_build_beside_a_cpu_torch(monkeypatch):
         pytest.skip("not built")
     monkeypatch.setattr(torch.version, "cuda", None)
     entry.build()
+
+
+def test_ctypes_signatures_are_the_headers():
+    """Every entry point that the Python operators call has the argument and result types of cuda/operators.h."""
+    import ctypes
+    import re
+
+    from tandem_b200.ops import _lib, attention
+    from tandem_b200.parallel.symm import cuda_lib
+
+    if not os.path.exists(build.CUDA_LIB):
+        pytest.skip("not built")
+    with open(build.OPS_HEADER) as f:
+        text = re.sub(r"//[^\n]*", "", f.read())
+    plain = {"int": ctypes.c_int, "unsigned": ctypes.c_uint, "long long": ctypes.c_longlong, "float": ctypes.c_float, "void": None}
+    pointers = {ctypes.c_void_p, ctypes.c_char_p, ctypes.POINTER(ctypes.c_int), ctypes.POINTER(ctypes.c_longlong), ctypes.POINTER(ctypes.c_void_p)}
+
+    def kind(declared):
+        declared = declared.strip()
+        return "pointer" if "*" in declared or declared.startswith("cudaStream_t") else plain[declared]
+
+    _lib.lib(), attention._fns()
+    declarations = re.findall(r"^([a-z][\w* ]*?)\b(tb_\w+)\(([^)]*)\);", text, re.M)
+    assert len(declarations) == 26
+    for result, name, arguments in declarations:
+        fn = getattr(cuda_lib(), name)
+        given = [re.sub(r"\w+$", "", a.strip()) if "*" not in a else a for a in arguments.split(",") if a.strip()]
+        want = [kind(a) for a in given]
+        got = ["pointer" if t in pointers else t for t in (fn.argtypes or [])]
+        assert got == want, name
+        assert ("pointer" if fn.restype in pointers else fn.restype) == kind(result), name

@@ -8,6 +8,7 @@ import pytest
 import torch
 
 from tandem_b200.ops import _lib, gemm
+from tandem_b200.utils import build
 
 pytestmark = pytest.mark.gpu
 HERE = os.path.dirname(os.path.abspath(__file__))
@@ -16,14 +17,12 @@ HERE = os.path.dirname(os.path.abspath(__file__))
 @pytest.fixture(scope="module")
 def fake_path(tmp_path_factory):
     out = str(tmp_path_factory.mktemp("fake") / "libfake_kernels.so")
-    subprocess.run(["g++", "-O1", "-std=c++17", "-fPIC", "-shared", os.path.join(HERE, "native", "fake_kernels.cpp"), "-o", out], check=True)
+    subprocess.run(["g++", "-O1", "-std=c++17", "-fPIC", "-shared", f"-I{build.CUDA}", f"-I{build.cuda_include()}", os.path.join(HERE, "native", "fake_kernels.cpp"), "-o", out], check=True)
     return out
 
 
 @pytest.fixture(params=["native", "python"])
 def kernels(request, fake_path, monkeypatch):
-    from tandem_b200.utils.build import CUDA_LIB
-
     fake = ctypes.CDLL(fake_path)
     fake.tb_gemm_last_error.restype = ctypes.c_char_p
     fake.tb_gemm_workspace_bytes.restype = ctypes.c_longlong
@@ -37,7 +36,7 @@ def kernels(request, fake_path, monkeypatch):
         monkeypatch.setattr(gemm, "lib", lambda: Untyped(fake))
     yield fake
     if request.param == "native":
-        _lib.native().bind(CUDA_LIB)
+        _lib.native().bind(build.CUDA_LIB)
 
 
 class Untyped:

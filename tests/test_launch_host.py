@@ -31,9 +31,8 @@ def fake(tmp_path_factory):
         pytest.skip("no compiler")
     objs = [o for o in build.cuda_objects() if os.path.basename(o) in ("gemm.o", "layers.o", "attention.o")]
     out = str(tmp_path_factory.mktemp("fake") / "libfake.so")
-    include = os.path.join(os.path.dirname(os.path.dirname(os.path.realpath(build.nvcc_path()))), "include")
     # -Bsymbolic: its own runtime, not one that torch may have brought into the process
-    r = subprocess.run(["g++", "-O1", "-std=c++17", "-fPIC", "-shared", "-Wl,-Bsymbolic", "-Wl,--no-undefined", f"-I{include}",
+    r = subprocess.run(["g++", "-O1", "-std=c++17", "-fPIC", "-shared", "-Wl,-Bsymbolic", "-Wl,--no-undefined", f"-I{build.cuda_include()}", f"-I{build.CUDA}",
                         os.path.join(HERE, "native", "fake_cuda.cpp"), *objs, "-o", out, "-lpthread"], capture_output=True, text=True)
     assert r.returncode == 0, r.stderr[-2000:]
     return signatures(ctypes.CDLL(out))
