@@ -1352,7 +1352,7 @@ __global__ void k_reciprocals(const float* d, float* out, long long pairs) {
 
 // Flag words for split-K.
 constexpr int SPLIT_FLAG_POOL = 1 << 16;
-__device__ unsigned g_split_flags[SPLIT_FLAG_POOL];
+__device__ unsigned g_split_flags[2 * SPLIT_FLAG_POOL];
 tb::WordPool g_flag_pool(SPLIT_FLAG_POOL);
 
 }  // namespace
@@ -1387,7 +1387,7 @@ int tb_gemm_bf16(const void* A, const void* B, void* out, int M, int N, int K, i
     if (workspace == nullptr || workspace_bytes < need || ((uintptr_t)workspace & 15) || words > SPLIT_FLAG_POOL) {
       splits = 1;  // no room to park partial tiles: compute unsplit (same result up to summation order)
     } else {
-      const cudaError_t e = g_flag_pool.take(words, &split_flags, [](void** at) { return cudaGetSymbolAddress(at, g_split_flags); });
+      const cudaError_t e = g_flag_pool.take(words, stream, &split_flags, [](void** at) { return cudaGetSymbolAddress(at, g_split_flags); });
       if (e != cudaSuccess) return (int)e;
     }
   }

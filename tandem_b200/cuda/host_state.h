@@ -72,17 +72,25 @@ class ErrorWord {
   int* dev_ = nullptr;
 };
 
-// Words of a __device__ array of `size` zeros, lent round-robin to launches that leave them zero again.  Launches in flight at
-// the same time never share one (a pool's worth of them would have to overlap).
+// Words of a __device__ array of 2 * `size` zeros, lent round-robin to launches that leave them zero again: launches in flight at
+// the same time share none (`size` words' worth of them would have to overlap).  A launch that is recorded into a graph keeps its
+// words for every replay, so those come from the second half: whatever is issued beside a replay has others.  Two graphs that are
+// replayed at the same time may share words, if between their recordings a whole half was lent.
 class WordPool {
  public:
   explicit WordPool(long long size) : size_(size) {}
-  // `words` <= size of them on the current device; `find(void**)` looks the array up there.
+  // `words` <= size of them for a launch on `stream` of the current device; `find(void**)` looks the array up there.
   template <typename Find>
-  cudaError_t take(long long words, unsigned** out, Find find) {
+  cudaError_t take(long long words, cudaStream_t stream, unsigned** out, Find find) {
     int dev = 0;
     cudaError_t e = cudaGetDevice(&dev);
     if (e != cudaSuccess) return e;
+    cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(stream, &status) != cudaSuccess) {  // the launch itself will meet the reason
+      cudaGetLastError();
+      status = cudaStreamCaptureStatusNone;
+    }
+    const int half = status != cudaStreamCaptureStatusNone;
     std::lock_guard<std::mutex> hold(lock_);
     if (device_ != dev) {
       void* at = nullptr;
@@ -90,9 +98,9 @@ class WordPool {
       pool_ = static_cast<unsigned*>(at);
       device_ = dev;
     }
-    if (next_ + words > size_) next_ = 0;
-    *out = pool_ + next_;
-    next_ += words;
+    if (next_[half] + words > size_) next_[half] = 0;
+    *out = pool_ + half * size_ + next_[half];
+    next_[half] += words;
     return cudaSuccess;
   }
 
@@ -101,7 +109,7 @@ class WordPool {
   const long long size_;
   unsigned* pool_ = nullptr;
   int device_ = -1;
-  long long next_ = 0;
+  long long next_[2] = {0, 0};
 };
 
 }  // namespace tb

@@ -396,7 +396,7 @@ k_reduce_partials(const float* __restrict__ part, int parts, int width, __nv_bfl
 // ------------------------------------------------------------------------------------ column sums
 // Ticket words for k_col_sum's single-launch mode.
 constexpr int TICKET_POOL = 8192;
-__device__ unsigned g_col_sum_tickets[TICKET_POOL];
+__device__ unsigned g_col_sum_tickets[2 * TICKET_POOL];
 tb::WordPool g_ticket_pool(TICKET_POOL);
 
 // part[blockIdx.y][c] = sum of x[r, c] over the block's row slice; 32 columns x 32 row lanes.
@@ -925,7 +925,7 @@ int tb_col_sum(const void* x, int M, int N, int ld, void* out_bf16, float* scrat
   // two-kernel path.
   if ((int)grid.x <= TICKET_POOL) {
     unsigned* tickets = nullptr;
-    const cudaError_t e = g_ticket_pool.take(grid.x, &tickets, [](void** at) { return cudaGetSymbolAddress(at, g_col_sum_tickets); });
+    const cudaError_t e = g_ticket_pool.take(grid.x, s, &tickets, [](void** at) { return cudaGetSymbolAddress(at, g_col_sum_tickets); });
     if (e != cudaSuccess) return (int)e;
     tb_note_launch(1);
     if (wide)

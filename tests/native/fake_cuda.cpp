@@ -26,7 +26,8 @@ std::map<const void*, unsigned long long> borrowed;      // the words of a pool 
 thread_local int device = 0;
 thread_local cudaError_t last = cudaSuccess;
 int refuse_allowing = 0;
-char words[1 << 19] __attribute__((aligned(256)));       // stands for every __device__ array
+std::atomic<int> recording{0};
+char words[1 << 20] __attribute__((aligned(256)));       // stands for every __device__ array
 
 CUresult encode(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*, const cuuint32_t*, const cuuint32_t*,
                 CUtensorMapInterleave, CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill) {
@@ -39,16 +40,19 @@ extern "C" {
 
 // ---------------------------------------------------------------- what a test asks and sets
 void fake_set_device(int d) { device = d; }
+void fake_record(int on) { recording = on; }  // every stream is being captured
 void fake_refuse_allowing(int n) { refuse_allowing = n; }  // the next n raises of a limit fail
-// How many different places of a pool were handed out, and the smallest and largest number of times that one was.
-void fake_borrowed(unsigned long long* out3) {
+// How many different places of a pool were handed out, the smallest and largest number of times that one was, and the first and the last.
+void fake_borrowed(unsigned long long* out5) {
   std::lock_guard<std::mutex> hold(lock);
-  out3[0] = borrowed.size();
-  out3[1] = ~0ull, out3[2] = 0;
+  out5[0] = borrowed.size();
+  out5[1] = ~0ull, out5[2] = 0;
   for (const auto& [at, n] : borrowed) {
-    if (n < out3[1]) out3[1] = n;
-    if (n > out3[2]) out3[2] = n;
+    if (n < out5[1]) out5[1] = n;
+    if (n > out5[2]) out5[2] = n;
   }
+  out5[3] = borrowed.empty() ? 0 : static_cast<const char*>(borrowed.begin()->first) - words;
+  out5[4] = borrowed.empty() ? 0 : static_cast<const char*>(borrowed.rbegin()->first) - words;
   borrowed.clear();
 }
 
@@ -99,6 +103,10 @@ cudaError_t cudaStreamWaitEvent(cudaStream_t, cudaEvent_t, unsigned) { return cu
 cudaError_t cudaGetDriverEntryPoint(const char*, void** out, unsigned long long, cudaDriverEntryPointQueryResult* q) {
   *out = (void*)encode;
   if (q != nullptr) *q = cudaDriverEntryPointSuccess;
+  return cudaSuccess;
+}
+cudaError_t cudaStreamIsCapturing(cudaStream_t, cudaStreamCaptureStatus* out) {
+  *out = recording ? cudaStreamCaptureStatusActive : cudaStreamCaptureStatusNone;
   return cudaSuccess;
 }
 cudaError_t cudaOccupancyMaxActiveClusters(int* n, const void*, const cudaLaunchConfig_t*) { *n = 74; return cudaSuccess; }

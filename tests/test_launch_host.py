@@ -42,13 +42,27 @@ def fake(tmp_path_factory):
 def test_threads_never_share_words(fake, products):
     """Tickets of column sums and flags of split products are handed out in turn, so every place of the pool is lent equally often,
     whatever the threads' timing.  A place lent twice in a round (two launches in flight would use the same words) is missing elsewhere."""
-    out = (ctypes.c_ulonglong * 3)()  # places, lent at least, lent at most
+    out = (ctypes.c_ulonglong * 5)()  # places, lent at least, lent at most, first, last
     fake.fake_borrowed(out)
     threads, each = 8, 20000
     assert fake.fake_threads(threads, each, products) == 0
     fake.fake_borrowed(out)
     assert out[0] > 50 and out[0] * out[1] <= threads * each <= out[0] * out[2]
     assert out[2] - out[1] <= 1, f"{out[0]} places, lent {out[1]} to {out[2]} times"
+
+
+@pytest.mark.parametrize("products", [0, 1])
+def test_recorded_launches_keep_their_words(fake, products):
+    """A graph's launches use theirs at every replay: none is lent to a launch that is not recorded, however many follow."""
+    out, ranges = (ctypes.c_ulonglong * 5)(), {}
+    fake.fake_borrowed(out)
+    for recorded in (0, 1, 0, 1):
+        fake.fake_record(recorded)
+        assert fake.fake_threads(1, 5000, products) == 0
+        fake.fake_borrowed(out)
+        assert ranges.setdefault(recorded, (out[3], out[4])) == (out[3], out[4])
+    fake.fake_record(0)
+    assert ranges[0][1] < ranges[1][0]
 
 
 def launches(lib):
