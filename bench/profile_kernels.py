@@ -1,6 +1,6 @@
 """Runs ONE kernel of this library a few times on a small, fixed case, so that a profiler can capture it:
 
-    python bench/profile_kernels.py gemm_fwd | gemm_dx | gemm_dw | attn | attn_long | adamw | layernorm |
+    python bench/profile_kernels.py gemm_fwd | gemm_gelu | gemm_dx | gemm_dw | attn | attn_long | adamw | layernorm |
                                                allreduce | reduce_scatter_adam | gather_gemm
 
 Inputs are larger than the 126 MB L2 where the kernel is memory-bound, and at most a few hundred MB in
@@ -28,13 +28,16 @@ def run(which, reps=3):
         return (torch.randn(*shape, device=dev) * scale).bfloat16()
 
     info = {}
-    if which in ("gemm_fwd", "gemm_dx", "gemm_dw"):
-        from tandem_b200.ops.gemm import BIAS, gemm
+    if which in ("gemm_fwd", "gemm_gelu", "gemm_dx", "gemm_dw"):
+        from tandem_b200.ops.gemm import BIAS, GELU, gemm
 
         M, N, K = 8192, 3072, 768
         if which == "gemm_fwd":
             a, b, bias = rnd(M, K), rnd(N, K), rnd(N)
             fn = lambda: gemm(a, b, M, N, K, K, K, False, False, BIAS, bias)
+        elif which == "gemm_gelu":  # the MLP's first product: GELU and its derivative
+            a, b, bias, slope = rnd(M, K), rnd(N, K), rnd(N), rnd(M, N)
+            fn = lambda: gemm(a, b, M, N, K, K, K, False, False, BIAS | GELU, bias, None, slope)
         elif which == "gemm_dx":
             M, N, K = 8192, 768, 3072
             a, b = rnd(M, K), rnd(K, N)
@@ -43,7 +46,7 @@ def run(which, reps=3):
             M, N, K = 3072, 768, 8192
             a, b = rnd(K, M), rnd(K, N)
             fn = lambda: gemm(a, b, M, N, K, M, N, True, True)
-        info = {"flops": 2.0 * M * N * K, "bytes": 2.0 * (M * K + N * K + M * N)}
+        info = {"flops": 2.0 * M * N * K, "bytes": 2.0 * (M * K + N * K + M * N * (2 if which == "gemm_gelu" else 1))}
     elif which in ("attn", "attn_long"):
         from tandem_b200.ops import causal_attention
 

@@ -341,10 +341,11 @@ __device__ __forceinline__ void bulk_store_2d(const CUtensorMap* map, const uint
 // What bounded it was waiting: for a chunk's aux_in, fetched by the lanes one chunk ahead and row by row, for the first bias, and
 // for the stores to release the blocks.  So begin(), called before the accumulator is complete, fetches the tile's bias and starts TMA
 // loads of aux_in into the blocks that the results will leave from (a lane replaces the values of its own row), and there are
-// BLOCKS blocks per warp, four where the ring keeps enough stages without their memory.  Before and after, us, cold: bias + residual
-// 3072 x 384 x 384 7.5, 5.4; 1024 x 768 x 768 8.1, 6.2; 4096 x 1024 x 1024 17.0, 12.5; 8192 x 768 x 3072 46.6, 39.0; times gelu'
-// 8192 x 3072 x 768 45.2, 39.0; GELU at that size 56, 47.4.  From there on shared memory's bandwidth bounds it beside a main loop of
-// twelve k-blocks, which leaves a quarter of that bandwidth.
+// BLOCKS blocks per warp, four where the ring keeps enough stages without their memory.  Before and after (with what this file gained
+// since: the deeper ring, the late trigger, the relaxed arrival), us, one after the other in a graph: bias + residual 3072 x 384 x 384 6.3, 4.9;
+// 1024 x 768 x 768 7.3, 5.9; 4096 x 1024 x 1024 14.2, 10.7; 8192 x 768 x 3072 46.1, 35.8; times gelu' 8192 x 3072 x 768 44.9, 37.5; GELU
+// at that size 55.9, 44.4.  What bounds GELU beside a main loop of twelve k-blocks is a warp's own chain (TMEM, special functions,
+// packed arithmetic, block; two warps per scheduler): the tensor pipe is active for 34 %, shared memory's pipes for 32 % and its banks for 12 %.
 template <int BLOCKS, int CHUNKS, int GELU_PAIRS = 2>
 struct Epilogue {
   uint8_t* staging;    // of all eight warps: blocks [8][BLOCKS][BLOCK_BYTES], bias values [8][32], barriers of the loads [8][BLOCKS]
@@ -1338,7 +1339,10 @@ GemmPlan plan_gemm(int M, int N, int K, int ctas) {
 }
 
 // Without a device (a build machine) the plan is the one a B200's 148 SMs would get.
-int planned_sms() { return tb::sm_count() > 0 ? tb::sm_count() : 148; }
+int planned_sms() {
+  const int n = tb::sm_count();
+  return n > 0 ? n : 148;
+}
 
 // reciprocal2 as the GELU epilogue uses it, for comparisons with a division.
 __global__ void k_reciprocals(const float* d, float* out, long long pairs) {
