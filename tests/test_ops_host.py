@@ -40,6 +40,28 @@ def test_host_tensors_are_refused_before_a_launch(kernels):
     assert set(kernels.calls) <= {"tb_gemm_workspace_bytes"}
 
 
+def test_elementwise_operands_that_do_not_fit_are_refused(kernels):
+    """One size is handed to the kernel for all arrays: none may be shorter, of another type or strided."""
+    p, g, m, v, scalars, shadow = (torch.zeros(16) for _ in range(6))
+    shadow = shadow.bfloat16()
+    good = dict(param=p, grad=g, exp_avg=m, exp_avg_sq=v, scalars=scalars, shadow=shadow)
+    bad = {"param": [p.double(), torch.zeros(32)[::2]], "grad": [g[:8], g.half()], "exp_avg": [m[:8], m.bfloat16(), torch.zeros(32)[::2]],
+           "exp_avg_sq": [v[:8], v.double()], "shadow": [shadow[:8], p, torch.zeros(32).bfloat16()[::2]], "scalars": [scalars[:7], scalars.double()]}
+    for name, values in bad.items():
+        for value in values:
+            with pytest.raises(ValueError) as e:
+                elementwise.adamw_step_dev(**{**good, name: value})
+            assert "cuda device" not in str(e.value), name
+    counter = torch.zeros(1, dtype=torch.float64)
+    for args in [(counter.float(), scalars), (counter, scalars[:7]), (counter, scalars.double())]:
+        with pytest.raises(ValueError, match="step counter"):
+            elementwise.adam_prepare(args[0], (1e-3, (0.9, 0.95), 1e-8, 0.1), args[1])
+    with pytest.raises(RuntimeError, match="size"):
+        elementwise.multi_copy(p, [(p[:8], g)])
+    elementwise.multi_copy(p, [(p, torch.ones(1))])  # as copy_ does
+    assert torch.equal(p, torch.ones(16)) and kernels.calls == []
+
+
 class Probe(torch.autograd.Function):
     """Tells whether a call went through the node (whose context torch makes) or through the forward alone."""
 
